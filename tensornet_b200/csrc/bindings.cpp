@@ -6,6 +6,7 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <atomic>
 #include <cstring>
 #include <string>
@@ -163,7 +164,12 @@ struct SparseCtx {
   void set_table(py::dict table) { keep["table"] = table; t = table_from_dict(table); upload_table(); }
 
   // Dedup, id dispatch and inverse map of a batch ahead of its pull (plain kernels on the current stream).
-  void front(at::Tensor ids, at::Tensor inverse) {
+  static const int* count_ptr(const c10::optional<at::Tensor>& n_dev) {
+    if (!n_dev.has_value()) return nullptr;
+    TORCH_CHECK(n_dev->is_cuda() && n_dev->scalar_type() == at::kInt && n_dev->numel() == 1, "n_dev: one int32 on the device");
+    return ptr_of<const int>(*n_dev);
+  }
+  void front(at::Tensor ids, at::Tensor inverse, c10::optional<at::Tensor> n_dev) {
     TORCH_CHECK(ids.is_cuda() && ids.scalar_type() == at::kLong && ids.is_contiguous(), "ids: contiguous int64 CUDA tensor");
     TORCH_CHECK(inverse.scalar_type() == at::kInt && inverse.numel() >= ids.numel(), "inverse: int32, one per id");
     c10::cuda::CUDAGuard guard(ids.device());
@@ -171,6 +177,7 @@ struct SparseCtx {
     a.c = c; a.tbl = t; a.opt = o;
     a.ids = ptr_of<const long long>(ids);
     a.n_ids = (int)ids.numel();
+    a.n_dev = count_ptr(n_dev);
     a.inverse = ptr_of<int>(inverse);
     a.training = 1;
     check(tn::launch_sparse_pull_front(a, cur_stream()), "sparse_pull_front launch");
@@ -178,7 +185,7 @@ struct SparseCtx {
   }
 
   void pull(at::Tensor ids, at::Tensor inverse, c10::optional<at::Tensor> labels, int label_mod, bool training, bool lookup_only,
-            bool front_done) {
+            bool front_done, c10::optional<at::Tensor> n_dev) {
     TORCH_CHECK(ids.is_cuda() && ids.scalar_type() == at::kLong && ids.is_contiguous(), "ids: contiguous int64 CUDA tensor");
     TORCH_CHECK(inverse.scalar_type() == at::kInt && inverse.numel() >= ids.numel(), "inverse: int32, one per id");
     c10::cuda::CUDAGuard guard(ids.device());
@@ -187,6 +194,7 @@ struct SparseCtx {
     a.tbl_dev = reinterpret_cast<const tn::TableView*>(tbl_dev.data_ptr());
     a.ids = ptr_of<const long long>(ids);
     a.n_ids = (int)ids.numel();
+    a.n_dev = count_ptr(n_dev);
     a.inverse = ptr_of<int>(inverse);
     a.labels = labels.has_value() ? ptr_of<const float>(*labels) : nullptr;
     a.label_mod = label_mod;
@@ -421,13 +429,13 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("set_opt", &SparseCtx::set_opt)
       .def("set_table", &SparseCtx::set_table)
       .def("pull", &SparseCtx::pull, py::arg("ids"), py::arg("inverse"), py::arg("labels"), py::arg("label_mod"), py::arg("training"),
-           py::arg("lookup_only") = false, py::arg("front_done") = false)
+           py::arg("lookup_only") = false, py::arg("front_done") = false, py::arg("n_dev") = py::none())
       .def("push", [](SparseCtx& self, int64_t work_hint, int max_ctas, py::object dense) {
         if (dense.is_none()) { self.push(work_hint, max_ctas, nullptr); return; }
         const tn::DenseStepArgs d = dense.cast<DenseCtx&>().rider_args();
         self.push(work_hint, max_ctas, &d);
       }, py::arg("work_hint"), py::arg("max_ctas") = 0, py::arg("dense") = py::none())
-      .def("front", &SparseCtx::front, py::arg("ids"), py::arg("inverse"));
+      .def("front", &SparseCtx::front, py::arg("ids"), py::arg("inverse"), py::arg("n_dev") = py::none());
   py::class_<BnCtx>(m, "BnCtx")
       .def(py::init<py::dict>())
       .def("push", &BnCtx::push)
@@ -489,10 +497,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     for (size_t i = 0; i < dsts.size(); ++i) {
       const at::Tensor& d = dsts[i];
       const at::Tensor& h = srcs[i];
-      TORCH_CHECK(d.is_cuda() && !h.is_cuda() && d.is_contiguous() && h.is_contiguous() && d.nbytes() == h.nbytes() &&
-                      d.scalar_type() == h.scalar_type(),
+      // a vector may be shorter than its static buffer (ids of a batch with ragged slots)
+      TORCH_CHECK(d.is_cuda() && !h.is_cuda() && d.is_contiguous() && h.is_contiguous() && d.scalar_type() == h.scalar_type() &&
+                      (d.nbytes() == h.nbytes() || (d.dim() == 1 && h.dim() == 1 && h.nbytes() <= d.nbytes())),
                   "stage_inputs: leaf ", i, " must be a contiguous host tensor of the static buffer's type and size");
-      check(cudaMemcpyAsync(d.data_ptr(), h.data_ptr(), d.nbytes(), cudaMemcpyHostToDevice, cs), "cudaMemcpyAsync");
+      if (h.nbytes() == 0) continue;
+      check(cudaMemcpyAsync(d.data_ptr(), h.data_ptr(), h.nbytes(), cudaMemcpyHostToDevice, cs), "cudaMemcpyAsync");
       // a page-locked source from torch's host allocator must not be handed out again before the copy has run
       // (what Tensor.copy_(non_blocking=True) does behind the scenes); a no-op for other host memory
       if (h.is_pinned())
@@ -501,6 +511,24 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     }
     check(cudaEventRecord(reinterpret_cast<cudaEvent_t>(copied_event), cs), "cudaEventRecord");
     check(cudaStreamWaitEvent(ms, reinterpret_cast<cudaEvent_t>(copied_event), 0), "cudaStreamWaitEvent");
+  });
+  // Numbers of ids of the ragged columns of a batch in host memory (values, offsets in turn), or an empty list when a
+  // column's last offset is not the length of its values: a Python-level read of every last offset costs more than the
+  // staging itself for batches of dozens of columns.
+  m.def("ragged_lengths", [](std::vector<at::Tensor> cols) {
+    std::vector<int64_t> n;
+    for (size_t i = 0; i + 1 < cols.size(); i += 2) {
+      const at::Tensor &v = cols[i], &o = cols[i + 1];
+      int64_t last = -1;
+      if (v.dim() == 1 && o.dim() == 1 && !o.is_cuda() && o.numel() >= 1) {
+        const char* p = static_cast<const char*>(o.data_ptr()) + (o.numel() - 1) * o.stride(0) * o.element_size();
+        if (o.scalar_type() == at::kInt) last = *reinterpret_cast<const int*>(p);
+        else if (o.scalar_type() == at::kLong) last = *reinterpret_cast<const int64_t*>(p);
+      }
+      if (last != v.numel()) return std::vector<int64_t>();
+      n.push_back(last);
+    }
+    return n;
   });
   // 4-byte device scalar -> slot of a pinned ring, then an event behind it (the loss of a step on its way to the host)
   // `wait_event` != 0: the copy runs on a stream of its own behind that event (the end of the step), so the compute
@@ -539,6 +567,38 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     return at::from_blob(ptr_of<void>(p), {nbytes}, opts);
   });
 
+  m.def("expand_bag_labels", [](at::Tensor y, at::Tensor offsets, int S, at::Tensor out) {
+    TORCH_CHECK(y.scalar_type() == at::kFloat && y.is_contiguous() && offsets.scalar_type() == at::kInt && offsets.is_contiguous() &&
+                    offsets.numel() == y.numel() * S + 1 && out.scalar_type() == at::kFloat && out.is_contiguous(), "expand_bag_labels");
+    c10::cuda::CUDAGuard guard(y.device());
+    tn::launch_expand_bag_labels(ptr_of<float>(y), ptr_of<int>(offsets), (int)y.numel(), (int)y.numel() * S, ptr_of<float>(out),
+                                 (int)out.numel(), cur_stream());
+  });
+  m.def("pack_columns", [](std::vector<at::Tensor> values, std::vector<c10::optional<at::Tensor>> offsets, std::vector<int> lens, int B,
+                           at::Tensor out_values, at::Tensor out_offsets) {
+    const int S = (int)values.size();
+    TORCH_CHECK(S >= 1 && (int)offsets.size() == S && (int)lens.size() == S && B >= 1 && out_values.scalar_type() == at::kLong &&
+                    out_values.is_contiguous() && out_offsets.scalar_type() == at::kInt && out_offsets.is_contiguous() &&
+                    out_offsets.numel() == (int64_t)S * B + 1, "pack_columns");
+    c10::cuda::CUDAGuard guard(out_values.device());
+    for (int s0 = 0; s0 < S; s0 += tn::kPackColumns) {
+      tn::PackColumns a{};
+      a.n = std::min(tn::kPackColumns, S - s0); a.B = B; a.first = s0;
+      a.out_values = ptr_of<long long>(out_values); a.out_offsets = ptr_of<int>(out_offsets); a.total_room = out_values.numel();
+      for (int c = 0; c < a.n; ++c) {
+        const at::Tensor& v = values[s0 + c];
+        TORCH_CHECK(v.is_cuda() && v.is_contiguous() && (v.scalar_type() == at::kLong || v.scalar_type() == at::kInt), "pack_columns: ids");
+        a.values[c] = v.data_ptr(); a.val64[c] = v.scalar_type() == at::kLong; a.room[c] = (int)v.numel(); a.len[c] = lens[s0 + c];
+        if (offsets[s0 + c].has_value()) {
+          const at::Tensor& o = *offsets[s0 + c];
+          TORCH_CHECK(o.is_cuda() && o.is_contiguous() && o.numel() == B + 1 && (o.scalar_type() == at::kLong || o.scalar_type() == at::kInt),
+                      "pack_columns: offsets");
+          a.offsets[c] = o.data_ptr(); a.off64[c] = o.scalar_type() == at::kLong;
+        }
+      }
+      tn::launch_pack_columns(a, cur_stream());
+    }
+  });
   m.def("pool_fwd", [](at::Tensor U, int ustride, at::Tensor inverse, c10::optional<at::Tensor> offsets, int B, int S, int pd,
                        int combiner, at::Tensor out, int out_ld) {
     c10::cuda::CUDAGuard guard(U.device());

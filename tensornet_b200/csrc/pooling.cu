@@ -162,6 +162,46 @@ __global__ void seq_bwd_kernel(float* __restrict__ gU, int gstride, const int* _
   }
 }
 
+// Per id the label of its example: one thread per bag writes its bag's few entries.
+__global__ void expand_bag_labels_kernel(const float* __restrict__ y, const int* __restrict__ offsets, int B, int nbags,
+                                         float* __restrict__ out, int room) {
+  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < nbags; g += gridDim.x * blockDim.x) {
+    const float v = y[g % B];
+    const int k1 = min(offsets[g + 1], room);
+    for (int k = max(offsets[g], 0); k < k1; ++k) out[k] = v;
+  }
+}
+
+__device__ __forceinline__ long long index_at(const void* p, int is64, long long i) {
+  return is64 ? reinterpret_cast<const long long*>(p)[i] : (long long)reinterpret_cast<const int*>(p)[i];
+}
+
+// Columns -> packed (values, offsets).  blockIdx.y = column; where it starts is the sum of the counts of the columns
+// before it, which only the device knows in a captured step: every block adds them up itself (a few hundred L2 reads),
+// which is cheaper than a second launch.  `first` columns of an earlier launch end at out_offsets[first * B].
+__global__ void pack_columns_kernel(const __grid_constant__ PackColumns a) {
+  __shared__ long long s_base;
+  const int c = blockIdx.y, B = a.B;
+  if (threadIdx.x == 0) s_base = a.first > 0 ? a.out_offsets[(size_t)a.first * B] : 0;
+  __syncthreads();
+  long long before = 0;
+  for (int j = threadIdx.x; j < c; j += blockDim.x)
+    before += a.offsets[j] != nullptr ? index_at(a.offsets[j], a.off64[j], B) : (long long)a.len[j] * B;
+  for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+  if ((threadIdx.x & 31) == 0 && before) atomicAdd(reinterpret_cast<unsigned long long*>(&s_base), (unsigned long long)before);
+  __syncthreads();
+  const long long base = s_base;
+  const void* off = a.offsets[c];
+  long long n = off != nullptr ? index_at(off, a.off64[c], B) : (long long)a.len[c] * B;
+  if (n > a.room[c]) n = a.room[c];
+  const int t0 = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+  for (long long k = t0; k < n && base + k < a.total_room; k += nt) a.out_values[base + k] = index_at(a.values[c], a.val64[c], k);
+  const size_t row = (size_t)(a.first + c) * B;
+  for (int b = t0; b < B; b += nt)
+    a.out_offsets[row + b] = (int)(base + (off != nullptr ? index_at(off, a.off64[c], b) : (long long)a.len[c] * b));
+  if (t0 == 0) a.out_offsets[row + B] = (int)(base + n);       // the next column writes the same value as its start
+}
+
 inline int grid_for(long long groups, int G, int threads) {
   long long blocks = (groups * G + threads - 1) / threads;
   if (blocks < 1) blocks = 1;
@@ -170,6 +210,17 @@ inline int grid_for(long long groups, int G, int threads) {
 }
 
 }  // namespace
+
+void launch_expand_bag_labels(const float* y, const int* offsets, int B, int nbags, float* out, int room, cudaStream_t st) {
+  expand_bag_labels_kernel<<<grid_for(nbags, 1, 256), 256, 0, st>>>(y, offsets, B, nbags, out, room);
+}
+void launch_pack_columns(const PackColumns& a, cudaStream_t st) {
+  long long most = a.B;
+  for (int c = 0; c < a.n; ++c) most = a.room[c] > most ? a.room[c] : most;
+  int bx = (int)((most + 1023) / 1024);          // four elements per thread of the longest column
+  if (bx > 64) bx = 64;
+  pack_columns_kernel<<<dim3(bx < 1 ? 1 : bx, a.n), 256, 0, st>>>(a);
+}
 
 void launch_pool_fwd(const float* U, int ustride, const int* inverse, const int* offsets, int B, int S, int pd,
                      int combiner, float* out, int out_ld, cudaStream_t st) {

@@ -43,6 +43,11 @@ __device__ __forceinline__ unsigned lanemask_lt() {
   return m;
 }
 
+// Number of ids of this batch: the launch's count, or less when the buffer of a captured step is not full.
+__device__ __forceinline__ int batch_ids(const PullArgs& a) {
+  return a.n_dev != nullptr ? min(a.n_ids, max(__ldg(a.n_dev), 0)) : a.n_ids;
+}
+
 // Warp-aggregated "counter += 1 for every lane in `mask`"; returns this lane's old value.
 // Must be called by all 32 lanes; lanes outside `mask` get an unspecified value.
 __device__ __forceinline__ int warp_alloc(int* counter, unsigned mask) {
@@ -170,6 +175,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_pull_fused_kernel(const __
   const int nth = gridDim.x * blockDim.x;
   const int lane = threadIdx.x & 31;
   const int W = c.world, R = c.rank, capo = c.capo;
+  const int n_ids = batch_ids(a);
   const unsigned long long epoch = __ldcg(c.epoch) + 1ull;
   const int dim = t.dim;
   const bool need_ou = a.training && W > 1;
@@ -182,9 +188,9 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_pull_fused_kernel(const __
     // show / click counts of the batch into the gradient records (the front runs while the previous step's records
     // are still in use, so it leaves them alone)
     if (a.training) {
-      for (int base = tid - lane; base < a.n_ids; base += nth) {
+      for (int base = tid - lane; base < n_ids; base += nth) {
         const int i = base + lane;
-        const bool valid = i < a.n_ids;
+        const bool valid = i < n_ids;
         const int v = valid ? a.inverse[i] : -1;
         const unsigned same = __match_any_sync(0xffffffffu, (valid && v >= 0) ? v : -2 - lane);
         if (valid && v >= 0) {
@@ -201,16 +207,16 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_pull_fused_kernel(const __
     prof_mark(c, 2);
   } else {
   // ---- phase A: dedup; first occurrence of a sign allocates a slot in its owner's segment --------
-  for (int base = tid - lane; base < a.n_ids; base += nth) {
+  for (int base = tid - lane; base < n_ids; base += nth) {
     const int i = base + lane;
     bool winner = false;
     unsigned hw = 0;
     unsigned long long key = 0;
-    if (i < a.n_ids) key = canon_key((unsigned long long)a.ids[i]);
+    if (i < n_ids) key = canon_key((unsigned long long)a.ids[i]);
     else key = kEmptyKey;
     // lanes of the warp that carry the same sign elect one representative: a hot sign costs one probe per warp
     const unsigned same = __match_any_sync(0xffffffffu, key);
-    if (i < a.n_ids && lane == __ffs(same) - 1) {
+    if (i < n_ids && lane == __ffs(same) - 1) {
       unsigned h = (unsigned)mix64(key ^ 0x2545F4914F6CDD1Dull) & c.dd_mask;
       bool done = false;
       for (unsigned probes = 0; probes <= c.dd_mask; ++probes) {
@@ -272,9 +278,9 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_pull_fused_kernel(const __
       st_release_sys_u64(sig_word(c.sig[p], kSigPullReq, R), (epoch << 32) | (unsigned long long)n);
     }
   }
-  for (int base = tid - lane; base < a.n_ids; base += nth) {
+  for (int base = tid - lane; base < n_ids; base += nth) {
     const int i = base + lane;
-    const bool valid = i < a.n_ids;
+    const bool valid = i < n_ids;
     const unsigned long long key = valid ? canon_key((unsigned long long)a.ids[i]) : kEmptyKey;
     const unsigned same = __match_any_sync(0xffffffffu, key);
     const int leader = __ffs(same) - 1;
@@ -570,15 +576,16 @@ __global__ void __launch_bounds__(kFrontThreads) pull_front_dedup_kernel(const _
   const int nth = gridDim.x * blockDim.x;
   const int lane = threadIdx.x & 31;
   const int W = c.world, capo = c.capo;
+  const int n_ids = batch_ids(a);
   if (c.prof != nullptr && tid == 0) c.prof[16] = globaltimer_ns();
-  for (int base = tid - lane; base < a.n_ids; base += nth) {
+  for (int base = tid - lane; base < n_ids; base += nth) {
     const int i = base + lane;
     bool winner = false;
     unsigned hw = 0;
     unsigned long long key = kEmptyKey;
-    if (i < a.n_ids) key = canon_key((unsigned long long)a.ids[i]);
+    if (i < n_ids) key = canon_key((unsigned long long)a.ids[i]);
     const unsigned same = __match_any_sync(0xffffffffu, key);
-    if (i < a.n_ids && lane == __ffs(same) - 1) {
+    if (i < n_ids && lane == __ffs(same) - 1) {
       unsigned h = (unsigned)mix64(key ^ 0x2545F4914F6CDD1Dull) & c.dd_mask;
       bool done = false;
       for (unsigned probes = 0; probes <= c.dd_mask; ++probes) {
@@ -629,6 +636,7 @@ __global__ void __launch_bounds__(kFrontThreads) pull_front_ship_kernel(const __
   const int nth = gridDim.x * blockDim.x;
   const int lane = threadIdx.x & 31;
   const int W = c.world, R = c.rank, capo = c.capo;
+  const int n_ids = batch_ids(a);
   const unsigned long long epoch = __ldcg(c.epoch) + 1ull;
   if (W > 1) {
     for (int p = 0; p < W; ++p) {
@@ -650,9 +658,9 @@ __global__ void __launch_bounds__(kFrontThreads) pull_front_ship_kernel(const __
       if (threadIdx.x == 0) c.bar[4] = 0;
     }
   }
-  for (int base = tid - lane; base < a.n_ids; base += nth) {
+  for (int base = tid - lane; base < n_ids; base += nth) {
     const int i = base + lane;
-    const bool valid = i < a.n_ids;
+    const bool valid = i < n_ids;
     const unsigned long long key = valid ? canon_key((unsigned long long)a.ids[i]) : kEmptyKey;
     const unsigned same = __match_any_sync(0xffffffffu, key);
     const int leader = __ffs(same) - 1;

@@ -15,6 +15,21 @@ void launch_seq_fwd(const float* U, int ustride, const int* inverse, const int* 
                     float* out, int* lengths, cudaStream_t st);
 void launch_seq_bwd(float* gU, int gstride, const int* inverse, const int* offsets, int B, int T, int pd, int dim,
                     const float* gout, cudaStream_t st);
+void launch_expand_bag_labels(const float* y, const int* offsets, int B, int nbags, float* out, int room, cudaStream_t st);
+// Up to kPackColumns id columns of a batch -> packed values and offsets (columns `first`, `first` + 1, ... of the result).
+constexpr int kPackColumns = 64;
+struct PackColumns {
+  int n, B, first;
+  const void* values[kPackColumns];      // int64 or int32 ids
+  const void* offsets[kPackColumns];     // [B + 1] int64 or int32, or null: every example has len[c] ids
+  int room[kPackColumns];                // ids the column's buffer can hold
+  int len[kPackColumns];
+  unsigned char val64[kPackColumns], off64[kPackColumns];
+  long long* out_values;
+  int* out_offsets;
+  long long total_room;                  // entries of out_values
+};
+void launch_pack_columns(const PackColumns& a, cudaStream_t st);
 
 // table_ops.cu
 void launch_table_insert_keys(const TableView& t, const long long* keys, int n, int* out_rows, int* status, cudaStream_t st);

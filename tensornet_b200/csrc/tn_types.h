@@ -70,6 +70,7 @@ struct PullArgs {
   SparseOptParams opt;
   const long long* ids;   // [n_ids] raw signs of the batch (all columns of the layer)
   int n_ids;
+  const int* n_dev;       // when not null: how many of the n_ids entries are there (buffers of captured steps have room to spare)
   int* inverse;           // [n_ids] out: virtual row (owner * capo + position) of every id
   const float* labels;    // optional click labels: labels[i % label_mod] (label_mod > 0) or labels[i]
   int label_mod;

@@ -48,7 +48,50 @@ class PackedFeatures:
 PACKED_KEY = "__packed__"
 
 
+class NeedsExactLengths(RuntimeError):
+    """Code other than the embedding layers looked into a padded feature of a captured step."""
+
+
+class PaddedRagged:
+    """The stand-in for a :class:`Ragged` column inside a captured step: ``values`` has room for more ids than the
+    batch holds, the last offset says how many are there.  Only :func:`gather_columns` reads it; anything that asks
+    for ``values`` / ``offsets`` expects exact lengths and is told so (the model then runs such batches uncaptured)."""
+
+    def __init__(self, values: torch.Tensor, offsets: torch.Tensor):
+        self._values, self._offsets = values, offsets
+
+    def _refuse(self, *_):
+        raise NeedsExactLengths("padded feature")
+
+    values = offsets = property(_refuse)
+    __getitem__ = __iter__ = __len__ = _refuse
+
+
+class PaddedPacked(PackedFeatures):
+    """:class:`PackedFeatures` of the ragged form with room for more ids than the batch holds; see :class:`PaddedRagged`."""
+
+    def __init__(self, keys: Sequence[str], values: torch.Tensor, offsets: torch.Tensor, batch_size: int):
+        self.keys, self.ids, self.batch_size = [str(k) for k in keys], None, int(batch_size)
+        self._values, self._offsets = values, offsets
+
+    def _refuse(self, *_):
+        raise NeedsExactLengths("padded features")
+
+    values = offsets = property(_refuse)
+    to = pin_memory = _refuse
+
+
+def padded_columns(features: Dict, keys: List[str]) -> bool:
+    """Do the slots ``keys`` come with room for more ids than the batch holds?  The last offset is then the count."""
+    packed = features.get(PACKED_KEY)
+    if packed is not None and packed.keys == keys:
+        return isinstance(packed, PaddedPacked)
+    return any(isinstance(features.get(k), PaddedRagged) for k in keys)
+
+
 def batch_size_of(feature) -> int:
+    if isinstance(feature, PaddedRagged):
+        return int(feature._offsets.numel()) - 1
     if isinstance(feature, Ragged) or (isinstance(feature, (tuple, list)) and len(feature) == 2):
         return int(feature[1].numel()) - 1
     return int(feature.shape[0])
@@ -61,6 +104,8 @@ def gather_columns(features: Dict, keys: List[str], device) -> Tuple[torch.Tenso
     if packed is not None and packed.keys == keys:
         if packed.ids is not None:
             return packed.ids.to(device, non_blocking=True).reshape(-1), None, packed.batch_size
+        if isinstance(packed, PaddedPacked):
+            return packed._values, packed._offsets.int(), packed.batch_size
         return (packed.values.to(device, non_blocking=True), packed.offsets.to(device, non_blocking=True).int(),
                 packed.batch_size)
     if packed is not None and packed.ids is not None and all(k in packed.keys for k in keys):
@@ -73,6 +118,8 @@ def gather_columns(features: Dict, keys: List[str], device) -> Tuple[torch.Tenso
     if single:
         ids = torch.stack([c.reshape(-1).to(device, non_blocking=True).long() for c in cols]).reshape(-1)
         return ids, None, B
+    if any(isinstance(c, PaddedRagged) for c in cols):
+        return _gather_padded(cols, B, device)
     vals, offs, base = [], [], 0
     for c in cols:
         if torch.is_tensor(c):
@@ -89,3 +136,31 @@ def gather_columns(features: Dict, keys: List[str], device) -> Tuple[torch.Tenso
         base += int(v.numel())
     offs.append(torch.tensor([base], device=device, dtype=torch.int64))
     return torch.cat(vals), torch.cat(offs).int(), B
+
+
+def _gather_padded(cols, B: int, device) -> Tuple[torch.Tensor, torch.Tensor, int]:
+    """Columns of a captured step -> packed layout.  Where a column starts depends on how many ids the columns before
+    it hold in THIS batch, so the packing is a kernel that reads the counts on the device."""
+    from .. import _build
+
+    vals, offs, lens, room = [], [], [], 0
+    for c in cols:
+        if isinstance(c, PaddedRagged):
+            v, o, n = c._values, c._offsets, 0
+        elif torch.is_tensor(c):
+            v, o = c.to(device, non_blocking=True).contiguous(), None
+            n = int(v.numel()) // B
+        else:
+            v, o, n = c[0].to(device, non_blocking=True).contiguous(), c[1].to(device, non_blocking=True).contiguous(), 0
+        if v.dtype not in (torch.int32, torch.int64):
+            v = v.long()
+        if o is not None and o.dtype not in (torch.int32, torch.int64):
+            o = o.long()
+        vals.append(v.reshape(-1))
+        offs.append(o)
+        lens.append(n)
+        room += int(v.numel())
+    values = torch.empty(room, dtype=torch.int64, device=device)
+    offsets = torch.empty(len(cols) * B + 1, dtype=torch.int32, device=device)
+    _build.cuda_ext().pack_columns(vals, offs, lens, B, values, offsets)
+    return values, offsets, B

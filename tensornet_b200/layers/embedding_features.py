@@ -18,9 +18,9 @@ import torch
 from torch import nn
 
 from .. import core
-from ..data.features import PACKED_KEY, gather_columns
+from ..data.features import PACKED_KEY, gather_columns, padded_columns
 from ..feature_column import EmbeddingColumn
-from ..ops.embedding import pull_pool
+from ..ops.embedding import expand_bag_labels, pull_pool
 
 
 class EmbeddingFeatures(nn.Module):
@@ -112,6 +112,8 @@ class EmbeddingFeatures(nn.Module):
             y = features[self._target_columns[0]].to(dev, non_blocking=True).reshape(-1).float()
             if offsets is None:
                 labels, label_mod = y, B
+            elif ids.is_cuda:
+                labels = expand_bag_labels(y, offsets, S, int(ids.numel()))
             else:
                 lens = (offsets[1:] - offsets[:-1]).long()
                 labels = torch.repeat_interleave(y.repeat(S), lens, output_size=int(ids.numel()))
@@ -129,7 +131,9 @@ class EmbeddingFeatures(nn.Module):
         self.table.set_training(training)
         ids, offsets, B, labels, label_mod, count = self._pull_args(features, training)
         S = len(self._keys)
-        out = pull_pool(self._anchor, self.link, ids, offsets, B, S, self.combiner, labels, label_mod, count)
+        # a captured step's buffers have room to spare: the last offset is the number of ids of this batch
+        n_dev = offsets[-1:] if offsets is not None and padded_columns(features, self._keys) else None
+        out = pull_pool(self._anchor, self.link, ids, offsets, B, S, self.combiner, labels, label_mod, count, n_dev)
         self._pending_push = count
         if self.is_concat:
             return out

@@ -24,7 +24,7 @@ from torch import nn
 
 from .. import core, metric as _metric
 from .._opentelemetry import phase, start_as_current_span
-from ..data.features import PackedFeatures, Ragged
+from ..data.features import PackedFeatures, PaddedPacked, PaddedRagged, Ragged
 from ..ops import functional as F
 from ..parallel.symm import verify_all_arenas
 
@@ -97,21 +97,62 @@ def _flatten(obj, out: List[torch.Tensor]):
     return ("const", obj)
 
 
-def _unflatten(spec, it):
+def _unflatten(spec, it, padded: bool = False):
+    """``padded``: ragged features come back as the padded stand-ins of a captured step."""
     kind = spec[0]
     if kind == "t":
         return next(it)
     if kind == "packed":
         _, keys, bs, sub = spec
         vals = [None if s is None else _unflatten(s, it) for s in sub]
+        if padded and vals[0] is None:
+            return PaddedPacked(list(keys), vals[1], vals[2], bs)
         return PackedFeatures(list(keys), vals[0], vals[1], vals[2], bs)
     if kind == "ragged":
-        return Ragged(*[_unflatten(s, it) for s in spec[1]])
+        return (PaddedRagged if padded else Ragged)(*[_unflatten(s, it) for s in spec[1]])
     if kind == "dict":
-        return {k: _unflatten(s, it) for k, s in spec[1]}
+        return {k: _unflatten(s, it, padded) for k, s in spec[1]}
     if kind == "list":
-        return [_unflatten(s, it) for s in spec[1]]
+        return [_unflatten(s, it, padded) for s in spec[1]]
     return spec[1]
+
+
+def _ragged_leaves(spec) -> List[int]:
+    """Positions, among the leaves of ``spec``, of the id vectors whose length differs from batch to batch; the leaf
+    behind each is its offsets."""
+    out, at = [], 0
+
+    def walk(s):
+        nonlocal at
+        kind = s[0]
+        if kind == "t":
+            at += 1
+        elif kind == "packed":
+            if s[3][0] is None:
+                out.append(at)
+            at += sum(x is not None for x in s[3])
+        elif kind == "ragged":
+            out.append(at)
+            at += 2
+        elif kind == "dict":
+            for _, x in s[1]:
+                walk(x)
+        elif kind == "list":
+            for x in s[1]:
+                walk(x)
+
+    walk(spec)
+    return out
+
+
+def _room_for(n: int, spare: bool) -> int:
+    """Length of the static buffer for a vector of ``n`` ids: the next multiple of an eighth of its magnitude; with
+    ``spare`` (lengths have been seen to differ) an eighth and six standard deviations of a Poisson count on top, so
+    that later batches fit as well."""
+    if spare:
+        n = n + n // 8 + int(6 * n ** 0.5)
+    g = max(32, 1 << max(0, int(n).bit_length() - 4))
+    return max(g, (int(n) + g - 1) // g * g)
 
 
 def _is_static(spec) -> bool:
@@ -173,6 +214,7 @@ class _GraphPair:
         self.done = [torch.cuda.Event(), torch.cuda.Event()]        # replay that last read set p has finished
         self.copied = [torch.cuda.Event(), torch.cuda.Event()]      # inputs of set p have landed
         self.done_recorded = [False, False]
+        self.read = [None, None]         # event behind the copy of set p's last loss to the host, when one was issued
         for e in self.copied:
             e.record()               # events get their CUDA handle at the first record
         self.turn = 0
@@ -198,6 +240,7 @@ class _GraphRing:
         self.done = [torch.cuda.Event() for _ in range(self.SETS)]       # the graph that ran set i as its step is over
         self.copied = [torch.cuda.Event() for _ in range(self.SETS)]     # inputs of set i have landed
         self.done_recorded = [False] * self.SETS
+        self.read = [None] * self.SETS                                   # as in _GraphPair
         for e in self.copied:
             e.record()
         self.sig: List[Any] = [None] * self.SETS                        # which batch (leaf addresses) set i holds
@@ -264,6 +307,9 @@ class Model(nn.Module):
         self._flat_cache = None                      # (batch object, its flattened form) of the batch named as next
         self._fronts_now = ()                        # (layer, next ids) of the step being issued
         self._last_done = None                       # event behind the last replayed step (None after an eager one)
+        self._last_set = None                        # (captured sets, index) of the last replayed step
+        self._padded_keys: Dict[Any, List[Any]] = {} # ragged batches: (structure, fixed shapes) -> [(rooms, key of ``_graphs``)]
+        self._padded_off = False                     # a captured step needed exact lengths
         self._max_graphs = 8
         self._graph_key = None
         self._static_leaves: List[torch.Tensor] = []
@@ -492,6 +538,35 @@ class Model(nn.Module):
         moved = [t.to(dev, non_blocking=True) for t in leaves]
         return _unflatten(spec, iter(moved)), spec, leaves
 
+    def _padded_plan(self, spec, leaves):
+        """For a batch with ragged slots in host memory: ``(key, rooms per ragged leaf)`` of the captured step it can run
+        in, or None.  The captured buffers have room to spare and the kernels read the number of ids from the last
+        offset, so that batches of many lengths share one capture.  One GPU only: with several, every rank would have
+        to capture at the same step."""
+        if self._padded_off or core.runtime().world > 1 or any(t.is_cuda for t in leaves):
+            return None
+        ragged = _ragged_leaves(spec)
+        if not ragged:
+            return None
+        # ids beyond the last offset (or missing ones) are the caller's to explain: such a batch runs at its exact length
+        from .. import _build
+        n = _build.cuda_ext().ragged_lengths([leaves[i + k] for i in ragged for k in (0, 1)])
+        if not n:
+            return None
+        at = set(ragged)
+        base = (spec, tuple((None if i in at else t.shape, t.dtype) for i, t in enumerate(leaves)))
+        known = self._padded_keys.setdefault(base, [])
+        best = None
+        for rooms, key in known:
+            # a much too large capture is not used: its kernels are launched for the room, not for the ids
+            if key in self._graphs and all(a <= r for a, r in zip(n, rooms)) and sum(rooms) <= 2 * sum(n) + 4096:
+                if best is None or sum(rooms) < sum(best[0]):
+                    best = (rooms, key)
+        if best is None:
+            rooms = tuple(_room_for(a, bool(known)) for a in n)
+            best = (rooms, (base, rooms))
+        return best[1], dict(zip(ragged, best[0]))
+
     def _eager_step(self, features, labels):
         self._last_done = None
         (f, y), _, _ = self._to_device((features, labels))
@@ -517,8 +592,13 @@ class Model(nn.Module):
         rt = core.runtime()
         leaves: List[torch.Tensor] = []
         spec = _flatten((features, labels), leaves)
-        key = (spec, tuple((t.shape, t.dtype) for t in leaves))
-        what = graph_decision(rt.world, key in self._graphs, _is_static(spec), len(self._graphs) + len(self._rings), self._max_graphs,
+        key, rooms = (spec, tuple((t.shape, t.dtype) for t in leaves)), None
+        static = _is_static(spec)
+        if not static:
+            plan = self._padded_plan(spec, leaves)
+            if plan is not None:
+                key, rooms = plan
+        what = graph_decision(rt.world, key in self._graphs, static or rooms is not None, len(self._graphs) + len(self._rings), self._max_graphs,
                               self._eager_steps, self._graph_warmup)
         if what == "eager":
             self._eager_steps += 1
@@ -527,8 +607,16 @@ class Model(nn.Module):
                 rt.check_status()      # surface device-side errors before the step is frozen into a graph
             return loss
         if what == "capture":
-            if _is_static(spec):
+            if static:
                 self._capture(spec, leaves, key)
+            elif rooms is not None:
+                try:
+                    self._capture(spec, leaves, key, rooms)
+                    self._padded_keys[key[0]].append((key[1], key))
+                except Exception:           # something in the step wants exact lengths (or cannot be captured): no padding any more
+                    torch.cuda.synchronize()
+                    self._padded_off = True
+                    return self._eager_step(features, labels)
             else:
                 try:
                     self._capture(spec, leaves, key)
@@ -541,20 +629,28 @@ class Model(nn.Module):
         p = gp.turn
         gp.turn ^= 1
         main = torch.cuda.current_stream()
+        if rooms is not None:
+            leaves = [t if t.is_contiguous() else t.contiguous() for t in leaves]
+        read = gp.read[p]                        # the set's last loss must have left before its memory is written again
         if any(t.is_cuda for t in leaves):
+            if read is not None:
+                main.wait_event(read)
             # inputs produced on the device come with the stream order of whatever produced them
             torch._foreach_copy_(gp.leaves[p], [t if t.is_cuda else t.to(rt.device, non_blocking=True) for t in leaves])
         elif core.config.native_step_path and all(t.is_contiguous() for t in leaves):
             # one native call: copy stream waits for the replay that last read this input set, the leaves go host ->
             # device, their arrival is recorded and the compute stream waits for it
             self._ext.stage_inputs(gp.leaves[p], leaves, self._copy_stream.cuda_stream, main.cuda_stream,
-                                   gp.done[p].cuda_event if gp.done_recorded[p] else 0, gp.copied[p].cuda_event, 0)
+                                   gp.done[p].cuda_event if gp.done_recorded[p] else 0, gp.copied[p].cuda_event,
+                                   read.cuda_event if read is not None else 0)
         else:
             copy = self._copy_stream
             copy.wait_event(gp.done[p])          # the replay that last read this input set is over
+            if read is not None:
+                copy.wait_event(read)
             with torch.cuda.stream(copy):
                 for dst, src in zip(gp.leaves[p], leaves):
-                    dst.copy_(src, non_blocking=True)
+                    (dst if dst.shape == src.shape else dst[: src.numel()]).copy_(src, non_blocking=True)
                 gp.copied[p].record(copy)
             main.wait_event(gp.copied[p])
         if self.optimizer is not None:
@@ -563,6 +659,7 @@ class Model(nn.Module):
         gp.done[p].record(main)
         gp.done_recorded[p] = True
         self._last_done = gp.done[p]
+        self._last_set, gp.read[p] = (gp, p), None
         if self.optimizer is not None:
             self.optimizer.iterations += 1
             self.optimizer.table.step_count += 1
@@ -578,14 +675,17 @@ class Model(nn.Module):
     def _stage(self, ring, i, leaves, sig, main):
         """Inputs ``leaves`` into static set i of the ring (host leaves: native staged copy on the copy stream; device
         leaves: one foreach copy in stream order)."""
+        read, ring.read[i] = ring.read[i], None
         if any(t.is_cuda for t in leaves):
+            if read is not None:
+                main.wait_event(read)
             dev = core.runtime().device
             torch._foreach_copy_(ring.leaves[i], [t if t.is_cuda else t.to(dev, non_blocking=True) for t in leaves])
         else:
             srcs = [t if t.is_contiguous() else t.contiguous() for t in leaves]
             self._ext.stage_inputs(ring.leaves[i], srcs, self._copy_stream.cuda_stream, main.cuda_stream,
                                    ring.done[i].cuda_event if ring.done_recorded[i] else 0, ring.copied[i].cuda_event,
-                                   0)
+                                   read.cuda_event if read is not None else 0)
         ring.sig[i] = sig
 
     def _flat(self, batch):
@@ -656,6 +756,7 @@ class Model(nn.Module):
         setattr_(self, "_static_leaves", ring.leaves[cur])
         setattr_(self, "_static_loss", loss)
         setattr_(self, "_last_done", ring.done[cur])
+        setattr_(self, "_last_set", (ring, cur))
         return loss
 
     def _capture_ring(self, spec, leaves, nleaves, key):
@@ -718,8 +819,9 @@ class Model(nn.Module):
         rt.barrier()                        # captures take a different time on every rank; line the ranks up again
         return ring
 
-    def _capture(self, spec, leaves, key):
-        """Capture the step twice (two sets of static inputs that take turns) into one memory pool."""
+    def _capture(self, spec, leaves, key, rooms=None):
+        """Capture the step twice (two sets of static inputs that take turns) into one memory pool.  ``rooms``: length
+        of the static buffer of every ragged leaf (a batch may hold fewer ids)."""
         dev = core.runtime().device
         gp = _GraphPair()
         from .. import _build
@@ -733,15 +835,25 @@ class Model(nn.Module):
         loss_steps0 = self._loss_steps
         pool = None
         for p in range(2):
-            static_leaves = [torch.empty(t.shape, dtype=t.dtype, device=dev) for t in leaves]
+            static_leaves = [torch.empty(t.shape, dtype=t.dtype, device=dev) if rooms is None or i not in rooms else
+                             torch.zeros((rooms[i],), dtype=t.dtype, device=dev) for i, t in enumerate(leaves)]
             for dst, src in zip(static_leaves, leaves):
-                dst.copy_(src, non_blocking=True)
-            f, y = _unflatten(spec, iter(static_leaves))
+                (dst if dst.shape == src.shape else dst[: src.numel()]).copy_(src, non_blocking=True)
+            f, y = _unflatten(spec, iter(static_leaves), padded=rooms is not None)
             torch.cuda.synchronize()
             g = torch.cuda.CUDAGraph()
             c0 = ext.launch_count()
-            with torch.cuda.graph(g, pool=pool):
-                static_loss = self._step_impl(f, y)
+            try:
+                with torch.cuda.graph(g, pool=pool):
+                    static_loss = self._step_impl(f, y)
+            except Exception:
+                if self.optimizer is not None:
+                    self.optimizer.iterations, self.optimizer.table.step_count = iters, steps0
+                self._loss_steps = loss_steps0
+                for layer in self.sparse_layers():
+                    if hasattr(layer, "_pending_push"):
+                        layer._pending_push = False
+                raise
             if p == 0:
                 self._launches_per_step = ext.launch_count() - c0
                 self._graph_loss_steps = self._loss_steps - loss_steps0
@@ -895,7 +1007,11 @@ class Model(nn.Module):
             return iter(())
         import itertools
         rest = itertools.chain([first], it)
-        return rest if _is_static(_flatten(first, [])) else self._prefetched(rest)
+        leaves: List[torch.Tensor] = []
+        spec = _flatten(first, leaves)
+        if _is_static(spec) or self._padded_plan(spec, leaves) is not None:
+            return rest
+        return self._prefetched(rest)
 
     def fit(self, dataset: Iterable, epochs: int = 1, steps_per_epoch: Optional[int] = None, callbacks: Sequence = (),
             verbose: int = 0, log_every: int = 100, prefetch: bool = True, record_step_loss: bool = False):
@@ -957,6 +1073,8 @@ class Model(nn.Module):
                                     # carries nothing between two replayed steps
                                     self._ext.read_scalar_async(pinned, slot, last, self._read_stream.cuda_stream,
                                                                 events[slot].cuda_event, self._last_done.cuda_event)
+                                    sets, k = self._last_set
+                                    sets.read[k] = events[slot]
                                 else:
                                     self._ext.read_scalar_async(pinned, slot, last, torch.cuda.current_stream().cuda_stream,
                                                                 events[slot].cuda_event, 0)

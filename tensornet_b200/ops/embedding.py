@@ -36,8 +36,9 @@ def _bag_scale(offsets, nbags, combiner, device):
 
 class _PullPool(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, anchor, table, ids, offsets, B, S, combiner, labels, label_mod, training):
-        inverse = table.pull(ids, labels, label_mod, training)
+    def forward(ctx, anchor, table, ids, offsets, B, S, combiner, labels, label_mod, training, n_dev):
+        inverse = table.pull(ids, labels, label_mod, training) if n_dev is None else \
+            table.pull(ids, labels, label_mod, training, n_dev=n_dev)
         pd = table.pdim
         if ids.is_cuda:
             out = torch.empty((B, S * pd), dtype=torch.float32, device=ids.device)
@@ -76,14 +77,22 @@ class _PullPool(torch.autograd.Function):
             inv = inverse.long()
             ok = inv >= 0
             table.gU[:, :dim].index_add_(0, inv[ok], gb[bag][ok])
-        return (None,) * 10
+        return (None,) * 11
 
 
-def pull_pool(anchor, table, ids, offsets, B, S, combiner="sum", labels=None, label_mod=0, training=True):
+def pull_pool(anchor, table, ids, offsets, B, S, combiner="sum", labels=None, label_mod=0, training=True, n_dev=None):
     """``ids``: all ids of the layer's S columns, column after column (bag ``s*B + b``).
-    ``offsets``: int32 ``[S*B + 1]`` bag boundaries, or None when every bag holds exactly one id."""
+    ``offsets``: int32 ``[S*B + 1]`` bag boundaries, or None when every bag holds exactly one id.  ``n_dev`` (GPU): one
+    int32 on the device saying how many of ``ids`` are there."""
     return _PullPool.apply(anchor, table, ids, offsets, B, S, COMBINERS[combiner] if isinstance(combiner, str) else combiner,
-                           labels, label_mod, training)
+                           labels, label_mod, training, n_dev)
+
+
+def expand_bag_labels(y: torch.Tensor, offsets: torch.Tensor, S: int, n_ids: int) -> torch.Tensor:
+    """Per id the label of its example (GPU): ``y`` fp32 ``[B]``, bag ``s*B + b`` of ``offsets`` belongs to example b."""
+    out = torch.zeros(n_ids, dtype=torch.float32, device=y.device)
+    _build.cuda_ext().expand_bag_labels(y, offsets, S, out)
+    return out
 
 
 class _PullSeq(torch.autograd.Function):

@@ -351,10 +351,11 @@ class GpuSparseLink:
             rt.barrier()
 
     def pull(self, ids: torch.Tensor, labels: Optional[torch.Tensor] = None, label_mod: int = 0, training: bool = True,
-             inverse: Optional[torch.Tensor] = None, lookup_only: bool = False) -> torch.Tensor:
+             inverse: Optional[torch.Tensor] = None, lookup_only: bool = False, n_dev: Optional[torch.Tensor] = None) -> torch.Tensor:
         """Dedup ``ids``, fetch (creating on miss) their rows from the owning GPUs into ``self.U`` and
         return ``inverse``: the row of ``self.U`` holding each id's embedding.  ``lookup_only`` (inference)
-        never creates rows: signs no shard holds come back as zeros."""
+        never creates rows: signs no shard holds come back as zeros.  ``n_dev``: one int32 on the device, the number
+        of ids that are there (``ids`` of a captured step has room for more)."""
         n = ids.numel()
         front, self._front = self._front, None
         front_done = False
@@ -368,7 +369,7 @@ class GpuSparseLink:
             inverse = torch.empty(n, dtype=torch.int32, device=self.dev)
         self._last_n_ids = n
         with phase("tn.sparse_pull"):
-            self.ctx.pull(ids.reshape(-1), inverse, labels, int(label_mod), bool(training), bool(lookup_only), front_done)
+            self.ctx.pull(ids.reshape(-1), inverse, labels, int(label_mod), bool(training), bool(lookup_only), front_done, n_dev)
         return inverse
 
     def fork_front(self):
