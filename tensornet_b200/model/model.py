@@ -27,6 +27,7 @@ from .._opentelemetry import phase, start_as_current_span
 from ..data.features import PackedFeatures, PaddedPacked, PaddedRagged, Ragged
 from ..ops import functional as F
 from ..parallel.symm import verify_all_arenas
+from ..utils.capture import capture
 
 
 # ----------------------------------------------------------------------------------------------
@@ -248,6 +249,25 @@ class _GraphRing:
         self.links: List[Any] = []
 
 
+class _PredictSets:
+    """Two captures of the scoring step that take turns, like :class:`_GraphPair`."""
+
+    def __init__(self):
+        self.graphs: List[Any] = []
+        self.leaves: List[List[torch.Tensor]] = []
+        self.pred: List[torch.Tensor] = []
+        self.done = [torch.cuda.Event(), torch.cuda.Event()]
+        self.copied = [torch.cuda.Event(), torch.cuda.Event()]
+        self.read = [None, None]         # event behind the copy of set p's last predictions to the host
+        self.used = [False, False]
+        for e in self.copied + self.done:
+            e.record()
+        self.turn = 0
+
+
+_PREDICT_RING = 16   # pinned buffers for predictions on their way to the host: how far the host may run ahead
+
+
 class _StatusPoll:
     """Looks at the device status words every few steps without stalling: an asynchronous copy into pinned memory
     now, read when the next poll comes round.  A device error therefore surfaces at most two polling periods
@@ -306,10 +326,15 @@ class Model(nn.Module):
         self._ring_refused = False
         self._flat_cache = None                      # (batch object, its flattened form) of the batch named as next
         self._fronts_now = ()                        # (layer, next ids) of the step being issued
+        self._loss_out = None                        # where the step being captured leaves its loss
+        self._loss_stream = None                     # the stream that copies it there
         self._last_done = None                       # event behind the last replayed step (None after an eager one)
         self._last_set = None                        # (captured sets, index) of the last replayed step
         self._padded_keys: Dict[Any, List[Any]] = {} # ragged batches: (structure, fixed shapes) -> [(rooms, key of ``_graphs``)]
         self._padded_off = False                     # a captured step needed exact lengths
+        self._predict_sets: Dict[Any, Any] = {}      # batch signature -> number of batches seen, then _PredictSets
+        self._predict_rooms: Dict[Any, List[Any]] = {}
+        self._predict_off = False                    # the scoring step cannot be captured
         self._max_graphs = 8
         self._graph_key = None
         self._static_leaves: List[torch.Tensor] = []
@@ -455,6 +480,9 @@ class Model(nn.Module):
             layer.link.next_ids = ids
         object.__setattr__(self, "_fronts_now", fronts)
         loss = self._step_body(features, labels)
+        if self._loss_stream is not None:      # the loss was copied out beside the backward pass
+            torch.cuda.current_stream().wait_stream(self._loss_stream)
+            object.__setattr__(self, "_loss_stream", None)
         object.__setattr__(self, "_fronts_now", ())
         for layer, _ in fronts:
             lk = layer.link
@@ -481,6 +509,15 @@ class Model(nn.Module):
             for m in self._host_metrics:
                 m.update_state(labels, pred)
         rt = core.runtime()
+        out = self._loss_out
+        if out is not None and loss.dtype == out.dtype and loss.numel() == 1:
+            # A captured step hands its loss over in memory of its own: the captures share one memory pool, in which the
+            # replay of the other capture writes its intermediates over this one's results.
+            main, side = torch.cuda.current_stream(), F._side_stream(rt.device)
+            side.wait_stream(main)
+            with torch.cuda.stream(side):
+                out.copy_(loss.detach().reshape(()))
+            object.__setattr__(self, "_loss_stream", side)
         for layer, _ in self._fronts_now:          # forward pass issued: the next batch's pull fronts start here
             layer.link.fork_front()
         with phase("tn.backward"):
@@ -529,7 +566,7 @@ class Model(nn.Module):
                     if rider is not None:
                         rider.dense_rider = None
                     self.optimizer.step(peers_past_backward=rt.peer_synced_pushes > before)
-        return loss.detach()
+        return loss.detach() if self._loss_stream is None else out.view(loss.shape)
 
     def _to_device(self, obj):
         dev = core.runtime().device
@@ -538,11 +575,13 @@ class Model(nn.Module):
         moved = [t.to(dev, non_blocking=True) for t in leaves]
         return _unflatten(spec, iter(moved)), spec, leaves
 
-    def _padded_plan(self, spec, leaves):
+    def _padded_plan(self, spec, leaves, captured=None, rooms_of=None):
         """For a batch with ragged slots in host memory: ``(key, rooms per ragged leaf)`` of the captured step it can run
         in, or None.  The captured buffers have room to spare and the kernels read the number of ids from the last
         offset, so that batches of many lengths share one capture.  One GPU only: with several, every rank would have
-        to capture at the same step."""
+        to capture at the same step.  ``captured`` / ``rooms_of``: the captures to look among (default: training steps)."""
+        captured = self._graphs if captured is None else captured
+        rooms_of = self._padded_keys if rooms_of is None else rooms_of
         if self._padded_off or core.runtime().world > 1 or any(t.is_cuda for t in leaves):
             return None
         ragged = _ragged_leaves(spec)
@@ -555,11 +594,11 @@ class Model(nn.Module):
             return None
         at = set(ragged)
         base = (spec, tuple((None if i in at else t.shape, t.dtype) for i, t in enumerate(leaves)))
-        known = self._padded_keys.setdefault(base, [])
+        known = rooms_of.setdefault(base, [])
         best = None
         for rooms, key in known:
             # a much too large capture is not used: its kernels are launched for the room, not for the ids
-            if key in self._graphs and all(a <= r for a, r in zip(n, rooms)) and sum(rooms) <= 2 * sum(n) + 4096:
+            if key in captured and all(a <= r for a, r in zip(n, rooms)) and sum(rooms) <= 2 * sum(n) + 4096:
                 if best is None or sum(rooms) < sum(best[0]):
                     best = (rooms, key)
         if best is None:
@@ -794,8 +833,12 @@ class Model(nn.Module):
             g = torch.cuda.CUDAGraph()
             c0 = ext.launch_count()
             f, y = feats[i]
-            with torch.cuda.graph(g, pool=pool):
-                static_loss = self._step_impl(f, y, next_features=feats[(i + 1) % ring.SETS][0])
+            self._loss_out = torch.empty((), dtype=torch.float32, device=dev)
+            try:
+                with capture(g, pool):
+                    static_loss = self._step_impl(f, y, next_features=feats[(i + 1) % ring.SETS][0])
+            finally:
+                self._loss_out = self._loss_stream = None
             if pool is None:
                 self._launches_per_step = ext.launch_count() - c0
                 self._graph_loss_steps = self._loss_steps - loss_steps0
@@ -843,8 +886,9 @@ class Model(nn.Module):
             torch.cuda.synchronize()
             g = torch.cuda.CUDAGraph()
             c0 = ext.launch_count()
+            self._loss_out = torch.empty((), dtype=torch.float32, device=dev)
             try:
-                with torch.cuda.graph(g, pool=pool):
+                with capture(g, pool):
                     static_loss = self._step_impl(f, y)
             except Exception:
                 if self.optimizer is not None:
@@ -854,6 +898,8 @@ class Model(nn.Module):
                     if hasattr(layer, "_pending_push"):
                         layer._pending_push = False
                 raise
+            finally:
+                self._loss_out = self._loss_stream = None
             if p == 0:
                 self._launches_per_step = ext.launch_count() - c0
                 self._graph_loss_steps = self._loss_steps - loss_steps0
@@ -901,6 +947,96 @@ class Model(nn.Module):
             pred = torch.sigmoid(self(f))
         return y, pred
 
+    # ---- captured scoring steps ---------------------------------------------------------------------------------
+    def _predict_captured(self, features):
+        """Issue the captured scoring step for a batch in host memory: ``(sets, index)`` whose ``pred[index]`` will hold
+        the predictions, or None when this batch is to be scored eagerly."""
+        rt = core.runtime()
+        if not self._use_graph or self._predict_off or rt.world > 1:
+            return None
+        leaves: List[torch.Tensor] = []
+        spec = _flatten(features, leaves)
+        if not leaves or any(t.is_cuda or not t.is_contiguous() for t in leaves):
+            return None
+        key, rooms = (spec, tuple((t.shape, t.dtype) for t in leaves)), None
+        try:
+            if not _is_static(spec):
+                plan = self._padded_plan(spec, leaves, self._predict_sets, self._predict_rooms)
+                if plan is None:
+                    return None
+                key, rooms = plan
+            sets = self._predict_sets.get(key)
+        except TypeError:                    # a feature that is no tensor and cannot be compared: nothing to recognise it by
+            return None
+        if not isinstance(sets, _PredictSets):
+            # the first batch of a kind runs eagerly, the second one is captured
+            if len(self._predict_sets) > 64:
+                self._predict_sets.clear()
+                self._predict_rooms.clear()
+                return None
+            if rooms is not None:
+                known = self._predict_rooms[key[0]]
+                if (key[1], key) not in known:
+                    known.append((key[1], key))
+            if sets is None:
+                self._predict_sets[key] = 1
+                return None
+            with torch.no_grad():            # shape and type of the result, from the batch itself
+                (f,), _, _ = self._to_device((features,))
+                like = torch.sigmoid(self(f))
+            self._predict_shape, self._predict_dtype = like.shape, like.dtype
+            held = [k for k, v in self._predict_sets.items() if isinstance(v, _PredictSets)]
+            if len(held) >= self._max_graphs > 0:
+                self._predict_sets.pop(held[0])
+            try:
+                sets = self._predict_sets[key] = self._capture_predict(spec, leaves, rooms)
+            except Exception:                # something in the forward pass cannot be captured
+                torch.cuda.synchronize()
+                self._predict_off = True
+                self._predict_sets.clear()
+                return None
+        for link in self._predict_links:
+            link.table.set_training(False)
+            if link._front is not None:      # a front that ran ahead for the next training batch
+                link.discard_front()
+        p = sets.turn
+        sets.turn ^= 1
+        main = torch.cuda.current_stream()
+        read, sets.read[p] = sets.read[p], None
+        self._ext.stage_inputs(sets.leaves[p], leaves, self._copy_stream.cuda_stream, main.cuda_stream,
+                               sets.done[p].cuda_event if sets.used[p] else 0, sets.copied[p].cuda_event,
+                               read.cuda_event if read is not None else 0)
+        sets.graphs[p].replay()
+        sets.done[p].record(main)
+        sets.used[p] = True
+        return sets, p
+
+    def _capture_predict(self, spec, leaves, rooms):
+        from .. import _build
+        self._ext = _build.cuda_ext()
+        dev = core.runtime().device
+        self._predict_links = [lk for layer in self.sparse_layers() for lk in (getattr(layer, "links", None) or [getattr(layer, "link", None)])
+                               if lk is not None and hasattr(lk, "discard_front")]
+        for lk in self._predict_links:
+            if lk._front is not None:
+                lk.discard_front()
+        sets, pool = _PredictSets(), None
+        for _ in range(2):
+            static = [torch.empty(t.shape, dtype=t.dtype, device=dev) if rooms is None or i not in rooms else
+                      torch.zeros((rooms[i],), dtype=t.dtype, device=dev) for i, t in enumerate(leaves)]
+            f = _unflatten(spec, iter(static), padded=rooms is not None)
+            torch.cuda.synchronize()
+            g = torch.cuda.CUDAGraph()
+            # the predictions live outside the captures' shared memory pool, where the other capture would overwrite them
+            pred = torch.empty(self._predict_shape, dtype=self._predict_dtype, device=dev)
+            with torch.no_grad(), capture(g, pool):
+                torch.sigmoid(self(f), out=pred)
+            pool = pool or g.pool()
+            sets.graphs.append(g)
+            sets.leaves.append(static)
+            sets.pred.append(pred)
+        return sets
+
     def predict_on_batch(self, x):
         with start_as_current_span("predict_on_batch"):
             return self.predict_step((x, None))[1]
@@ -915,13 +1051,43 @@ class Model(nn.Module):
                 cb.set_model(self)
                 cb.on_predict_begin()
             ys, ps = [], []
+            self.eval()
+            ring, flying = [], []            # pinned buffers; (position in ps, buffer, event) of copies on their way
             for i, batch in enumerate(dataset):
                 if steps is not None and i >= steps:
                     break
-                y, p = self.predict_step(batch)
-                ps.append(p.cpu())
-                if y is not None:
-                    ys.append(y.cpu())
+                features, labels = batch if isinstance(batch, (tuple, list)) and len(batch) == 2 else (batch, None)
+                issued = self._predict_captured(features) if not self.training else None
+                if issued is None:
+                    y, p = self.predict_step(batch)
+                    ps.append(p.cpu())
+                    if y is not None:
+                        ys.append(y.cpu())
+                    continue
+                # predictions go to the host behind the step on a stream of their own; the host runs ahead meanwhile
+                sets, k = issued
+                pred = sets.pred[k]
+                if len(flying) >= _PREDICT_RING:
+                    at, buf, ev = flying.pop(0)
+                    ev.synchronize()
+                    ps[at] = buf.clone()
+                    ring.append((buf, ev))
+                fit = [j for j, (b, _) in enumerate(ring) if b.shape == pred.shape and b.dtype == pred.dtype]
+                buf, ev = ring.pop(fit[0]) if fit else (torch.empty(pred.shape, dtype=pred.dtype, pin_memory=True), torch.cuda.Event())
+                if getattr(self, "_read_stream", None) is None:
+                    self._read_stream = torch.cuda.Stream(device=pred.device)
+                with torch.cuda.stream(self._read_stream):
+                    self._read_stream.wait_event(sets.done[k])
+                    buf.copy_(pred, non_blocking=True)
+                    ev.record()
+                sets.read[k] = ev
+                flying.append((len(ps), buf, ev))
+                ps.append(None)
+                if labels is not None:
+                    ys.append(labels.cpu())
+            for at, buf, ev in flying:
+                ev.synchronize()
+                ps[at] = buf
             core.runtime().check_status()
             for cb in callbacks:
                 cb.on_predict_end()
@@ -1040,7 +1206,8 @@ class Model(nn.Module):
                         e.record()           # events get their CUDA handle at the first record
                     from .. import _build
                     self._ext = _build.cuda_ext()
-                    self._read_stream = torch.cuda.Stream(device=rt.device)
+                    if getattr(self, "_read_stream", None) is None:
+                        self._read_stream = torch.cuda.Stream(device=rt.device)
                 pinned = self._pinned_loss
                 events = self._loss_events
             for cb in callbacks:

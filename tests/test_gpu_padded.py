@@ -62,3 +62,27 @@ def test_a_model_that_reads_exact_lengths_is_not_padded(tn_gpu, status_ok):
     m.compile(optimizer=tn.optimizer.Optimizer(tn.core.Adam(learning_rate=1e-3)))
     losses = [float(m.train_on_batch(f, y)) for f, y in data]
     assert m._padded_off and all(l == l for l in losses)
+
+
+@pytest.mark.parametrize("form", ["packed", "columns", "single"])
+def test_captured_scoring_equals_the_eager_scoring(tn_gpu, status_ok, form):
+    """More batches than there are pinned buffers, a shorter last batch, training in between (whose run-ahead front the
+    scoring must not take for its own).  Same kernels on the same numbers: equal to bf16 rounding of the towers."""
+    tn = tn_gpu
+    slots, B = ["a", "b", "c"], 48
+    if form == "single":
+        g = torch.Generator().manual_seed(5)
+        data = [({tn.data.PACKED_KEY: tn.data.PackedFeatures(slots, ids=torch.randint(0, 300, (3, B if k < 21 else 7), generator=g))},
+                 (torch.rand(B if k < 21 else 7, generator=g) < 0.3).float()) for k in range(22)]
+    else:
+        data = _batches(tn, slots, B, 22, form)
+    torch.manual_seed(2)
+    m = tn.models.DeepFM(slots, slots, dnn_hidden_units=(32, 16), embedding_dim=8, bucket_size=5 * B, table_rows=1 << 13)
+    m.compile(optimizer=tn.optimizer.Optimizer(tn.core.Adam(learning_rate=1e-3)))
+    for _ in range(2):
+        m.fit(data[:10])
+        y, p = m.predict(data)
+        assert m._predict_sets and not m._predict_off
+        want = torch.cat([m.predict_on_batch(f).cpu() for f, _ in data])
+        assert p.shape == want.shape and torch.equal(y, torch.cat([l for _, l in data]))
+        assert torch.allclose(p, want, atol=1e-5), float((p - want).abs().max())
