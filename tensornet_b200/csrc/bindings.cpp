@@ -354,7 +354,7 @@ void gemm(at::Tensor A, at::Tensor B, at::Tensor C, int M, int N, int K, int lda
           bool accumulate, bool relu, c10::optional<at::Tensor> bias, c10::optional<at::Tensor> mask_aux,
           c10::optional<at::Tensor> had_x0, c10::optional<at::Tensor> had_xl, int ld_aux, int ones_col, int n_store,
           int split_k, int BN, at::Tensor status, c10::optional<at::Tensor> prof, c10::optional<at::Tensor> gate_flags,
-          c10::optional<at::Tensor> gate_epoch, int gate_world, uint64_t gate_wait_ns, int m_halves, c10::optional<at::Tensor> aux_out) {
+          c10::optional<at::Tensor> gate_epoch, int gate_world, uint64_t gate_wait_ns, int m_halves, c10::optional<at::Tensor> aux_out, int cluster_k) {
   TORCH_CHECK(A.is_cuda() && B.is_cuda() && C.is_cuda(), "gemm: CUDA tensors");
   TORCH_CHECK(A.scalar_type() == at::kBFloat16 && B.scalar_type() == at::kBFloat16, "gemm: bf16 operands");
   c10::cuda::CUDAGuard guard(A.device());
@@ -372,6 +372,7 @@ void gemm(at::Tensor A, at::Tensor B, at::Tensor C, int M, int N, int K, int lda
   d.status = ptr_of<int>(status);
   d.prof = prof.has_value() ? ptr_of<unsigned long long>(*prof) : nullptr;
   d.m_halves = m_halves;
+  d.cluster_k = cluster_k;
   if (aux_out.has_value()) {
     TORCH_CHECK(aux_out->scalar_type() == at::kBFloat16 && aux_out->stride(0) == ld_aux, "gemm: aux_out must be bf16 with row stride ld_aux");
     d.aux_out = aux_out->data_ptr();
@@ -480,7 +481,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("mask_aux"), py::arg("had_x0"), py::arg("had_xl"), py::arg("ld_aux"), py::arg("ones_col"), py::arg("n_store"),
         py::arg("split_k"), py::arg("BN"), py::arg("status"), py::arg("prof") = py::none(),
         py::arg("gate_flags") = py::none(), py::arg("gate_epoch") = py::none(), py::arg("gate_world") = 0, py::arg("gate_wait_ns") = 0,
-        py::arg("m_halves") = 0, py::arg("aux_out") = py::none());
+        py::arg("m_halves") = 0, py::arg("aux_out") = py::none(), py::arg("cluster_k") = 0);
   m.def("launch_count", []() { return g_launches.load(); });
 
   // ---- per-step host path of a replayed training step --------------------------------------------

