@@ -343,6 +343,151 @@ struct BnCtx {
   }
 };
 
+// Device address of a host tensor that kernels may read in place (page-locked and mapped), else null.
+const void* mapped_host_ptr(const at::Tensor& t) {
+  if (t.is_cuda() || t.numel() == 0 || !t.is_contiguous() || !t.is_pinned()) return nullptr;
+  void* p = nullptr;
+  if (cudaHostGetDevicePointer(&p, t.data_ptr(), 0) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+  return p;
+}
+
+// InferenceEngine's request path: lookup + pooling, the layers of the tower, head and sigmoid, launched from one call.
+// Holds the dictionary's descriptor; weights come with every call (training may have re-pointed them).
+struct ServeCtx {
+  tn::TableView t{};
+  py::dict keep;
+  int S, combiner;
+  std::vector<int> dims;           // tower widths, input first
+  bool relu_last;
+  ServeCtx(py::dict table, int S_, int combiner_, std::vector<int> dims_, bool relu_last_)
+      : keep(table), S(S_), combiner(combiner_), dims(std::move(dims_)), relu_last(relu_last_) {
+    t = table_from_dict(table);
+    TORCH_CHECK(t.dim % 4 == 0 && t.stride % 4 == 0, "serving: dim must be a multiple of 4");
+    TORCH_CHECK(dims.size() >= 2 && dims.size() <= (size_t)tn::kServeMaxLayers + 1 && dims[0] == S * t.dim, "serving: tower input width");
+  }
+  static int pad8(int n) { return (n + 7) / 8 * 8; }
+  struct CopyLane { cudaStream_t stream = nullptr; cudaEvent_t begin = nullptr, end = nullptr; };
+  // one per thread and device: threads that serve side by side do not wait for one another's copies
+  static CopyLane& copy_lane(int device) {
+    static thread_local CopyLane lanes[64];
+    CopyLane& c = lanes[device & 63];
+    if (c.stream == nullptr) {
+      check(cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking), "serving: stream");
+      check(cudaEventCreateWithFlags(&c.begin, cudaEventDisableTiming), "serving: event");
+      check(cudaEventCreateWithFlags(&c.end, cudaEventDisableTiming), "serving: event");
+    }
+    return c;
+  }
+
+  // `weights`: fp32 [N, pad8(K + 1)] per layer; `shadows`: their bf16 copies when something keeps them current, else empty.
+  at::Tensor forward(at::Tensor ids, c10::optional<at::Tensor> offsets, int B, const std::vector<at::Tensor>& weights,
+                     const std::vector<at::Tensor>& shadows, at::Tensor head_w, at::Tensor status) {
+    const int L = (int)dims.size() - 1;
+    const bool cast_needed = shadows.empty();
+    TORCH_CHECK((int)weights.size() == L && (cast_needed || (int)shadows.size() == L) && head_w.numel() == dims[L] + 1 && head_w.is_cuda() &&
+                    head_w.is_contiguous() && head_w.scalar_type() == at::kFloat, "serving: weights");
+    TORCH_CHECK(ids.scalar_type() == at::kLong && ids.is_contiguous() && B >= 1, "serving: contiguous int64 ids");
+    TORCH_CHECK(offsets.has_value() ? offsets->numel() == (int64_t)S * B + 1 && offsets->is_contiguous() && offsets->scalar_type() == at::kInt
+                                    : ids.numel() == (int64_t)S * B, "serving: one bag per slot and example");
+    c10::cuda::CUDAGuard guard(head_w.device());
+    const cudaStream_t st = at::cuda::getCurrentCUDAStream().stream();
+    const auto dev = head_w.device();
+    // Ids and offsets: small ones in place when the kernels can reach them (a copy costs its launch and a wait, 3 us);
+    // beyond that the copy engine is the faster reader (44 against 22 GB/s at 819 KB).
+    const bool on_host = !ids.is_cuda() && ids.numel() > 0;
+    const size_t in_bytes = (size_t)ids.numel() * 8 + (offsets.has_value() ? (size_t)offsets->numel() * 4 : 0);
+    at::Tensor hold_ids = ids, hold_off = offsets.has_value() ? *offsets : at::Tensor();
+    const bool off_host = hold_off.defined() && !hold_off.is_cuda();
+    const void *mid = nullptr, *moff = nullptr;
+    if (in_bytes <= 128 * 1024) {
+      if (on_host) mid = mapped_host_ptr(ids);
+      if (off_host) moff = mapped_host_ptr(hold_off);
+    }
+    const bool copy_ids = on_host && !mid, copy_off = off_host && !moff;
+    if (copy_ids) hold_ids = at::empty(ids.sizes(), ids.options().device(dev));
+    if (copy_off) hold_off = at::empty(hold_off.sizes(), hold_off.options().device(dev));
+    const long long* pid = static_cast<const long long*>(mid ? mid : hold_ids.data_ptr());
+    const int* poff = hold_off.defined() ? static_cast<const int*>(moff ? moff : hold_off.data_ptr()) : nullptr;
+    const bool skinny = B <= tn::kServeSkinnyRows;
+    // one workspace: activations, row indices and offsets of a ragged request, bf16 weights
+    auto up = [](size_t n) { return (n + 255) / 256 * 256; };
+    std::vector<size_t> at_act(L + 1), at_w(L);
+    size_t bytes = 0;
+    for (int l = 0; l <= L; ++l) { at_act[l] = bytes; bytes += up((size_t)B * pad8(dims[l] + 1) * 2); }
+    size_t at_rows = 0, at_off = 0;
+    if (poff) { at_rows = bytes; bytes += up((size_t)ids.numel() * 4); at_off = bytes; bytes += up(((size_t)S * B + 1) * 4); }
+    const bool cast_now = cast_needed && !skinny;
+    if (cast_now)
+      for (int l = 0; l < L; ++l) { at_w[l] = bytes; bytes += up((size_t)weights[l].numel() * 2); }
+    at::Tensor ws = at::empty({(int64_t)bytes}, at::TensorOptions().dtype(at::kByte).device(dev));
+    at::Tensor prob = at::empty({B}, at::TensorOptions().dtype(at::kFloat).device(dev));
+    uint8_t* w0 = static_cast<uint8_t*>(ws.data_ptr());
+    for (int l = 0; l < L; ++l) {
+      const at::Tensor& w = cast_needed ? weights[l] : shadows[l];
+      TORCH_CHECK(w.is_cuda() && w.dim() == 2 && w.is_contiguous() && w.size(0) == dims[l + 1] && w.size(1) == pad8(dims[l] + 1) &&
+                      w.scalar_type() == (cast_needed ? at::kFloat : at::kBFloat16) && (reinterpret_cast<uintptr_t>(w.data_ptr()) & 15) == 0,
+                  "serving: layer ", l, " weights");
+    }
+    if (copy_ids || copy_off) {
+      // on a stream of its own: the weights are converted meanwhile
+      CopyLane& cl = copy_lane(dev.index());
+      const bool side = cast_now;
+      const cudaStream_t cs = side ? cl.stream : st;
+      if (side) {
+        check(cudaEventRecord(cl.begin, st), "serving: event");        // the buffers' former users are done
+        check(cudaStreamWaitEvent(cs, cl.begin, 0), "serving: wait");
+      }
+      auto put = [&](const at::Tensor& d, const at::Tensor& h) {
+        check(cudaMemcpyAsync(d.data_ptr(), h.data_ptr(), h.nbytes(), cudaMemcpyHostToDevice, cs), "serving: copy");
+        if (h.is_pinned())
+          at::getHostAllocator(at::kCUDA)->record_event(const_cast<void*>(h.storage().data()), h.storage().data_ptr().get_context(),
+                                                        c10::cuda::getStreamFromExternal(cs, dev.index()).unwrap());
+      };
+      if (copy_ids) put(hold_ids, ids);
+      if (copy_off) put(hold_off, *offsets);
+      if (side) check(cudaEventRecord(cl.end, cs), "serving: event");
+    }
+    if (cast_now) {
+      tn::ServeCast c{};
+      c.n = L;
+      for (int l = 0; l < L; ++l) { c.src[l] = ptr_of<const float>(weights[l]); c.dst[l] = w0 + at_w[l]; c.n8[l] = weights[l].numel() / 8; }
+      tn::launch_serve_cast(c, st);
+      if (copy_ids || copy_off) check(cudaStreamWaitEvent(st, copy_lane(dev.index()).end, 0), "serving: wait");
+    }
+    // behind a copy the lookup is launched the ordinary way; the conversion is then complete anyway
+    const bool behind_cast = cast_now && !copy_ids && !copy_off;
+    const int ld0 = pad8(dims[0] + 1);
+    if (poff)
+      tn::launch_serve_lookup_ragged(t, pid, (int)ids.numel(), poff, B, S, combiner, reinterpret_cast<int*>(w0 + at_rows),
+                                     moff ? reinterpret_cast<int*>(w0 + at_off) : nullptr, w0 + at_act[0], ld0, dims[0], behind_cast, st);
+    else
+      tn::launch_serve_lookup_single(t, pid, B, S, w0 + at_act[0], ld0, dims[0], behind_cast, st);
+    // host memory read in place must not be handed out again before the kernels are done with it
+    for (const at::Tensor* h : {mid ? &hold_ids : nullptr, moff ? &hold_off : nullptr})
+      if (h != nullptr)
+        at::getHostAllocator(at::kCUDA)->record_event(const_cast<void*>(h->storage().data()), h->storage().data_ptr().get_context(),
+                                                      at::cuda::getCurrentCUDAStream().unwrap());
+    for (int l = 0; l < L; ++l) {
+      const int N = dims[l + 1], K = dims[l] + 1, ldx = pad8(K), ldy = pad8(N + 1), relu = relu_last || l < L - 1;
+      void *x = w0 + at_act[l], *y = w0 + at_act[l + 1];
+      const void* w = cast_now ? (const void*)(w0 + at_w[l]) : (cast_needed ? weights[l].data_ptr() : shadows[l].data_ptr());
+      if (skinny) {
+        tn::launch_serve_skinny(x, ldx, w, cast_needed ? 1 : 0, ldx, B, N, K, relu, y, ldy, ldy, st);
+      } else {
+        tn::GemmDesc d;
+        d.M = B; d.N = N; d.K = K; d.A = x; d.B = w; d.lda = ldx; d.ldb = ldx; d.C = y; d.ldc = ldy; d.relu = relu;
+        d.ones_col = N; d.n_store = ldy; d.split_k = 1; d.status = ptr_of<int>(status);
+        const char* err = tn::gemm_bf16(d, st);
+        if (err) throw std::runtime_error(err);
+      }
+    }
+    tn::launch_serve_head(w0 + at_act[L], pad8(dims[L] + 1), B, dims[L] + 1, ptr_of<const float>(head_w), ptr_of<float>(prob), st);
+    check(cudaGetLastError(), "serving launch");
+    g_launches.fetch_add(L + 2 + (cast_now ? 1 : 0) + (poff ? 1 : 0), std::memory_order_relaxed);
+    return prob;
+  }
+};
+
 // A metric-sum buffer is fp32[4] or fp32[4 + 2 * nbins]: the tail holds the two u32 prediction histograms of the AUC.
 static int hist_bins(const at::Tensor& sums) {
   TORCH_CHECK(sums.scalar_type() == at::kFloat && sums.is_contiguous() && sums.numel() >= 4 && (sums.numel() - 4) % 2 == 0,
@@ -437,6 +582,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         self.push(work_hint, max_ctas, &d);
       }, py::arg("work_hint"), py::arg("max_ctas") = 0, py::arg("dense") = py::none())
       .def("front", &SparseCtx::front, py::arg("ids"), py::arg("inverse"), py::arg("n_dev") = py::none());
+  py::class_<ServeCtx>(m, "ServeCtx")
+      .def(py::init<py::dict, int, int, std::vector<int>, bool>())
+      .def("forward", &ServeCtx::forward);
   py::class_<BnCtx>(m, "BnCtx")
       .def(py::init<py::dict>())
       .def("push", &BnCtx::push)

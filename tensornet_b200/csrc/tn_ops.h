@@ -97,6 +97,23 @@ void launch_bn_apply_bwd(const float* dy, int ldd, const float* x, int ldx, int 
 // serving.cu
 void launch_dict_lookup_pool(const TableView& t, const long long* ids, const int* offsets, int B, int S, int combiner, void* out,
                              int ld_out, int ones_col, cudaStream_t st);
+// The kernels of InferenceEngine's request path (in launch order); `ids` / `offsets` may be pinned host memory.
+constexpr int kServeMaxLayers = 8;
+constexpr int kServeSkinnyRows = 2;      // requests of up to this many rows take launch_serve_skinny for their layers
+struct ServeCast {
+  int n;
+  const float* src[kServeMaxLayers];
+  void* dst[kServeMaxLayers];
+  long long n8[kServeMaxLayers];         // groups of eight elements
+};
+void launch_serve_cast(const ServeCast& a, cudaStream_t st);
+void launch_serve_lookup_single(const TableView& t, const long long* ids, int B, int S, void* out, int ld_out, int ones_col, bool behind_cast,
+                                cudaStream_t st);
+void launch_serve_lookup_ragged(const TableView& t, const long long* ids, int n, const int* offsets, int B, int S, int combiner, int* rows,
+                                int* offsets_dev, void* out, int ld_out, int ones_col, bool behind_cast, cudaStream_t st);
+void launch_serve_skinny(const void* x, int ldx, const void* w, int w_f32, int ldw, int M, int N, int K, int relu, void* y, int ldy, int n_store,
+                         cudaStream_t st);
+void launch_serve_head(const void* z, int ld, int B, int K, const float* w, float* prob, cudaStream_t st);
 void launch_sigmoid(const float* x, float* y, int n, cudaStream_t st);
 
 }  // namespace tn

@@ -8,8 +8,10 @@ import torch
 
 from .. import _build
 from ..core.runtime import runtime
+from ..layers.dense import DenseHead, MLP
 from ..ops import functional as F
 from ..tools import merge_sparse
+from ..utils.capture import capture
 
 
 def export_sparse_dictionary(checkpoint_dir: str, table_name: str, out_file: str, **kw) -> int:
@@ -87,14 +89,35 @@ class EmbeddingDictionary:
 class InferenceEngine:
     """``ids [S, B]`` (or ragged) -> click probabilities, for a dense tower ``MLP`` + ``DenseHead``.
 
-    The first call for a batch shape captures lookup + towers + sigmoid in a CUDA graph; later calls copy
-    the ids into the static buffer and replay it."""
+    On a GPU a request is one native call that launches lookup, layers and head as a chain of dependent kernels; ids in
+    pinned host memory are read in place.  (A captured graph per batch shape, which this replaces, took longer to start
+    than the chain takes to issue, and served ragged requests not at all.)  Towers other than ``MLP`` + ``DenseHead``
+    run as the modules they are, captured per batch shape."""
 
     def __init__(self, dictionary: EmbeddingDictionary, mlp, head, n_slots: int, combiner: str = "mean"):
         self.dict, self.mlp, self.head, self.S = dictionary, mlp, head, n_slots
         self.combiner = {"sum": 0, "mean": 1, "sqrtn": 2}[combiner]
         self._graphs = {}
         assert mlp.in_dim == n_slots * dictionary.dim, "tower input width must equal slots * dim"
+        self._ctx = None
+        if dictionary.on_gpu and type(mlp) is MLP and type(head) is DenseHead and len(mlp.hidden_units) <= 8:
+            self._ctx = _build.cuda_ext().ServeCtx(dictionary.table_dict(), n_slots, self.combiner,
+                                                   [mlp.in_dim, *mlp.hidden_units], bool(mlp.relu_last))
+
+    def _native(self, ids, offsets, B: int):
+        """The request through the native chain, or None when something about it is out of the ordinary."""
+        ws = list(self.mlp.weights._parameters.values())
+        hw = self.head.weight
+        if self.mlp.weight_gate is not None or not all(w.is_cuda and w.dtype == torch.float32 and w.is_contiguous() for w in (*ws, hw)):
+            return None
+        if ids.dtype != torch.int64 or not ids.is_contiguous():
+            ids = ids.to(torch.int64).contiguous()
+        if offsets is not None and (offsets.dtype != torch.int32 or not offsets.is_contiguous()):
+            offsets = offsets.to(torch.int32).contiguous()
+        shadows = [getattr(w, "_tn_bf16", None) for w in ws]
+        if any(s is None for s in shadows):
+            shadows = []
+        return self._ctx.forward(ids, offsets, B, ws, shadows, hw, runtime().status)
 
     def _forward_gpu(self, ids, offsets, B):
         ext = _build.cuda_ext()
@@ -125,6 +148,11 @@ class InferenceEngine:
             x = pooled.permute(1, 0, 2).reshape(B, -1)
             return torch.sigmoid(self.head(self.mlp(F.concat_cast([x], ones=True)))).view(-1)
         dev = rt.device
+        if self._ctx is not None:
+            n = int(ids.shape[1]) if offsets is None else (offsets.numel() - 1) // self.S
+            prob = self._native(ids, offsets, n) if n > 0 else None
+            if prob is not None:
+                return prob
         if offsets is not None or not use_graph:
             B = ids.shape[1] if offsets is None else (offsets.numel() - 1) // self.S
             return self._forward_gpu(ids.to(dev).reshape(-1), None if offsets is None else offsets.to(dev).int(), B)
@@ -137,7 +165,7 @@ class InferenceEngine:
                 self._forward_gpu(static_ids, None, B)
             torch.cuda.synchronize()
             g = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(g):
+            with capture(g):
                 out = self._forward_gpu(static_ids, None, B)
             entry = (g, static_ids, out)
             self._graphs[B] = entry
@@ -217,7 +245,7 @@ class ShardedInferenceEngine:
             torch.cuda.synchronize()
             rt.check_status()
             g = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(g):
+            with capture(g):
                 out = self._forward(static_ids, None, B)
             entry = (g, static_ids, out)
             self._graphs[B] = entry

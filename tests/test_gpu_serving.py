@@ -1,0 +1,53 @@
+"""The native request path against the module path (same dictionary, same tower)."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("B", [1, 2, 3, 17, 130, 1024])
+@pytest.mark.parametrize("where", ["pinned", "pageable", "device"])
+@pytest.mark.parametrize("ragged", [False, True])
+def test_native_requests_equal_the_modules(tn_gpu, status_ok, B, where, ragged):
+    """Both round rows and weights to bf16 and accumulate in fp32: logits differ by the order of the sums and by roundings
+    of the hidden activations that flip with it, a bf16 step (2^-8) of a few of them; probabilities by a quarter of that."""
+    from tensornet_b200.layers import DenseHead, MLP
+    from tensornet_b200.serving import EmbeddingDictionary, InferenceEngine
+
+    tn = tn_gpu
+    dev = tn.core.runtime().device
+    S, D = 37, 12
+    rng = np.random.default_rng(B)
+    signs = np.unique(rng.integers(1, 2 ** 40, 20_000).astype(np.uint64))
+    torch.manual_seed(B)
+    mlp, head = MLP(S * D, [200, 64, 33]).to(dev), DenseHead(33).to(dev)
+    d = EmbeddingDictionary(signs, rng.standard_normal((len(signs), D)).astype(np.float32))
+    eng = InferenceEngine(d, mlp, head, S, combiner="mean")
+    assert eng._ctx is not None
+    lens = torch.from_numpy(rng.integers(0, 40 if B < 20 else 6, S * B)) if ragged else torch.ones(S * B, dtype=torch.int64)
+    offs = torch.cat([torch.zeros(1, dtype=torch.int64), lens.cumsum(0)]).int()
+    n = int(offs[-1])
+    ids = np.where(rng.random(n) < 0.8, signs[rng.integers(0, len(signs), n)].view(np.int64), rng.integers(2 ** 41, 2 ** 42, n))
+    ids = torch.from_numpy(ids)
+    with torch.no_grad():
+        want = eng._forward_gpu(ids.to(dev), offs.to(dev) if ragged else None, B)
+    if not ragged:
+        ids = ids.view(S, B)
+    move = {"pinned": lambda t: t.pin_memory(), "pageable": lambda t: t, "device": lambda t: t.to(dev)}[where]
+    got = eng.infer(move(ids), move(offs) if ragged else None)
+    assert torch.allclose(got, want, atol=2 ** -10), float((got - want).abs().max())
+
+
+def test_weights_written_between_requests_are_seen(tn_gpu, status_ok):
+    from tensornet_b200.layers import DenseHead, MLP
+    from tensornet_b200.serving import EmbeddingDictionary, InferenceEngine
+
+    dev = tn_gpu.core.runtime().device
+    mlp, head = MLP(8, [16]).to(dev), DenseHead(16).to(dev)
+    eng = InferenceEngine(EmbeddingDictionary(np.arange(1, 9, dtype=np.uint64), np.ones((8, 4), np.float32)), mlp, head, 2)
+    for B in (1, 40):
+        ids = torch.randint(1, 9, (2, B))
+        a = eng.infer(ids).clone()
+        mlp.weights[0].data.mul_(-1.0)
+        assert not torch.equal(a, eng.infer(ids))
