@@ -132,47 +132,142 @@ __device__ __forceinline__ float concat_src(const ConcatArgs& a, int b, int c) {
   }
   return 0.f;
 }
-// one thread = 8 consecutive output columns = one 16-byte store (ld_out is a multiple of 8)
+
+// The piece that holds all of columns [c0, c0 + 8), or -1; `off`: its first column.
+__device__ __forceinline__ int piece_of_chunk(const ConcatArgs& a, int c0, int& off) {
+  int found = -1, at = 0;
+#pragma unroll
+  for (int p = 0; p < kMaxPieces; ++p) {
+    if (p < a.n_pieces) {
+      const int w = a.width[p];
+      if (c0 >= at && c0 + 8 <= at + w) { found = p; off = at; }
+      at += w;
+    }
+  }
+  return found;
+}
+
+// Position (row, 8-column chunk) of a grid-stride loop: one division before the loop, additions inside it (a 64-bit
+// division per chunk was a third of these kernels).
+struct ChunkWalk {
+  int b, j, db, dj, cpr;
+  __device__ __forceinline__ explicit ChunkWalk(int cpr_) : cpr(cpr_) {
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x, n = (long long)gridDim.x * blockDim.x;
+    b = (int)(i / cpr); j = (int)(i - (long long)b * cpr);
+    db = (int)(n / cpr); dj = (int)(n - (long long)db * cpr);
+  }
+  __device__ __forceinline__ void next() {
+    b += db; j += dj;
+    if (j >= cpr) { j -= cpr; ++b; }
+  }
+};
+
+// One thread = 8 consecutive output columns = one 16-byte store (ld_out is a multiple of 8).  Bound by memory: a chunk
+// that lies in one piece, which is nearly every chunk, is fetched with the widest loads its address allows (16, 8 or 4
+// bytes); only chunks across a seam look up each column.  8192 x 6413: 96 us with a lookup per column,
+// 45 us now (7 TB/s counting what L2 still holds).
 __global__ void concat_cast_kernel(const ConcatArgs a) {
   pdl_sync();
-  const int cpr = a.ld_out >> 3;
-  const long long total = (long long)a.B * cpr;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int b = (int)(i / cpr), c0 = (int)(i - (long long)b * cpr) * 8;
-    float v[8];
+  for (ChunkWalk at(a.ld_out >> 3); at.b < a.B; at.next()) {
+    const int b = at.b, c0 = at.j * 8;
+    uint4 o;
+    int off = 0;
+    const int p = piece_of_chunk(a, c0, off);
+    const size_t idx = p >= 0 ? (size_t)b * a.ld[p] + (c0 - off) : 0;
+    if (p >= 0 && a.is_bf16[p]) {
+      const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(a.ptr[p]) + idx;
+      if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+        o = *reinterpret_cast<const uint4*>(src);
+      } else {
+        const unsigned short* h = reinterpret_cast<const unsigned short*>(src);
+        unsigned x[4];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) v[k] = concat_src(a, b, c0 + k);
-    __nv_bfloat162 p0 = __floats2bfloat162_rn(v[0], v[1]), p1 = __floats2bfloat162_rn(v[2], v[3]);
-    __nv_bfloat162 p2 = __floats2bfloat162_rn(v[4], v[5]), p3 = __floats2bfloat162_rn(v[6], v[7]);
-    uint4 o = make_uint4(*reinterpret_cast<uint32_t*>(&p0), *reinterpret_cast<uint32_t*>(&p1),
-                         *reinterpret_cast<uint32_t*>(&p2), *reinterpret_cast<uint32_t*>(&p3));
+        for (int k = 0; k < 4; ++k) x[k] = (unsigned)h[2 * k] | ((unsigned)h[2 * k + 1] << 16);
+        o = make_uint4(x[0], x[1], x[2], x[3]);
+      }
+    } else {
+      float v[8];
+      if (p >= 0) {
+        const float* src = reinterpret_cast<const float*>(a.ptr[p]) + idx;
+        if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+          const float4 x = *reinterpret_cast<const float4*>(src), y = *reinterpret_cast<const float4*>(src + 4);
+          v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
+        } else if ((reinterpret_cast<uintptr_t>(src) & 7) == 0) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const float2 x = *reinterpret_cast<const float2*>(src + 2 * k);
+            v[2 * k] = x.x; v[2 * k + 1] = x.y;
+          }
+        } else {
+#pragma unroll
+          for (int k = 0; k < 8; ++k) v[k] = src[k];
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = concat_src(a, b, c0 + k);
+      }
+      __nv_bfloat162 p0 = __floats2bfloat162_rn(v[0], v[1]), p1 = __floats2bfloat162_rn(v[2], v[3]);
+      __nv_bfloat162 p2 = __floats2bfloat162_rn(v[4], v[5]), p3 = __floats2bfloat162_rn(v[6], v[7]);
+      o = make_uint4(*reinterpret_cast<uint32_t*>(&p0), *reinterpret_cast<uint32_t*>(&p1),
+                     *reinterpret_cast<uint32_t*>(&p2), *reinterpret_cast<uint32_t*>(&p3));
+    }
     *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.out) + (size_t)b * a.ld_out + c0) = o;
   }
 }
-// reverse: bf16 [B, ld_out] -> pieces (each piece written with its own ld); 8 columns per thread
+
+// Reverse: bf16 [B, ld_out] -> pieces (each piece written with its own ld), 8 columns per thread, with the widest
+// stores the address allows.  8192 x 6413: 259 us with one 4-byte store per column, 70 us now.
 __global__ void split_cast_kernel(const ConcatArgs a) {
   pdl_sync();
-  const int cpr = a.ld_out >> 3;
-  const long long total = (long long)a.B * cpr;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int b = (int)(i / cpr), c0 = (int)(i - (long long)b * cpr) * 8;
+  for (ChunkWalk at(a.ld_out >> 3); at.b < a.B; at.next()) {
+    const int b = at.b, c0 = at.j * 8;
+    int off = 0;
+    const int p = piece_of_chunk(a, c0, off);
+    if (p >= 0 && a.ptr[p] == nullptr) continue;           // nobody asked for this piece
     const uint4 raw = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.out) + (size_t)b * a.ld_out + c0);
     const __nv_bfloat16* x = reinterpret_cast<const __nv_bfloat16*>(&raw);
+    if (p >= 0) {
+      const size_t idx = (size_t)b * a.ld[p] + (c0 - off);
+      if (a.is_bf16[p]) {
+        __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(const_cast<void*>(a.ptr[p])) + idx;
+        if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) *reinterpret_cast<uint4*>(dst) = raw;
+        else {
+#pragma unroll
+          for (int k = 0; k < 8; ++k) dst[k] = x[k];
+        }
+        continue;
+      }
+      float* dst = reinterpret_cast<float*>(const_cast<void*>(a.ptr[p])) + idx;
+      float v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = __bfloat162float(x[k]);
+      if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+        *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+        *reinterpret_cast<float4*>(dst + 4) = make_float4(v[4], v[5], v[6], v[7]);
+      } else if ((reinterpret_cast<uintptr_t>(dst) & 7) == 0) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) *reinterpret_cast<float2*>(dst + 2 * k) = make_float2(v[2 * k], v[2 * k + 1]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) dst[k] = v[k];
+      }
+      continue;
+    }
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       const int c = c0 + k;
-      int off = 0;
-      for (int p = 0; p < a.n_pieces; ++p) {
-        const int w = a.width[p];
-        if (c >= off && c < off + w) {
-          if (a.ptr[p]) {
-            const size_t idx = (size_t)b * a.ld[p] + (c - off);
-            if (a.is_bf16[p]) reinterpret_cast<__nv_bfloat16*>(const_cast<void*>(a.ptr[p]))[idx] = x[k];
-            else reinterpret_cast<float*>(const_cast<void*>(a.ptr[p]))[idx] = __bfloat162float(x[k]);
+      int at_col = 0;
+      for (int q = 0; q < a.n_pieces; ++q) {
+        const int w = a.width[q];
+        if (c >= at_col && c < at_col + w) {
+          if (a.ptr[q]) {
+            const size_t idx = (size_t)b * a.ld[q] + (c - at_col);
+            if (a.is_bf16[q]) reinterpret_cast<__nv_bfloat16*>(const_cast<void*>(a.ptr[q]))[idx] = x[k];
+            else reinterpret_cast<float*>(const_cast<void*>(a.ptr[q]))[idx] = __bfloat162float(x[k]);
           }
           break;
         }
-        off += w;
+        at_col += w;
       }
     }
   }
@@ -315,25 +410,65 @@ __global__ void cross_v1_fwd_kernel(const float* __restrict__ x0, const float* _
     for (int d = lane; d < D; d += 32) y[(size_t)b * D + d] = a[d] * s + bias[d] + c[d];
   }
 }
-// gx0 += gy * s ; gxl = gy + w * (gy . x0) ; gw += xl * (gy . x0) ; gb += gy
-__global__ void cross_v1_bwd_kernel(const float* __restrict__ x0, const float* __restrict__ xl, const float* __restrict__ w,
-                                    const float* __restrict__ dot, const float* __restrict__ gy, int B, int D,
-                                    float* __restrict__ gx0, float* __restrict__ gxl, float* __restrict__ gw, float* __restrict__ gb) {
+// gx0 = gy * s ; gxl = gy + w * (gy . x0) ; gw += xl * (gy . x0) ; gb += gy.   One warp per row.
+// Adding every row's contribution to the D words of gw and gb was all this kernel did: 1.6 M atomics on 400 words, 39 us
+// for 4096 x 200.  A lane now keeps the sums of its NC columns in registers over the warp's rows, the warps of a block
+// meet in shared memory, and a block adds to gw / gb once: 5.8 us.  Rows wider than 32 * NC columns are walked in
+// tiles of that width (with the dot product taken once per tile).
+template <int NC>
+__global__ void __launch_bounds__(256) cross_v1_bwd_kernel(const float* __restrict__ x0, const float* __restrict__ xl,
+                                                           const float* __restrict__ w, const float* __restrict__ dot,
+                                                           const float* __restrict__ gy, int B, int D, float* __restrict__ gx0,
+                                                           float* __restrict__ gxl, float* __restrict__ gw, float* __restrict__ gb) {
   pdl_sync();
+  __shared__ float s_w[32 * NC], s_b[32 * NC];
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (int b = warp; b < B; b += nwarps) {
-    const float* a = x0 + (size_t)b * D; const float* c = xl + (size_t)b * D; const float* g = gy + (size_t)b * D;
-    float t = 0.f;
-    for (int d = lane; d < D; d += 32) t += g[d] * a[d];
-    t = warp_sum(t);
-    const float s = dot[b];
-    for (int d = lane; d < D; d += 32) {
-      gx0[(size_t)b * D + d] = g[d] * s;
-      gxl[(size_t)b * D + d] = g[d] + w[d] * t;
-      atomicAdd(gw + d, c[d] * t);
-      atomicAdd(gb + d, g[d]);
+  for (int d0 = 0; d0 < D; d0 += 32 * NC) {
+    for (int k = threadIdx.x; k < 32 * NC; k += blockDim.x) { s_w[k] = 0.f; s_b[k] = 0.f; }
+    __syncthreads();
+    float aw[NC], ab[NC];
+#pragma unroll
+    for (int i = 0; i < NC; ++i) { aw[i] = 0.f; ab[i] = 0.f; }
+    for (int b = warp; b < B; b += nwarps) {
+      const float* a = x0 + (size_t)b * D; const float* c = xl + (size_t)b * D; const float* g = gy + (size_t)b * D;
+      float gv[NC], cv[NC];
+      float t = 0.f;
+#pragma unroll
+      for (int i = 0; i < NC; ++i) {
+        const int d = d0 + lane + 32 * i;
+        gv[i] = d < D ? g[d] : 0.f;
+        cv[i] = d < D ? c[d] : 0.f;
+        t += d < D ? gv[i] * a[d] : 0.f;
+      }
+      if (D > 32 * NC) {
+        for (int d = lane; d < D; d += 32)
+          if (d < d0 || d >= d0 + 32 * NC) t += g[d] * a[d];
+      }
+      t = warp_sum(t);
+      const float s = dot[b];
+#pragma unroll
+      for (int i = 0; i < NC; ++i) {
+        const int d = d0 + lane + 32 * i;
+        if (d < D) {
+          gx0[(size_t)b * D + d] = gv[i] * s;
+          gxl[(size_t)b * D + d] = gv[i] + __ldg(w + d) * t;
+        }
+        aw[i] += cv[i] * t;
+        ab[i] += gv[i];
+      }
     }
+#pragma unroll
+    for (int i = 0; i < NC; ++i) {
+      atomicAdd(&s_w[lane + 32 * i], aw[i]);
+      atomicAdd(&s_b[lane + 32 * i], ab[i]);
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < 32 * NC && d0 + k < D; k += blockDim.x) {
+      atomicAdd(gw + d0 + k, s_w[k]);
+      atomicAdd(gb + d0 + k, s_b[k]);
+    }
+    __syncthreads();
   }
 }
 
@@ -470,7 +605,12 @@ void launch_cross_v1_fwd(const float* x0, const float* xl, const float* w, const
 }
 void launch_cross_v1_bwd(const float* x0, const float* xl, const float* w, const float* dot, const float* gy, int B, int D,
                          float* gx0, float* gxl, float* gw, float* gb, cudaStream_t st) {
-  launch_pdl(cross_v1_bwd_kernel, dim3(blocks_for(B, 8)), dim3(256), 0, st, x0, xl, w, dot, gy, B, D, gx0, gxl, gw, gb);
+  // two rows per warp: fewer blocks would leave SMs idle, more would add to gw / gb more often
+  int blocks = (B + 15) / 16;
+  if (blocks > 148 * 2) blocks = 148 * 2;
+  if (blocks < 1) blocks = 1;
+  auto* kernel = D <= 256 ? cross_v1_bwd_kernel<8> : D <= 512 ? cross_v1_bwd_kernel<16> : cross_v1_bwd_kernel<32>;
+  launch_pdl(kernel, dim3(blocks), dim3(256), 0, st, x0, xl, w, dot, gy, B, D, gx0, gxl, gw, gb);
 }
 
 }  // namespace tn

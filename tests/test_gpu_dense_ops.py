@@ -140,3 +140,49 @@ def test_dense_table_step(tn_gpu, status_ok, kind):
             assert torch.allclose(p.detach().cpu(), w, rtol=1e-4, atol=1e-5)
             assert float(p.grad.abs().sum()) == 0.0
             assert torch.equal(p._tn_bf16.float(), p.detach().bfloat16().float())
+
+
+@pytest.mark.parametrize("widths", [(416, 13), (390, 5), (7, 9, 1), (8,), (64, 3, 24, 1)])
+@pytest.mark.parametrize("shift", [0, 1, 2])
+def test_concat_split_every_alignment(tn_gpu, status_ok, widths, shift):
+    """Pieces that start at any column, on any 4-byte boundary, fp32 and bf16 in turn, rows longer than the piece:
+    exactly the rounded values, and gradients exactly the operand's columns."""
+    from tensornet_b200.ops import functional as F
+
+    dev = tn_gpu.core.runtime().device
+    B = 131
+    leaves, pieces = [], []
+    for k, w in enumerate(widths):
+        base = torch.randn(B, w + 3, device=dev, dtype=torch.float32 if k % 2 == 0 else torch.bfloat16, requires_grad=True)
+        leaves.append((base, w))
+        pieces.append(base[:, shift: shift + w])
+    x = F.concat_cast(pieces, ones=True)
+    want = torch.cat([p.detach().bfloat16() for p in pieces], dim=1)
+    K = want.shape[1]
+    assert torch.equal(x[:, :K], want) and torch.all(x[:, K] == 1) and torch.all(x[:, K + 1:] == 0)
+    g = torch.randn_like(x, dtype=torch.float32).bfloat16()
+    x.backward(g)
+    at = 0
+    for base, w in leaves:
+        assert torch.equal(base.grad[:, shift: shift + w], g[:, at: at + w].to(base.dtype))
+        at += w
+
+
+@pytest.mark.parametrize("B,D", [(1, 1), (33, 31), (700, 200), (64, 256), (40, 257), (130, 777), (20, 1024), (50, 2500)])
+def test_cross_v1_backward_against_fp64(tn_gpu, status_ok, B, D):
+    """Sums of at most max(B, D) 32-bit products: error below 4 * sqrt(n) * 2^-24 of the sum of absolute values."""
+    from tensornet_b200.ops import functional as F
+
+    dev = tn_gpu.core.runtime().device
+    g = torch.Generator(device=dev).manual_seed(B * 4096 + D)
+    x0, xl = (torch.randn(B, D, generator=g, device=dev).requires_grad_(True) for _ in range(2))
+    w, b = torch.randn(D, 1, generator=g, device=dev).requires_grad_(True), torch.randn(D, generator=g, device=dev).requires_grad_(True)
+    gy = torch.randn(B, D, generator=g, device=dev)
+    F.cross_v1(x0, xl, w, b).backward(gy)
+    d = [t.detach().double() for t in (x0, xl, w.view(-1), gy)]
+    t, s = (d[3] * d[0]).sum(1, keepdim=True), (d[1] * d[2]).sum(1, keepdim=True)
+    eps = 4 * max(B, D) ** 0.5 * 2.0 ** -24
+    ta, sa = (d[3] * d[0]).abs().sum(1, keepdim=True), (d[1] * d[2]).abs().sum(1, keepdim=True)
+    for got, want, size in [(x0.grad, d[3] * s, d[3].abs() * sa), (xl.grad, d[3] + d[2] * t, d[3].abs() + d[2].abs() * ta),
+                            (w.grad.view(-1), (d[1] * t).sum(0), (d[1].abs() * ta).sum(0)), (b.grad, d[3].sum(0), d[3].abs().sum(0))]:
+        assert bool(((got.double() - want).abs() <= 2 * eps * size + 1e-30).all())
