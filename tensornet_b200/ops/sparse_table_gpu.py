@@ -307,7 +307,9 @@ class GpuSparseLink:
             ("sig", (4 * 8,), torch.int64),
         ])
         d = self.dev
-        dd_cap = next_pow2(2 * self.max_unique + 16)
+        # at most two thirds full: the scratch is probed at random and cleared every batch, so what counts is that it stays
+        # in L2 (4.1 M ids of 4.9 M that fit: 67 MB of keys instead of 134, pull 627 -> 570 us)
+        dd_cap = next_pow2(max(self.max_unique * 3 // 2, 32))
         loc = dict(
             stage_ids=torch.zeros(n_seg, dtype=torch.int64, device=d),
             gU=arena.tensor("gU").zero_(),

@@ -327,3 +327,28 @@ def test_pull_front_run_ahead_matches_the_one_kernel_pull(tn_gpu, status_ok, dim
     assert rows_a.keys() == rows_b.keys()
     for k in rows_a:
         assert np.allclose(rows_a[k], rows_b[k], rtol=1e-5, atol=1e-6)
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 5000, 151553, 460001, 700001])
+@pytest.mark.parametrize("front", [False, True])
+def test_dedup_over_several_ids_per_lane(tn_gpu, status_ok, n, front):
+    """One to four ids per lane, whole and broken warps: as many rows as distinct ids, every id mapped to the row of its
+    sign, show and click counts exact, the scratch left empty."""
+    tn = tn_gpu
+    t, lk = _mk(tn, tn.core.AdaGrad(learning_rate=0.05, initial_g2sum=0.1, initial_scale=0.3), 4, rows=1 << 20, max_unique=n)
+    g = torch.Generator(device=t.dev).manual_seed(n)
+    ids = torch.randint(0, max(1, n // 2), (n,), generator=g, device=t.dev) ** 2 // max(1, n // 2) * 7919 + 3
+    labels = (torch.rand(n, generator=g, device=t.dev) < 0.3).float()
+    if front:
+        lk.prefetch(ids)
+    inv = lk.pull(ids, labels=labels, training=True)
+    uniq, counts = torch.unique(ids, return_counts=True)
+    n_u = lk.unique_counts()[0]
+    assert n_u == uniq.numel() == t.n_rows
+    stage = lk.comm["stage_ids"][:n_u]
+    assert torch.equal(stage.sort().values, uniq) and torch.equal(stage[inv.long()], ids)
+    order = stage.argsort()
+    assert torch.equal(lk.cnts[:n_u, 0][order].long(), counts)
+    clicks = torch.zeros(n_u, device=t.dev).index_add_(0, inv.long(), labels)
+    assert torch.equal(lk.cnts[:n_u, 1], clicks)
+    assert bool((lk.comm["dd_keys"] == -1).all())
