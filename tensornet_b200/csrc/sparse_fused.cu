@@ -695,6 +695,27 @@ __device__ __forceinline__ float fast_sqrt(float x) {
 }
 __device__ __forceinline__ float fast_div(float a, float b) { return __fdividef(a, b); }
 
+// The element-wise optimizers on one 16-byte chunk of a row (w, two slots) and its gradient x.
+__device__ __forceinline__ void adam_chunk(const SparseOptParams& o, const float4& x, float4& w, float4& mm, float4& vv) {
+  const float c1 = 1.f - o.beta1, c2 = 1.f - o.beta2;
+#define TN_SADAM(cmp) \
+  mm.cmp = o.beta1 * mm.cmp + c1 * x.cmp; vv.cmp = o.beta2 * vv.cmp + c2 * x.cmp * x.cmp; \
+  w.cmp -= fast_div(o.lr * mm.cmp, o.eps + fast_sqrt(vv.cmp));
+  TN_SADAM(x) TN_SADAM(y) TN_SADAM(z) TN_SADAM(w)
+#undef TN_SADAM
+}
+__device__ __forceinline__ void ftrl_chunk(const SparseOptParams& o, const float4& x, float4& w, float4& zz, float4& nn) {
+#define TN_SFTRL(cmp) { \
+  const float g2 = x.cmp * x.cmp; \
+  const float sn = fast_sqrt(nn.cmp + g2); \
+  zz.cmp += x.cmp - o.lr * (sn - fast_sqrt(nn.cmp)) * w.cmp; \
+  nn.cmp += g2; \
+  const float shr = zz.cmp > 0.f ? zz.cmp - o.lambda1 : zz.cmp + o.lambda1; \
+  w.cmp = fabsf(zz.cmp) > o.lambda1 ? -fast_div(shr, (o.ftrl_beta + sn) * o.lr + o.lambda2) : 0.f; }
+  TN_SFTRL(x) TN_SFTRL(y) TN_SFTRL(z) TN_SFTRL(w)
+#undef TN_SFTRL
+}
+
 // One optimizer step on one row by a group of G lanes.  `g` points at the gradient (dim floats), bshow / bclick
 // are the batch's show and click counts of the sign.   Math as in the reference's Sparse*Value::Apply.
 // VEC: dim is a multiple of 4, every lane works on float4 chunks.
@@ -771,11 +792,7 @@ __device__ __forceinline__ void apply_row(const SparseOptParams& o, float* row, 
         const float4 x = *reinterpret_cast<const float4*>(g + 4 * ch);
         float4 mm = *reinterpret_cast<float4*>(m + 4 * ch), vv = *reinterpret_cast<float4*>(v + 4 * ch);
         float4 w = *reinterpret_cast<float4*>(row + 4 * ch);
-#define TN_SADAM(cmp) \
-        mm.cmp = o.beta1 * mm.cmp + c1 * x.cmp; vv.cmp = o.beta2 * vv.cmp + c2 * x.cmp * x.cmp; \
-        w.cmp -= fast_div(o.lr * mm.cmp, o.eps + fast_sqrt(vv.cmp));
-        TN_SADAM(x) TN_SADAM(y) TN_SADAM(z) TN_SADAM(w)
-#undef TN_SADAM
+        adam_chunk(o, x, w, mm, vv);
         *reinterpret_cast<float4*>(m + 4 * ch) = mm;
         *reinterpret_cast<float4*>(v + 4 * ch) = vv;
         *reinterpret_cast<float4*>(row + 4 * ch) = w;
@@ -800,15 +817,7 @@ __device__ __forceinline__ void apply_row(const SparseOptParams& o, float* row, 
         const float4 x = *reinterpret_cast<const float4*>(g + 4 * ch);
         float4 zz = *reinterpret_cast<float4*>(z + 4 * ch), nn = *reinterpret_cast<float4*>(n + 4 * ch);
         float4 w = *reinterpret_cast<float4*>(row + 4 * ch);
-#define TN_SFTRL(cmp) { \
-        const float g2 = x.cmp * x.cmp; \
-        const float sn = fast_sqrt(nn.cmp + g2); \
-        zz.cmp += x.cmp - o.lr * (sn - fast_sqrt(nn.cmp)) * w.cmp; \
-        nn.cmp += g2; \
-        const float shr = zz.cmp > 0.f ? zz.cmp - o.lambda1 : zz.cmp + o.lambda1; \
-        w.cmp = fabsf(zz.cmp) > o.lambda1 ? -fast_div(shr, (o.ftrl_beta + sn) * o.lr + o.lambda2) : 0.f; }
-        TN_SFTRL(x) TN_SFTRL(y) TN_SFTRL(z) TN_SFTRL(w)
-#undef TN_SFTRL
+          ftrl_chunk(o, x, w, zz, nn);
         *reinterpret_cast<float4*>(z + 4 * ch) = zz;
         *reinterpret_cast<float4*>(n + 4 * ch) = nn;
         *reinterpret_cast<float4*>(row + 4 * ch) = w;
@@ -833,6 +842,152 @@ __device__ __forceinline__ void apply_row(const SparseOptParams& o, float* row, 
 
 }  // namespace
 
+// One GPU: every distinct sign of the batch maps to exactly one row, so there is nothing to exchange and nothing to wait
+// for: an ordinary kernel updates the rows in place.  What bounds it is random access to gradient, row and optimizer slots:
+// all loads of a row, its counters included, are issued before the first use (one chunk of 16 bytes per lane: dim a
+// multiple of 4, at most 128), and the grid is one wave of resident blocks.  Rows in flight against blocks per SM, and
+// whether the next round's rows are asked for from L2 meanwhile, were measured: 1.1 M AdaGrad rows of 128 take 515 us
+// with one row, six blocks and prefetching (two rows, four blocks: 544 without, 570 with; four rows, two blocks: 682); 2.2 M
+// Ftrl rows of 64, three times the bytes and registers, 930-980 us with two rows, three blocks and none (with: 1057; one
+// row, six blocks: 1253).  As a branch of the cooperative kernel, one row per group after the other: 702 and 1371 us.
+template <int KIND> struct LocalPush { static constexpr int kRows = 2, kBlocks = 3; static constexpr bool kPrefetch = false; };
+template <> struct LocalPush<kAdaGrad> { static constexpr int kRows = 1, kBlocks = 6; static constexpr bool kPrefetch = true; };
+
+template <int KIND>
+__global__ void __launch_bounds__(256, LocalPush<KIND>::kBlocks) sparse_push_local_kernel(const __grid_constant__ PushArgs a) {
+  constexpr int R = LocalPush<KIND>::kRows;
+  pdl_sync();
+  const SparseCommView& c = a.c;
+  const SparseOptParams& o = a.opt;
+  prof_mark(c, 8);
+  __shared__ TableView s_tbl;
+  if (threadIdx.x == 0) s_tbl = a.tbl_dev != nullptr ? *a.tbl_dev : a.tbl;
+  __syncthreads();
+  const TableView& t = s_tbl;
+  const int n = __ldcg(&c.cnt_saved[0]);
+  const int G = a.lanes, lane = threadIdx.x % G;
+  const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / G, ngroups = gridDim.x * blockDim.x / G;
+  const unsigned gmask = group_mask(G);
+  const int dim = t.dim, stride = t.stride, gstride = c.gstride;
+  const bool has = 4 * lane < dim;                  // lanes of a group beyond the row only take part in the shuffles
+  const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int j0 = gid; j0 < n; j0 += R * ngroups) {
+    float* row[R];
+    float4 x[R], w[R], s1[R], s2[R];
+    float4 tail[R];                  // AdaGrad: accumulator, show, click, days without show
+    int delta[R];                    // Adam, Ftrl: shows since the last save
+    float2 cn[R];
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      const int j = j0 + q * ngroups;
+      row[q] = nullptr;
+      x[q] = zero4;
+      if (j >= n) continue;
+      const int rr = __ldcg(&c.req_row[j]);
+      if (has) x[q] = ldcg_f4(c.gU + (size_t)j * gstride + 4 * lane);
+      if (lane == 0) cn[q] = __ldcg(reinterpret_cast<const float2*>(c.cnts) + j);
+      if (rr != kReqNone && rr != kReqPending) row[q] = t.rows + (size_t)(rr & kReqRowMask) * stride;
+    }
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      w[q] = s1[q] = s2[q] = zero4;
+      tail[q] = zero4;
+      delta[q] = 0;
+      if (row[q] == nullptr) continue;
+      if (has) {
+        w[q] = ldcg_f4(row[q] + 4 * lane);
+        if (KIND != kAdaGrad) {
+          s1[q] = ldcg_f4(row[q] + dim + 4 * lane);
+          s2[q] = ldcg_f4(row[q] + 2 * dim + 4 * lane);
+        }
+      }
+      if (KIND == kAdaGrad) tail[q] = ldcg_f4(row[q] + dim);
+      else if (lane == 0) delta[q] = __ldcg(reinterpret_cast<const int*>(row[q]) + 3 * dim + 1);
+    }
+#pragma unroll
+    for (int q = 0; LocalPush<KIND>::kPrefetch && q < R; ++q) {
+      const int j = j0 + (R + q) * ngroups;
+      if (j >= n) continue;
+      const int rr = __ldcg(&c.req_row[j]);
+      prefetch_row_l2(c.gU + (size_t)j * gstride, dim, lane, G);
+      if (rr != kReqNone && rr != kReqPending) prefetch_row_l2(t.rows + (size_t)(rr & kReqRowMask) * stride, stride, lane, G);
+    }
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      const int j = j0 + q * ngroups;
+      if (j >= n) continue;                         // the same for all lanes of a group
+      if (KIND == kAdaGrad) {
+        float ss = x[q].x * x[q].x + x[q].y * x[q].y + x[q].z * x[q].z + x[q].w * x[q].w;
+        for (int off = G >> 1; off > 0; off >>= 1) ss += __shfl_xor_sync(gmask, ss, off);
+        tail[q].x += ss / (float)dim;
+        const float scale = fast_div(o.lr, o.eps + fast_sqrt(tail[q].x));
+        w[q].x -= scale * x[q].x; w[q].y -= scale * x[q].y; w[q].z -= scale * x[q].z; w[q].w -= scale * x[q].w;
+      } else if (KIND == kAdam) {
+        adam_chunk(o, x[q], w[q], s1[q], s2[q]);
+      } else {
+        ftrl_chunk(o, x[q], w[q], s1[q], s2[q]);
+      }
+      if (row[q] != nullptr) {
+        if (has) {
+          *reinterpret_cast<float4*>(row[q] + 4 * lane) = w[q];
+          if (KIND != kAdaGrad) {
+            *reinterpret_cast<float4*>(row[q] + dim + 4 * lane) = s1[q];
+            *reinterpret_cast<float4*>(row[q] + 2 * dim + 4 * lane) = s2[q];
+          }
+        }
+        if (lane == 0) {
+          if (KIND == kAdaGrad) {
+            *reinterpret_cast<float4*>(row[q] + dim) = make_float4(tail[q].x, tail[q].y + cn[q].x, tail[q].z + cn[q].y, 0.f);
+          } else {
+            reinterpret_cast<int*>(row[q])[3 * dim + 1] = delta[q] + (int)cn[q].x;
+          }
+        }
+      }
+      if (has) *reinterpret_cast<float4*>(c.gU + (size_t)j * gstride + 4 * lane) = zero4;
+      if (lane == 0) reinterpret_cast<float2*>(c.cnts)[j] = make_float2(0.f, 0.f);
+    }
+  }
+  prof_mark(c, 13);
+}
+
+// The other row widths (no multiple of 4, or above 128): one row per group at a time, the next one asked for from L2.
+__global__ void __launch_bounds__(256) sparse_push_local_rows_kernel(const __grid_constant__ PushArgs a) {
+  pdl_sync();
+  const SparseCommView& c = a.c;
+  prof_mark(c, 8);
+  __shared__ TableView s_tbl;
+  if (threadIdx.x == 0) s_tbl = a.tbl_dev != nullptr ? *a.tbl_dev : a.tbl;
+  __syncthreads();
+  const TableView& t = s_tbl;
+  const int n = __ldcg(&c.cnt_saved[0]);
+  const int G = a.lanes, lane = threadIdx.x % G;
+  const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / G, ngroups = gridDim.x * blockDim.x / G;
+  const unsigned gmask = group_mask(G);
+  const int dim = t.dim, gstride = c.gstride, gch = gstride >> 2;
+  const bool vec = (dim & 3) == 0;
+  const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int j = gid; j < n; j += ngroups) {
+    const int rr = __ldcg(&c.req_row[j]);
+    if (j + ngroups < n) {
+      const int r2 = __ldcg(&c.req_row[j + ngroups]);
+      if (r2 != kReqNone && r2 != kReqPending) prefetch_row_l2(t.rows + (size_t)(r2 & kReqRowMask) * t.stride, t.stride, lane, G);
+    }
+    float* g = c.gU + (size_t)j * gstride;
+    float* cn = c.cnts + 2 * (size_t)j;
+    if (rr != kReqNone && rr != kReqPending) {
+      float* row = t.rows + (size_t)(rr & kReqRowMask) * t.stride;
+      const float bshow = cn[0], bclick = cn[1];
+      if (vec) apply_row<true>(a.opt, row, g, bshow, bclick, dim, lane, G, gmask);
+      else apply_row<false>(a.opt, row, g, bshow, bclick, dim, lane, G, gmask);
+    }
+    __syncwarp(gmask);
+    for (int ch = lane; ch < gch; ch += G) *reinterpret_cast<float4*>(g + 4 * ch) = zero4;
+    if (lane == 0) { cn[0] = 0.f; cn[1] = 0.f; }
+  }
+  prof_mark(c, 13);
+}
+
+// Several GPUs.
 // `dense_ctas` > 0: the last `dense_ctas` CTAs of the grid run the dense step `d` of the same training step (reduce-
 // scatter of the flat gradient, optimizer on the owned chunk, all-gather of the new weights) while the others push.
 // Both exchanges wait on the same peers at the same point of the step, so side by side they cost one wait instead
@@ -868,30 +1023,6 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_push_fused_kernel(const __
   const bool vec = (dim & 3) == 0;
 
   prof_mark(c, 8);
-  if (W == 1) {
-    // single GPU: every unique sign of the batch maps to exactly one row; update in place
-    const int n = __ldcg(&c.cnt_saved[0]);
-    for (int j = gid; j < n; j += ngroups) {
-      int rr = __ldcg(&c.req_row[j]);
-      if (j + ngroups < n) {
-        const int r2 = __ldcg(&c.req_row[j + ngroups]);
-        if (r2 != kReqNone && r2 != kReqPending) prefetch_row_l2(t.rows + (size_t)(r2 & kReqRowMask) * t.stride, t.stride, lane, G);
-      }
-      float* g = c.gU + (size_t)j * gstride;
-      float* cn = c.cnts + 2 * (size_t)j;
-      if (rr != kReqNone && rr != kReqPending) {
-        float* row = t.rows + (size_t)(rr & kReqRowMask) * t.stride;
-        const float bshow = cn[0], bclick = cn[1];
-        if (vec) apply_row<true>(a.opt, row, g, bshow, bclick, dim, lane, G, gmask);
-        else apply_row<false>(a.opt, row, g, bshow, bclick, dim, lane, G, gmask);
-      }
-      __syncwarp(gmask);
-      for (int ch = lane; ch < gch; ch += G) *reinterpret_cast<float4*>(g + 4 * ch) = zero4;
-      if (lane == 0) { cn[0] = 0.f; cn[1] = 0.f; }
-    }
-    goto done;
-  }
-
   // ---- phase A: tell every owner that this GPU's gradient records are complete.  They are: the backward pass that
   // wrote them precedes this kernel in the stream.  The records stay where they are; each owner READS its segment of
   // every GPU's records over NVLink and sums as it reads.  (Shipping them into inboxes first cost a pass of peer
@@ -1082,9 +1213,29 @@ cudaError_t launch_sparse_pull_front(const PullArgs& args, cudaStream_t stream) 
   return cudaMemsetAsync(args.c.dd_keys, 0xFF, ((size_t)args.c.dd_mask + 1u) * sizeof(unsigned long long), stream);
 }
 
+static cudaError_t launch_sparse_push_local(PushArgs args, long long rows, int max_ctas, cudaStream_t stream) {
+  const int dim = args.tbl.dim, kind = args.opt.kind;
+  const bool chunk_per_lane = (dim & 3) == 0 && dim <= 128;
+  if (chunk_per_lane) args.lanes = lanes_for_width(dim);
+  void (*kernel)(PushArgs) = sparse_push_local_rows_kernel;
+  int rows_per_group = 1, per_sm = 4;
+  auto take = [&](void (*k)(PushArgs), int r, int blocks) { kernel = k; rows_per_group = r; per_sm = blocks; };
+  if (chunk_per_lane) {
+    if (kind == kAdaGrad) take(sparse_push_local_kernel<kAdaGrad>, LocalPush<kAdaGrad>::kRows, LocalPush<kAdaGrad>::kBlocks);
+    else if (kind == kAdam) take(sparse_push_local_kernel<kAdam>, LocalPush<kAdam>::kRows, LocalPush<kAdam>::kBlocks);
+    else take(sparse_push_local_kernel<kFtrl>, LocalPush<kFtrl>::kRows, LocalPush<kFtrl>::kBlocks);
+  }
+  long long blocks = (rows * args.lanes + 256ll * rows_per_group - 1) / (256ll * rows_per_group);
+  if (blocks < 1) blocks = 1;
+  if (blocks > 148ll * per_sm) blocks = 148ll * per_sm;
+  if (max_ctas > 0 && blocks > (long long)max_ctas * per_sm) blocks = (long long)max_ctas * per_sm;
+  return launch_pdl(kernel, dim3((unsigned)blocks), dim3(256), 0, stream, args);
+}
+
 // `max_ctas` > 0 caps the grid below the SM count, leaving whole SMs to a kernel running on another stream.
 // `dense` != null (several GPUs only): the dense step rides on `dense_ctas` extra CTAs of the same cooperative grid.
 cudaError_t launch_sparse_push(const PushArgs& args, int work_items, int max_ctas, const DenseStepArgs* dense, cudaStream_t stream) {
+  if (args.c.world == 1 && dense == nullptr) return launch_sparse_push_local(args, work_items / args.lanes, max_ctas, stream);
   int dev = 0;
   cudaGetDevice(&dev);
   static int grid_max[64] = {0};

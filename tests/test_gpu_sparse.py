@@ -352,3 +352,55 @@ def test_dedup_over_several_ids_per_lane(tn_gpu, status_ok, n, front):
     clicks = torch.zeros(n_u, device=t.dev).index_add_(0, inv.long(), labels)
     assert torch.equal(lk.cnts[:n_u, 1], clicks)
     assert bool((lk.comm["dd_keys"] == -1).all())
+
+
+@pytest.mark.parametrize("kind", ["AdaGrad", "Adam", "Ftrl"])
+@pytest.mark.parametrize("dim,n_ids", [(1, 3), (4, 1), (10, 700), (12, 5000), (20, 33), (100, 2000), (124, 31), (128, 90000), (132, 500), (160, 900)])
+def test_push_every_row_width(tn_gpu, status_ok, kind, dim, n_ids):
+    """Row updates of one GPU against the same mathematics in 64 bits: widths with and without whole 16-byte chunks, up
+    to and beyond 128, fewer rows than a group takes at once and more than the grid takes in one round."""
+    tn = tn_gpu
+    opt = {"AdaGrad": tn.core.AdaGrad(learning_rate=0.05, initial_g2sum=0.1, initial_scale=0.3),
+           "Adam": tn.core.Adam(learning_rate=0.01, initial_scale=0.3),
+           "Ftrl": tn.core.Ftrl(learning_rate=0.05, initial_scale=0.3, lambda1=0.001)}[kind]
+    t, lk = _mk(tn, opt, dim, rows=1 << 17, max_unique=n_ids)
+    ids = (torch.arange(n_ids, device=t.dev) * 104729 + 5) * 1000003
+    g = torch.Generator(device=t.dev).manual_seed(dim)
+    for _ in range(2):
+        lk.pull(ids, labels=torch.ones(n_ids, device=t.dev), training=True)
+        at = t.lookup_rows(lk.comm["stage_ids"][:n_ids]).long()
+        before = t.rows[at].double()
+        lk.gU[:n_ids, :dim] = torch.randn((n_ids, dim), generator=g, device=t.dev)
+        x = lk.gU[:n_ids, :dim].double()
+        lk.push()
+        got = t.rows[at]
+        assert float(lk.gU.abs().sum()) == 0.0 and float(lk.cnts.abs().sum()) == 0.0
+        w, s1, s2 = before[:, :dim], before[:, dim:2 * dim], before[:, 2 * dim:3 * dim]
+        # the update terms are good to a few ulp of 2^-24: the error stays below 2^-19 of the magnitudes that enter
+        if kind == "AdaGrad":
+            acc = before[:, dim] + (x * x).mean(1)
+            step = opt.learning_rate * x / (opt.epsilon + acc.sqrt())[:, None]
+            want = [(got[:, :dim], w - step, w.abs() + step.abs()), (got[:, dim], acc, acc),
+                    (got[:, dim + 1: dim + 3], before[:, dim + 1: dim + 3] + 1, before[:, dim + 1: dim + 3] + 1)]
+            assert bool((got[:, dim + 3].contiguous().view(torch.int32) == 0).all())
+        elif kind == "Adam":
+            b1, b2 = float(np.float32(opt.beta1)), float(np.float32(opt.beta2))      # 1 - beta2 is 5e-5 off its 64-bit value
+            m, v = b1 * s1 + (1 - b1) * x, b2 * s2 + (1 - b2) * x * x
+            step = opt.learning_rate * m / (opt.epsilon + v.sqrt())
+            want = [(got[:, dim:2 * dim], m, s1.abs() + x.abs()), (got[:, 2 * dim:3 * dim], v, v)]
+            ok = v > 1e-8                      # elsewhere the quotient magnifies the rounding of m and v
+            want.append((got[:, :dim][ok], (w - step)[ok], (w.abs() + opt.learning_rate * (s1.abs() + x.abs()) / v.sqrt())[ok]))
+        else:
+            n2 = s2 + x * x
+            z = s1 + x - opt.learning_rate * (n2.sqrt() - s2.sqrt()) * w
+            size = s1.abs() + x.abs() + opt.learning_rate * n2.sqrt() * w.abs()
+            shrunk = torch.where(z > 0, z - opt.lambda1, z + opt.lambda1)
+            scale = (opt.beta + n2.sqrt()) * opt.learning_rate + opt.lambda2
+            ok = (z.abs() - opt.lambda1).abs() > 1e-5          # not on the edge of the dead zone
+            nw = torch.where(z.abs() > opt.lambda1, -shrunk / scale, torch.zeros_like(z))
+            want = [(got[:, dim:2 * dim], z, size), (got[:, 2 * dim:3 * dim], n2, n2), (got[:, :dim][ok], nw[ok], ((size + opt.lambda1) / scale)[ok])]
+        if kind != "AdaGrad":
+            delta = got[:, 3 * dim + 1].contiguous().view(torch.int32)
+            assert bool((delta == before.float()[:, 3 * dim + 1].contiguous().view(torch.int32) + 1).all())
+        for a, b, size in want:
+            assert bool(((a.double() - b).abs() <= 2.0 ** -19 * size + 1e-12).all()), (kind, dim)
