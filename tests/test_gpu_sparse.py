@@ -404,3 +404,37 @@ def test_push_every_row_width(tn_gpu, status_ok, kind, dim, n_ids):
             assert bool((delta == before.float()[:, 3 * dim + 1].contiguous().view(torch.int32) + 1).all())
         for a, b, size in want:
             assert bool(((a.double() - b).abs() <= 2.0 ** -19 * size + 1e-12).all()), (kind, dim)
+
+
+@pytest.mark.parametrize("B,S,dim", [(1, 1, 4), (37, 3, 8), (70001, 3, 32), (1001, 5, 132)])
+@pytest.mark.parametrize("ragged", [False, True])
+@pytest.mark.parametrize("combiner", [0, 1, 2])
+def test_pooling_with_several_rows_in_flight(tn_gpu, status_ok, B, S, dim, ragged, combiner):
+    """Bags of none to nine ids and of exactly one, ids without a row (-1) among them; 32-bit sums of at most nine terms."""
+    from tensornet_b200._build import cuda_ext
+
+    dev, ext = tn_gpu.core.runtime().device, cuda_ext()
+    g = torch.Generator(device=dev).manual_seed(B + dim)
+    lens = torch.randint(0, 10, (B * S,), generator=g, device=dev) if ragged else torch.ones(B * S, dtype=torch.int64, device=dev)
+    offsets = torch.cat([torch.zeros(1, dtype=torch.int64, device=dev), lens.cumsum(0)])
+    nnz, rows = int(offsets[-1]), 1000
+    inverse = torch.randint(-1, rows, (max(nnz, 1),), generator=g, device=dev, dtype=torch.int32)[:nnz]
+    U = torch.randn((rows, dim), generator=g, device=dev)
+    off32 = offsets.int() if ragged else None
+    out = torch.empty((B, S * dim), device=dev)
+    ext.pool_fwd(U, dim, inverse, off32, B, S, dim, combiner, out, S * dim)
+    bag = torch.arange(B * S, device=dev).repeat_interleave(lens)
+    ok = inverse >= 0
+    scale = torch.ones(B * S, device=dev, dtype=torch.float64)
+    if combiner:
+        scale = lens.clamp(min=1).double() ** (-1.0 if combiner == 1 else -0.5)
+    want = torch.zeros((B * S, dim), dtype=torch.float64, device=dev).index_add_(0, bag[ok], U[inverse[ok].long()].double()) * scale[:, None]
+    got = out.view(B, S, dim).transpose(0, 1).reshape(B * S, dim)
+    assert bool(((got.double() - want).abs() <= 16 * 2.0 ** -24 * (want.abs() + 40)).all())
+    gU = torch.zeros((rows, dim), device=dev)
+    gout = torch.randn((B, S * dim), generator=g, device=dev)
+    ext.pool_bwd(gU, dim, inverse, off32, B, S, dim, dim, combiner, gout, S * dim)
+    go = gout.view(B, S, dim).transpose(0, 1).reshape(B * S, dim).double() * scale[:, None]
+    wantg = torch.zeros((rows, dim), dtype=torch.float64, device=dev).index_add_(0, inverse[ok].long(), go[bag[ok]])
+    size = torch.zeros((rows, dim), dtype=torch.float64, device=dev).index_add_(0, inverse[ok].long(), go[bag[ok]].abs())
+    assert bool(((gU.double() - wantg).abs() <= 64 * 2.0 ** -24 * size + 1e-12).all())
