@@ -920,6 +920,29 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     c10::cuda::CUDAGuard guard(g.device());
     tn::launch_cross_v2_bwd_elem(g.data_ptr(), u.data_ptr(), x0.data_ptr(), ptr_of<float>(gx0), du.data_ptr(), g.numel(), first ? 1 : 0, cur_stream());
   });
+  m.def("cross_v2_du", [](at::Tensor g, at::Tensor x0, at::Tensor du) {
+    TORCH_CHECK(g.is_contiguous() && x0.is_contiguous() && du.is_contiguous(), "contiguous operands");
+    TORCH_CHECK(g.numel() % 8 == 0 && x0.numel() == g.numel() && du.numel() == g.numel(), "sizes");
+    TORCH_CHECK(g.scalar_type() == at::kBFloat16 && x0.scalar_type() == at::kBFloat16 && du.scalar_type() == at::kBFloat16, "g / x0 / du are bf16");
+    c10::cuda::CUDAGuard guard(g.device());
+    tn::launch_cross_v2_du(g.data_ptr(), x0.data_ptr(), du.data_ptr(), g.numel(), cur_stream());
+  });
+  m.attr("MAX_CROSS_LAYERS") = (int)tn::kMaxCrossLayers;
+  m.def("cross_v2_bwd_sum", [](std::vector<at::Tensor> g, std::vector<at::Tensor> u, at::Tensor g0, at::Tensor out) {
+    TORCH_CHECK(g.size() == u.size() && g.size() <= (size_t)tn::kMaxCrossLayers, "cross_v2_bwd_sum: one u per g, at most 8 layers");
+    TORCH_CHECK(g0.is_contiguous() && out.is_contiguous() && g0.numel() % 8 == 0 && out.numel() == g0.numel(), "operands");
+    TORCH_CHECK(g0.scalar_type() == at::kBFloat16 && out.scalar_type() == at::kBFloat16, "bf16 operands");
+    tn::CrossTerms t{};
+    t.n = (int)g.size();
+    for (size_t l = 0; l < g.size(); ++l) {
+      for (const at::Tensor* x : {&g[l], &u[l]})
+        TORCH_CHECK(x->is_contiguous() && x->numel() == g0.numel() && x->scalar_type() == at::kBFloat16, "cross_v2_bwd_sum: contiguous bf16 terms");
+      t.g[l] = g[l].data_ptr();
+      t.u[l] = u[l].data_ptr();
+    }
+    c10::cuda::CUDAGuard guard(g0.device());
+    tn::launch_cross_v2_bwd_sum(t, g0.data_ptr(), out.data_ptr(), g0.numel(), cur_stream());
+  });
   m.def("cross_v2_bwd_final", [](at::Tensor gx0, at::Tensor g, at::Tensor out) {
     TORCH_CHECK(gx0.is_contiguous() && g.is_contiguous() && out.is_contiguous() && g.numel() % 8 == 0 && gx0.numel() == g.numel() && out.numel() == g.numel(), "operands");
     c10::cuda::CUDAGuard guard(g.device());

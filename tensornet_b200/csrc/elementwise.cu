@@ -534,6 +534,59 @@ __global__ void cross_v2_bwd_final_kernel(const float4* __restrict__ gx0, const 
   }
 }
 
+// The same backward pass with the Hadamard terms left to the end (networks of up to kMaxCrossLayers layers): per layer only
+// du = g * x0, and once  out = bf16(g_0 + sum_l g_l * u_l), summed in fp32 in the order of the layers above.  The fp32
+// accumulator, read and written once per layer, is gone: three layers at 8192 x 6416 take 275 us per step instead of
+// 463 (49 us and 127 us a kernel, 6.4 TB/s).
+__global__ void cross_v2_du_kernel(const uint4* __restrict__ g, const uint4* __restrict__ x0, uint4* __restrict__ du, long long n8) {
+  pdl_sync();
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n8; i += (long long)gridDim.x * blockDim.x) {
+    const uint4 gv = g[i], xv = x0[i];
+    const __nv_bfloat162* gp = reinterpret_cast<const __nv_bfloat162*>(&gv);
+    const __nv_bfloat162* xp = reinterpret_cast<const __nv_bfloat162*>(&xv);
+    uint4 dv;
+    uint32_t* dp = reinterpret_cast<uint32_t*>(&dv);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float2 gf = __bfloat1622float2(gp[k]), xf = __bfloat1622float2(xp[k]);
+      __nv_bfloat162 d = __floats2bfloat162_rn(gf.x * xf.x, gf.y * xf.y);
+      dp[k] = *reinterpret_cast<uint32_t*>(&d);
+    }
+    du[i] = dv;
+  }
+}
+__global__ void cross_v2_bwd_sum_kernel(const __grid_constant__ CrossTerms t, const uint4* __restrict__ g0, uint4* __restrict__ out,
+                                        long long n8) {
+  pdl_sync();
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n8; i += (long long)gridDim.x * blockDim.x) {
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    const uint4 last = g0[i];
+#pragma unroll
+    for (int l = 0; l < kMaxCrossLayers; ++l) {
+      if (l >= t.n) continue;
+      const uint4 gv = reinterpret_cast<const uint4*>(t.g[l])[i], uv = reinterpret_cast<const uint4*>(t.u[l])[i];
+      const __nv_bfloat162* gp = reinterpret_cast<const __nv_bfloat162*>(&gv);
+      const __nv_bfloat162* up = reinterpret_cast<const __nv_bfloat162*>(&uv);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float2 gf = __bfloat1622float2(gp[k]), uf = __bfloat1622float2(up[k]);
+        acc[2 * k] += gf.x * uf.x;
+        acc[2 * k + 1] += gf.y * uf.y;
+      }
+    }
+    const __nv_bfloat162* gp = reinterpret_cast<const __nv_bfloat162*>(&last);
+    uint4 ov;
+    uint32_t* op = reinterpret_cast<uint32_t*>(&ov);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float2 gf = __bfloat1622float2(gp[k]);
+      __nv_bfloat162 d = __floats2bfloat162_rn(acc[2 * k] + gf.x, acc[2 * k + 1] + gf.y);
+      op[k] = *reinterpret_cast<uint32_t*>(&d);
+    }
+    out[i] = ov;
+  }
+}
+
 inline int blocks_for(long long work, int per_block) {
   long long b = (work + per_block - 1) / per_block;
   if (b < 1) b = 1;
@@ -598,6 +651,14 @@ void launch_cross_v2_bwd_elem(const void* g, const void* u, const void* x0, floa
 void launch_cross_v2_bwd_final(const float* gx0, const void* g, void* out, long long n, cudaStream_t st) {
   launch_pdl(cross_v2_bwd_final_kernel, dim3(blocks_for(n / 8, 256)), dim3(256), 0, st, reinterpret_cast<const float4*>(gx0),
              reinterpret_cast<const uint4*>(g), reinterpret_cast<uint4*>(out), n / 8);
+}
+void launch_cross_v2_du(const void* g, const void* x0, void* du, long long n, cudaStream_t st) {
+  launch_pdl(cross_v2_du_kernel, dim3(blocks_for(n / 8, 256)), dim3(256), 0, st, reinterpret_cast<const uint4*>(g),
+             reinterpret_cast<const uint4*>(x0), reinterpret_cast<uint4*>(du), n / 8);
+}
+void launch_cross_v2_bwd_sum(const CrossTerms& t, const void* g0, void* out, long long n, cudaStream_t st) {
+  launch_pdl(cross_v2_bwd_sum_kernel, dim3(blocks_for(n / 8, 256)), dim3(256), 0, st, t, reinterpret_cast<const uint4*>(g0),
+             reinterpret_cast<uint4*>(out), n / 8);
 }
 void launch_cross_v1_fwd(const float* x0, const float* xl, const float* w, const float* bias, int B, int D, float* y, float* dot,
                          cudaStream_t st) {

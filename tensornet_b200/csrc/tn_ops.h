@@ -68,6 +68,14 @@ void launch_cross_v1_bwd(const float* x0, const float* xl, const float* w, const
                          float* gx0, float* gxl, float* gw, float* gb, cudaStream_t st);
 void launch_relu_mask(void* g, const void* y, long long n, cudaStream_t st);
 void launch_cross_v2_bwd_elem(const void* g, const void* u, const void* x0, float* gx0, void* du, long long n, int first, cudaStream_t st);
+constexpr int kMaxCrossLayers = 8;
+struct CrossTerms {              // gradient of each layer's output and its u, last layer first; bf16
+  const void* g[kMaxCrossLayers];
+  const void* u[kMaxCrossLayers];
+  int n;
+};
+void launch_cross_v2_du(const void* g, const void* x0, void* du, long long n, cudaStream_t st);
+void launch_cross_v2_bwd_sum(const CrossTerms& t, const void* g0, void* out, long long n, cudaStream_t st);
 void launch_cross_v2_bwd_final(const float* gx0, const void* g, void* out, long long n, cudaStream_t st);
 
 // deepfm_fused.cu  (return nullptr or a static error string)

@@ -465,14 +465,21 @@ class _CrossV2(torch.autograd.Function):
         x0 = xs[0]
         B, Dp = x0.shape[0], int(x0.stride(0))
         g = g.contiguous()
-        gx0 = torch.empty((B, Dp), dtype=torch.float32, device=g.device)
+        # the gradients of the layers' outputs are kept and their Hadamard terms summed at the end, in one pass, unless
+        # there are more layers than that kernel takes
+        late = L <= ext.MAX_CROSS_LAYERS
+        gs = []
+        gx0 = None if late else torch.empty((B, Dp), dtype=torch.float32, device=g.device)
         du = torch.empty((B, Dp), dtype=torch.bfloat16, device=g.device)
         for l in range(L - 1, -1, -1):
             w, xl = weights[l], xs[l]
             wb = _bf16_of(w)
             Kp = int(w.shape[1])
-            # gx0 (+)= g * u ; du = g * x0   in one pass
-            ext.cross_v2_bwd_elem(g, us[l], x0, gx0, du, l == L - 1)
+            if late:
+                ext.cross_v2_du(g, x0, du)
+                gs.append(g)
+            else:       # gx0 (+)= g * u ; du = g * x0   in one pass
+                ext.cross_v2_bwd_elem(g, us[l], x0, gx0, du, l == L - 1)
             if w.requires_grad:
                 ext.gemm(du, xl, _grad_buffer(w), dim, dim + 1, B, Dp, Dp, Kp, True, True, True, False, None, None, None, None, 0, -1,
                          dim + 1, 0, 0, st)
@@ -481,7 +488,10 @@ class _CrossV2(torch.autograd.Function):
             ext.gemm(du, wb, gn, B, min(Kp, Dp), dim, Dp, Kp, Dp, False, True, False, False, None, None, None, g, Dp, -1, Dp, 1, 0, st)
             g = gn
         out = torch.empty((B, Dp), dtype=torch.bfloat16, device=g.device)
-        ext.cross_v2_bwd_final(gx0, g, out)
+        if late:
+            ext.cross_v2_bwd_sum(gs, list(us[::-1]), g, out)
+        else:
+            ext.cross_v2_bwd_final(gx0, g, out)
         return (out, None, *([None] * L))
 
 

@@ -268,3 +268,23 @@ def test_head_forward_backward_wide(tn_gpu, status_ok, K):
     gw = F._grad_buffer(w)
     gw_ref = z.detach().float()[:, :K].t() @ gy.view(-1)
     assert torch.allclose(gw[:K], gw_ref, rtol=2e-2, atol=5e-2)
+
+
+@pytest.mark.parametrize("layers", [1, 3, 8])
+def test_cross_v2_backward_terms_summed_at_the_end(tn_gpu, status_ok, layers):
+    """out = bf16(g_0 + sum g_l * u_l): one rounding to bf16 (half of 2^-7) on top of a 32-bit sum."""
+    dev = tn_gpu.core.runtime().device
+    n = 257 * 136
+    gen = torch.Generator(device="cpu").manual_seed(layers)
+    draw = lambda: torch.randn(n, generator=gen).bfloat16().to(dev)
+    gs, us, g0, x0 = [draw() for _ in range(layers)], [draw() for _ in range(layers)], draw(), draw()
+    out, du = torch.empty_like(g0), torch.empty_like(g0)
+    _ext().cross_v2_bwd_sum(gs, us, g0, out)
+    want = g0.double() + sum(a.double() * b.double() for a, b in zip(gs, us))
+    size = g0.double().abs() + sum((a.double() * b.double()).abs() for a, b in zip(gs, us))
+    assert bool(((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -20 * size).all())
+    _ext().cross_v2_du(g0, x0, du)
+    assert torch.equal(du, (g0.float() * x0.float()).bfloat16())
+    if layers == 8:
+        with pytest.raises(RuntimeError):
+            _ext().cross_v2_bwd_sum(gs + [g0], us + [x0], g0, out)
