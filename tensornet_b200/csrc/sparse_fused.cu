@@ -2,7 +2,8 @@
 // all-to-all exchange with the owning GPUs over NVLink peer memory, the owner-side hash
 // probe (insert on miss) and the optimizer update each run as ONE persistent cooperative
 // kernel per direction.  Peer traffic is plain ld/st to symmetric-heap addresses with
-// release/acquire flags at system scope; no collective library is involved.
+// release/acquire flags at system scope; no collective library is involved.  On one GPU there is nothing to push to
+// anybody: the row updates are an ordinary kernel there (sparse_push_local_kernel).
 //
 // What these kernels replace in the reference:
 //   pull : SparsePullVarInfo dedup + per-shard RPC fan-out + SparseTable::Pull + scatter back
