@@ -265,6 +265,28 @@ class _PredictSets:
         self.turn = 0
 
 
+_OWN_CODE = (__name__.split(".")[0] + ".", "torch.nn.")
+
+
+def _own_code(fn) -> bool:
+    return (getattr(fn, "__module__", None) or "").startswith(_OWN_CODE)
+
+
+def _scored_by_own_code(model) -> bool:
+    """Is all Python that scores a batch with ``model`` this package's or torch.nn's?  Such code does nothing but launch
+    kernels, so a replay of its launches stands for it.  Code of the user's (an overridden ``predict_step``, a forward
+    pass or a hook of its own) may count, keep or branch on what it sees, and has to run for every batch."""
+    hooks = torch.nn.modules.module
+    if hooks._global_forward_hooks or hooks._global_forward_pre_hooks or torch.is_autocast_enabled("cuda"):
+        return False
+    if not _own_code(type(model).predict_step) or "predict_step" in model.__dict__:
+        return False
+    for m in model.modules():
+        if not (_own_code(type(m)) and _own_code(type(m).forward)) or "forward" in m.__dict__ or m._forward_hooks or m._forward_pre_hooks:
+            return False
+    return True
+
+
 _PREDICT_RING = 16   # pinned buffers for predictions on their way to the host: how far the host may run ahead
 
 
@@ -948,11 +970,14 @@ class Model(nn.Module):
         return y, pred
 
     # ---- captured scoring steps ---------------------------------------------------------------------------------
-    def _predict_captured(self, features):
+    def _predict_captured(self, features, check: bool = True):
         """Issue the captured scoring step for a batch in host memory: ``(sets, index)`` whose ``pred[index]`` will hold
-        the predictions, or None when this batch is to be scored eagerly."""
+        the predictions, or None when this batch is to be scored eagerly.  ``check``: code of the user's may have run
+        since the last batch, so look again at whether it takes part in the scoring."""
         rt = core.runtime()
         if not self._use_graph or self._predict_off or rt.world > 1:
+            return None
+        if check and not _scored_by_own_code(self):
             return None
         leaves: List[torch.Tensor] = []
         spec = _flatten(features, leaves)
@@ -1052,12 +1077,14 @@ class Model(nn.Module):
                 cb.on_predict_begin()
             ys, ps = [], []
             self.eval()
+            own = False                      # nothing of the user's runs between the batches of a list
             ring, flying = [], []            # pinned buffers; (position in ps, buffer, event) of copies on their way
             for i, batch in enumerate(dataset):
                 if steps is not None and i >= steps:
                     break
                 features, labels = batch if isinstance(batch, (tuple, list)) and len(batch) == 2 else (batch, None)
-                issued = self._predict_captured(features) if not self.training else None
+                issued = self._predict_captured(features, check=not own) if not self.training else None
+                own = issued is not None and type(dataset) in (list, tuple)
                 if issued is None:
                     y, p = self.predict_step(batch)
                     ps.append(p.cpu())
