@@ -272,19 +272,46 @@ def _own_code(fn) -> bool:
     return (getattr(fn, "__module__", None) or "").startswith(_OWN_CODE)
 
 
-def _scored_by_own_code(model) -> bool:
-    """Is all Python that scores a batch with ``model`` this package's or torch.nn's?  Such code does nothing but launch
-    kernels, so a replay of its launches stands for it.  Code of the user's (an overridden ``predict_step``, a forward
-    pass or a hook of its own) may count, keep or branch on what it sees, and has to run for every batch."""
+_PLAIN = (int, float, bool, str)
+# what training and compile change on the modules of a model without any bearing on its predictions
+_NOT_SCORED = {"stop_training", "is_loaded_from_checkpoint", "metrics", "optimizer", "loss_fn", "batch_counter"}
+
+
+def _scoring_state(model) -> Optional[list]:
+    """What a captured scoring step of ``model`` is made from: its modules, the storage of their parameters and buffers,
+    and the public attributes their forward passes go by.  None when a replay cannot stand for scoring a batch: that
+    takes Python which does nothing but launch kernels, as this package's and torch.nn's does.  Code of the user's (an
+    overridden ``predict_step``, a forward pass or a hook of its own) may count, keep or branch on what it sees, and has
+    to run for every batch."""
     hooks = torch.nn.modules.module
     if hooks._global_forward_hooks or hooks._global_forward_pre_hooks or torch.is_autocast_enabled("cuda"):
-        return False
+        return None
     if not _own_code(type(model).predict_step) or "predict_step" in model.__dict__:
-        return False
+        return None
+    out: list = [torch.get_float32_matmul_precision()]
     for m in model.modules():
         if not (_own_code(type(m)) and _own_code(type(m).forward)) or "forward" in m.__dict__ or m._forward_hooks or m._forward_pre_hooks:
-            return False
-    return True
+            return None
+        out.append(m)
+        for held in (m._parameters, m._buffers):
+            for t in held.values():
+                out.append(t)
+                if t is not None:
+                    out.append(t.data_ptr())
+                    out.append(getattr(t, "_tn_bf16", None))
+        for k, v in m.__dict__.items():
+            if k[0] != "_" and k not in _NOT_SCORED:
+                if type(v) in (list, tuple):
+                    out.extend(v)
+                else:
+                    out.append(v)
+                    if torch.is_tensor(v):
+                        out.append(v.data_ptr())
+    return out
+
+
+def _same_state(a: list, b: list) -> bool:
+    return len(a) == len(b) and all(x is y or (type(x) is type(y) and type(x) in _PLAIN and x == y) for x, y in zip(a, b))
 
 
 _PREDICT_RING = 16   # pinned buffers for predictions on their way to the host: how far the host may run ahead
@@ -357,6 +384,7 @@ class Model(nn.Module):
         self._predict_sets: Dict[Any, Any] = {}      # batch signature -> number of batches seen, then _PredictSets
         self._predict_rooms: Dict[Any, List[Any]] = {}
         self._predict_off = False                    # the scoring step cannot be captured
+        self._predict_state = None                   # what the captured scoring steps were recorded from
         self._max_graphs = 8
         self._graph_key = None
         self._static_leaves: List[torch.Tensor] = []
@@ -380,6 +408,7 @@ class Model(nn.Module):
         ``acc, mse, mae, mape`` and any other metric object get ``update_state(labels, predictions)`` after every
         step; such a model runs its steps without CUDA graphs."""
         rt = core.runtime()
+        self._drop_captures()
         self.to(rt.device)
         self.optimizer = optimizer
         self.loss_fn = loss
@@ -428,6 +457,27 @@ class Model(nn.Module):
                     for lk in getattr(layer, "links", None) or [layer.link]:
                         lk.push_cta_cap = torch.cuda.get_device_properties(rt.device).multi_processor_count - dense_sms
         return self
+
+    def _drop_captures(self):
+        """Captured steps read the parameters, metric sums and optimizer arrays they were recorded with; ``compile`` puts
+        others in their place.  Training then starts over with its eager steps, on every rank alike."""
+        if self._graphs or self._rings:
+            torch.cuda.synchronize()
+        self._graphs.clear()
+        self._rings.clear()
+        self._padded_keys.clear()
+        self._ring_refused = self._padded_off = self._predict_off = False
+        self._graph = self._graph_key = self._flat_cache = self._last_done = self._last_set = self._static_loss = None
+        self._static_leaves = []
+        self._max_graphs, self._eager_steps = 8, 0
+        self._drop_scoring()
+
+    def _drop_scoring(self):
+        if any(isinstance(v, _PredictSets) for v in self._predict_sets.values()):
+            torch.cuda.synchronize()         # replays and copies of predictions under way
+        self._predict_sets.clear()
+        self._predict_rooms.clear()
+        self._predict_state = None
 
     def sparse_layers(self):
         return [m for m in self.modules() if hasattr(m, "backwards") and m is not self]
@@ -973,11 +1023,9 @@ class Model(nn.Module):
     def _predict_captured(self, features, check: bool = True):
         """Issue the captured scoring step for a batch in host memory: ``(sets, index)`` whose ``pred[index]`` will hold
         the predictions, or None when this batch is to be scored eagerly.  ``check``: code of the user's may have run
-        since the last batch, so look again at whether it takes part in the scoring."""
+        since the last batch, so look again at what the model is made of."""
         rt = core.runtime()
         if not self._use_graph or self._predict_off or rt.world > 1:
-            return None
-        if check and not _scored_by_own_code(self):
             return None
         leaves: List[torch.Tensor] = []
         spec = _flatten(features, leaves)
@@ -994,6 +1042,12 @@ class Model(nn.Module):
         except TypeError:                    # a feature that is no tensor and cannot be compared: nothing to recognise it by
             return None
         if not isinstance(sets, _PredictSets):
+            state = _scoring_state(self)
+            if state is None:
+                return None
+            if self._predict_state is not None and not _same_state(state, self._predict_state):
+                self._drop_scoring()
+                return None
             # the first batch of a kind runs eagerly, the second one is captured
             if len(self._predict_sets) > 64:
                 self._predict_sets.clear()
@@ -1015,15 +1069,12 @@ class Model(nn.Module):
                 self._predict_sets.pop(held[0])
             try:
                 sets = self._predict_sets[key] = self._capture_predict(spec, leaves, rooms)
+                self._predict_state, check = state, False
             except Exception:                # something in the forward pass cannot be captured
                 torch.cuda.synchronize()
                 self._predict_off = True
                 self._predict_sets.clear()
                 return None
-        for link in self._predict_links:
-            link.table.set_training(False)
-            if link._front is not None:      # a front that ran ahead for the next training batch
-                link.discard_front()
         p = sets.turn
         sets.turn ^= 1
         main = torch.cuda.current_stream()
@@ -1031,6 +1082,17 @@ class Model(nn.Module):
         self._ext.stage_inputs(sets.leaves[p], leaves, self._copy_stream.cuda_stream, main.cuda_stream,
                                sets.done[p].cuda_event if sets.used[p] else 0, sets.copied[p].cuda_event,
                                read.cuda_event if read is not None else 0)
+        if check:                            # the inputs are on their way meanwhile
+            state = _scoring_state(self)
+            if state is None:
+                return None
+            if not _same_state(state, self._predict_state):
+                self._drop_scoring()
+                return None
+        for link in self._predict_links:
+            link.table.set_training(False)
+            if link._front is not None:      # a front that ran ahead for the next training batch
+                link.discard_front()
         sets.graphs[p].replay()
         sets.done[p].record(main)
         sets.used[p] = True

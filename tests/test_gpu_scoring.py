@@ -72,3 +72,53 @@ def test_code_of_the_users_runs_for_every_batch(tn_gpu, status_ok):
     m.predict(data)
     m.predict_step = lambda batch: (batch[1], torch.full((48, 1), 0.25))
     assert float(m.predict(data)[1].max()) == 0.25
+
+
+def _held(m):
+    """Keeps the storage a model scores from alive, so that a step captured from it reads what it read before."""
+    return [p.data for p in m.parameters()] + [getattr(p, "_tn_bf16", None) for p in m.parameters()]
+
+
+def test_scoring_follows_what_the_model_is_made_of(tn_gpu, status_ok):
+    """Parameters re-pointed by an optimizer, a replaced sub-module, an attribute the forward pass goes by."""
+    from tensornet_b200.layers import DenseHead
+
+    tn = tn_gpu
+    data = _data(tn, 20)
+    m = _model(tn, compiled=False)
+    m.compile()
+    keep = [_held(m)]
+    m.predict(data)
+    for _ in range(2):
+        keep.append((m.optimizer, _held(m)))
+        m.compile(optimizer=tn.optimizer.Optimizer(tn.core.Adam(learning_rate=3e-2)))
+        before = m.predict(data)[1]
+        _same(before, _eager(m, data))
+        m.fit(data)
+        after = m.predict(data)[1]
+        _same(after, _eager(m, data))
+        assert float((after - before).abs().max()) > 1e-3
+    keep.append(m.sub_model.head)
+    m.sub_model.head = DenseHead(m.sub_model.head.in_dim).cuda()
+    _same(m.predict(data)[1], _eager(m, data))
+    m.sub_model.mlp.relu_last = False
+    _same(m.predict(data)[1], _eager(m, data))
+    m.predict(data)
+    sets = dict(m._predict_sets)
+    m.fit(data)                                       # training writes the weights in place: nothing to capture again
+    _same(m.predict(data)[1], _eager(m, data))
+    assert sets == m._predict_sets and not m._predict_off
+
+
+def test_training_follows_a_second_optimizer(tn_gpu, status_ok):
+    tn = tn_gpu
+    data = _data(tn, 12)
+    m = _model(tn)
+    m.fit(data)
+    keep = (m.optimizer, _held(m))
+    m.compile(optimizer=tn.optimizer.Optimizer(tn.core.Adam(learning_rate=1e-2)))
+    before = [p.detach().clone() for p in m.parameters()]
+    m.fit(data, epochs=2)
+    assert m._graphs or m._rings
+    assert all(not torch.equal(a, b) for a, b in zip(before, m.parameters()))
+    del keep
