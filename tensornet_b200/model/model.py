@@ -1021,8 +1021,8 @@ class Model(nn.Module):
 
     # ---- captured scoring steps ---------------------------------------------------------------------------------
     def _predict_captured(self, features, check: bool = True):
-        """Issue the captured scoring step for a batch in host memory: ``(sets, index)`` whose ``pred[index]`` will hold
-        the predictions, or None when this batch is to be scored eagerly.  ``check``: code of the user's may have run
+        """Issue the captured scoring step for a batch in host memory: ``(sets, index, inputs)``, where ``sets.pred[index]``
+        will hold the predictions and ``sets.copied[index]`` tells when the inputs have been read; or None when this batch is to be scored eagerly.  ``check``: code of the user's may have run
         since the last batch, so look again at what the model is made of."""
         rt = core.runtime()
         if not self._use_graph or self._predict_off or rt.world > 1:
@@ -1096,7 +1096,7 @@ class Model(nn.Module):
         sets.graphs[p].replay()
         sets.done[p].record(main)
         sets.used[p] = True
-        return sets, p
+        return sets, p, leaves
 
     def _capture_predict(self, spec, leaves, rooms):
         from .. import _build
@@ -1154,7 +1154,7 @@ class Model(nn.Module):
                         ys.append(y.cpu())
                     continue
                 # predictions go to the host behind the step on a stream of their own; the host runs ahead meanwhile
-                sets, k = issued
+                sets, k, leaves = issued
                 pred = sets.pred[k]
                 if len(flying) >= _PREDICT_RING:
                     at, buf, ev = flying.pop(0)
@@ -1173,7 +1173,9 @@ class Model(nn.Module):
                 flying.append((len(ps), buf, ev))
                 ps.append(None)
                 if labels is not None:
-                    ys.append(labels.cpu())
+                    ys.append(labels.cpu() if labels.is_cuda else labels.clone())
+                if not own and any(t.is_pinned() for t in leaves):
+                    sets.copied[k].synchronize()     # a reader may fill the same page-locked buffers with the next batch
             for at, buf, ev in flying:
                 ev.synchronize()
                 ps[at] = buf

@@ -122,3 +122,27 @@ def test_training_follows_a_second_optimizer(tn_gpu, status_ok):
     assert m._graphs or m._rings
     assert all(not torch.equal(a, b) for a, b in zip(before, m.parameters()))
     del keep
+
+
+@pytest.mark.parametrize("pinned", [False, True])
+def test_a_reader_may_fill_the_same_buffers_again(tn_gpu, status_ok, pinned):
+    """Ids and labels of every batch in one buffer each, overwritten as soon as the next batch is asked for."""
+    tn = tn_gpu
+    data = _data(tn, 30)
+    m = _model(tn)
+    want = _eager(m, data)
+    ids = torch.empty((3, 48), dtype=torch.int64, pin_memory=pinned)
+    y = torch.empty(48, pin_memory=pinned)
+
+    def reader():
+        for f, labels in data:
+            ids.copy_(f[tn.data.PACKED_KEY].ids)
+            y.copy_(labels)
+            yield {tn.data.PACKED_KEY: tn.data.PackedFeatures(SLOTS, ids=ids)}, y
+        ids.fill_(7)
+        y.fill_(0.5)
+
+    for _ in range(2):
+        labels, got = m.predict(reader())
+        _same(got, want)
+        assert torch.equal(labels, torch.cat([l for _, l in data]))
