@@ -1050,8 +1050,7 @@ class Model(nn.Module):
                 return None
             # the first batch of a kind runs eagerly, the second one is captured
             if len(self._predict_sets) > 64:
-                self._predict_sets.clear()
-                self._predict_rooms.clear()
+                self._drop_scoring()
                 return None
             if rooms is not None:
                 known = self._predict_rooms[key[0]]
@@ -1066,6 +1065,7 @@ class Model(nn.Module):
             self._predict_shape, self._predict_dtype = like.shape, like.dtype
             held = [k for k, v in self._predict_sets.items() if isinstance(v, _PredictSets)]
             if len(held) >= self._max_graphs > 0:
+                torch.cuda.synchronize()
                 self._predict_sets.pop(held[0])
             try:
                 sets = self._predict_sets[key] = self._capture_predict(spec, leaves, rooms)
@@ -1102,6 +1102,8 @@ class Model(nn.Module):
         from .. import _build
         self._ext = _build.cuda_ext()
         dev = core.runtime().device
+        if getattr(self, "_read_stream", None) is None:
+            self._read_stream = torch.cuda.Stream(device=dev)
         self._predict_links = [lk for layer in self.sparse_layers() for lk in (getattr(layer, "links", None) or [getattr(layer, "link", None)])
                                if lk is not None and hasattr(lk, "discard_front")]
         for lk in self._predict_links:
@@ -1116,6 +1118,7 @@ class Model(nn.Module):
             g = torch.cuda.CUDAGraph()
             # the predictions live outside the captures' shared memory pool, where the other capture would overwrite them
             pred = torch.empty(self._predict_shape, dtype=self._predict_dtype, device=dev)
+            pred.record_stream(self._read_stream)      # copied to the host from there: not to be handed out before
             with torch.no_grad(), capture(g, pool):
                 torch.sigmoid(self(f), out=pred)
             pool = pool or g.pool()
@@ -1163,8 +1166,6 @@ class Model(nn.Module):
                     ring.append((buf, ev))
                 fit = [j for j, (b, _) in enumerate(ring) if b.shape == pred.shape and b.dtype == pred.dtype]
                 buf, ev = ring.pop(fit[0]) if fit else (torch.empty(pred.shape, dtype=pred.dtype, pin_memory=True), torch.cuda.Event())
-                if getattr(self, "_read_stream", None) is None:
-                    self._read_stream = torch.cuda.Stream(device=pred.device)
                 with torch.cuda.stream(self._read_stream):
                     self._read_stream.wait_event(sets.done[k])
                     buf.copy_(pred, non_blocking=True)

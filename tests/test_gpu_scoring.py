@@ -146,3 +146,30 @@ def test_a_reader_may_fill_the_same_buffers_again(tn_gpu, status_ok, pinned):
         labels, got = m.predict(reader())
         _same(got, want)
         assert torch.equal(labels, torch.cat([l for _, l in data]))
+
+
+def test_predictions_outlive_the_captures_they_came_from(tn_gpu, status_ok, monkeypatch):
+    """Captured steps that go while the copies of their predictions still wait for their turn on the read-back stream."""
+    tn = tn_gpu
+    data = _data(tn, 40, B=512)
+    m = _model(tn, B=512)
+    want = _eager(m, data)
+    m.predict(data)
+    issue = type(m)._predict_captured
+
+    def late(self, features, check=True):
+        got = issue(self, features, check)
+        with torch.cuda.stream(self._read_stream):
+            torch.cuda._sleep(2_000_000)               # about a millisecond: the copy of this batch's predictions is late
+        if len(calls) % 5 == 4:
+            torch.cuda.current_stream().synchronize()  # the replays are over, the copies are not
+            self._predict_sets.clear()                 # the last reference but the one predict holds for this batch
+            torch.full((512, 1), 9.0, device="cuda")   # whoever gets the memory next writes it at once
+            torch.full((512, 1), 9.0, device="cuda")
+        calls.append(got is not None)
+        return got
+
+    calls = []
+    monkeypatch.setattr(tn.model.Model, "_predict_captured", late)
+    _same(m.predict(data)[1], want)
+    assert sum(calls) >= 10
