@@ -314,6 +314,31 @@ def _same_state(a: list, b: list) -> bool:
     return len(a) == len(b) and all(x is y or (type(x) is type(y) and type(x) in _PLAIN and x == y) for x, y in zip(a, b))
 
 
+_PADDED_SETS = 3     # captured steps per kind of ragged batch: short, usual and long ones
+_KINDS = 64          # kinds of batches whose history is kept
+
+
+class _Kind:
+    """The batches of one structure and fixed shapes, as far as captured steps go."""
+
+    __slots__ = ("sets", "sights")
+
+    def __init__(self):
+        self.sets: List[Any] = []        # ragged batches: (rooms, key of the captured step), one per capture
+        self.sights = 0                  # batches that found no captured step
+
+    @staticmethod
+    def of(kinds: Dict[Any, "_Kind"], base) -> "_Kind":
+        kind = kinds.get(base)
+        if kind is None:
+            if len(kinds) >= _KINDS:     # batch sizes that never come back
+                for k in [k for k, v in kinds.items() if not v.sets]:
+                    del kinds[k]
+            kind = kinds[base] = _Kind()
+        return kind
+
+
+_PREDICT_SETS = 8    # captured scoring steps per model; batches of further kinds are scored eagerly
 _PREDICT_RING = 16   # pinned buffers for predictions on their way to the host: how far the host may run ahead
 
 
@@ -379,10 +404,10 @@ class Model(nn.Module):
         self._loss_stream = None                     # the stream that copies it there
         self._last_done = None                       # event behind the last replayed step (None after an eager one)
         self._last_set = None                        # (captured sets, index) of the last replayed step
-        self._padded_keys: Dict[Any, List[Any]] = {} # ragged batches: (structure, fixed shapes) -> [(rooms, key of ``_graphs``)]
+        self._padded_kinds: Dict[Any, _Kind] = {}    # ragged batches, by structure and fixed shapes
         self._padded_off = False                     # a captured step needed exact lengths
-        self._predict_sets: Dict[Any, Any] = {}      # batch signature -> number of batches seen, then _PredictSets
-        self._predict_rooms: Dict[Any, List[Any]] = {}
+        self._predict_sets: Dict[Any, _PredictSets] = {}    # batch signature -> the two captures of the scoring step
+        self._predict_kinds: Dict[Any, _Kind] = {}
         self._predict_off = False                    # the scoring step cannot be captured
         self._predict_state = None                   # what the captured scoring steps were recorded from
         self._max_graphs = 8
@@ -465,7 +490,7 @@ class Model(nn.Module):
             torch.cuda.synchronize()
         self._graphs.clear()
         self._rings.clear()
-        self._padded_keys.clear()
+        self._padded_kinds.clear()
         self._ring_refused = self._padded_off = self._predict_off = False
         self._graph = self._graph_key = self._flat_cache = self._last_done = self._last_set = self._static_loss = None
         self._static_leaves = []
@@ -473,10 +498,10 @@ class Model(nn.Module):
         self._drop_scoring()
 
     def _drop_scoring(self):
-        if any(isinstance(v, _PredictSets) for v in self._predict_sets.values()):
+        if self._predict_sets:
             torch.cuda.synchronize()         # replays and copies of predictions under way
         self._predict_sets.clear()
-        self._predict_rooms.clear()
+        self._predict_kinds.clear()
         self._predict_state = None
 
     def sparse_layers(self):
@@ -647,13 +672,9 @@ class Model(nn.Module):
         moved = [t.to(dev, non_blocking=True) for t in leaves]
         return _unflatten(spec, iter(moved)), spec, leaves
 
-    def _padded_plan(self, spec, leaves, captured=None, rooms_of=None):
-        """For a batch with ragged slots in host memory: ``(key, rooms per ragged leaf)`` of the captured step it can run
-        in, or None.  The captured buffers have room to spare and the kernels read the number of ids from the last
-        offset, so that batches of many lengths share one capture.  One GPU only: with several, every rank would have
-        to capture at the same step.  ``captured`` / ``rooms_of``: the captures to look among (default: training steps)."""
-        captured = self._graphs if captured is None else captured
-        rooms_of = self._padded_keys if rooms_of is None else rooms_of
+    def _padded_lengths(self, spec, leaves):
+        """``(positions, lengths)`` of the ragged leaves of a batch in host memory that could run in a padded captured
+        step, else None.  One GPU only: with several, every rank would have to capture at the same step."""
         if self._padded_off or core.runtime().world > 1 or any(t.is_cuda for t in leaves):
             return None
         ragged = _ragged_leaves(spec)
@@ -662,21 +683,30 @@ class Model(nn.Module):
         # ids beyond the last offset (or missing ones) are the caller's to explain: such a batch runs at its exact length
         from .. import _build
         n = _build.cuda_ext().ragged_lengths([leaves[i + k] for i in ragged for k in (0, 1)])
-        if not n:
+        return (ragged, n) if n else None
+
+    def _padded_plan(self, spec, leaves, kinds, full: bool):
+        """For a batch with ragged slots in host memory: ``(kind, key, rooms)`` of the captured step to run it in, None
+        when it does not take that path.  The captured buffers have room to spare and the kernels read the number of ids
+        from the last offset, so that batches of many lengths share one capture.  ``key`` is None for a batch that fits
+        none of its kind's captures when there are as many as there may be (``full``: of the whole model)."""
+        got = self._padded_lengths(spec, leaves)
+        if got is None:
             return None
+        ragged, n = got
         at = set(ragged)
         base = (spec, tuple((None if i in at else t.shape, t.dtype) for i, t in enumerate(leaves)))
-        known = rooms_of.setdefault(base, [])
-        best = None
-        for rooms, key in known:
-            # a much too large capture is not used: its kernels are launched for the room, not for the ids
-            if key in captured and all(a <= r for a, r in zip(n, rooms)) and sum(rooms) <= 2 * sum(n) + 4096:
-                if best is None or sum(rooms) < sum(best[0]):
-                    best = (rooms, key)
-        if best is None:
-            rooms = tuple(_room_for(a, bool(known)) for a in n)
-            best = (rooms, (base, rooms))
-        return best[1], dict(zip(ragged, best[0]))
+        kind = _Kind.of(kinds, base)
+        fits = sorted((sum(rooms), rooms, k) for k, (rooms, _) in enumerate(kind.sets) if all(a <= r for a, r in zip(n, rooms)))
+        # a much too large capture is the second choice: its kernels are launched for the room, not for the ids
+        if fits and (fits[0][0] <= 2 * sum(n) + 4096 or full or len(kind.sets) >= _PADDED_SETS):
+            rooms, key = kind.sets[fits[0][2]]
+        elif full or len(kind.sets) >= _PADDED_SETS:
+            return kind, None, None
+        else:
+            rooms = tuple(_room_for(a, bool(kind.sets)) for a in n)
+            key = (base, rooms)
+        return kind, key, dict(zip(ragged, rooms))
 
     def _eager_step(self, features, labels):
         self._last_done = None
@@ -703,14 +733,15 @@ class Model(nn.Module):
         rt = core.runtime()
         leaves: List[torch.Tensor] = []
         spec = _flatten((features, labels), leaves)
-        key, rooms = (spec, tuple((t.shape, t.dtype) for t in leaves)), None
+        key, rooms, kind = (spec, tuple((t.shape, t.dtype) for t in leaves)), None, None
         static = _is_static(spec)
+        held = len(self._graphs) + len(self._rings)
         if not static:
-            plan = self._padded_plan(spec, leaves)
+            plan = self._padded_plan(spec, leaves, self._padded_kinds, held >= self._max_graphs)
             if plan is not None:
-                key, rooms = plan
-        what = graph_decision(rt.world, key in self._graphs, static or rooms is not None, len(self._graphs) + len(self._rings), self._max_graphs,
-                              self._eager_steps, self._graph_warmup)
+                kind, key, rooms = plan
+        what = "eager" if key is None else graph_decision(rt.world, key in self._graphs, static, held, self._max_graphs,
+                                                          self._eager_steps, self._graph_warmup)
         if what == "eager":
             self._eager_steps += 1
             loss = self._eager_step(features, labels)
@@ -723,7 +754,7 @@ class Model(nn.Module):
             elif rooms is not None:
                 try:
                     self._capture(spec, leaves, key, rooms)
-                    self._padded_keys[key[0]].append((key[1], key))
+                    kind.sets.append((key[1], key))
                 except Exception:           # something in the step wants exact lengths (or cannot be captured): no padding any more
                     torch.cuda.synchronize()
                     self._padded_off = True
@@ -985,6 +1016,8 @@ class Model(nn.Module):
         self._loss_steps = loss_steps0
         if len(self._graphs) >= self._max_graphs:          # static shapes beyond the cap replace the oldest capture
             self._graphs.pop(next(iter(self._graphs)))
+            for kind in self._padded_kinds.values():
+                kind.sets = [x for x in kind.sets if x[1] in self._graphs]
         self._graphs[key] = gp
         # Capture takes a different time on every rank; the first replay's kernels wait for their peers on the
         # device with a finite budget, so line the ranks up on the host first.
@@ -1022,8 +1055,9 @@ class Model(nn.Module):
     # ---- captured scoring steps ---------------------------------------------------------------------------------
     def _predict_captured(self, features, check: bool = True):
         """Issue the captured scoring step for a batch in host memory: ``(sets, index, inputs)``, where ``sets.pred[index]``
-        will hold the predictions and ``sets.copied[index]`` tells when the inputs have been read; or None when this batch is to be scored eagerly.  ``check``: code of the user's may have run
-        since the last batch, so look again at what the model is made of."""
+        will hold the predictions and ``sets.copied[index]`` tells when the inputs have been read; or None when this batch
+        is to be scored eagerly.  ``check``: code of the user's may have run since the last batch, so look again at what
+        the model is made of."""
         rt = core.runtime()
         if not self._use_graph or self._predict_off or rt.world > 1:
             return None
@@ -1031,49 +1065,42 @@ class Model(nn.Module):
         spec = _flatten(features, leaves)
         if not leaves or any(t.is_cuda or not t.is_contiguous() for t in leaves):
             return None
-        key, rooms = (spec, tuple((t.shape, t.dtype) for t in leaves)), None
+        key, rooms, kind = (spec, tuple((t.shape, t.dtype) for t in leaves)), None, None
+        full = len(self._predict_sets) >= _PREDICT_SETS
         try:
             if not _is_static(spec):
-                plan = self._padded_plan(spec, leaves, self._predict_sets, self._predict_rooms)
-                if plan is None:
+                plan = self._padded_plan(spec, leaves, self._predict_kinds, full)
+                if plan is None or plan[1] is None:
                     return None
-                key, rooms = plan
+                kind, key, rooms = plan
             sets = self._predict_sets.get(key)
+            if sets is None and kind is None:
+                kind = _Kind.of(self._predict_kinds, key)
         except TypeError:                    # a feature that is no tensor and cannot be compared: nothing to recognise it by
             return None
-        if not isinstance(sets, _PredictSets):
+        if sets is None:
             state = _scoring_state(self)
             if state is None:
                 return None
             if self._predict_state is not None and not _same_state(state, self._predict_state):
                 self._drop_scoring()
                 return None
-            # the first batch of a kind runs eagerly, the second one is captured
-            if len(self._predict_sets) > 64:
-                self._drop_scoring()
-                return None
-            if rooms is not None:
-                known = self._predict_rooms[key[0]]
-                if (key[1], key) not in known:
-                    known.append((key[1], key))
-            if sets is None:
-                self._predict_sets[key] = 1
+            kind.sights += 1
+            if full or kind.sights < 2:      # the first batch of a kind runs eagerly, the second one is captured
                 return None
             with torch.no_grad():            # shape and type of the result, from the batch itself
                 (f,), _, _ = self._to_device((features,))
                 like = torch.sigmoid(self(f))
             self._predict_shape, self._predict_dtype = like.shape, like.dtype
-            held = [k for k, v in self._predict_sets.items() if isinstance(v, _PredictSets)]
-            if len(held) >= self._max_graphs > 0:
-                torch.cuda.synchronize()
-                self._predict_sets.pop(held[0])
             try:
                 sets = self._predict_sets[key] = self._capture_predict(spec, leaves, rooms)
                 self._predict_state, check = state, False
+                if rooms is not None:
+                    kind.sets.append((key[1], key))
             except Exception:                # something in the forward pass cannot be captured
                 torch.cuda.synchronize()
+                self._drop_scoring()
                 self._predict_off = True
-                self._predict_sets.clear()
                 return None
         p = sets.turn
         sets.turn ^= 1
@@ -1267,7 +1294,7 @@ class Model(nn.Module):
         rest = itertools.chain([first], it)
         leaves: List[torch.Tensor] = []
         spec = _flatten(first, leaves)
-        if _is_static(spec) or self._padded_plan(spec, leaves) is not None:
+        if _is_static(spec) or self._padded_lengths(spec, leaves) is not None:
             return rest
         return self._prefetched(rest)
 

@@ -86,3 +86,66 @@ def test_captured_scoring_equals_the_eager_scoring(tn_gpu, status_ok, form):
         want = torch.cat([m.predict_on_batch(f).cpu() for f, _ in data])
         assert p.shape == want.shape and torch.equal(y, torch.cat([l for _, l in data]))
         assert torch.allclose(p, want, atol=1e-5), float((p - want).abs().max())
+
+
+def _count(monkeypatch, tn, name):
+    made, orig = [], getattr(tn.model.Model, name)
+
+    def counted(self, *a, **kw):
+        made.append(1)
+        return orig(self, *a, **kw)
+
+    monkeypatch.setattr(tn.model.Model, name, counted)
+    return made
+
+
+def _model(tn, slots, B, cls=None):
+    torch.manual_seed(1)
+    m = (cls or tn.models.WideDeep)(slots, slots, dnn_hidden_units=(16,), embedding_dim=4, bucket_size=40 * B, table_rows=1 << 14, use_bn=False)
+    m.compile(optimizer=tn.optimizer.Optimizer(tn.core.Adam(learning_rate=2e-3)))
+    return m
+
+
+def test_the_number_of_captures_is_bounded(tn_gpu, status_ok, monkeypatch):
+    """Twelve batch sizes in turn, more than are captured: the rest runs eagerly, no capture makes way for another."""
+    tn = tn_gpu
+    slots = ["a", "b"]
+    data = [_batches(tn, slots, B, 4, "packed", seed=B)[k] for k in range(4) for B in range(20, 32)]
+    made = _count(monkeypatch, tn, "_capture")
+    m = _model(tn, slots, 32)
+    for _ in range(3):
+        m.fit(data)
+    assert 1 <= len(made) <= 8 and len(m._graphs) <= 8
+    made = _count(monkeypatch, tn, "_capture_predict")
+    for _ in range(3):
+        p = m.predict(data)[1]
+    want = torch.cat([m.predict_on_batch(f).cpu() for f, _ in data])
+    assert 1 <= len(made) <= 8 and torch.allclose(p, want, atol=1e-5)
+    for B in range(200, 300):                            # sizes that never come back leave nothing behind
+        f, y = _batches(tn, slots, B, 1, "packed", seed=B)[0]
+        m.train_on_batch(f, y)
+    assert len(m._padded_kinds) <= 80
+
+
+def test_lengths_of_a_heavy_tail(tn_gpu, status_ok, monkeypatch):
+    """Now and then one column many times its usual length: a handful of captures, and the steps of an eager run."""
+    tn = tn_gpu
+    slots, B = [f"s{k}" for k in range(12)], 16
+    g = torch.Generator().manual_seed(8)
+    data = []
+    for _ in range(60):
+        f = {}
+        for s in slots:
+            most = int(torch.empty(1).exponential_(1.0, generator=g).exp().clamp(1, 30))
+            lens = torch.randint(1, most + 1, (B,), generator=g)
+            offs = torch.cat([torch.zeros(1, dtype=torch.long), lens.cumsum(0)])
+            f[s] = tn.data.Ragged(torch.randint(0, 400, (int(offs[-1]),), generator=g), offs)
+        data.append((f, (torch.rand(B, generator=g) < 0.3).float()))
+    made = _count(monkeypatch, tn, "_capture")
+    m = _model(tn, slots, B)
+    got = m.fit(data, epochs=2, record_step_loss=True)["step_loss"]
+    assert 1 <= len(made) <= 3
+    e = _model(tn, slots, B)
+    e._use_graph = False
+    want = e.fit(data, epochs=2, record_step_loss=True)["step_loss"]
+    assert all(abs(a - b) < 5e-2 * max(1.0, abs(a)) for a, b in zip(want, got)), (want, got)
