@@ -149,3 +149,24 @@ def test_lengths_of_a_heavy_tail(tn_gpu, status_ok, monkeypatch):
     e._use_graph = False
     want = e.fit(data, epochs=2, record_step_loss=True)["step_loss"]
     assert all(abs(a - b) < 5e-2 * max(1.0, abs(a)) for a, b in zip(want, got)), (want, got)
+
+
+def test_lengths_within_a_fifth_of_one_another_share_a_capture(tn_gpu, status_ok, monkeypatch):
+    tn = tn_gpu
+    slots, B = ["a", "b"], 64
+    g = torch.Generator().manual_seed(9)
+    data = []
+    for k in range(40):
+        lens = torch.poisson(torch.full((2 * B,), 3.0 + 0.3 * (k % 2)), generator=g).long().clamp_(min=1)
+        offs = torch.cat([torch.zeros(1, dtype=torch.long), lens.cumsum(0)])
+        p = tn.data.PackedFeatures(slots, values=torch.randint(0, 400, (int(offs[-1]),), generator=g), offsets=offs.int(), batch_size=B)
+        data.append(({tn.data.PACKED_KEY: p}, (torch.rand(B, generator=g) < 0.3).float()))
+    made = _count(monkeypatch, tn, "_capture")
+    m = _model(tn, slots, B)
+    m.fit(data)
+    assert len(made) == 1
+    made = _count(monkeypatch, tn, "_capture_predict")
+    m.predict(data[:7])
+    assert not made                                      # a short pass does not pay for captures
+    m.predict(data)
+    assert len(made) == 1
