@@ -2,11 +2,35 @@
 from __future__ import annotations
 
 import gc
+import threading
 from contextlib import contextmanager
 
 import torch
 
 _STREAMS = {}
+
+
+class _CollectorOff:
+    """The garbage collector is off while any thread is inside, and then back as the first one found it."""
+
+    def __init__(self):
+        self.lock, self.inside, self.was_on = threading.Lock(), 0, False
+
+    def __enter__(self):
+        with self.lock:
+            if self.inside == 0:
+                self.was_on = gc.isenabled()
+                gc.disable()
+            self.inside += 1
+
+    def __exit__(self, *_):
+        with self.lock:
+            self.inside -= 1
+            if self.inside == 0 and self.was_on:
+                gc.enable()
+
+
+_collector_off = _CollectorOff()
 
 
 @contextmanager
@@ -26,15 +50,9 @@ def capture(graph: "torch.cuda.CUDAGraph", pool=None):
     if free < max(torch.cuda.memory_reserved(dev), total // 8):
         gc.collect()
         torch.cuda.empty_cache()
-    held = gc.isenabled()
-    gc.disable()
-    try:
-        with torch.cuda.stream(stream):
-            graph.capture_begin(*(() if pool is None else (pool,)))
-            try:
-                yield
-            finally:
-                graph.capture_end()
-    finally:
-        if held:
-            gc.enable()
+    with _collector_off, torch.cuda.stream(stream):
+        graph.capture_begin(*(() if pool is None else (pool,)))
+        try:
+            yield
+        finally:
+            graph.capture_end()

@@ -42,3 +42,21 @@ def test_cached_memory_goes_back_where_memory_is_short(device, free, reserved, g
     with C.capture(_Graph(device.log)):
         device.log.append("body")
     assert device.log == (["empty"] if gives_back else []) + ["begin", "body", "end"]
+
+
+def test_two_threads_leave_the_collector_as_they_found_it(device):
+    """The second capture begins inside the first and ends after it."""
+    import gc
+
+    assert gc.isenabled()
+    first, second = C.capture(_Graph(device.log)), C.capture(_Graph(device.log))
+    first.__enter__()
+    second.__enter__()
+    first.__exit__(None, None, None)
+    assert not gc.isenabled()              # the second one is still recording
+    second.__exit__(None, None, None)
+    assert gc.isenabled()
+    with pytest.raises(ValueError):
+        with C.capture(_Graph(device.log)):
+            raise ValueError
+    assert gc.isenabled() and device.log[-1] == "end"
