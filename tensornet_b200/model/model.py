@@ -17,6 +17,7 @@ from __future__ import annotations
 
 import json
 import os
+import warnings
 from typing import Any, Callable, Dict, Iterable, List, Optional, Sequence
 
 import torch
@@ -24,7 +25,7 @@ from torch import nn
 
 from .. import core, metric as _metric
 from .._opentelemetry import phase, start_as_current_span
-from ..data.features import PackedFeatures, PaddedPacked, PaddedRagged, Ragged
+from ..data.features import NeedsExactLengths, PackedFeatures, PaddedPacked, PaddedRagged, Ragged
 from ..ops import functional as F
 from ..parallel.symm import verify_all_arenas
 from ..utils.capture import capture
@@ -316,18 +317,26 @@ def _same_state(a: list, b: list) -> bool:
 
 _PADDED_SETS = 3     # captured steps per kind of ragged batch: short, usual and long ones
 _KINDS = 64          # kinds of batches whose history is kept
+_OOM_HOLD = 1000     # batches of a kind that run eagerly after its capture ran out of memory, before the next attempt
 
 
 class _Kind:
     """The batches of one structure and fixed shapes, as far as captured steps go."""
 
-    __slots__ = ("sets", "sights", "most", "differ")
+    __slots__ = ("sets", "sights", "most", "differ", "hold")
 
     def __init__(self):
         self.sets: List[Any] = []        # ragged batches: (rooms, key of the captured step), one per capture
         self.sights = 0                  # batches that found no captured step
         self.most: List[int] = []        # most ids such a batch had, per ragged leaf
         self.differ = False              # their lengths were not all the same
+        self.hold = 0                    # batches that run eagerly before a capture is tried (again)
+
+    def held_off(self) -> bool:
+        if self.hold > 0:
+            self.hold -= 1
+            return True
+        return False
 
     def note(self, n: List[int]):
         self.sights += 1
@@ -714,11 +723,13 @@ class Model(nn.Module):
         at = set(ragged)
         base = (spec, tuple((None if i in at else t.shape, t.dtype) for i, t in enumerate(leaves)))
         kind = _Kind.of(kinds, base)
+        if not kind.sets and kind.held_off():
+            return kind, None, None
         fits = sorted((sum(rooms), rooms, k) for k, (rooms, _) in enumerate(kind.sets) if all(a <= r for a, r in zip(n, rooms)))
         # a much too large capture is the second choice: its kernels are launched for the room, not for the ids
         if fits and (fits[0][0] <= 2 * sum(n) + 4096 or full or len(kind.sets) >= _PADDED_SETS):
             rooms, key = kind.sets[fits[0][2]]
-        elif full or len(kind.sets) >= _PADDED_SETS:
+        elif full or len(kind.sets) >= _PADDED_SETS or kind.held_off():
             return kind, None, None
         else:
             rooms = kind.rooms(n, not fits)
@@ -727,6 +738,28 @@ class Model(nn.Module):
                 return kind, key, dict(zip(ragged, rooms))
             kind.note(n)
         return kind, key, dict(zip(ragged, rooms))
+
+    @staticmethod
+    def _tried(kind, what: str, record: Callable) -> bool:
+        """Capture a step that can also run uncaptured.  When that fails, ``kind`` is held off captures for a while where
+        memory ran out, and for good otherwise; an error of the step itself then shows in the uncaptured one.  (A step
+        that wants exact lengths is an ordinary case, anything else worth a warning: eager steps take several times as long.)"""
+        why = None
+        try:
+            record()
+            return True
+        except NeedsExactLengths:
+            kind.hold = float("inf")
+        except torch.OutOfMemoryError as e:
+            kind.hold, why = _OOM_HOLD, str(e)
+        except Exception as e:
+            kind.hold, why = float("inf"), f"{type(e).__name__}: {e}"
+        torch.cuda.synchronize()
+        if kind.hold == _OOM_HOLD:
+            torch.cuda.empty_cache()     # what the attempt held went with the frames of its traceback
+        if why is not None:
+            warnings.warn(f"{what} step could not be captured and runs without: {why}", RuntimeWarning, stacklevel=3)
+        return False
 
     def _eager_step(self, features, labels):
         self._last_done = None
@@ -772,13 +805,10 @@ class Model(nn.Module):
             if static:
                 self._capture(spec, leaves, key)
             elif rooms is not None:
-                try:
-                    self._capture(spec, leaves, key, rooms)
-                    kind.sets.append((key[1], key))
-                except Exception:           # something in the step wants exact lengths (or cannot be captured): no padding any more
-                    torch.cuda.synchronize()
-                    self._padded_off = True
+                if not self._tried(kind, "training", lambda: self._capture(spec, leaves, key, rooms)):
+                    self._padded_off = kind.hold == float("inf")
                     return self._eager_step(features, labels)
+                kind.sets.append((key[1], key))
             else:
                 try:
                     self._capture(spec, leaves, key)
@@ -1107,22 +1137,22 @@ class Model(nn.Module):
                 return None
             if rooms is None:
                 kind.sights += 1
-            if full or kind.sights <= _PREDICT_SIGHTS:
+            if full or kind.sights <= _PREDICT_SIGHTS or (rooms is None and kind.held_off()):
                 return None
             with torch.no_grad():            # shape and type of the result, from the batch itself
                 (f,), _, _ = self._to_device((features,))
                 like = torch.sigmoid(self(f))
             self._predict_shape, self._predict_dtype = like.shape, like.dtype
-            try:
-                sets = self._predict_sets[key] = self._capture_predict(spec, leaves, rooms)
-                self._predict_state, check = state, False
-                if rooms is not None:
-                    kind.sets.append((key[1], key))
-            except Exception:                # something in the forward pass cannot be captured
-                torch.cuda.synchronize()
-                self._drop_scoring()
-                self._predict_off = True
+
+            def record():
+                self._predict_sets[key] = self._capture_predict(spec, leaves, rooms)
+
+            if not self._tried(kind, "scoring", record):
+                self._predict_off = kind.hold == float("inf")
                 return None
+            sets, self._predict_state, check = self._predict_sets[key], state, False
+            if rooms is not None:
+                kind.sets.append((key[1], key))
         p = sets.turn
         sets.turn ^= 1
         main = torch.cuda.current_stream()

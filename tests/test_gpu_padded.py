@@ -170,3 +170,39 @@ def test_lengths_within_a_fifth_of_one_another_share_a_capture(tn_gpu, status_ok
     assert not made                                      # a short pass does not pay for captures
     m.predict(data)
     assert len(made) == 1
+
+
+@pytest.mark.parametrize("name", ["_capture", "_capture_predict"])
+def test_a_capture_that_fails_says_so(tn_gpu, status_ok, monkeypatch, name):
+    """Out of memory: eager for a while, then tried again.  Anything else: no padding and no captured scoring for good
+    (training goes on at exact lengths), with the reason."""
+    import warnings
+
+    tn = tn_gpu
+    slots, B = ["a", "b"], 32
+    data = _batches(tn, slots, B, 24, "packed")
+    orig = getattr(tn.model.Model, name)
+    step = (lambda m: m.fit(data)) if name == "_capture" else (lambda m: m.predict(data))
+    captured = (lambda m: m._graphs) if name == "_capture" else (lambda m: m._predict_sets)
+    for error, again in ((torch.OutOfMemoryError("no memory for it"), True), (ValueError("no such thing"), False)):
+        tries = []
+
+        def fails_once(self, *a, **kw):
+            tries.append(1)
+            if len(tries) == 1:
+                raise error
+            return orig(self, *a, **kw)
+
+        monkeypatch.setattr(tn.model.Model, name, fails_once)
+        monkeypatch.setattr(tn.model.model, "_OOM_HOLD", 30, raising=False)
+        m = _model(tn, slots, B)
+        with warnings.catch_warnings(record=True) as said:
+            warnings.simplefilter("always")
+            step(m)
+            assert any(str(error) in str(w.message) for w in said)
+            assert (m._padded_off or m._predict_off) != again
+            if again:
+                assert len(tries) == 1 and not captured(m)
+                for _ in range(3):
+                    step(m)
+                assert len(tries) == 2 and captured(m)
