@@ -52,19 +52,23 @@ class NeedsExactLengths(RuntimeError):
     """Code other than the embedding layers looked into a padded feature of a captured step."""
 
 
-class PaddedRagged:
+class PaddedRagged(Ragged):
     """The stand-in for a :class:`Ragged` column inside a captured step: ``values`` has room for more ids than the
-    batch holds, the last offset says how many are there.  Only :func:`gather_columns` reads it; anything that asks
-    for ``values`` / ``offsets`` expects exact lengths and is told so (the model then runs such batches uncaptured)."""
+    batch holds, the last offset says how many are there.  Only :func:`gather_columns` reads it.  It is a ``Ragged`` to
+    code that looks at the type, and tells whatever asks for ``values`` / ``offsets`` that exact lengths are not to be
+    had (the model then runs such batches uncaptured)."""
 
-    def __init__(self, values: torch.Tensor, offsets: torch.Tensor):
+    def __new__(cls, values: torch.Tensor, offsets: torch.Tensor):
+        self = super().__new__(cls, None, None)
         self._values, self._offsets = values, offsets
+        return self
 
-    def _refuse(self, *_):
+    def _refuse(self, *_, **__):
         raise NeedsExactLengths("padded feature")
 
     values = offsets = property(_refuse)
-    __getitem__ = __iter__ = __len__ = _refuse
+    __getitem__ = __iter__ = __len__ = __eq__ = __ne__ = __hash__ = __contains__ = _refuse
+    _replace = _asdict = index = count = _refuse
 
 
 class PaddedPacked(PackedFeatures):

@@ -51,3 +51,23 @@ def test_loss_helpers_shape_labels_weights_and_masks():
     assert torch.equal(tn.model.apply_mask(y_p, sw, mask), torch.tensor([[1.0], [0.0], [3.0], [4.0]]))
     assert torch.equal(tn.model.apply_mask(y_p, None, mask), mask.float())
     assert tn.model.apply_mask(y_p, sw, None) is sw
+
+
+def test_padded_column_of_a_captured_step_is_a_ragged_one():
+    """Code that looks at the type takes its ragged branch, and there learns that exact lengths are not to be had."""
+    import pytest
+    import torch
+
+    from tensornet_b200.data.features import NeedsExactLengths, PaddedRagged, Ragged, batch_size_of, padded_columns
+
+    f = PaddedRagged(torch.zeros(64, dtype=torch.long), torch.tensor([0, 2, 3]))
+    assert isinstance(f, Ragged) and isinstance(f, tuple)
+    assert batch_size_of(f) == 2 and padded_columns({"a": f}, ["a"])
+    for look in (lambda: f.values, lambda: f.offsets, lambda: f[0], lambda: list(f), lambda: len(f), lambda: f._replace(values=0),
+                 lambda: [v for v in f], lambda: f == f):
+        with pytest.raises(NeedsExactLengths):
+            look()
+    with pytest.raises(NeedsExactLengths):
+        v, o = f
+    with pytest.raises(NeedsExactLengths):
+        (lambda a, b: None)(*f)
