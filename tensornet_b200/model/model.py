@@ -432,6 +432,7 @@ class Model(nn.Module):
         self._last_set = None                        # (captured sets, index) of the last replayed step
         self._padded_kinds: Dict[Any, _Kind] = {}    # ragged batches, by structure and fixed shapes
         self._padded_off = False                     # a captured step needed exact lengths
+        self._uncaptured = 0                         # ragged batches in a row, after the warm-up, that fitted no captured step
         self._predict_sets: Dict[Any, _PredictSets] = {}    # batch signature -> the two captures of the scoring step
         self._predict_kinds: Dict[Any, _Kind] = {}
         self._predict_off = False                    # the scoring step cannot be captured
@@ -520,7 +521,7 @@ class Model(nn.Module):
         self._ring_refused = self._padded_off = self._predict_off = False
         self._graph = self._graph_key = self._flat_cache = self._last_done = self._last_set = self._static_loss = None
         self._static_leaves = []
-        self._max_graphs, self._eager_steps = 8, 0
+        self._max_graphs, self._eager_steps, self._uncaptured = 8, 0, 0
         self._drop_scoring()
 
     def _drop_scoring(self):
@@ -795,6 +796,8 @@ class Model(nn.Module):
                 kind, key, rooms = plan
         what = "eager" if key is None else graph_decision(rt.world, key in self._graphs, static, held, self._max_graphs,
                                                           self._eager_steps, self._graph_warmup)
+        if kind is not None and not kind.hold:       # (a kind held off captures is not to be captured at its exact lengths either)
+            self._uncaptured = self._uncaptured + 1 if key is None else 0
         if what == "eager":
             self._eager_steps += 1
             loss = self._eager_step(features, labels)
@@ -1345,9 +1348,19 @@ class Model(nn.Module):
         rest = itertools.chain([first], it)
         leaves: List[torch.Tensor] = []
         spec = _flatten(first, leaves)
-        if _is_static(spec) or self._padded_lengths(spec, leaves) is not None:
+        if _is_static(spec):
             return rest
+        if self._padded_lengths(spec, leaves) is not None:
+            return self._while_captured(rest)
         return self._prefetched(rest)
+
+    def _while_captured(self, batches):
+        """Ragged batches as they are while captured steps take them, staged one batch ahead from then on."""
+        for batch in batches:
+            yield batch
+            if self._padded_off or self._uncaptured >= 8:
+                break
+        yield from self._prefetched(batches)
 
     def fit(self, dataset: Iterable, epochs: int = 1, steps_per_epoch: Optional[int] = None, callbacks: Sequence = (),
             verbose: int = 0, log_every: int = 100, prefetch: bool = True, record_step_loss: bool = False):

@@ -206,3 +206,27 @@ def test_a_capture_that_fails_says_so(tn_gpu, status_ok, monkeypatch, name):
                 for _ in range(3):
                     step(m)
                 assert len(tries) == 2 and captured(m)
+
+
+@pytest.mark.parametrize("why", ["exact lengths", "too many kinds"])
+def test_batches_that_run_uncaptured_are_staged_ahead(tn_gpu, status_ok, monkeypatch, why):
+    """``fit`` hands them over on the device, copied beside the step before."""
+    tn = tn_gpu
+    slots = ["a", "b"]
+
+    class Mean(tn.models.WideDeep):
+        def forward(self, features):
+            return super().forward(features) + features["a"].values.numel() * 0.0
+
+    sizes = [16] * 40 if why == "exact lengths" else list(range(16, 56))
+    data = [_batches(tn, slots, B, 1, "columns", seed=k)[0] for k, B in enumerate(sizes)]
+    m = _model(tn, slots, 56, Mean if why == "exact lengths" else None)
+    step, on_gpu = tn.model.Model.train_step, []
+
+    def seen(self, batch, next_batch=None):
+        on_gpu.append(batch[0]["a"].values.is_cuda)
+        return step(self, batch, next_batch)
+
+    monkeypatch.setattr(tn.model.Model, "train_step", seen)
+    assert all(l == l for l in m.fit(data, record_step_loss=True)["step_loss"])
+    assert len(on_gpu) == 40 and not on_gpu[0] and all(on_gpu[-15:])
