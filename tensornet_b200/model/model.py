@@ -633,14 +633,12 @@ class Model(nn.Module):
             for m in self._host_metrics:
                 m.update_state(labels, pred)
         rt = core.runtime()
-        out = self._loss_out
-        if out is not None and loss.dtype == out.dtype and loss.numel() == 1:
-            # A captured step hands its loss over in memory of its own: the captures share one memory pool, in which the
-            # replay of the other capture writes its intermediates over this one's results.
+        out = self._own_loss(loss)
+        if out is not None:
             main, side = torch.cuda.current_stream(), F._side_stream(rt.device)
             side.wait_stream(main)
             with torch.cuda.stream(side):
-                out.copy_(loss.detach().reshape(()))
+                out.copy_(loss.detach())
             object.__setattr__(self, "_loss_stream", side)
         for layer, _ in self._fronts_now:          # forward pass issued: the next batch's pull fronts start here
             layer.link.fork_front()
@@ -690,7 +688,14 @@ class Model(nn.Module):
                     if rider is not None:
                         rider.dense_rider = None
                     self.optimizer.step(peers_past_backward=rt.peer_synced_pushes > before)
-        return loss.detach() if self._loss_stream is None else out.view(loss.shape)
+        return loss.detach() if out is None else out
+
+    def _own_loss(self, loss):
+        """Where a step that is being captured is to leave its loss: the captures share one memory pool, in which the
+        replay of the other capture writes its intermediates over this one's results.  None for an eager step."""
+        if self._loss_out is None:
+            return None
+        return self._loss_out[: loss.numel() * loss.element_size()].view(loss.dtype).view(loss.shape)
 
     def _to_device(self, obj):
         dev = core.runtime().device
@@ -989,7 +994,7 @@ class Model(nn.Module):
             g = torch.cuda.CUDAGraph()
             c0 = ext.launch_count()
             f, y = feats[i]
-            self._loss_out = torch.empty((), dtype=torch.float32, device=dev)
+            self._loss_out = torch.empty(8, dtype=torch.uint8, device=dev)      # a scalar of any type
             try:
                 with capture(g, pool):
                     static_loss = self._step_impl(f, y, next_features=feats[(i + 1) % ring.SETS][0])
@@ -1042,7 +1047,7 @@ class Model(nn.Module):
             torch.cuda.synchronize()
             g = torch.cuda.CUDAGraph()
             c0 = ext.launch_count()
-            self._loss_out = torch.empty((), dtype=torch.float32, device=dev)
+            self._loss_out = torch.empty(8, dtype=torch.uint8, device=dev)      # a scalar of any type
             try:
                 with capture(g, pool):
                     static_loss = self._step_impl(f, y)
@@ -1653,4 +1658,6 @@ class PCGradModel(Model):
             torch.stack(losses).sum().backward()
             self.optimizer.step()
         self.backwards()
-        return torch.stack(losses).sum().detach()
+        total = torch.stack(losses).sum().detach()
+        out = self._own_loss(total)
+        return total if out is None else out.copy_(total)

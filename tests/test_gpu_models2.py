@@ -148,3 +148,45 @@ def test_sharded_serving_matches_single_dictionary(tn_gpu, status_ok):
         assert torch.allclose(a, b, atol=2e-3), float((a - b).abs().max())
     assert eng.table.n_rows == n0                      # nothing was inserted
     assert B in eng._graphs
+
+
+def _two_task(tn, slots, B):
+    class TwoTask(tn.model.PCGradModel):
+        def __init__(self):
+            super().__init__()
+            cols = [tn.feature_column.embedding_column(tn.feature_column.category_column(key=s, bucket_size=4 * B), 8, "sum") for s in slots]
+            self.emb = tn.layers.EmbeddingFeatures(cols, tn.core.AdaGrad(learning_rate=0.05), name="emb", is_concat=True, rows=1 << 12)
+            self.body = torch.nn.Sequential(torch.nn.Linear(16, 32), torch.nn.ReLU(), torch.nn.Linear(32, 2))
+
+        def forward(self, features):
+            return self.body(self.emb(features))
+
+    return TwoTask
+
+
+@pytest.mark.parametrize("kind", ["two tasks", "fp64 loss"])
+def test_losses_of_captured_steps_stay_what_they_were(tn_gpu, kind):
+    """The losses of two steps in a row, read after both have run: the captures take turns in one memory pool, so a loss
+    in that pool could be written over by the step after it."""
+    tn = tn_gpu
+    slots, B = ["a", "b"], 64
+
+    g = torch.Generator().manual_seed(3)
+    data = [({tn.data.PACKED_KEY: tn.data.PackedFeatures(slots, ids=torch.randint(0, 200, (2, B), generator=g))},
+             (torch.rand(B, 2, generator=g) < 0.4).float()) for _ in range(24)]
+    runs = []
+    for graph in (False, True):
+        torch.manual_seed(6)
+        if kind == "two tasks":
+            m, loss = _two_task(tn, slots, B)(), "binary_crossentropy"
+        else:
+            m = tn.models.DeepFM(slots, slots, dnn_hidden_units=(32, 16), embedding_dim=8, bucket_size=4 * B, table_rows=1 << 12)
+            loss = lambda logits, y: torch.nn.functional.binary_cross_entropy_with_logits(logits.double(), y[:, :1].double())
+        m.compile(optimizer=tn.optimizer.Optimizer(tn.core.Adam(learning_rate=1e-2)), loss=loss, cuda_graph=graph)
+        got = []
+        for k in range(0, 24, 2):
+            pair = [m.train_on_batch(f, y) for f, y in data[k: k + 2]]
+            got += [float(l) for l in pair]
+        runs.append(got)
+        assert bool(m._graphs) == graph
+    assert all(abs(a - b) < 1e-3 * abs(a) for a, b in zip(*runs)), runs
