@@ -476,7 +476,8 @@ class Model(nn.Module):
         self._steps_seen = self._loss_steps = 0
         self._unit_grad = torch.ones((), dtype=torch.float32, device=rt.device)
         # metrics that read every step's predictions on the host cannot run inside a captured step
-        self._use_graph = rt.on_gpu and (core.config.cuda_graph if cuda_graph is None else cuda_graph) and not self._host_metrics
+        self._use_graph = (rt.on_gpu and (core.config.cuda_graph if cuda_graph is None else cuda_graph) and not self._host_metrics and
+                           getattr(optimizer, "capturable", True))
         self._graph_warmup = graph_warmup
         if rt.on_gpu:
             tables = {id(l.table): l.table for l in self.sparse_layers() if hasattr(l, "table")}

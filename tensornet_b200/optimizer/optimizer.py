@@ -66,6 +66,8 @@ class PCGrad(Optimizer):
     plane of each other task gradient it conflicts with (negative inner product), in random
     order, and the projected gradients are summed."""
 
+    capturable = False      # the order is drawn and the inner products are looked at on the host, every step anew
+
     def project(self, task_grads: Sequence[torch.Tensor]) -> torch.Tensor:
         """``task_grads``: one flat gradient per task over the same parameters."""
         out = []

@@ -190,3 +190,16 @@ def test_losses_of_captured_steps_stay_what_they_were(tn_gpu, kind):
         runs.append(got)
         assert bool(m._graphs) == graph
     assert all(abs(a - b) < 1e-3 * abs(a) for a, b in zip(*runs)), runs
+
+
+def test_gradient_surgery_runs_past_the_warm_up_steps(tn_gpu):
+    tn = tn_gpu
+    slots, B = ["a", "b"], 64
+    g = torch.Generator().manual_seed(3)
+    f = {tn.data.PACKED_KEY: tn.data.PackedFeatures(slots, ids=torch.randint(0, 200, (2, B), generator=g))}
+    y = (torch.rand(B, 2, generator=g) < 0.4).float()
+    torch.manual_seed(6)
+    m = _two_task(tn, slots, B)()
+    m.compile(optimizer=tn.optimizer.PCGrad(tn.core.Adam(learning_rate=1e-2)))
+    losses = [float(m.train_on_batch(f, y)) for _ in range(12)]
+    assert losses[-1] < losses[0]
