@@ -203,3 +203,38 @@ def test_gradient_surgery_runs_past_the_warm_up_steps(tn_gpu):
     m.compile(optimizer=tn.optimizer.PCGrad(tn.core.Adam(learning_rate=1e-2)))
     losses = [float(m.train_on_batch(f, y)) for _ in range(12)]
     assert losses[-1] < losses[0]
+
+
+@pytest.mark.parametrize("layers", [1, 8, 9, 11])
+def test_cross_v2_gradients_of_many_layers(tn_gpu, status_ok, layers):
+    """Up to eight layers their Hadamard terms are summed in one pass, beyond that layer by layer into an fp32 array.
+    Against autograd of the same network in fp64 on the bf16 values the kernels get: every layer rounds its output and its
+    gradient to bf16 (2^-9 each, relative), so the error grows with the layers, as 2^-8 of the result each at most."""
+    from tensornet_b200.ops import functional as F
+
+    torch.manual_seed(layers)
+    B, dim = 33, 30
+    ld = F.pad8(dim + 1)
+    x = torch.zeros(B, ld, device="cuda")
+    x[:, :dim] = torch.randn(B, dim, device="cuda") * 0.5
+    x[:, dim] = 1.0
+    xb = x.to(torch.bfloat16).requires_grad_(True)
+    ws = [torch.zeros(dim, ld, device="cuda") for _ in range(layers)]
+    for w in ws:
+        w[:, : dim + 1] = (torch.randn(dim, dim + 1, device="cuda") * 0.05).to(torch.bfloat16).float()
+        w.requires_grad_(True)
+    gy = torch.zeros(B, ld, device="cuda", dtype=torch.bfloat16)
+    gy[:, :dim] = torch.randn(B, dim, device="cuda").to(torch.bfloat16)
+    F.cross_v2(xb, ws, dim).backward(gy)
+    x0 = xb.detach().double()[:, : dim + 1].clone().requires_grad_(True)
+    wd = [w.detach().double()[:, : dim + 1].clone().requires_grad_(True) for w in ws]
+    xl = x0[:, :dim]
+    one = torch.ones(B, 1, device="cuda", dtype=torch.float64)
+    for w in wd:
+        xl = x0[:, :dim] * (torch.cat([xl, one], dim=1) @ w.t()) + xl
+    xl.backward(gy.double()[:, :dim])
+    err = lambda a, b: float((a.double() - b).norm() / b.norm())
+    bound = 2.0 ** -8 * (layers + 1)
+    assert err(xb.grad[:, :dim], x0.grad[:, :dim]) < bound
+    for w, d in zip(ws, wd):
+        assert err(w.grad[:, : dim + 1], d.grad) < bound
