@@ -109,7 +109,7 @@ class EmbeddingFeatures(nn.Module):
         S = len(self._keys)
         labels, label_mod = None, 0
         if self._target_columns:
-            y = features[self._target_columns[0]].to(dev, non_blocking=True).reshape(-1).float()
+            y = features[self._target_columns[0]].to(dev, non_blocking=True).reshape(-1).float().contiguous()
             if offsets is None:
                 labels, label_mod = y, B
             elif ids.is_cuda:

@@ -438,3 +438,31 @@ def test_pooling_with_several_rows_in_flight(tn_gpu, status_ok, B, S, dim, ragge
     wantg = torch.zeros((rows, dim), dtype=torch.float64, device=dev).index_add_(0, inverse[ok].long(), go[bag[ok]])
     size = torch.zeros((rows, dim), dtype=torch.float64, device=dev).index_add_(0, inverse[ok].long(), go[bag[ok]].abs())
     assert bool(((gU.double() - wantg).abs() <= 64 * 2.0 ** -24 * size + 1e-12).all())
+
+
+@pytest.mark.parametrize("ragged", [False, True])
+def test_labels_of_the_click_counts_may_be_a_column(tn_gpu, status_ok, ragged):
+    """Labels that are a strided view on the device: the same counts as from a contiguous tensor."""
+    tn = tn_gpu
+    dev = tn.core.runtime().device
+    slots, B, dim = ["a", "b"], 40, 4
+    g = torch.Generator().manual_seed(4)
+    lens = torch.randint(1, 4, (2 * B,), generator=g) if ragged else torch.ones(2 * B, dtype=torch.long)
+    offs = torch.cat([torch.zeros(1, dtype=torch.long), lens.cumsum(0)]).int()
+    ids = torch.randint(1, 30, (int(offs[-1]),), generator=g)
+    both = torch.rand((B, 2), generator=g).round().to(dev)
+    rows = []
+    for y in (both[:, 1], both[:, 1].clone()):
+        cols = [tn.feature_column.embedding_column(tn.feature_column.category_column(key=s, bucket_size=4 * B), dim, "sum") for s in slots]
+        layer = tn.layers.EmbeddingFeatures(cols, tn.core.AdaGrad(learning_rate=0.01, initial_scale=0.1), name="e", is_concat=True,
+                                            target_columns=["label"], rows=1 << 10)
+        p = (tn.data.PackedFeatures(slots, values=ids.to(dev), offsets=offs.to(dev), batch_size=B) if ragged else
+             tn.data.PackedFeatures(slots, ids=ids.view(2, B).to(dev)))
+        out = layer({tn.data.PACKED_KEY: p, "label": y}, training=True)
+        out.backward(torch.ones_like(out))
+        layer.backwards()
+        at = layer.table.lookup_rows(torch.unique(ids).to(dev)).long()
+        rows.append(layer.table.rows[at][:, dim + 1: dim + 3].cpu())          # show, click
+    want = torch.zeros(30)
+    want.index_add_(0, ids, torch.repeat_interleave(both[:, 1].cpu().repeat(2), lens))
+    assert torch.equal(rows[1][:, 1], want[torch.unique(ids)]) and torch.equal(rows[0], rows[1])
