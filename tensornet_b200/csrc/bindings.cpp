@@ -380,8 +380,9 @@ struct ServeCtx {
   }
 
   // `weights`: fp32 [N, pad8(K + 1)] per layer; `shadows`: their bf16 copies when something keeps them current, else empty.
-  at::Tensor forward(at::Tensor ids, c10::optional<at::Tensor> offsets, int B, const std::vector<at::Tensor>& weights,
-                     const std::vector<at::Tensor>& shadows, at::Tensor head_w, at::Tensor status) {
+  // Nothing comes back when they do not start on 16 bytes, which the kernels' loads ask for.
+  c10::optional<at::Tensor> forward(at::Tensor ids, c10::optional<at::Tensor> offsets, int B, const std::vector<at::Tensor>& weights,
+                                    const std::vector<at::Tensor>& shadows, at::Tensor head_w, at::Tensor status) {
     const int L = (int)dims.size() - 1;
     const bool cast_needed = shadows.empty();
     TORCH_CHECK((int)weights.size() == L && (cast_needed || (int)shadows.size() == L) && head_w.numel() == dims[L] + 1 && head_w.is_cuda() &&
@@ -389,6 +390,8 @@ struct ServeCtx {
     TORCH_CHECK(ids.scalar_type() == at::kLong && ids.is_contiguous() && B >= 1, "serving: contiguous int64 ids");
     TORCH_CHECK(offsets.has_value() ? offsets->numel() == (int64_t)S * B + 1 && offsets->is_contiguous() && offsets->scalar_type() == at::kInt
                                     : ids.numel() == (int64_t)S * B, "serving: one bag per slot and example");
+    for (const at::Tensor& w : cast_needed ? weights : shadows)
+      if (reinterpret_cast<uintptr_t>(w.data_ptr()) & 15) return c10::nullopt;
     c10::cuda::CUDAGuard guard(head_w.device());
     const cudaStream_t st = at::cuda::getCurrentCUDAStream().stream();
     const auto dev = head_w.device();
@@ -425,7 +428,7 @@ struct ServeCtx {
     for (int l = 0; l < L; ++l) {
       const at::Tensor& w = cast_needed ? weights[l] : shadows[l];
       TORCH_CHECK(w.is_cuda() && w.dim() == 2 && w.is_contiguous() && w.size(0) == dims[l + 1] && w.size(1) == pad8(dims[l] + 1) &&
-                      w.scalar_type() == (cast_needed ? at::kFloat : at::kBFloat16) && (reinterpret_cast<uintptr_t>(w.data_ptr()) & 15) == 0,
+                      w.scalar_type() == (cast_needed ? at::kFloat : at::kBFloat16),
                   "serving: layer ", l, " weights");
     }
     if (copy_ids || copy_off) {

@@ -99,13 +99,30 @@ class InferenceEngine:
         self.combiner = {"sum": 0, "mean": 1, "sqrtn": 2}[combiner]
         self._graphs = {}
         assert mlp.in_dim == n_slots * dictionary.dim, "tower input width must equal slots * dim"
-        self._ctx = None
-        if dictionary.on_gpu and type(mlp) is MLP and type(head) is DenseHead and len(mlp.hidden_units) <= 8:
-            self._ctx = _build.cuda_ext().ServeCtx(dictionary.table_dict(), n_slots, self.combiner,
-                                                   [mlp.in_dim, *mlp.hidden_units], bool(mlp.relu_last))
+        self._ctx, self._ctx_of = None, ()
+        if dictionary.on_gpu:
+            self._context()
+
+    def _context(self):
+        """The native chain for what the engine is made of now (a dictionary or a tower may be put in another's place
+        between requests), or None when that takes Python to run: modules of another kind, or with hooks."""
+        d, mlp, head = self.dict, self.mlp, self.head
+        if type(mlp) is not MLP or type(head) is not DenseHead or len(mlp.hidden_units) > 8 or d.dim % 4:
+            return None
+        if (mlp._forward_hooks or mlp._forward_pre_hooks or head._forward_hooks or head._forward_pre_hooks or
+                "forward" in mlp.__dict__ or "forward" in head.__dict__):
+            return None
+        of = (id(d.keys), id(d.slots), id(d.rows), id(mlp), self.S, self.combiner, mlp.relu_last)
+        if of != self._ctx_of:
+            self._ctx = _build.cuda_ext().ServeCtx(d.table_dict(), self.S, self.combiner, [mlp.in_dim, *mlp.hidden_units], bool(mlp.relu_last))
+            self._ctx_of, self._ctx_mlp = of, mlp           # the chain holds the arrays: an id stands for one object
+        return self._ctx
 
     def _native(self, ids, offsets, B: int):
         """The request through the native chain, or None when something about it is out of the ordinary."""
+        ctx = self._context()
+        if ctx is None:
+            return None
         ws = list(self.mlp.weights._parameters.values())
         hw = self.head.weight
         if self.mlp.weight_gate is not None or not all(w.is_cuda and w.dtype == torch.float32 and w.is_contiguous() for w in (*ws, hw)):
@@ -117,7 +134,7 @@ class InferenceEngine:
         shadows = [getattr(w, "_tn_bf16", None) for w in ws]
         if any(s is None for s in shadows):
             shadows = []
-        return self._ctx.forward(ids, offsets, B, ws, shadows, hw, runtime().status)
+        return ctx.forward(ids, offsets, B, ws, shadows, hw, runtime().status)
 
     def _forward_gpu(self, ids, offsets, B):
         ext = _build.cuda_ext()
@@ -148,11 +165,10 @@ class InferenceEngine:
             x = pooled.permute(1, 0, 2).reshape(B, -1)
             return torch.sigmoid(self.head(self.mlp(F.concat_cast([x], ones=True)))).view(-1)
         dev = rt.device
-        if self._ctx is not None:
-            n = int(ids.shape[1]) if offsets is None else (offsets.numel() - 1) // self.S
-            prob = self._native(ids, offsets, n) if n > 0 else None
-            if prob is not None:
-                return prob
+        n = int(ids.shape[1]) if offsets is None else (offsets.numel() - 1) // self.S
+        prob = self._native(ids, offsets, n) if n > 0 else None
+        if prob is not None:
+            return prob
         if offsets is not None or not use_graph:
             B = ids.shape[1] if offsets is None else (offsets.numel() - 1) // self.S
             return self._forward_gpu(ids.to(dev).reshape(-1), None if offsets is None else offsets.to(dev).int(), B)

@@ -51,3 +51,50 @@ def test_weights_written_between_requests_are_seen(tn_gpu, status_ok):
         a = eng.infer(ids).clone()
         mlp.weights[0].data.mul_(-1.0)
         assert not torch.equal(a, eng.infer(ids))
+
+
+def test_requests_follow_what_the_engine_is_made_of(tn_gpu, status_ok):
+    """Another dictionary, another tower, an attribute of it, a hook on it: between two requests, ragged and not."""
+    from tensornet_b200.layers import DenseHead, MLP
+    from tensornet_b200.serving import EmbeddingDictionary, InferenceEngine
+
+    dev = tn_gpu.core.runtime().device
+    torch.manual_seed(1)
+    make = lambda: (MLP(8, [16, 8]).to(dev), DenseHead(8).to(dev))
+    signs = np.arange(1, 9, dtype=np.uint64)
+    rows = lambda seed: np.random.default_rng(seed).standard_normal((8, 4)).astype(np.float32)
+    mlp, head = make()
+    eng = InferenceEngine(EmbeddingDictionary(signs, rows(0)), mlp, head, 2)
+    ids = torch.randint(1, 9, (2, 40))
+    offs = torch.arange(81, dtype=torch.int32)
+
+    def follows():
+        with torch.no_grad():
+            want = eng._forward_gpu(ids.to(dev).reshape(-1), offs.to(dev), 40)
+        for got in (eng.infer(ids), eng.infer(ids.reshape(-1), offs)):
+            assert torch.allclose(got, want, atol=2 ** -10), float((got - want).abs().max())      # bound: see above
+        return want
+
+    seen = [follows()]
+
+    def changed():
+        seen.append(follows())
+        assert not torch.allclose(seen[-1], seen[-2], atol=2 ** -8)
+
+    eng.dict = EmbeddingDictionary(signs, rows(1))
+    changed()
+    eng.mlp, eng.head = make()
+    changed()
+    eng.mlp.relu_last = False
+    changed()
+    flat = torch.zeros(16 * 16 + 1, device=dev)[1:].view(16, 16)          # weights off the 16-byte boundary
+    flat.copy_(eng.mlp.weights[0].detach())
+    eng.mlp.weights[0].data = flat
+    follows()
+    calls = []
+    handle = eng.mlp.register_forward_hook(lambda *_: calls.append(1))
+    for k in range(3):
+        eng.infer(ids.reshape(-1), offs)
+    assert len(calls) == 3
+    handle.remove()
+    follows()
