@@ -273,46 +273,61 @@ def _own_code(fn) -> bool:
     return (getattr(fn, "__module__", None) or "").startswith(_OWN_CODE)
 
 
-_PLAIN = (int, float, bool, str)
 # what training and compile change on the modules of a model without any bearing on its predictions
 _NOT_SCORED = {"stop_training", "is_loaded_from_checkpoint", "metrics", "optimizer", "loss_fn", "batch_counter"}
+_PLAIN = {int, float, bool, str}
 
 
-def _scoring_state(model) -> Optional[list]:
-    """What a captured scoring step of ``model`` is made from: its modules, the storage of their parameters and buffers,
-    and the public attributes their forward passes go by.  None when a replay cannot stand for scoring a batch: that
-    takes Python which does nothing but launch kernels, as this package's and torch.nn's does.  Code of the user's (an
-    overridden ``predict_step``, a forward pass or a hook of its own) may count, keep or branch on what it sees, and has
-    to run for every batch."""
+def _scoring_state(model) -> list:
+    """What a captured scoring step of ``model`` is made from: its modules and their code, the storage of their parameters
+    and buffers, and the public attributes their forward passes go by.  (Looked at in every pass over a dataset, so
+    written to take little: 20 us for a DeepFM.)"""
     hooks = torch.nn.modules.module
-    if hooks._global_forward_hooks or hooks._global_forward_pre_hooks or torch.is_autocast_enabled("cuda"):
-        return None
-    if not _own_code(type(model).predict_step) or "predict_step" in model.__dict__:
-        return None
-    out: list = [torch.get_float32_matmul_precision()]
-    for m in model.modules():
-        if not (_own_code(type(m)) and _own_code(type(m).forward)) or "forward" in m.__dict__ or m._forward_hooks or m._forward_pre_hooks:
-            return None
-        out.append(m)
-        for held in (m._parameters, m._buffers):
+    out = [len(hooks._global_forward_hooks) + len(hooks._global_forward_pre_hooks), torch.is_autocast_enabled("cuda"),
+           torch.get_float32_matmul_precision(), type(model).predict_step, "predict_step" in model.__dict__]
+    todo = [model]
+    for m in todo:
+        d, cls = m.__dict__, type(m)
+        out += (m, cls, cls.forward, len(d["_forward_hooks"]) + len(d["_forward_pre_hooks"]))
+        for held in (d["_parameters"], d["_buffers"]):
             for t in held.values():
-                out.append(t)
-                if t is not None:
-                    out.append(t.data_ptr())
-                    out.append(getattr(t, "_tn_bf16", None))
-        for k, v in m.__dict__.items():
-            if k[0] != "_" and k not in _NOT_SCORED:
-                if type(v) in (list, tuple):
-                    out.extend(v)
+                if t is None:
+                    out.append(None)
                 else:
-                    out.append(v)
-                    if torch.is_tensor(v):
-                        out.append(v.data_ptr())
+                    out += (t, t.data_ptr(), getattr(t, "_tn_bf16", None))
+        for v in [v for k, v in d.items() if k[0] != "_" and k not in _NOT_SCORED]:
+            if type(v) in (list, tuple):
+                out += v
+            else:
+                out.append(v)
+                if isinstance(v, torch.Tensor):
+                    out.append(v.data_ptr())
+        todo += [c for c in d["_modules"].values() if c is not None]
     return out
 
 
 def _same_state(a: list, b: list) -> bool:
-    return len(a) == len(b) and all(x is y or (type(x) is type(y) and type(x) in _PLAIN and x == y) for x, y in zip(a, b))
+    if len(a) != len(b):
+        return False
+    for x, y in zip(a, b):
+        if x is not y and not (type(x) in _PLAIN and type(x) is type(y) and x == y):
+            return False
+    return True
+
+
+def _scored_by_own_code(model) -> bool:
+    """Can a replay stand for scoring a batch with ``model``?  That takes Python which does nothing but launch kernels, as
+    this package's and torch.nn's does.  Code of the user's (an overridden ``predict_step``, a forward pass or a hook of
+    its own) may count, keep or branch on what it sees, and has to run for every batch."""
+    hooks = torch.nn.modules.module
+    if hooks._global_forward_hooks or hooks._global_forward_pre_hooks or torch.is_autocast_enabled("cuda"):
+        return False
+    if not _own_code(type(model).predict_step) or "predict_step" in model.__dict__:
+        return False
+    for m in model.modules():
+        if not (_own_code(type(m)) and _own_code(type(m).forward)) or "forward" in m.__dict__ or m._forward_hooks or m._forward_pre_hooks:
+            return False
+    return True
 
 
 _PADDED_SETS = 3     # captured steps per kind of ragged batch: short, usual and long ones
@@ -362,8 +377,8 @@ class _Kind:
 
 
 _PREDICT_SETS = 8    # captured scoring steps per model; batches of further kinds are scored eagerly
-# Batches of a kind that are scored eagerly before the step is captured.  Two captures take 1.9 to 2.7 ms and save 250 to
-# 350 us a batch (Wide&Deep of 32 and 1024, DeepFM of 8192, static and ragged): a shorter pass would not get them back.
+# Batches of a kind, seen or still to come in a pass over a list, that make the captures of its scoring step worth while:
+# two of them take 1.9 to 2.7 ms and save 250 to 350 us a batch (Wide&Deep of 32 and 1024, DeepFM of 8192, static and ragged).
 _PREDICT_SIGHTS = 8
 _PREDICT_RING = 16   # pinned buffers for predictions on their way to the host: how far the host may run ahead
 
@@ -1112,11 +1127,11 @@ class Model(nn.Module):
         return y, pred
 
     # ---- captured scoring steps ---------------------------------------------------------------------------------
-    def _predict_captured(self, features, check: bool = True):
+    def _predict_captured(self, features, check: bool = True, left: int = 0):
         """Issue the captured scoring step for a batch in host memory: ``(sets, index, inputs)``, where ``sets.pred[index]``
         will hold the predictions and ``sets.copied[index]`` tells when the inputs have been read; or None when this batch
         is to be scored eagerly.  ``check``: code of the user's may have run since the last batch, so look again at what
-        the model is made of."""
+        the model is made of.  ``left``: batches that are known to follow."""
         rt = core.runtime()
         if not self._use_graph or self._predict_off or rt.world > 1:
             return None
@@ -1138,15 +1153,15 @@ class Model(nn.Module):
         except TypeError:                    # a feature that is no tensor and cannot be compared: nothing to recognise it by
             return None
         if sets is None:
-            state = _scoring_state(self)
-            if state is None:
+            if not _scored_by_own_code(self):
                 return None
+            state = _scoring_state(self)
             if self._predict_state is not None and not _same_state(state, self._predict_state):
                 self._drop_scoring()
                 return None
             if rooms is None:
                 kind.sights += 1
-            if full or kind.sights <= _PREDICT_SIGHTS or (rooms is None and kind.held_off()):
+            if full or kind.sights + left <= _PREDICT_SIGHTS or (rooms is None and kind.held_off()):
                 return None
             with torch.no_grad():            # shape and type of the result, from the batch itself
                 (f,), _, _ = self._to_device((features,))
@@ -1169,13 +1184,9 @@ class Model(nn.Module):
         self._ext.stage_inputs(sets.leaves[p], leaves, self._copy_stream.cuda_stream, main.cuda_stream,
                                sets.done[p].cuda_event if sets.used[p] else 0, sets.copied[p].cuda_event,
                                read.cuda_event if read is not None else 0)
-        if check:                            # the inputs are on their way meanwhile
-            state = _scoring_state(self)
-            if state is None:
-                return None
-            if not _same_state(state, self._predict_state):
-                self._drop_scoring()
-                return None
+        if check and not _same_state(_scoring_state(self), self._predict_state):      # the inputs are on their way meanwhile
+            self._drop_scoring()
+            return None
         for link in self._predict_links:
             link.table.set_training(False)
             if link._front is not None:      # a front that ran ahead for the next training batch
@@ -1229,14 +1240,17 @@ class Model(nn.Module):
                 cb.on_predict_begin()
             ys, ps = [], []
             self.eval()
+            listed = len(dataset) if type(dataset) in (list, tuple) else 0
+            if steps is not None:
+                listed = min(listed, steps)
             own = False                      # nothing of the user's runs between the batches of a list
             ring, flying = [], []            # pinned buffers; (position in ps, buffer, event) of copies on their way
             for i, batch in enumerate(dataset):
                 if steps is not None and i >= steps:
                     break
                 features, labels = batch if isinstance(batch, (tuple, list)) and len(batch) == 2 else (batch, None)
-                issued = self._predict_captured(features, check=not own) if not self.training else None
-                own = issued is not None and type(dataset) in (list, tuple)
+                issued = self._predict_captured(features, not own, max(0, listed - i - 1)) if not self.training else None
+                own = issued is not None and listed > 0
                 if issued is None:
                     y, p = self.predict_step(batch)
                     ps.append(p.cpu())

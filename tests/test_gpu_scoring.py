@@ -157,8 +157,8 @@ def test_predictions_outlive_the_captures_they_came_from(tn_gpu, status_ok, monk
     m.predict(data)
     issue = type(m)._predict_captured
 
-    def late(self, features, check=True):
-        got = issue(self, features, check)
+    def late(self, features, *a):
+        got = issue(self, features, *a)
         with torch.cuda.stream(self._read_stream):
             torch.cuda._sleep(2_000_000)               # about a millisecond: the copy of this batch's predictions is late
         if len(calls) % 5 == 4:
