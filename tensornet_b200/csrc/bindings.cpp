@@ -964,8 +964,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("cross_v1_bwd", [](at::Tensor x0, at::Tensor xl, at::Tensor w, at::Tensor dot, at::Tensor gy, at::Tensor gx0,
                            at::Tensor gxl, at::Tensor gw, at::Tensor gb) {
     c10::cuda::CUDAGuard guard(x0.device());
+    at::Tensor scratch;
+    if (x0.size(1) > tn::kCrossV1OneTile) scratch = at::empty({x0.size(0)}, x0.options());
     tn::launch_cross_v1_bwd(ptr_of<float>(x0), ptr_of<float>(xl), ptr_of<float>(w), ptr_of<float>(dot), ptr_of<float>(gy),
                             (int)x0.size(0), (int)x0.size(1), ptr_of<float>(gx0), ptr_of<float>(gxl), ptr_of<float>(gw),
-                            ptr_of<float>(gb), cur_stream());
+                            ptr_of<float>(gb), scratch.defined() ? ptr_of<float>(scratch) : nullptr, cur_stream());
   });
 }

@@ -413,60 +413,79 @@ __global__ void cross_v1_fwd_kernel(const float* __restrict__ x0, const float* _
 // gx0 = gy * s ; gxl = gy + w * (gy . x0) ; gw += xl * (gy . x0) ; gb += gy.   One warp per row.
 // Adding every row's contribution to the D words of gw and gb was all this kernel did: 1.6 M atomics on 400 words, 39 us
 // for 4096 x 200.  A lane now keeps the sums of its NC columns in registers over the warp's rows, the warps of a block
-// meet in shared memory, and a block adds to gw / gb once: 5.8 us.  Rows wider than 32 * NC columns are walked in
-// tiles of that width (with the dot product taken once per tile).
-template <int NC>
+// meet in shared memory, and a block adds to gw / gb once: 5.8 us.  Rows wider than 1024 columns are cut into tiles
+// (blockIdx.y), for which the rows' dot products are taken beforehand (kTiled: `t_row`): 4096 x 2048 50 us, 4096 x 6416
+// 140, 1024 x 16384 91, a third to a quarter of the time with atomics (126, 279, 390); as tiles that each took the whole
+// row's product again they were 96, 889 and 2331.
+template <int NC, bool kTiled>
 __global__ void __launch_bounds__(256) cross_v1_bwd_kernel(const float* __restrict__ x0, const float* __restrict__ xl,
                                                            const float* __restrict__ w, const float* __restrict__ dot,
                                                            const float* __restrict__ gy, int B, int D, float* __restrict__ gx0,
-                                                           float* __restrict__ gxl, float* __restrict__ gw, float* __restrict__ gb) {
+                                                           float* __restrict__ gxl, float* __restrict__ gw, float* __restrict__ gb,
+                                                           const float* __restrict__ t_row) {
   pdl_sync();
   __shared__ float s_w[32 * NC], s_b[32 * NC];
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (int d0 = 0; d0 < D; d0 += 32 * NC) {
-    for (int k = threadIdx.x; k < 32 * NC; k += blockDim.x) { s_w[k] = 0.f; s_b[k] = 0.f; }
-    __syncthreads();
-    float aw[NC], ab[NC];
+  const int d0 = kTiled ? (int)blockIdx.y * 32 * NC : 0;
+  for (int k = threadIdx.x; k < 32 * NC; k += blockDim.x) { s_w[k] = 0.f; s_b[k] = 0.f; }
+  __syncthreads();
+  float aw[NC], ab[NC];
 #pragma unroll
-    for (int i = 0; i < NC; ++i) { aw[i] = 0.f; ab[i] = 0.f; }
-    for (int b = warp; b < B; b += nwarps) {
-      const float* a = x0 + (size_t)b * D; const float* c = xl + (size_t)b * D; const float* g = gy + (size_t)b * D;
-      float gv[NC], cv[NC];
-      float t = 0.f;
-#pragma unroll
-      for (int i = 0; i < NC; ++i) {
-        const int d = d0 + lane + 32 * i;
-        gv[i] = d < D ? g[d] : 0.f;
-        cv[i] = d < D ? c[d] : 0.f;
-        t += d < D ? gv[i] * a[d] : 0.f;
-      }
-      if (D > 32 * NC) {
-        for (int d = lane; d < D; d += 32)
-          if (d < d0 || d >= d0 + 32 * NC) t += g[d] * a[d];
-      }
-      t = warp_sum(t);
-      const float s = dot[b];
-#pragma unroll
-      for (int i = 0; i < NC; ++i) {
-        const int d = d0 + lane + 32 * i;
-        if (d < D) {
-          gx0[(size_t)b * D + d] = gv[i] * s;
-          gxl[(size_t)b * D + d] = gv[i] + __ldg(w + d) * t;
-        }
-        aw[i] += cv[i] * t;
-        ab[i] += gv[i];
-      }
-    }
+  for (int i = 0; i < NC; ++i) { aw[i] = 0.f; ab[i] = 0.f; }
+  for (int b = warp; b < B; b += nwarps) {
+    const float* a = x0 + (size_t)b * D; const float* c = xl + (size_t)b * D; const float* g = gy + (size_t)b * D;
+    float gv[NC], cv[NC];
+    float t = kTiled ? __ldg(t_row + b) : 0.f;
 #pragma unroll
     for (int i = 0; i < NC; ++i) {
-      atomicAdd(&s_w[lane + 32 * i], aw[i]);
-      atomicAdd(&s_b[lane + 32 * i], ab[i]);
+      const int d = d0 + lane + 32 * i;
+      gv[i] = d < D ? g[d] : 0.f;
+      cv[i] = d < D ? c[d] : 0.f;
+      if (!kTiled) t += d < D ? gv[i] * a[d] : 0.f;
     }
+    if (!kTiled) t = warp_sum(t);
+    const float s = dot[b];
+#pragma unroll
+    for (int i = 0; i < NC; ++i) {
+      const int d = d0 + lane + 32 * i;
+      if (d < D) {
+        gx0[(size_t)b * D + d] = gv[i] * s;
+        gxl[(size_t)b * D + d] = gv[i] + __ldg(w + d) * t;
+      }
+      aw[i] += cv[i] * t;
+      ab[i] += gv[i];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < NC; ++i) {
+    atomicAdd(&s_w[lane + 32 * i], aw[i]);
+    atomicAdd(&s_b[lane + 32 * i], ab[i]);
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < 32 * NC && d0 + k < D; k += blockDim.x) {
+    atomicAdd(gw + d0 + k, s_w[k]);
+    atomicAdd(gb + d0 + k, s_b[k]);
+  }
+}
+// t[b] = gy[b] . x0[b] for rows of many columns, a block per row
+__global__ void __launch_bounds__(256) cross_v1_rowdot_kernel(const float* __restrict__ gy, const float* __restrict__ x0, int B, int D,
+                                                              float* __restrict__ t) {
+  pdl_sync();
+  __shared__ float s_part[8];
+  for (int b = blockIdx.x; b < B; b += gridDim.x) {
+    const float* g = gy + (size_t)b * D; const float* a = x0 + (size_t)b * D;
+    float v = 0.f;
+#pragma unroll 4
+    for (int d = threadIdx.x; d < D; d += 256) v += g[d] * a[d];
+    v = warp_sum(v);
+    if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = v;
     __syncthreads();
-    for (int k = threadIdx.x; k < 32 * NC && d0 + k < D; k += blockDim.x) {
-      atomicAdd(gw + d0 + k, s_w[k]);
-      atomicAdd(gb + d0 + k, s_b[k]);
+    if (threadIdx.x == 0) {
+      float sum = 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) sum += s_part[k];
+      t[b] = sum;
     }
     __syncthreads();
   }
@@ -665,13 +684,24 @@ void launch_cross_v1_fwd(const float* x0, const float* xl, const float* w, const
   launch_pdl(cross_v1_fwd_kernel, dim3(blocks_for(B, 8)), dim3(256), 0, st, x0, xl, w, bias, B, D, y, dot);
 }
 void launch_cross_v1_bwd(const float* x0, const float* xl, const float* w, const float* dot, const float* gy, int B, int D,
-                         float* gx0, float* gxl, float* gw, float* gb, cudaStream_t st) {
+                         float* gx0, float* gxl, float* gw, float* gb, float* row_scratch, cudaStream_t st) {
+  if (D > kCrossV1OneTile) {
+    // 256 columns a tile; with the rows split over blocks until four blocks per SM have work
+    const int tiles = (D + 255) / 256;
+    int by_rows = (B + 15) / 16, most = (148 * 4 + tiles - 1) / tiles;
+    if (by_rows > most) by_rows = most;
+    if (by_rows < 1) by_rows = 1;
+    launch_pdl(cross_v1_rowdot_kernel, dim3(blocks_for(B, 1)), dim3(256), 0, st, gy, x0, B, D, row_scratch);
+    launch_pdl(cross_v1_bwd_kernel<8, true>, dim3(by_rows, tiles), dim3(256), 0, st, x0, xl, w, dot, gy, B, D, gx0, gxl, gw, gb,
+               static_cast<const float*>(row_scratch));
+    return;
+  }
   // two rows per warp: fewer blocks would leave SMs idle, more would add to gw / gb more often
   int blocks = (B + 15) / 16;
   if (blocks > 148 * 2) blocks = 148 * 2;
   if (blocks < 1) blocks = 1;
-  auto* kernel = D <= 256 ? cross_v1_bwd_kernel<8> : D <= 512 ? cross_v1_bwd_kernel<16> : cross_v1_bwd_kernel<32>;
-  launch_pdl(kernel, dim3(blocks), dim3(256), 0, st, x0, xl, w, dot, gy, B, D, gx0, gxl, gw, gb);
+  auto* kernel = D <= 256 ? cross_v1_bwd_kernel<8, false> : D <= 512 ? cross_v1_bwd_kernel<16, false> : cross_v1_bwd_kernel<32, false>;
+  launch_pdl(kernel, dim3(blocks), dim3(256), 0, st, x0, xl, w, dot, gy, B, D, gx0, gxl, gw, gb, static_cast<const float*>(nullptr));
 }
 
 }  // namespace tn

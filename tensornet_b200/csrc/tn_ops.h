@@ -64,8 +64,9 @@ void launch_bce(const float* logit, const float* label, int B, float* pred, floa
                 int nbins, cudaStream_t st);
 void launch_cross_v1_fwd(const float* x0, const float* xl, const float* w, const float* bias, int B, int D, float* y, float* dot,
                          cudaStream_t st);
+constexpr int kCrossV1OneTile = 1024;   // wider rows take `row_scratch`: fp32 [B]
 void launch_cross_v1_bwd(const float* x0, const float* xl, const float* w, const float* dot, const float* gy, int B, int D,
-                         float* gx0, float* gxl, float* gw, float* gb, cudaStream_t st);
+                         float* gx0, float* gxl, float* gw, float* gb, float* row_scratch, cudaStream_t st);
 void launch_relu_mask(void* g, const void* y, long long n, cudaStream_t st);
 void launch_cross_v2_bwd_elem(const void* g, const void* u, const void* x0, float* gx0, void* du, long long n, int first, cudaStream_t st);
 constexpr int kMaxCrossLayers = 8;

@@ -186,3 +186,9 @@ def test_cross_v1_backward_against_fp64(tn_gpu, status_ok, B, D):
     for got, want, size in [(x0.grad, d[3] * s, d[3].abs() * sa), (xl.grad, d[3] + d[2] * t, d[3].abs() + d[2].abs() * ta),
                             (w.grad.view(-1), (d[1] * t).sum(0), (d[1].abs() * ta).sum(0)), (b.grad, d[3].sum(0), d[3].abs().sum(0))]:
         assert bool(((got.double() - want).abs() <= 2 * eps * size + 1e-30).all())
+
+
+@pytest.mark.parametrize("B,D", [(1, 1025), (7, 1280), (33, 1281), (600, 2048), (20, 6413)])
+def test_cross_v1_backward_of_rows_in_tiles(tn_gpu, status_ok, B, D):
+    """Above 1024 columns: edges of the 256-column tiles, one row and more rows than a block's warps."""
+    test_cross_v1_backward_against_fp64(tn_gpu, status_ok, B, D)
