@@ -164,12 +164,7 @@ struct SparseCtx {
   void set_table(py::dict table) { keep["table"] = table; t = table_from_dict(table); upload_table(); }
 
   // Dedup, id dispatch and inverse map of a batch ahead of its pull (plain kernels on the current stream).
-  static const int* count_ptr(const c10::optional<at::Tensor>& n_dev) {
-    if (!n_dev.has_value()) return nullptr;
-    TORCH_CHECK(n_dev->is_cuda() && n_dev->scalar_type() == at::kInt && n_dev->numel() == 1, "n_dev: one int32 on the device");
-    return ptr_of<const int>(*n_dev);
-  }
-  void front(at::Tensor ids, at::Tensor inverse, c10::optional<at::Tensor> n_dev) {
+  void front(at::Tensor ids, at::Tensor inverse) {
     TORCH_CHECK(ids.is_cuda() && ids.scalar_type() == at::kLong && ids.is_contiguous(), "ids: contiguous int64 CUDA tensor");
     TORCH_CHECK(inverse.scalar_type() == at::kInt && inverse.numel() >= ids.numel(), "inverse: int32, one per id");
     c10::cuda::CUDAGuard guard(ids.device());
@@ -177,13 +172,17 @@ struct SparseCtx {
     a.c = c; a.tbl = t; a.opt = o;
     a.ids = ptr_of<const long long>(ids);
     a.n_ids = (int)ids.numel();
-    a.n_dev = count_ptr(n_dev);
     a.inverse = ptr_of<int>(inverse);
     a.training = 1;
     check(tn::launch_sparse_pull_front(a, cur_stream()), "sparse_pull_front launch");
     g_launches.fetch_add(1, std::memory_order_relaxed);      // two kernels
   }
 
+  static const int* count_ptr(const c10::optional<at::Tensor>& n_dev) {
+    if (!n_dev.has_value()) return nullptr;
+    TORCH_CHECK(n_dev->is_cuda() && n_dev->scalar_type() == at::kInt && n_dev->numel() == 1, "n_dev: one int32 on the device");
+    return ptr_of<const int>(*n_dev);
+  }
   void pull(at::Tensor ids, at::Tensor inverse, c10::optional<at::Tensor> labels, int label_mod, bool training, bool lookup_only,
             bool front_done, c10::optional<at::Tensor> n_dev) {
     TORCH_CHECK(ids.is_cuda() && ids.scalar_type() == at::kLong && ids.is_contiguous(), "ids: contiguous int64 CUDA tensor");
@@ -584,7 +583,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         const tn::DenseStepArgs d = dense.cast<DenseCtx&>().rider_args();
         self.push(work_hint, max_ctas, &d);
       }, py::arg("work_hint"), py::arg("max_ctas") = 0, py::arg("dense") = py::none())
-      .def("front", &SparseCtx::front, py::arg("ids"), py::arg("inverse"), py::arg("n_dev") = py::none());
+      .def("front", &SparseCtx::front, py::arg("ids"), py::arg("inverse"));
   py::class_<ServeCtx>(m, "ServeCtx")
       .def(py::init<py::dict, int, int, std::vector<int>, bool>())
       .def("forward", &ServeCtx::forward);

@@ -415,8 +415,7 @@ __global__ void cross_v1_fwd_kernel(const float* __restrict__ x0, const float* _
 // for 4096 x 200.  A lane now keeps the sums of its NC columns in registers over the warp's rows, the warps of a block
 // meet in shared memory, and a block adds to gw / gb once: 5.8 us.  Rows wider than 1024 columns are cut into tiles
 // (blockIdx.y), for which the rows' dot products are taken beforehand (kTiled: `t_row`): 4096 x 2048 50 us, 4096 x 6416
-// 140, 1024 x 16384 91, a third to a quarter of the time with atomics (126, 279, 390); as tiles that each took the whole
-// row's product again they were 96, 889 and 2331.
+// 140, 1024 x 16384 91 us (126, 279 and 390 with the atomics).
 template <int NC, bool kTiled>
 __global__ void __launch_bounds__(256) cross_v1_bwd_kernel(const float* __restrict__ x0, const float* __restrict__ xl,
                                                            const float* __restrict__ w, const float* __restrict__ dot,

@@ -432,7 +432,8 @@ const char* gemm_bf16(const GemmDesc& d, cudaStream_t stream) {
   int stages = 3;
   if (halves == 1) {
     const int most = gemm_ring_stages(BN), want = ktps < most ? ktps : most;
-    stages = most < 4 ? 3 : (want <= 4 ? 4 : (want <= 6 || most < 8 ? (most >= 6 ? 6 : 4) : 8));
+    static_assert((200 * 1024) / (128 * 128 + 256 * 128) >= 4, "the widest tile has four stages");
+    stages = want <= 4 ? 4 : (want <= 6 || most < 8 ? (most >= 6 ? 6 : 4) : 8);
   }
   size_t smem = stages * (a_stage + b_bytes) + 1024;
   if (smem < epi_bytes) smem = epi_bytes;
@@ -441,7 +442,6 @@ const char* gemm_bf16(const GemmDesc& d, cudaStream_t stream) {
     cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
     cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<6, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
     cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<4, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<3, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
     cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<3, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
     attr_set = true;
   }
@@ -463,8 +463,7 @@ const char* gemm_bf16(const GemmDesc& d, cudaStream_t stream) {
   if (halves == 2) e = cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_kernel<3, 2>, tmA, tmB, p);
   else if (stages == 8) e = cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_kernel<8, 1>, tmA, tmB, p);
   else if (stages == 6) e = cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_kernel<6, 1>, tmA, tmB, p);
-  else if (stages == 4) e = cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_kernel<4, 1>, tmA, tmB, p);
-  else e = cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_kernel<3, 1>, tmA, tmB, p);
+  else e = cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_kernel<4, 1>, tmA, tmB, p);
   if (e == cudaSuccess) e = cudaGetLastError();
   return e == cudaSuccess ? nullptr : cudaGetErrorString(e);
 }

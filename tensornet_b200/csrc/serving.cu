@@ -179,14 +179,14 @@ __device__ __forceinline__ float4 bf16x4(uint2 v) {
   return make_float4(a.x, a.y, b.x, b.y);
 }
 
-// A layer of a request of at most 8 rows, y[m, n] = relu(sum_k x[m, k] w[n, k]): a 128-row MMA tile would be all
+// A layer of a request of at most kServeSkinnyRows rows, y[m, n] = relu(sum_k x[m, k] w[n, k]): a 128-row MMA tile would be all
 // padding, and what counts is streaming the weights once through every SM.  A warp takes kRows weight rows, eight loads
 // in flight per lane; a block's warps share a group of rows and split K (`ksplit` ways), the parts meet in shared
 // memory.  fp32 weights are rounded to bf16 on the way, as the MMA operands are.  The bias sits in column K - 1.
 template <int kM, bool kF32>
 __global__ void __launch_bounds__(256) serve_skinny_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const void* __restrict__ w, int ldw, int M,
                                                            int N, int K, int relu, __nv_bfloat16* __restrict__ y, int ldy, int n_store, int ksplit) {
-  constexpr int kRows = kM <= 2 ? 2 : 1;
+  constexpr int kRows = 2;
   __shared__ float s_part[8][kRows * kM];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int groups = 8 / ksplit;                                 // row groups per block
@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(256) serve_skinny_kernel(const __nv_bfloat16* 
   const int per = (n4 + ksplit - 1) / ksplit;
   const int c0 = kp * per, c1 = min(n4, c0 + per);
   // the weights do not depend on the kernel before this one: the first ones are on their way before its results are waited for
-  constexpr int kUn = kRows == 2 ? 4 : 8;
+  constexpr int kUn = 4;
   float4 wv[kRows][kUn];
   auto load_w = [&](int c) {
 #pragma unroll
@@ -336,7 +336,7 @@ void launch_serve_lookup_ragged(const TableView& t, const long long* ids, int n,
 template <int kM>
 static void skinny(const void* x, int ldx, const void* w, int w_f32, int ldw, int M, int N, int K, int relu, void* y, int ldy, int n_store,
                    cudaStream_t st) {
-  constexpr int kRows = kM <= 2 ? 2 : 1;
+  constexpr int kRows = 2;               // as in the kernel
   // long rows are split over the warps of a block until every SM has a block (a row group is read by one warp otherwise)
   int ks = 1;
   while (ks < 8 && (n_store + (8 / ks) * kRows - 1) / ((8 / ks) * kRows) < 148 && K / (2 * ks) >= 256) ks *= 2;
@@ -348,10 +348,9 @@ static void skinny(const void* x, int ldx, const void* w, int w_f32, int ldw, in
 }
 void launch_serve_skinny(const void* x, int ldx, const void* w, int w_f32, int ldw, int M, int N, int K, int relu, void* y, int ldy, int n_store,
                          cudaStream_t st) {
+  static_assert(kServeSkinnyRows == 2, "one instantiation per row count");
   if (M <= 1) skinny<1>(x, ldx, w, w_f32, ldw, M, N, K, relu, y, ldy, n_store, st);
-  else if (M <= 2) skinny<2>(x, ldx, w, w_f32, ldw, M, N, K, relu, y, ldy, n_store, st);
-  else if (M <= 4) skinny<4>(x, ldx, w, w_f32, ldw, M, N, K, relu, y, ldy, n_store, st);
-  else skinny<8>(x, ldx, w, w_f32, ldw, M, N, K, relu, y, ldy, n_store, st);
+  else skinny<2>(x, ldx, w, w_f32, ldw, M, N, K, relu, y, ldy, n_store, st);
 }
 void launch_serve_head(const void* z, int ld, int B, int K, const float* w, float* prob, cudaStream_t st) {
   launch_pdl(serve_head_kernel, dim3(capped((B + 7) / 8, 148 * 4)), dim3(256), 0, st, reinterpret_cast<const __nv_bfloat16*>(z), ld, B, K, w, prob);

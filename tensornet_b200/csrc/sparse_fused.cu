@@ -639,7 +639,7 @@ __global__ void __launch_bounds__(kFrontThreads) pull_front_dedup_kernel(const _
   if (s_bad != 0) return;
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int nth = gridDim.x * blockDim.x;
-  const int n_ids = batch_ids(a);
+  const int n_ids = a.n_ids;
   if (c.prof != nullptr && tid == 0) c.prof[16] = globaltimer_ns();
   dedup_assign(a, n_ids, tid, nth);
   if (c.prof != nullptr && threadIdx.x == 0) atomicMax(&c.prof[17], globaltimer_ns());      // last CTA's end
@@ -655,7 +655,7 @@ __global__ void __launch_bounds__(kFrontThreads) pull_front_ship_kernel(const __
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int nth = gridDim.x * blockDim.x;
   const int W = c.world, R = c.rank, capo = c.capo;
-  const int n_ids = batch_ids(a);
+  const int n_ids = a.n_ids;
   const unsigned long long epoch = __ldcg(c.epoch) + 1ull;
   if (W > 1) {
     for (int p = 0; p < W; ++p) {
