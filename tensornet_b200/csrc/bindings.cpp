@@ -365,7 +365,7 @@ struct ServeCtx {
     TORCH_CHECK(dims.size() >= 2 && dims.size() <= (size_t)tn::kServeMaxLayers + 1 && dims[0] == S * t.dim, "serving: tower input width");
   }
   static int pad8(int n) { return (n + 7) / 8 * 8; }
-  struct CopyLane { cudaStream_t stream = nullptr; cudaEvent_t begin = nullptr, end = nullptr; };
+  struct CopyLane { cudaStream_t stream = nullptr; cudaEvent_t begin = nullptr, end = nullptr, read = nullptr; };
   // one per thread and device: threads that serve side by side do not wait for one another's copies
   static CopyLane& copy_lane(int device) {
     static thread_local CopyLane lanes[64];
@@ -374,18 +374,22 @@ struct ServeCtx {
       check(cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking), "serving: stream");
       check(cudaEventCreateWithFlags(&c.begin, cudaEventDisableTiming), "serving: event");
       check(cudaEventCreateWithFlags(&c.end, cudaEventDisableTiming), "serving: event");
+      check(cudaEventCreateWithFlags(&c.read, cudaEventDisableTiming), "serving: event");
     }
     return c;
   }
 
   // `weights`: fp32 [N, pad8(K + 1)] per layer; `shadows`: their bf16 copies when something keeps them current, else empty.
-  // Nothing comes back when they do not start on 16 bytes, which the kernels' loads ask for.
+  // Nothing comes back for weights of another kind, or that do not start on 16 bytes, which the kernels' loads ask for.
+  // `wait_read`: return only when page-locked ids and offsets have been read, so that the caller may fill them again.
   c10::optional<at::Tensor> forward(at::Tensor ids, c10::optional<at::Tensor> offsets, int B, const std::vector<at::Tensor>& weights,
-                                    const std::vector<at::Tensor>& shadows, at::Tensor head_w, at::Tensor status) {
+                                    const std::vector<at::Tensor>& shadows, at::Tensor head_w, at::Tensor status, bool wait_read) {
     const int L = (int)dims.size() - 1;
     const bool cast_needed = shadows.empty();
-    TORCH_CHECK((int)weights.size() == L && (cast_needed || (int)shadows.size() == L) && head_w.numel() == dims[L] + 1 && head_w.is_cuda() &&
-                    head_w.is_contiguous() && head_w.scalar_type() == at::kFloat, "serving: weights");
+    if (!head_w.is_cuda() || !head_w.is_contiguous() || head_w.scalar_type() != at::kFloat) return c10::nullopt;
+    for (const at::Tensor& w : weights)
+      if (!w.is_cuda() || !w.is_contiguous() || w.scalar_type() != at::kFloat) return c10::nullopt;
+    TORCH_CHECK((int)weights.size() == L && (cast_needed || (int)shadows.size() == L) && head_w.numel() == dims[L] + 1, "serving: weights");
     TORCH_CHECK(ids.scalar_type() == at::kLong && ids.is_contiguous() && B >= 1, "serving: contiguous int64 ids");
     TORCH_CHECK(offsets.has_value() ? offsets->numel() == (int64_t)S * B + 1 && offsets->is_contiguous() && offsets->scalar_type() == at::kInt
                                     : ids.numel() == (int64_t)S * B, "serving: one bag per slot and example");
@@ -430,6 +434,8 @@ struct ServeCtx {
                       w.scalar_type() == (cast_needed ? at::kFloat : at::kBFloat16),
                   "serving: layer ", l, " weights");
     }
+    cudaEvent_t read = nullptr;                // behind the last reader of page-locked memory
+    bool pinned = mid != nullptr || moff != nullptr;
     if (copy_ids || copy_off) {
       // on a stream of its own: the weights are converted meanwhile
       CopyLane& cl = copy_lane(dev.index());
@@ -441,13 +447,19 @@ struct ServeCtx {
       }
       auto put = [&](const at::Tensor& d, const at::Tensor& h) {
         check(cudaMemcpyAsync(d.data_ptr(), h.data_ptr(), h.nbytes(), cudaMemcpyHostToDevice, cs), "serving: copy");
-        if (h.is_pinned())
+        if (h.is_pinned()) {
+          pinned = true;
           at::getHostAllocator(at::kCUDA)->record_event(const_cast<void*>(h.storage().data()), h.storage().data_ptr().get_context(),
                                                         c10::cuda::getStreamFromExternal(cs, dev.index()).unwrap());
+        }
       };
       if (copy_ids) put(hold_ids, ids);
       if (copy_off) put(hold_off, *offsets);
       if (side) check(cudaEventRecord(cl.end, cs), "serving: event");
+      if (wait_read && pinned) {
+        read = side ? cl.end : cl.read;
+        if (!side) check(cudaEventRecord(cl.read, st), "serving: event");
+      }
     }
     if (cast_now) {
       tn::ServeCast c{};
@@ -459,11 +471,14 @@ struct ServeCtx {
     // behind a copy the lookup is launched the ordinary way; the conversion is then complete anyway
     const bool behind_cast = cast_now && !copy_ids && !copy_off;
     const int ld0 = pad8(dims[0] + 1);
+    const bool in_place = mid != nullptr || moff != nullptr;
+    if (wait_read && in_place) read = copy_lane(dev.index()).read;
     if (poff)
       tn::launch_serve_lookup_ragged(t, pid, (int)ids.numel(), poff, B, S, combiner, reinterpret_cast<int*>(w0 + at_rows),
-                                     moff ? reinterpret_cast<int*>(w0 + at_off) : nullptr, w0 + at_act[0], ld0, dims[0], behind_cast, st);
+                                     moff ? reinterpret_cast<int*>(w0 + at_off) : nullptr, w0 + at_act[0], ld0, dims[0], behind_cast,
+                                     wait_read && in_place ? read : nullptr, st);
     else
-      tn::launch_serve_lookup_single(t, pid, B, S, w0 + at_act[0], ld0, dims[0], behind_cast, st);
+      tn::launch_serve_lookup_single(t, pid, B, S, w0 + at_act[0], ld0, dims[0], behind_cast, wait_read && in_place ? read : nullptr, st);
     // host memory read in place must not be handed out again before the kernels are done with it
     for (const at::Tensor* h : {mid ? &hold_ids : nullptr, moff ? &hold_off : nullptr})
       if (h != nullptr)
@@ -486,6 +501,12 @@ struct ServeCtx {
     tn::launch_serve_head(w0 + at_act[L], pad8(dims[L] + 1), B, dims[L] + 1, ptr_of<const float>(head_w), ptr_of<float>(prob), st);
     check(cudaGetLastError(), "serving launch");
     g_launches.fetch_add(L + 2 + (cast_now ? 1 : 0) + (poff ? 1 : 0), std::memory_order_relaxed);
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (read != nullptr) check(cudaStreamIsCapturing(st, &capturing), "serving: stream");
+    if (read != nullptr && capturing == cudaStreamCaptureStatusNone) {
+      py::gil_scoped_release others_may_run;
+      check(cudaEventSynchronize(read), "serving: inputs");
+    }
     return prob;
   }
 };

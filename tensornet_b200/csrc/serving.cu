@@ -51,12 +51,13 @@ __global__ void dict_lookup_pool_kernel(TableView t, const long long* __restrict
 // The request path of InferenceEngine: lookup -> layers -> head, a handful of kernels chained as programmatic
 // dependents.  What bounds a request is latency, so every stage is shaped for parallel misses: one lane per id probes
 // (its key and its row index are loaded together, not one behind the other), then all rows of a warp's bags are in
-// flight at once.  Ids may be read straight from pinned host memory, which takes the copy and the wait for it out of
-// the chain: the PCIe reads of all warps are in flight together.
+// flight at once.  The ids of a small request (128 KB at most) may be read straight from pinned host memory, which takes
+// the copy and the wait for it out of the chain: the PCIe reads of all warps are in flight together.  Larger ones are
+// copied first, beside the conversion of the weights where there is one.
 // The first kernel of the chain is launched the ordinary way: it starts when everything before the request is complete,
 // so that the ones behind it may write their buffers and read weights before their own predecessor is done.
-// 200 slots x 512 examples, dim 32 (102 K ids, 2 M rows): copy 18.6 us + lookup 17.3 us before, one kernel of that
-// transfer's length now.
+// 200 slots x 512 examples, dim 32 (102 K ids, 2 M rows): lookup 17.3 us as one probe after the other, 9.4 to 9.9 now,
+// behind a copy of 18 to 36 us (the host link differs from machine to machine).
 // ---------------------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ int find_row(const TableView& t, unsigned long long key) {
   unsigned h = table_home(t, key);
@@ -313,7 +314,7 @@ void launch_serve_cast(const ServeCast& a, cudaStream_t st) {
   serve_cast_kernel<<<capped((n8 + 255) / 256, 148 * 4), 256, 0, st>>>(a);
 }
 void launch_serve_lookup_single(const TableView& t, const long long* ids, int B, int S, void* out, int ld_out, int ones_col, bool behind_cast,
-                                cudaStream_t st) {
+                                cudaEvent_t read, cudaStream_t st) {
   const int G = lanes_for_width(t.dim);
   const long long nbags = (long long)B * S;
   int wb = 32;                                                   // enough warps for every SM to have a few
@@ -322,14 +323,16 @@ void launch_serve_lookup_single(const TableView& t, const long long* ids, int B,
   __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(out);
   if (behind_cast) launch_pdl(serve_lookup_single_kernel, grid, dim3(256), 0, st, t, ids, B, S, o, ld_out, ones_col, G, wb);
   else serve_lookup_single_kernel<<<grid, 256, 0, st>>>(t, ids, B, S, o, ld_out, ones_col, G, wb);
+  if (read != nullptr) cudaEventRecord(read, st);
 }
 void launch_serve_lookup_ragged(const TableView& t, const long long* ids, int n, const int* offsets, int B, int S, int combiner, int* rows,
-                                int* offsets_dev, void* out, int ld_out, int ones_col, bool behind_cast, cudaStream_t st) {
+                                int* offsets_dev, void* out, int ld_out, int ones_col, bool behind_cast, cudaEvent_t read, cudaStream_t st) {
   const int G = lanes_for_width(t.dim);
   const long long nbags = (long long)B * S;
   const dim3 grid(capped(((n > nbags ? n : nbags) + 255) / 256, 148 * 8));
   if (behind_cast) launch_pdl(serve_probe_kernel, grid, dim3(256), 0, st, t, ids, n, offsets, (int)nbags + 1, rows, offsets_dev);
   else serve_probe_kernel<<<grid, 256, 0, st>>>(t, ids, n, offsets, (int)nbags + 1, rows, offsets_dev);
+  if (read != nullptr) cudaEventRecord(read, st);
   launch_pdl(serve_pool_kernel, dim3(capped((nbags * G + 255) / 256, 148 * 8)), dim3(256), 0, st, t, rows, n,
              static_cast<const int*>(offsets_dev != nullptr ? offsets_dev : offsets), B, S, combiner, reinterpret_cast<__nv_bfloat16*>(out), ld_out, ones_col, G);
 }

@@ -116,10 +116,11 @@ struct ServeCast {
   long long n8[kServeMaxLayers];         // groups of eight elements
 };
 void launch_serve_cast(const ServeCast& a, cudaStream_t st);
+// `read` (may be null): recorded once ids and offsets have been read
 void launch_serve_lookup_single(const TableView& t, const long long* ids, int B, int S, void* out, int ld_out, int ones_col, bool behind_cast,
-                                cudaStream_t st);
+                                cudaEvent_t read, cudaStream_t st);
 void launch_serve_lookup_ragged(const TableView& t, const long long* ids, int n, const int* offsets, int B, int S, int combiner, int* rows,
-                                int* offsets_dev, void* out, int ld_out, int ones_col, bool behind_cast, cudaStream_t st);
+                                int* offsets_dev, void* out, int ld_out, int ones_col, bool behind_cast, cudaEvent_t read, cudaStream_t st);
 void launch_serve_skinny(const void* x, int ldx, const void* w, int w_f32, int ldw, int M, int N, int K, int relu, void* y, int ldy, int n_store,
                          cudaStream_t st);
 void launch_serve_head(const void* z, int ld, int B, int K, const float* w, float* prob, cudaStream_t st);

@@ -89,10 +89,10 @@ class EmbeddingDictionary:
 class InferenceEngine:
     """``ids [S, B]`` (or ragged) -> click probabilities, for a dense tower ``MLP`` + ``DenseHead``.
 
-    On a GPU a request is one native call that launches lookup, layers and head as a chain of dependent kernels; ids in
-    pinned host memory are read in place.  (A captured graph per batch shape, which this replaces, took longer to start
-    than the chain takes to issue, and served ragged requests not at all.)  Towers other than ``MLP`` + ``DenseHead``
-    run as the modules they are, captured per batch shape."""
+    On a GPU a request is one native call that launches lookup, layers and head as a chain of dependent kernels; up to
+    128 KB of ids in pinned host memory are read in place, more are copied first.  (A captured graph per batch shape, which this replaces, took longer to start
+    than the chain takes to issue, and served ragged requests not at all.)  Towers other than ``MLP`` + ``DenseHead``,
+    or with hooks, run as the modules they are, captured per batch shape."""
 
     def __init__(self, dictionary: EmbeddingDictionary, mlp, head, n_slots: int, combiner: str = "mean"):
         self.dict, self.mlp, self.head, self.S = dictionary, mlp, head, n_slots
@@ -118,15 +118,14 @@ class InferenceEngine:
             self._ctx_of, self._ctx_mlp = of, mlp           # the chain holds the arrays: an id stands for one object
         return self._ctx
 
-    def _native(self, ids, offsets, B: int):
+    def _native(self, ids, offsets, B: int, wait_read: bool):
         """The request through the native chain, or None when something about it is out of the ordinary."""
         ctx = self._context()
         if ctx is None:
             return None
-        ws = list(self.mlp.weights._parameters.values())
-        hw = self.head.weight
-        if self.mlp.weight_gate is not None or not all(w.is_cuda and w.dtype == torch.float32 and w.is_contiguous() for w in (*ws, hw)):
+        if self.mlp.weight_gate is not None:
             return None
+        ws = list(self.mlp.weights._parameters.values())
         if ids.dtype != torch.int64 or not ids.is_contiguous():
             ids = ids.to(torch.int64).contiguous()
         if offsets is not None and (offsets.dtype != torch.int32 or not offsets.is_contiguous()):
@@ -134,7 +133,7 @@ class InferenceEngine:
         shadows = [getattr(w, "_tn_bf16", None) for w in ws]
         if any(s is None for s in shadows):
             shadows = []
-        return ctx.forward(ids, offsets, B, ws, shadows, hw, runtime().status)
+        return ctx.forward(ids, offsets, B, ws, shadows, self.head.weight, runtime().status, wait_read)
 
     def _forward_gpu(self, ids, offsets, B):
         ext = _build.cuda_ext()
@@ -166,7 +165,8 @@ class InferenceEngine:
             return torch.sigmoid(self.head(self.mlp(F.concat_cast([x], ones=True)))).view(-1)
         dev = rt.device
         n = int(ids.shape[1]) if offsets is None else (offsets.numel() - 1) // self.S
-        prob = self._native(ids, offsets, n) if n > 0 else None
+        # a request with offsets, or outside a graph, has always been through with the caller's buffers on return
+        prob = self._native(ids, offsets, n, offsets is not None or not use_graph) if n > 0 else None
         if prob is not None:
             return prob
         if offsets is not None or not use_graph:

@@ -98,3 +98,32 @@ def test_requests_follow_what_the_engine_is_made_of(tn_gpu, status_ok):
     assert len(calls) == 3
     handle.remove()
     follows()
+
+
+@pytest.mark.parametrize("B", [2, 40, 700])
+@pytest.mark.parametrize("ragged", [False, True])
+def test_page_locked_buffers_may_be_filled_again(tn_gpu, status_ok, B, ragged):
+    """A request with offsets, or one outside a graph, that is queued behind other work: its buffers are written over as
+    soon as the call returns.  2: read in place; 40: in place, layers on the tensor cores; 700: copied."""
+    from tensornet_b200.layers import DenseHead, MLP
+    from tensornet_b200.serving import EmbeddingDictionary, InferenceEngine
+
+    dev = tn_gpu.core.runtime().device
+    S = 40
+    torch.manual_seed(B)
+    mlp, head = MLP(S * 4, [32, 16]).to(dev), DenseHead(16).to(dev)
+    rows = np.random.default_rng(0).standard_normal((100, 4)).astype(np.float32)
+    eng = InferenceEngine(EmbeddingDictionary(np.arange(1, 101, dtype=np.uint64), rows), mlp, head, S)
+    ids = torch.randint(1, 101, (S, B)).pin_memory()
+    offs = torch.arange(S * B + 1, dtype=torch.int32).pin_memory()
+    args = (ids.reshape(-1), offs) if ragged else (ids,)
+    want = eng.infer(*args, use_graph=False).clone()
+    for _ in range(3):
+        keep = ids.clone(), offs.clone()
+        torch.cuda._sleep(1_000_000)                  # half a millisecond of other work in front
+        got = eng.infer(*args, use_graph=False)
+        ids.fill_(7)
+        offs.fill_(0)
+        assert torch.equal(got, want)
+        ids.copy_(keep[0])
+        offs.copy_(keep[1])
