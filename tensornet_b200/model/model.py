@@ -1275,7 +1275,7 @@ class Model(nn.Module):
                 flying.append((len(ps), buf, ev))
                 ps.append(None)
                 if labels is not None:
-                    ys.append(labels.cpu() if labels.is_cuda else labels.clone())
+                    ys.append(labels if own else labels.cpu() if labels.is_cuda else labels.clone())
                 if not own and any(t.is_pinned() for t in leaves):
                     sets.copied[k].synchronize()     # a reader may fill the same page-locked buffers with the next batch
             for at, buf, ev in flying:

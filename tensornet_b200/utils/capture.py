@@ -45,11 +45,12 @@ def capture(graph: "torch.cuda.CUDAGraph", pool=None):
     if stream is None:
         stream = _STREAMS[dev] = torch.cuda.Stream(device=dev)
     torch.cuda.synchronize()
-    free, total = torch.cuda.mem_get_info(dev)
-    # no step so far has needed more than the allocator holds; an eighth of the device for steps that are larger
-    if free < max(torch.cuda.memory_reserved(dev), total // 8):
-        gc.collect()
-        torch.cuda.empty_cache()
+    if pool is None:               # (the first capture of a group: the others find what it needed in their common pool)
+        free, total = torch.cuda.mem_get_info(dev)
+        # no step so far has needed more than the allocator holds; an eighth of the device for steps that are larger
+        if free < max(torch.cuda.memory_reserved(dev), total // 8):
+            gc.collect()
+            torch.cuda.empty_cache()
     with _collector_off, torch.cuda.stream(stream):
         graph.capture_begin(*(() if pool is None else (pool,)))
         try:
