@@ -132,3 +132,14 @@ def test_native_dense_step_matches_the_reference_formulas(kind):
         assert np.allclose(s0, c, rtol=1e-5) and np.allclose(s1, q, rtol=1e-5) and np.allclose(s2, m, rtol=1e-5, atol=1e-6)
         assert np.allclose(w, w0 - lr * m / (np.sqrt(q) / np.sqrt(c) + eps), rtol=1e-5, atol=1e-6)
     assert not g.any()
+
+
+def test_dedup_scratch_holds_every_sign_that_a_batch_may_have():
+    """One GPU: all of a segment, with a third to spare (a full scratch is walked from end to end by every further id).
+    Several GPUs: twice the declared number of distinct signs, as long as there have been such segments."""
+    from tensornet_b200.ops.sparse_table_gpu import dedup_slots, round_up
+
+    for m in list(range(1, 300)) + [4096, 49216, 1 << 20, 4_921_600]:
+        capo = round_up(m + 4, 32)
+        assert dedup_slots(m, capo, 1) * 2 >= capo * 3
+        assert all(dedup_slots(m, capo, w) >= 2 * m + 16 for w in (2, 8))
