@@ -163,18 +163,37 @@ struct SparseCtx {
   // The shard's arrays were replaced (growth, compaction): launches already recorded in CUDA graphs pick the new ones up.
   void set_table(py::dict table) { keep["table"] = table; t = table_from_dict(table); upload_table(); }
 
-  // Dedup, id dispatch and inverse map of a batch ahead of its pull (plain kernels on the current stream).
-  void front(at::Tensor ids, at::Tensor inverse) {
+  // One GPU: the pull is ordinary kernels, and pooling reads the rows where they are (staged returns keep the exchange kernel).
+  bool in_place() const { return c.world == 1 && tile_rows == 0; }
+
+  // `req`: rows of the batch's distinct signs, for a batch whose pull started ahead of its step (in place only)
+  int* req_ptr(const c10::optional<at::Tensor>& req) const {
+    if (!req.has_value()) return c.req_row;
+    TORCH_CHECK(in_place() && req->is_cuda() && req->scalar_type() == at::kInt && req->numel() >= c.capo, "req: int32, one per distinct sign");
+    return ptr_of<int>(*req);
+  }
+  tn::PullArgs pull_args(const at::Tensor& ids, const at::Tensor& inverse, const c10::optional<at::Tensor>& req) const {
     TORCH_CHECK(ids.is_cuda() && ids.scalar_type() == at::kLong && ids.is_contiguous(), "ids: contiguous int64 CUDA tensor");
     TORCH_CHECK(inverse.scalar_type() == at::kInt && inverse.numel() >= ids.numel(), "inverse: int32, one per id");
-    c10::cuda::CUDAGuard guard(ids.device());
     tn::PullArgs a{};
     a.c = c; a.tbl = t; a.opt = o;
+    a.c.req_row = req_ptr(req);
+    a.tbl_dev = reinterpret_cast<const tn::TableView*>(tbl_dev.data_ptr());
     a.ids = ptr_of<const long long>(ids);
     a.n_ids = (int)ids.numel();
     a.inverse = ptr_of<int>(inverse);
+    a.lanes = pull_lanes;
+    return a;
+  }
+
+  // The part of a batch's pull that needs only its ids, ahead of its step (plain kernels on the current stream).
+  void front(at::Tensor ids, at::Tensor inverse, c10::optional<at::Tensor> req) {
+    c10::cuda::CUDAGuard guard(ids.device());
+    tn::PullArgs a = pull_args(ids, inverse, req);
     a.training = 1;
-    check(tn::launch_sparse_pull_front(a, cur_stream()), "sparse_pull_front launch");
+    a.front_done = 1;
+    check(in_place() ? tn::launch_sparse_pull_local_front(a, cur_stream()) : tn::launch_sparse_pull_front(a, cur_stream()),
+          "sparse_pull_front launch");
     g_launches.fetch_add(1, std::memory_order_relaxed);      // two kernels
   }
 
@@ -183,35 +202,49 @@ struct SparseCtx {
     TORCH_CHECK(n_dev->is_cuda() && n_dev->scalar_type() == at::kInt && n_dev->numel() == 1, "n_dev: one int32 on the device");
     return ptr_of<const int>(*n_dev);
   }
+  // `rows`: the pulled rows are wanted in the per-batch matrix (always the case where they are not read in place)
   void pull(at::Tensor ids, at::Tensor inverse, c10::optional<at::Tensor> labels, int label_mod, bool training, bool lookup_only,
-            bool front_done, c10::optional<at::Tensor> n_dev) {
-    TORCH_CHECK(ids.is_cuda() && ids.scalar_type() == at::kLong && ids.is_contiguous(), "ids: contiguous int64 CUDA tensor");
-    TORCH_CHECK(inverse.scalar_type() == at::kInt && inverse.numel() >= ids.numel(), "inverse: int32, one per id");
+            bool front_done, c10::optional<at::Tensor> n_dev, bool rows, c10::optional<at::Tensor> req) {
     c10::cuda::CUDAGuard guard(ids.device());
-    tn::PullArgs a{};
-    a.c = c; a.tbl = t; a.opt = o;
-    a.tbl_dev = reinterpret_cast<const tn::TableView*>(tbl_dev.data_ptr());
-    a.ids = ptr_of<const long long>(ids);
-    a.n_ids = (int)ids.numel();
+    tn::PullArgs a = pull_args(ids, inverse, req);
     a.n_dev = count_ptr(n_dev);
-    a.inverse = ptr_of<int>(inverse);
     a.labels = labels.has_value() ? ptr_of<const float>(*labels) : nullptr;
     a.label_mod = label_mod;
     a.training = training ? 1 : 0;
     a.lookup_only = lookup_only ? 1 : 0;
     TORCH_CHECK(!(training && lookup_only), "a training pull creates rows; lookup_only is for inference");
     a.front_done = front_done ? 1 : 0;
-    a.lanes = pull_lanes;
+    if (in_place()) {
+      check(tn::launch_sparse_pull_local(a, rows, cur_stream()), "sparse_pull_local launch");
+      g_launches.fetch_add((front_done ? 0 : 1) + (rows ? 1 : 0), std::memory_order_relaxed);
+      return;
+    }
     a.tile_rows = tile_rows;
     long long work = (long long)a.n_ids * (pull_lanes > 4 ? pull_lanes / 2 : 2);
     if (work > (1ll << 30)) work = 1ll << 30;
     check(tn::launch_sparse_pull(a, (int)work, cur_stream()), "sparse_pull_fused launch");
   }
 
+  // The rows of the last pull as the pooling kernels are to read them.
+  tn::RowSource source(const c10::optional<at::Tensor>& req) const {
+    tn::RowSource s{};
+    s.U = c.U[c.rank];
+    s.ustride = c.ustride;
+    if (in_place()) {
+      s.row_of = req_ptr(req);
+      s.tbl = reinterpret_cast<const tn::TableView*>(tbl_dev.data_ptr());
+    }
+    s.stride = t.stride;
+    s.dim = t.dim;
+    s.cvm = !t.use_cvm ? 0 : o.kind == tn::kAdaGrad ? 1 : 2;
+    return s;
+  }
+
   // `dense`: the dense step of the same training step (DenseCtx::rider_args), carried by a few CTAs of this launch.
-  void push(int64_t work_hint, int max_ctas, const tn::DenseStepArgs* dense) {
+  void push(int64_t work_hint, int max_ctas, const tn::DenseStepArgs* dense, const c10::optional<at::Tensor>& req) {
     tn::PushArgs a{};
     a.c = c; a.tbl = t; a.opt = o; a.lanes = push_lanes;
+    a.c.req_row = req_ptr(req);
     a.tbl_dev = reinterpret_cast<const tn::TableView*>(tbl_dev.data_ptr());
     long long work = work_hint * push_lanes;
     if (work > (1ll << 30)) work = 1ll << 30;
@@ -598,13 +631,40 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("set_opt", &SparseCtx::set_opt)
       .def("set_table", &SparseCtx::set_table)
       .def("pull", &SparseCtx::pull, py::arg("ids"), py::arg("inverse"), py::arg("labels"), py::arg("label_mod"), py::arg("training"),
-           py::arg("lookup_only") = false, py::arg("front_done") = false, py::arg("n_dev") = py::none())
-      .def("push", [](SparseCtx& self, int64_t work_hint, int max_ctas, py::object dense) {
-        if (dense.is_none()) { self.push(work_hint, max_ctas, nullptr); return; }
+           py::arg("lookup_only") = false, py::arg("front_done") = false, py::arg("n_dev") = py::none(), py::arg("rows") = true,
+           py::arg("req") = py::none())
+      .def("push", [](SparseCtx& self, int64_t work_hint, int max_ctas, py::object dense, c10::optional<at::Tensor> req) {
+        if (dense.is_none()) { self.push(work_hint, max_ctas, nullptr, req); return; }
         const tn::DenseStepArgs d = dense.cast<DenseCtx&>().rider_args();
-        self.push(work_hint, max_ctas, &d);
-      }, py::arg("work_hint"), py::arg("max_ctas") = 0, py::arg("dense") = py::none())
-      .def("front", &SparseCtx::front, py::arg("ids"), py::arg("inverse"));
+        self.push(work_hint, max_ctas, &d, req);
+      }, py::arg("work_hint"), py::arg("max_ctas") = 0, py::arg("dense") = py::none(), py::arg("req") = py::none())
+      .def("front", &SparseCtx::front, py::arg("ids"), py::arg("inverse"), py::arg("req") = py::none())
+      .def("in_place", &SparseCtx::in_place)
+      .def("pool_fwd", [](SparseCtx& self, at::Tensor inverse, c10::optional<at::Tensor> offsets, int B, int S, int combiner, at::Tensor out,
+                          c10::optional<at::Tensor> req) {
+        c10::cuda::CUDAGuard guard(out.device());
+        const int pd = self.t.dim + 2 * self.t.use_cvm;
+        TORCH_CHECK(out.scalar_type() == at::kFloat && out.is_contiguous() && out.numel() == (int64_t)B * S * pd, "pool_fwd: out must be fp32 [B, S * width]");
+        tn::launch_pool_fwd(self.source(req), ptr_of<int>(inverse), offsets ? ptr_of<int>(*offsets) : nullptr, B, S, pd, combiner,
+                            ptr_of<float>(out), S * pd, cur_stream());
+      })
+      .def("seq_fwd", [](SparseCtx& self, at::Tensor inverse, at::Tensor offsets, int B, int T, at::Tensor out, at::Tensor lengths,
+                         c10::optional<at::Tensor> req) {
+        c10::cuda::CUDAGuard guard(out.device());
+        tn::launch_seq_fwd(self.source(req), ptr_of<int>(inverse), ptr_of<int>(offsets), B, T, self.t.dim + 2 * self.t.use_cvm,
+                           ptr_of<float>(out), ptr_of<int>(lengths), cur_stream());
+      })
+      .def("deepfm_input_fwd", [](SparseCtx& self, at::Tensor inverse, int B, int S, int D, c10::optional<at::Tensor> dense, at::Tensor X0,
+                                  at::Tensor fm, int lin_col, c10::optional<at::Tensor> Lout, at::Tensor E, c10::optional<at::Tensor> req) {
+        c10::cuda::CUDAGuard guard(X0.device());
+        const int Dd = dense ? (int)dense->size(1) : 0;
+        TORCH_CHECK(E.scalar_type() == at::kFloat && E.is_contiguous() && E.numel() == (int64_t)B * S * D, "deepfm_input: E must be fp32 [B, S * D]");
+        const char* err = tn::launch_deepfm_input_fwd(self.source(req), ptr_of<int>(inverse), B, S, D, dense ? ptr_of<float>(*dense) : nullptr,
+                                                      Dd, dense ? (int)dense->stride(0) : 0, X0.data_ptr(), (int)X0.stride(0),
+                                                      ptr_of<float>(fm), Lout ? lin_col : -1, Lout ? ptr_of<float>(*Lout) : nullptr,
+                                                      ptr_of<float>(E), cur_stream());
+        if (err) throw std::runtime_error(err);
+      });
   py::class_<ServeCtx>(m, "ServeCtx")
       .def(py::init<py::dict, int, int, std::vector<int>, bool>())
       .def("forward", &ServeCtx::forward);
@@ -774,20 +834,19 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("pool_fwd", [](at::Tensor U, int ustride, at::Tensor inverse, c10::optional<at::Tensor> offsets, int B, int S, int pd,
                        int combiner, at::Tensor out, int out_ld) {
     c10::cuda::CUDAGuard guard(U.device());
-    tn::launch_pool_fwd(ptr_of<float>(U), ustride, ptr_of<int>(inverse), offsets ? ptr_of<int>(*offsets) : nullptr, B, S, pd,
+    TORCH_CHECK(ustride % 4 == 0 && reinterpret_cast<uintptr_t>(U.data_ptr()) % 16 == 0, "pool_fwd: rows of U must be whole 16-byte pieces");
+    tn::RowSource src{};
+    src.U = ptr_of<float>(U);
+    src.ustride = ustride;
+    tn::launch_pool_fwd(src, ptr_of<int>(inverse), offsets ? ptr_of<int>(*offsets) : nullptr, B, S, pd,
                         combiner, ptr_of<float>(out), out_ld, cur_stream());
   });
   m.def("pool_bwd", [](at::Tensor gU, int gstride, at::Tensor inverse, c10::optional<at::Tensor> offsets, int B, int S, int pd,
                        int dim, int combiner, at::Tensor gout, int gout_ld) {
     c10::cuda::CUDAGuard guard(gU.device());
+    TORCH_CHECK(gstride % 4 == 0 && reinterpret_cast<uintptr_t>(gU.data_ptr()) % 16 == 0, "pool_bwd: rows of gU must be whole 16-byte pieces");
     tn::launch_pool_bwd(ptr_of<float>(gU), gstride, ptr_of<int>(inverse), offsets ? ptr_of<int>(*offsets) : nullptr, B, S, pd,
                         dim, combiner, ptr_of<float>(gout), gout_ld, cur_stream());
-  });
-  m.def("seq_fwd", [](at::Tensor U, int ustride, at::Tensor inverse, at::Tensor offsets, int B, int T, int pd, at::Tensor out,
-                      at::Tensor lengths) {
-    c10::cuda::CUDAGuard guard(U.device());
-    tn::launch_seq_fwd(ptr_of<float>(U), ustride, ptr_of<int>(inverse), ptr_of<int>(offsets), B, T, pd, ptr_of<float>(out),
-                       ptr_of<int>(lengths), cur_stream());
   });
   m.def("seq_bwd", [](at::Tensor gU, int gstride, at::Tensor inverse, at::Tensor offsets, int B, int T, int pd, int dim,
                       at::Tensor gout) {
@@ -876,20 +935,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     tn::launch_bce(ptr_of<float>(logit), ptr_of<float>(label), (int)logit.numel(), pred ? ptr_of<float>(*pred) : nullptr,
                    dlogit ? ptr_of<float>(*dlogit) : nullptr, grad_scale, ptr_of<float>(sums), hist_bins(sums), cur_stream());
   });
-  m.def("deepfm_input_fwd", [](at::Tensor U, int ustride, at::Tensor inverse, int B, int S, int D, c10::optional<at::Tensor> dense,
-                               at::Tensor X0, at::Tensor fm, int lin_col, c10::optional<at::Tensor> Lout) {
-    c10::cuda::CUDAGuard guard(U.device());
-    const int Dd = dense ? (int)dense->size(1) : 0;
-    const char* err = tn::launch_deepfm_input_fwd(ptr_of<float>(U), ustride, ptr_of<int>(inverse), B, S, D,
-                                                  dense ? ptr_of<float>(*dense) : nullptr, Dd, dense ? (int)dense->stride(0) : 0,
-                                                  X0.data_ptr(), (int)X0.stride(0), ptr_of<float>(fm), Lout ? lin_col : -1,
-                                                  Lout ? ptr_of<float>(*Lout) : nullptr, cur_stream());
-    if (err) throw std::runtime_error(err);
-  });
-  m.def("deepfm_input_bwd", [](at::Tensor U, int ustride, at::Tensor inverse, int B, int S, int D, at::Tensor dX0, at::Tensor gfm,
+  m.def("deepfm_input_bwd", [](at::Tensor E, at::Tensor inverse, int B, int S, int D, at::Tensor dX0, at::Tensor gfm,
                                at::Tensor gU, int gstride, int lin_col, c10::optional<at::Tensor> dL) {
-    c10::cuda::CUDAGuard guard(U.device());
-    const char* err = tn::launch_deepfm_input_bwd(ptr_of<float>(U), ustride, ptr_of<int>(inverse), B, S, D, dX0.data_ptr(),
+    c10::cuda::CUDAGuard guard(E.device());
+    const char* err = tn::launch_deepfm_input_bwd(ptr_of<float>(E), ptr_of<int>(inverse), B, S, D, dX0.data_ptr(),
                                                   (int)dX0.stride(0), ptr_of<float>(gfm), ptr_of<float>(gU), gstride, dL ? lin_col : -1,
                                                   dL ? ptr_of<float>(*dL) : nullptr, cur_stream());
     if (err) throw std::runtime_error(err);

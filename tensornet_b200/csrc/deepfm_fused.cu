@@ -12,7 +12,7 @@
 //                      dFM, weight gradient) in one kernel - the logit gradient depends on nothing
 //                      but the logit and the label, so forward and backward of the head are one pass.
 #include <cuda_bf16.h>
-#include "tn_device.cuh"
+#include "sparse_table.cuh"
 #include "tn_ops.h"
 
 namespace tn {
@@ -25,11 +25,14 @@ __device__ __forceinline__ float wsum(float v) {
   return v;
 }
 
-// D % 4 == 0, dq = D/4 a power of two <= 32.  One warp per example.
-__global__ void deepfm_input_fwd_kernel(const float* __restrict__ U, int ustride, const int* __restrict__ inverse, int B, int S,
-                                        int D, const float* __restrict__ dense, int Dd, int ld_dense,
-                                        __nv_bfloat16* __restrict__ X0, int ld, float* __restrict__ fm, int lin_col,
-                                        float* __restrict__ Lout) {
+// D % 4 == 0, dq = D/4 a power of two <= 32.  One warp per example.  The rows it has read are left in `E` as they are: the
+// backward pass then reads them as one run per example instead of gathering them once more (and does not depend on
+// what happens to the pulled rows in between).
+template <bool kInPlace>
+__global__ void __launch_bounds__(256, 6) deepfm_input_fwd_kernel(const RowSource src, const int* __restrict__ inverse, int B, int S, int D,
+                                        const float* __restrict__ dense, int Dd, int ld_dense, __nv_bfloat16* __restrict__ X0, int ld,
+                                        float* __restrict__ fm, int lin_col, float* __restrict__ Lout, float* __restrict__ E) {
+  const PulledRows<kInPlace> rows(src);
   pdl_sync();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -39,25 +42,28 @@ __global__ void deepfm_input_fwd_kernel(const float* __restrict__ U, int ustride
     float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
     float sq = 0.f;
     // batches of 4 x 32 chunks: first all row indices, then all row gathers, then the arithmetic, so that a
-    // warp has four independent loads in flight at each of the two dependent steps
+    // warp has four independent loads in flight at each of the dependent steps
     for (int c0 = 0; c0 < nch; c0 += 128) {
-      int v[4];
+      int r[4];
       float4 x[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const int c = c0 + 32 * k + lane;
-        v[k] = c < nch ? __ldg(inverse + (size_t)(c / dq) * B + b) : -1;
+        r[k] = c < nch ? __ldg(inverse + (size_t)(c / dq) * B + b) : -1;
       }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) r[k] = rows.row(r[k]);
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const int c = c0 + 32 * k + lane;
         x[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (v[k] >= 0) x[k] = ldcg_f4(U + (size_t)v[k] * ustride + 4 * (c % dq));
+        if (r[k] >= 0) x[k] = ldcg_f4(rows.base + (size_t)r[k] * rows.stride + 4 * (c % dq));
       }
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const int c = c0 + 32 * k + lane;
         if (c >= nch) continue;
+        *reinterpret_cast<float4*>(E + (size_t)b * S * D + 4 * c) = x[k];
         s.x += x[k].x; s.y += x[k].y; s.z += x[k].z; s.w += x[k].w;
         sq += x[k].x * x[k].x + x[k].y * x[k].y + x[k].z * x[k].z + x[k].w * x[k].w;
         __nv_bfloat162 lo = __floats2bfloat162_rn(x[k].x, x[k].y), hi = __floats2bfloat162_rn(x[k].z, x[k].w);
@@ -73,8 +79,8 @@ __global__ void deepfm_input_fwd_kernel(const float* __restrict__ U, int ustride
     if (lane == 0) fm[b] = 0.5f * part;
     if (lin_col >= 0) {   // the slot's linear weight rides in column `lin_col` of the same row
       for (int f = lane; f < S; f += 32) {
-        const int v = __ldg(inverse + (size_t)f * B + b);
-        Lout[(size_t)b * S + f] = v >= 0 ? __ldcg(U + (size_t)v * ustride + lin_col) : 0.f;
+        const int r = rows.row(__ldg(inverse + (size_t)f * B + b));
+        Lout[(size_t)b * S + f] = r >= 0 ? __ldcg(rows.base + (size_t)r * rows.stride + lin_col) : 0.f;
       }
     }
     const int tail0 = S * D;
@@ -87,8 +93,8 @@ __global__ void deepfm_input_fwd_kernel(const float* __restrict__ U, int ustride
   }
 }
 
-__global__ void deepfm_input_bwd_kernel(const float* __restrict__ U, int ustride, const int* __restrict__ inverse, int B, int S,
-                                        int D, const __nv_bfloat16* __restrict__ dX0, int ld, const float* __restrict__ gfm,
+__global__ void deepfm_input_bwd_kernel(const float* __restrict__ E, const int* __restrict__ inverse, int B, int S, int D,
+                                        const __nv_bfloat16* __restrict__ dX0, int ld, const float* __restrict__ gfm,
                                         float* __restrict__ gU, int gstride, int lin_col, const float* __restrict__ dL) {
   pdl_sync();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
@@ -96,6 +102,7 @@ __global__ void deepfm_input_bwd_kernel(const float* __restrict__ U, int ustride
   const int dq = D >> 2, nch = S * dq;
   for (int b = warp; b < B; b += nwarps) {
     const __nv_bfloat16* grow = dX0 + (size_t)b * ld;
+    const float* e = E + (size_t)b * S * D;
     const float gf = gfm[b];
     float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
     if (nch <= 128) {
@@ -108,12 +115,10 @@ __global__ void deepfm_input_bwd_kernel(const float* __restrict__ U, int ustride
         const int c = 32 * k + lane;
         v[k] = c < nch ? __ldg(inverse + (size_t)(c / dq) * B + b) : -1;
         raw[k] = c < nch ? *reinterpret_cast<const uint2*>(grow + 4 * c) : make_uint2(0u, 0u);
+        x[k] = c < nch ? ldcg_f4(e + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const int c = 32 * k + lane;
-        x[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (v[k] >= 0) x[k] = ldcg_f4(U + (size_t)v[k] * ustride + 4 * (c % dq));
         s.x += x[k].x; s.y += x[k].y; s.z += x[k].z; s.w += x[k].w;
       }
       for (int o = 16; o >= dq; o >>= 1) {
@@ -135,12 +140,8 @@ __global__ void deepfm_input_bwd_kernel(const float* __restrict__ U, int ustride
       }
     } else {
       for (int c = lane; c < nch; c += 32) {
-        const int f = c / dq, dc = c - f * dq;
-        const int v = __ldg(inverse + (size_t)f * B + b);
-        if (v >= 0) {
-          const float4 x = ldcg_f4(U + (size_t)v * ustride + 4 * dc);
-          s.x += x.x; s.y += x.y; s.z += x.z; s.w += x.w;
-        }
+        const float4 x = ldcg_f4(e + 4 * c);
+        s.x += x.x; s.y += x.y; s.z += x.z; s.w += x.w;
       }
       for (int o = 16; o >= dq; o >>= 1) {
         s.x += __shfl_xor_sync(0xffffffffu, s.x, o); s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
@@ -150,7 +151,7 @@ __global__ void deepfm_input_bwd_kernel(const float* __restrict__ U, int ustride
         const int f = c / dq, dc = c - f * dq;
         const int v = __ldg(inverse + (size_t)f * B + b);
         if (v < 0) continue;
-        const float4 x = ldcg_f4(U + (size_t)v * ustride + 4 * dc);
+        const float4 x = ldcg_f4(e + 4 * c);
         const uint2 raw = *reinterpret_cast<const uint2*>(grow + 4 * c);
         const float2 g01 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
         const float2 g23 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
@@ -307,22 +308,22 @@ __global__ void deepfm_head_loss_kernel(const __nv_bfloat16* __restrict__ H, int
 
 }  // namespace
 
-const char* launch_deepfm_input_fwd(const float* U, int ustride, const int* inverse, int B, int S, int D, const float* dense, int Dd,
-                                    int ld_dense, void* X0, int ld, float* fm, int lin_col, float* Lout, cudaStream_t st) {
+const char* launch_deepfm_input_fwd(const RowSource& src, const int* inverse, int B, int S, int D, const float* dense, int Dd, int ld_dense,
+                                    void* X0, int ld, float* fm, int lin_col, float* Lout, float* E, cudaStream_t st) {
   const int dq = D >> 2;
   if ((D & 3) || dq < 1 || dq > 32 || (dq & (dq - 1))) return "deepfm_input: embedding dim must be 4 * 2^k, at most 128";
   if (ld < S * D + Dd + 1 || (ld & 3)) return "deepfm_input: operand row too short";
   int blocks = (B + 7) / 8; if (blocks > 148 * 8) blocks = 148 * 8; if (blocks < 1) blocks = 1;
-  cudaError_t e = launch_pdl(deepfm_input_fwd_kernel, dim3(blocks), dim3(256), 0, st, U, ustride, inverse, B, S, D, dense, Dd, ld_dense,
-                             reinterpret_cast<__nv_bfloat16*>(X0), ld, fm, lin_col, Lout);
+  cudaError_t e = launch_pdl(src.row_of != nullptr ? deepfm_input_fwd_kernel<true> : deepfm_input_fwd_kernel<false>, dim3(blocks), dim3(256), 0,
+                             st, src, inverse, B, S, D, dense, Dd, ld_dense, reinterpret_cast<__nv_bfloat16*>(X0), ld, fm, lin_col, Lout, E);
   return e == cudaSuccess ? nullptr : cudaGetErrorString(e);
 }
-const char* launch_deepfm_input_bwd(const float* U, int ustride, const int* inverse, int B, int S, int D, const void* dX0, int ld,
-                                    const float* gfm, float* gU, int gstride, int lin_col, const float* dL, cudaStream_t st) {
+const char* launch_deepfm_input_bwd(const float* E, const int* inverse, int B, int S, int D, const void* dX0, int ld, const float* gfm,
+                                    float* gU, int gstride, int lin_col, const float* dL, cudaStream_t st) {
   const int dq = D >> 2;
   if ((D & 3) || dq < 1 || dq > 32 || (dq & (dq - 1))) return "deepfm_input: embedding dim must be 4 * 2^k, at most 128";
   int blocks = (B + 7) / 8; if (blocks > 148 * 8) blocks = 148 * 8; if (blocks < 1) blocks = 1;
-  cudaError_t e = launch_pdl(deepfm_input_bwd_kernel, dim3(blocks), dim3(256), 0, st, U, ustride, inverse, B, S, D,
+  cudaError_t e = launch_pdl(deepfm_input_bwd_kernel, dim3(blocks), dim3(256), 0, st, E, inverse, B, S, D,
                              reinterpret_cast<const __nv_bfloat16*>(dX0), ld, gfm, gU, gstride, lin_col, dL);
   return e == cudaSuccess ? nullptr : cudaGetErrorString(e);
 }

@@ -3,7 +3,7 @@
 // safe_embedding_lookup_sparse / sequence lookups that the reference calls on its batch
 // variable (tensornet/layers/embedding_features.py:283-284,
 // tensornet/layers/sequence_embedding_features.py:99-137).
-#include "tn_device.cuh"
+#include "sparse_table.cuh"
 #include "tn_ops.h"
 
 namespace tn {
@@ -17,11 +17,59 @@ __device__ __forceinline__ float bag_scale(int combiner, int len) {
   return 1.f;
 }
 
-// One group of G lanes per bag.  Bag g = s * B + b, its ids are positions
-// [offsets[g], offsets[g+1]) of `inverse` (or exactly position g when offsets == nullptr).
-__global__ void pool_fwd_kernel(const float* __restrict__ U, int ustride, const int* __restrict__ inverse,
-                                const int* __restrict__ offsets, int B, int S, int pd, int combiner,
-                                float* __restrict__ out, int out_ld, int G) {
+// One group of G lanes per bag, a lane moves four columns at a time: rows and gradient rows are whole 16-byte pieces whatever
+// their width, only the pooled columns are written (and their gradient read) SV = 4, 2 or 1 at a time, as their address
+// allows.  Bag g = s * B + b, its ids are positions [offsets[g], offsets[g+1]) of `inverse` (or exactly position g when
+// offsets == nullptr).  Bound by random row reads (or reductions), so a group keeps kPoolFlight of them in flight: that many
+// bags when every bag holds one id, that many ids of a bag otherwise.  Ids of a bag are added in their order, one after
+// the other, whatever the number in flight.
+// 2.1 M single-id bags of 128: forward 399 us with one row at a time, 312 now (326 with the rows read in place, a
+// dependent load more but no copy of the rows beforehand); backward 474 us, 445 now.  0.8 M bags of five ids and 64
+// columns: forward 251 -> 205 us (5.1 to 6.2 TB/s), backward unchanged: the reductions bound it.
+constexpr int kPoolFlight = 4;
+
+template <bool kInPlace, int SV>
+__global__ void __launch_bounds__(256, 6) pool_fwd_single_kernel(const RowSource src, const int* __restrict__ inverse, int B, int S,
+                                                                 int pd, int combiner, float* __restrict__ out, int out_ld, int G) {
+  const PulledRows<kInPlace> rows(src);
+  pdl_sync();
+  const int lane = threadIdx.x % G;
+  const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / G;
+  const int ngroups = (gridDim.x * blockDim.x) / G;
+  const int nbags = B * S;
+  const float sc = bag_scale(combiner, 1);
+  for (long long g0 = gid; g0 < nbags; g0 += (long long)kPoolFlight * ngroups) {
+    int r[kPoolFlight];
+#pragma unroll
+    for (int q = 0; q < kPoolFlight; ++q) {
+      const long long g = g0 + (long long)q * ngroups;
+      r[q] = g < nbags ? __ldg(inverse + g) : -1;
+    }
+#pragma unroll
+    for (int q = 0; q < kPoolFlight; ++q) r[q] = rows.row(r[q]);
+    for (int d = 4 * lane; d < pd; d += 4 * G) {
+      float4 x[kPoolFlight];
+#pragma unroll
+      for (int q = 0; q < kPoolFlight; ++q) {
+        x[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r[q] >= 0) x[q] = rows.load4(r[q], d);
+      }
+#pragma unroll
+      for (int q = 0; q < kPoolFlight; ++q) {
+        const long long g = g0 + (long long)q * ngroups;
+        if (g >= nbags) continue;
+        const int s = (int)g / B, b = (int)g - s * B;
+        store_cols<SV>(out + (size_t)b * out_ld + (size_t)s * pd + d, make_float4(x[q].x * sc, x[q].y * sc, x[q].z * sc, x[q].w * sc), pd - d);
+      }
+    }
+  }
+}
+
+template <bool kInPlace, int SV>
+__global__ void __launch_bounds__(256, 5) pool_fwd_bags_kernel(const RowSource src, const int* __restrict__ inverse,
+                                                               const int* __restrict__ offsets, int B, int S, int pd, int combiner,
+                                                               float* __restrict__ out, int out_ld, int G) {
+  const PulledRows<kInPlace> rows(src);
   pdl_sync();
   const int lane = threadIdx.x % G;
   const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / G;
@@ -29,110 +77,41 @@ __global__ void pool_fwd_kernel(const float* __restrict__ U, int ustride, const 
   const int nbags = B * S;
   for (int g = gid; g < nbags; g += ngroups) {
     const int s = g / B, b = g - s * B;
-    int k0 = g, k1 = g + 1;
-    if (offsets) { k0 = offsets[g]; k1 = offsets[g + 1]; }
-    const float sc = bag_scale(combiner, k1 - k0);
-    float* o = out + (size_t)b * out_ld + (size_t)s * pd;
-    for (int d = lane; d < pd; d += G) {
-      float acc = 0.f;
-      for (int k = k0; k < k1; ++k) {
-        int v = inverse[k];
-        if (v >= 0) acc += __ldcg(U + (size_t)v * ustride + d);
-      }
-      o[d] = acc * sc;
-    }
-  }
-}
-
-// The variants for pd % 4 == 0: every lane moves float4 chunks.  Bound by random row reads (or reductions), so a group of
-// lanes keeps kPoolFlight of them in flight: that many bags when every bag holds one id, that many ids of a bag
-// otherwise.  Ids of a bag are added in their order, one after the other, whatever the number in flight.
-// 2.1 M single-id bags of 128: forward 399 us with one row at a time, 316 now; backward 474 us, 445 now.  0.8 M bags of
-// five ids and 64 columns: forward 251 -> 205 us (5.1 to 6.2 TB/s), backward unchanged: the reductions bound it.
-constexpr int kPoolFlight = 4;
-
-__global__ void __launch_bounds__(256) pool_fwd_single_vec4_kernel(const float* __restrict__ U, int ustride,
-                                                                   const int* __restrict__ inverse, int B, int S, int pd,
-                                                                   int combiner, float* __restrict__ out, int out_ld, int G) {
-  pdl_sync();
-  const int lane = threadIdx.x % G;
-  const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / G;
-  const int ngroups = (gridDim.x * blockDim.x) / G;
-  const int nbags = B * S, nch = pd >> 2;
-  const float sc = bag_scale(combiner, 1);
-  for (long long g0 = gid; g0 < nbags; g0 += (long long)kPoolFlight * ngroups) {
-    int v[kPoolFlight];
-    float* o[kPoolFlight];
-#pragma unroll
-    for (int q = 0; q < kPoolFlight; ++q) {
-      const long long gl = g0 + (long long)q * ngroups;
-      o[q] = nullptr;
-      v[q] = -1;
-      if (gl < nbags) {
-        const int g = (int)gl, s = g / B, b = g - s * B;
-        v[q] = __ldg(inverse + g);
-        o[q] = out + (size_t)b * out_ld + (size_t)s * pd;
-      }
-    }
-    for (int ch = lane; ch < nch; ch += G) {
-      float4 x[kPoolFlight];
-#pragma unroll
-      for (int q = 0; q < kPoolFlight; ++q) {
-        x[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (v[q] >= 0) x[q] = ldcg_f4(U + (size_t)v[q] * ustride + 4 * ch);
-      }
-#pragma unroll
-      for (int q = 0; q < kPoolFlight; ++q) {
-        if (o[q] != nullptr)
-          *reinterpret_cast<float4*>(o[q] + 4 * ch) = make_float4(x[q].x * sc, x[q].y * sc, x[q].z * sc, x[q].w * sc);
-      }
-    }
-  }
-}
-
-__global__ void __launch_bounds__(256) pool_fwd_bags_vec4_kernel(const float* __restrict__ U, int ustride,
-                                                                 const int* __restrict__ inverse, const int* __restrict__ offsets,
-                                                                 int B, int S, int pd, int combiner, float* __restrict__ out,
-                                                                 int out_ld, int G) {
-  pdl_sync();
-  const int lane = threadIdx.x % G;
-  const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / G;
-  const int ngroups = (gridDim.x * blockDim.x) / G;
-  const int nbags = B * S, nch = pd >> 2;
-  for (int g = gid; g < nbags; g += ngroups) {
-    const int s = g / B, b = g - s * B;
     const int k0 = offsets[g], k1 = offsets[g + 1];
     const float sc = bag_scale(combiner, k1 - k0);
     float* o = out + (size_t)b * out_ld + (size_t)s * pd;
-    for (int ch = lane; ch < nch; ch += G) {
+    for (int d = 4 * lane; d < pd; d += 4 * G) {
       float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
       for (int k = k0; k < k1; k += kPoolFlight) {
-        int v[kPoolFlight];
+        int r[kPoolFlight];
         float4 x[kPoolFlight];
 #pragma unroll
-        for (int q = 0; q < kPoolFlight; ++q) v[q] = k + q < k1 ? __ldg(inverse + k + q) : -1;
+        for (int q = 0; q < kPoolFlight; ++q) r[q] = k + q < k1 ? __ldg(inverse + k + q) : -1;
+#pragma unroll
+        for (int q = 0; q < kPoolFlight; ++q) r[q] = rows.row(r[q]);
 #pragma unroll
         for (int q = 0; q < kPoolFlight; ++q)
-          if (v[q] >= 0) x[q] = ldcg_f4(U + (size_t)v[q] * ustride + 4 * ch);
+          if (r[q] >= 0) x[q] = rows.load4(r[q], d);
 #pragma unroll
         for (int q = 0; q < kPoolFlight; ++q)
-          if (v[q] >= 0) { acc.x += x[q].x; acc.y += x[q].y; acc.z += x[q].z; acc.w += x[q].w; }
+          if (r[q] >= 0) { acc.x += x[q].x; acc.y += x[q].y; acc.z += x[q].z; acc.w += x[q].w; }
       }
       acc.x *= sc; acc.y *= sc; acc.z *= sc; acc.w *= sc;
-      *reinterpret_cast<float4*>(o + 4 * ch) = acc;
+      store_cols<SV>(o + d, acc, pd - d);
     }
   }
 }
 
-// dim % 4 == 0 and pd % 4 == 0: vector reductions into the unique-gradient rows.
-__global__ void __launch_bounds__(256) pool_bwd_single_vec4_kernel(float* __restrict__ gU, int gstride,
-                                                                   const int* __restrict__ inverse, int B, int S, int pd, int dim,
-                                                                   int combiner, const float* __restrict__ gout, int gout_ld, int G) {
+// Backward: vector reductions into the unique-gradient rows.  CVM columns (d >= dim) carry no gradient.
+template <int SV>
+__global__ void __launch_bounds__(256) pool_bwd_single_kernel(float* __restrict__ gU, int gstride, const int* __restrict__ inverse,
+                                                              int B, int S, int pd, int dim, int combiner,
+                                                              const float* __restrict__ gout, int gout_ld, int G) {
   pdl_sync();
   const int lane = threadIdx.x % G;
   const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / G;
   const int ngroups = (gridDim.x * blockDim.x) / G;
-  const int nbags = B * S, nch = dim >> 2;
+  const int nbags = B * S;
   const float sc = bag_scale(combiner, 1);
   for (long long g0 = gid; g0 < nbags; g0 += (long long)kPoolFlight * ngroups) {
     int v[kPoolFlight];
@@ -148,51 +127,23 @@ __global__ void __launch_bounds__(256) pool_bwd_single_vec4_kernel(float* __rest
         go[q] = gout + (size_t)b * gout_ld + (size_t)s * pd;
       }
     }
-    for (int ch = lane; ch < nch; ch += G) {
+    for (int d = 4 * lane; d < dim; d += 4 * G) {
       float4 x[kPoolFlight];
 #pragma unroll
       for (int q = 0; q < kPoolFlight; ++q)
-        if (v[q] >= 0) x[q] = *reinterpret_cast<const float4*>(go[q] + 4 * ch);
+        if (v[q] >= 0) x[q] = load_cols<SV>(go[q] + d, dim - d);
 #pragma unroll
       for (int q = 0; q < kPoolFlight; ++q)
         if (v[q] >= 0)
-          red_add_f32x4(gU + (size_t)v[q] * gstride + 4 * ch, make_float4(x[q].x * sc, x[q].y * sc, x[q].z * sc, x[q].w * sc));
+          red_add_cols(gU + (size_t)v[q] * gstride + d, make_float4(x[q].x * sc, x[q].y * sc, x[q].z * sc, x[q].w * sc), dim - d);
     }
   }
 }
 
-__global__ void __launch_bounds__(256) pool_bwd_bags_vec4_kernel(float* __restrict__ gU, int gstride,
-                                                                 const int* __restrict__ inverse, const int* __restrict__ offsets,
-                                                                 int B, int S, int pd, int dim, int combiner,
-                                                                 const float* __restrict__ gout, int gout_ld, int G) {
-  pdl_sync();
-  const int lane = threadIdx.x % G;
-  const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / G;
-  const int ngroups = (gridDim.x * blockDim.x) / G;
-  const int nbags = B * S, nch = dim >> 2;
-  for (int g = gid; g < nbags; g += ngroups) {
-    const int s = g / B, b = g - s * B;
-    const int k0 = offsets[g], k1 = offsets[g + 1];
-    const float sc = bag_scale(combiner, k1 - k0);
-    const float* go = gout + (size_t)b * gout_ld + (size_t)s * pd;
-    for (int ch = lane; ch < nch; ch += G) {
-      float4 x = *reinterpret_cast<const float4*>(go + 4 * ch);
-      x.x *= sc; x.y *= sc; x.z *= sc; x.w *= sc;
-      for (int k = k0; k < k1; k += kPoolFlight) {
-        int v[kPoolFlight];
-#pragma unroll
-        for (int q = 0; q < kPoolFlight; ++q) v[q] = k + q < k1 ? __ldg(inverse + k + q) : -1;
-#pragma unroll
-        for (int q = 0; q < kPoolFlight; ++q)
-          if (v[q] >= 0) red_add_f32x4(gU + (size_t)v[q] * gstride + 4 * ch, x);
-      }
-    }
-  }
-}
-
-__global__ void pool_bwd_kernel(float* __restrict__ gU, int gstride, const int* __restrict__ inverse,
-                                const int* __restrict__ offsets, int B, int S, int pd, int dim, int combiner,
-                                const float* __restrict__ gout, int gout_ld, int G) {
+template <int SV>
+__global__ void __launch_bounds__(256) pool_bwd_bags_kernel(float* __restrict__ gU, int gstride, const int* __restrict__ inverse,
+                                                            const int* __restrict__ offsets, int B, int S, int pd, int dim,
+                                                            int combiner, const float* __restrict__ gout, int gout_ld, int G) {
   pdl_sync();
   const int lane = threadIdx.x % G;
   const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / G;
@@ -200,15 +151,19 @@ __global__ void pool_bwd_kernel(float* __restrict__ gU, int gstride, const int* 
   const int nbags = B * S;
   for (int g = gid; g < nbags; g += ngroups) {
     const int s = g / B, b = g - s * B;
-    int k0 = g, k1 = g + 1;
-    if (offsets) { k0 = offsets[g]; k1 = offsets[g + 1]; }
+    const int k0 = offsets[g], k1 = offsets[g + 1];
     const float sc = bag_scale(combiner, k1 - k0);
     const float* go = gout + (size_t)b * gout_ld + (size_t)s * pd;
-    for (int d = lane; d < dim; d += G) {   // CVM columns (d >= dim) carry no gradient
-      const float x = go[d] * sc;
-      for (int k = k0; k < k1; ++k) {
-        int v = inverse[k];
-        if (v >= 0) atomicAdd(gU + (size_t)v * gstride + d, x);
+    for (int d = 4 * lane; d < dim; d += 4 * G) {
+      float4 x = load_cols<SV>(go + d, dim - d);
+      x.x *= sc; x.y *= sc; x.z *= sc; x.w *= sc;
+      for (int k = k0; k < k1; k += kPoolFlight) {
+        int v[kPoolFlight];
+#pragma unroll
+        for (int q = 0; q < kPoolFlight; ++q) v[q] = k + q < k1 ? __ldg(inverse + k + q) : -1;
+#pragma unroll
+        for (int q = 0; q < kPoolFlight; ++q)
+          if (v[q] >= 0) red_add_cols(gU + (size_t)v[q] * gstride + d, x, dim - d);
       }
     }
   }
@@ -216,9 +171,10 @@ __global__ void pool_bwd_kernel(float* __restrict__ gU, int gstride, const int* 
 
 // Sequence gather of one column: element t of example b -> out[b, t, :]; t >= T is dropped,
 // positions past the length stay zero (caller zero-fills).  lengths[b] = min(len, T).
-__global__ void seq_fwd_kernel(const float* __restrict__ U, int ustride, const int* __restrict__ inverse,
-                               const int* __restrict__ offsets, int B, int T, int pd, float* __restrict__ out,
-                               int* __restrict__ lengths, int G) {
+template <bool kInPlace>
+__global__ void seq_fwd_kernel(const RowSource src, const int* __restrict__ inverse, const int* __restrict__ offsets, int B, int T,
+                               int pd, float* __restrict__ out, int* __restrict__ lengths, int G) {
+  const PulledRows<kInPlace> rows(src);
   pdl_sync();
   const int lane = threadIdx.x % G;
   const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / G;
@@ -228,9 +184,10 @@ __global__ void seq_fwd_kernel(const float* __restrict__ U, int ustride, const i
     const int k0 = offsets[b], len = offsets[b + 1] - k0;
     if (tt == 0 && lane == 0 && lengths) lengths[b] = len < T ? len : T;
     if (tt >= len) continue;
-    const int v = inverse[k0 + tt];
+    const int r = rows.row(inverse[k0 + tt]);
     float* o = out + ((size_t)b * T + tt) * pd;
-    for (int d = lane; d < pd; d += G) o[d] = v >= 0 ? __ldcg(U + (size_t)v * ustride + d) : 0.f;
+    for (int d = 4 * lane; d < pd; d += 4 * G)
+      store_cols<1>(o + d, r >= 0 ? rows.load4(r, d) : make_float4(0.f, 0.f, 0.f, 0.f), pd - d);
   }
 }
 
@@ -317,43 +274,60 @@ void launch_pack_columns(const PackColumns& a, cudaStream_t st) {
   pack_columns_kernel<<<dim3(bx < 1 ? 1 : bx, a.n), 256, 0, st>>>(a);
 }
 
-void launch_pool_fwd(const float* U, int ustride, const int* inverse, const int* offsets, int B, int S, int pd,
-                     int combiner, float* out, int out_ld, cudaStream_t st) {
-  if ((pd & 3) == 0 && (out_ld & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
-    const int G = lanes_for_width(pd);
-    if (offsets == nullptr)
-      launch_pdl(pool_fwd_single_vec4_kernel, dim3(grid_for(single_groups((long long)B * S, G), G, 256)), dim3(256), 0, st, U, ustride,
-                 inverse, B, S, pd, combiner, out, out_ld, G);
-    else
-      launch_pdl(pool_fwd_bags_vec4_kernel, dim3(grid_for((long long)B * S, G, 256)), dim3(256), 0, st, U, ustride, inverse, offsets, B, S,
-                 pd, combiner, out, out_ld, G);
-    return;
+// Columns that move at a time where bags lie in memory next to each other: 4, 2 or 1.
+static int cols_at_once(int pd, int ld, const void* p) {
+  const int all = pd | ld;
+  const uintptr_t at = reinterpret_cast<uintptr_t>(p);
+  return (all & 3) == 0 && (at & 15) == 0 ? 4 : (all & 1) == 0 && (at & 7) == 0 ? 2 : 1;
+}
+
+template <bool kInPlace, int SV>
+static void pool_fwd(const RowSource& src, const int* inverse, const int* offsets, int B, int S, int pd, int combiner, float* out,
+                     int out_ld, cudaStream_t st) {
+  const int G = lanes_for_width(pd);
+  const long long bags = (long long)B * S;
+  if (offsets == nullptr)
+    launch_pdl(pool_fwd_single_kernel<kInPlace, SV>, dim3(grid_for(single_groups(bags, G), G, 256)), dim3(256), 0, st, src, inverse, B, S,
+               pd, combiner, out, out_ld, G);
+  else
+    launch_pdl(pool_fwd_bags_kernel<kInPlace, SV>, dim3(grid_for(bags, G, 256)), dim3(256), 0, st, src, inverse, offsets, B, S, pd,
+               combiner, out, out_ld, G);
+}
+void launch_pool_fwd(const RowSource& src, const int* inverse, const int* offsets, int B, int S, int pd, int combiner, float* out,
+                     int out_ld, cudaStream_t st) {
+  const bool in_place = src.row_of != nullptr;
+  switch (cols_at_once(pd, out_ld, out)) {
+    case 4: (in_place ? pool_fwd<true, 4> : pool_fwd<false, 4>)(src, inverse, offsets, B, S, pd, combiner, out, out_ld, st); break;
+    case 2: (in_place ? pool_fwd<true, 2> : pool_fwd<false, 2>)(src, inverse, offsets, B, S, pd, combiner, out, out_ld, st); break;
+    default: (in_place ? pool_fwd<true, 1> : pool_fwd<false, 1>)(src, inverse, offsets, B, S, pd, combiner, out, out_ld, st);
   }
-  int G = pd >= 32 ? 32 : (pd >= 16 ? 16 : (pd >= 8 ? 8 : (pd >= 4 ? 4 : (pd >= 2 ? 2 : 1))));
-  launch_pdl(pool_fwd_kernel, dim3(grid_for((long long)B * S, G, 256)), dim3(256), 0, st, U, ustride, inverse, offsets, B, S, pd, combiner,
-                                                                        out, out_ld, G);
+}
+
+template <int SV>
+static void pool_bwd(float* gU, int gstride, const int* inverse, const int* offsets, int B, int S, int pd, int dim, int combiner,
+                     const float* gout, int gout_ld, cudaStream_t st) {
+  const int G = lanes_for_width(dim);
+  const long long bags = (long long)B * S;
+  if (offsets == nullptr)
+    launch_pdl(pool_bwd_single_kernel<SV>, dim3(grid_for(single_groups(bags, G), G, 256)), dim3(256), 0, st, gU, gstride, inverse, B, S, pd,
+               dim, combiner, gout, gout_ld, G);
+  else
+    launch_pdl(pool_bwd_bags_kernel<SV>, dim3(grid_for(bags, G, 256)), dim3(256), 0, st, gU, gstride, inverse, offsets, B, S, pd, dim,
+               combiner, gout, gout_ld, G);
 }
 void launch_pool_bwd(float* gU, int gstride, const int* inverse, const int* offsets, int B, int S, int pd, int dim,
                      int combiner, const float* gout, int gout_ld, cudaStream_t st) {
-  if ((pd & 3) == 0 && (dim & 3) == 0 && (gout_ld & 3) == 0 && (reinterpret_cast<uintptr_t>(gout) & 15) == 0) {
-    const int G = lanes_for_width(dim);
-    if (offsets == nullptr)
-      launch_pdl(pool_bwd_single_vec4_kernel, dim3(grid_for(single_groups((long long)B * S, G), G, 256)), dim3(256), 0, st, gU, gstride,
-                 inverse, B, S, pd, dim, combiner, gout, gout_ld, G);
-    else
-      launch_pdl(pool_bwd_bags_vec4_kernel, dim3(grid_for((long long)B * S, G, 256)), dim3(256), 0, st, gU, gstride, inverse, offsets, B,
-                 S, pd, dim, combiner, gout, gout_ld, G);
-    return;
+  switch (cols_at_once(pd, gout_ld, gout)) {
+    case 4: pool_bwd<4>(gU, gstride, inverse, offsets, B, S, pd, dim, combiner, gout, gout_ld, st); break;
+    case 2: pool_bwd<2>(gU, gstride, inverse, offsets, B, S, pd, dim, combiner, gout, gout_ld, st); break;
+    default: pool_bwd<1>(gU, gstride, inverse, offsets, B, S, pd, dim, combiner, gout, gout_ld, st);
   }
-  int G = dim >= 32 ? 32 : (dim >= 16 ? 16 : (dim >= 8 ? 8 : (dim >= 4 ? 4 : (dim >= 2 ? 2 : 1))));
-  launch_pdl(pool_bwd_kernel, dim3(grid_for((long long)B * S, G, 256)), dim3(256), 0, st, gU, gstride, inverse, offsets, B, S, pd, dim,
-                                                                        combiner, gout, gout_ld, G);
 }
-void launch_seq_fwd(const float* U, int ustride, const int* inverse, const int* offsets, int B, int T, int pd,
-                    float* out, int* lengths, cudaStream_t st) {
-  int G = pd >= 32 ? 32 : (pd >= 16 ? 16 : (pd >= 8 ? 8 : (pd >= 4 ? 4 : (pd >= 2 ? 2 : 1))));
-  launch_pdl(seq_fwd_kernel, dim3(grid_for((long long)B * T, G, 256)), dim3(256), 0, st, U, ustride, inverse, offsets, B, T, pd, out,
-                                                                       lengths, G);
+void launch_seq_fwd(const RowSource& src, const int* inverse, const int* offsets, int B, int T, int pd, float* out, int* lengths,
+                    cudaStream_t st) {
+  const int G = lanes_for_width(pd);
+  launch_pdl(src.row_of != nullptr ? seq_fwd_kernel<true> : seq_fwd_kernel<false>, dim3(grid_for((long long)B * T, G, 256)), dim3(256), 0, st,
+             src, inverse, offsets, B, T, pd, out, lengths, G);
 }
 void launch_seq_bwd(float* gU, int gstride, const int* inverse, const int* offsets, int B, int T, int pd, int dim,
                     const float* gout, cudaStream_t st) {

@@ -76,15 +76,25 @@ __device__ __forceinline__ int dedup_ids_per_lane(int n_ids, int nth) {
 // First occurrence of a sign allocates a position in its owner's segment.  The slot of the dedup table that holds an
 // id's sign is left in inverse[] as -2 - slot (negative: "no row" to every reader until dedup_resolve has run), so
 // that the second pass is one load per id instead of another probe: 65 -> 31 us for 2.1 M ids.
-__device__ __forceinline__ void dedup_assign(const PullArgs& a, int n_ids, int tid, int nth) {
+// kLocal (one GPU): whoever allocates a position also looks the sign up in the table `t` and leaves its row in
+// req_row[position]; positions of signs that have no row yet are listed in req_ou[0 .. *ocount).  The table is only read.
+// A warp waits for the longest of its chains of dependent accesses, so a lane with one id saves what it can of them: it
+// goes to the dedup table with a compare-and-swap at once (in a large batch the later occurrences of a hot sign had better
+// find it without queueing an atomic on the same word) and asks for the sign's home slot in the table meanwhile: 10 K ids
+// 16.7 -> 13.0 us, but 2.1 M ids, four to a lane, 126 -> 149 us.
+template <bool kLocal>
+__device__ __forceinline__ void dedup_assign(const PullArgs& a, const TableView& t, int n_ids, int tid, int nth) {
   const SparseCommView& c = a.c;
-  const int lane = threadIdx.x & 31, W = c.world, capo = c.capo;
+  const int lane = threadIdx.x & 31, W = kLocal ? 1 : c.world, capo = c.capo;
   const int per = dedup_ids_per_lane(n_ids, nth);
+  const bool early = kLocal && per == 1;
   for (long long base = (long long)(tid - lane) * per; base < n_ids; base += (long long)nth * per) {
     unsigned long long key[kDedupIds], old[kDedupIds];
     unsigned hw[kDedupIds];
     unsigned lead = 0, win = 0;              // bit k: this lane probes for / allocates its k-th id
     int from[kDedupIds];
+    unsigned long long tkey[kDedupIds];      // kLocal: the table slot a new sign has got to, and its row
+    int trow[kDedupIds];
 #pragma unroll
     for (int k = 0; k < kDedupIds; ++k) {
       const long long i = base + 32 * k + lane;
@@ -98,25 +108,51 @@ __device__ __forceinline__ void dedup_assign(const PullArgs& a, int n_ids, int t
       hw[k] = (unsigned)mix64(key[k] ^ 0x2545F4914F6CDD1Dull) & c.dd_mask;
       if (key[k] != kEmptyKey && lane == from[k]) {
         lead |= 1u << k;
+        old[k] = early ? atomicCAS(&c.dd_keys[hw[k]], kEmptyKey, key[k]) : __ldcg(&c.dd_keys[hw[k]]);
+        if (early) {
+          const unsigned h = table_home(t, key[k]);
+          tkey[k] = __ldcg(&t.keys[h]);
+          trow[k] = __ldcg(&t.slots[h]);
+        }
+      }
+    }
+    if (early && (lead & 1u) && old[0] == kEmptyKey) { win = 1u; old[0] = key[0]; }
+    // Rounds: all of the lane's ids that are still on their way take a step side by side.  One that stands before an empty
+    // slot takes it with a compare-and-swap, one that has met another sign moves on to the next slot.
+    unsigned todo = lead;
+    for (unsigned probes = 0; todo != 0; ++probes) {
+      unsigned tried = 0;
+#pragma unroll
+      for (int k = 0; k < kDedupIds; ++k) {
+        if (!((todo >> k) & 1u) || old[k] != kEmptyKey) continue;
+        old[k] = atomicCAS(&c.dd_keys[hw[k]], kEmptyKey, key[k]);
+        tried |= 1u << k;
+      }
+#pragma unroll
+      for (int k = 0; k < kDedupIds; ++k) {
+        if (!((todo >> k) & 1u)) continue;
+        if (((tried >> k) & 1u) && old[k] == kEmptyKey) { win |= 1u << k; todo &= ~(1u << k); continue; }
+        if (old[k] == key[k]) { todo &= ~(1u << k); continue; }
+        hw[k] = (hw[k] + 1) & c.dd_mask;
         old[k] = __ldcg(&c.dd_keys[hw[k]]);
       }
-    }
+      if (todo != 0 && probes > c.dd_mask) {
+        set_status(c.status, kDedupOverflow, 1, 0);
 #pragma unroll
-    for (int k = 0; k < kDedupIds; ++k) {
-      if (k >= per || !((lead >> k) & 1u)) continue;
-      bool done = false;
-      unsigned long long o = old[k];
-      for (unsigned probes = 0; probes <= c.dd_mask; ++probes) {
-        // read first: later occurrences of a hot sign find it without queueing an atomic on the same word
-        if (o == kEmptyKey) o = atomicCAS(&c.dd_keys[hw[k]], kEmptyKey, key[k]);
-        if (o == kEmptyKey) { win |= 1u << k; done = true; break; }
-        if (o == key[k]) { done = true; break; }
-        hw[k] = (hw[k] + 1) & c.dd_mask;
-        o = __ldcg(&c.dd_keys[hw[k]]);
+        for (int k = 0; k < kDedupIds; ++k) if ((todo >> k) & 1u) hw[k] = 0xffffffffu;
+        break;
       }
-      if (!done) { set_status(c.status, kDedupOverflow, 1, 0); hw[k] = 0xffffffffu; }
     }
     __syncwarp();
+    if (kLocal && !early) {                  // the home slots of the new signs, while their positions are handed out
+#pragma unroll
+      for (int k = 0; k < kDedupIds; ++k) {
+        if (!((win >> k) & 1u)) continue;
+        const unsigned h = table_home(t, key[k]);
+        tkey[k] = __ldcg(&t.keys[h]);
+        trow[k] = __ldcg(&t.slots[h]);
+      }
+    }
     int pos0 = 0;                            // one owner: positions of all the warp's winners in one go
     if (W == 1) {
       int total = 0;
@@ -125,6 +161,19 @@ __device__ __forceinline__ void dedup_assign(const PullArgs& a, int n_ids, int t
       if (total > 0) {
         if (lane == 0) pos0 = atomicAdd(&c.cnt[0], total);
         pos0 = __shfl_sync(0xffffffffu, pos0, 0);
+      }
+    }
+    if (kLocal) {                            // walk on from home slots that hold another sign, in rounds as well
+      unsigned walk = win;
+      for (unsigned probes = 1; walk != 0 && probes <= t.cap_mask; ++probes) {
+#pragma unroll
+        for (int k = 0; k < kDedupIds; ++k) {
+          if (!((walk >> k) & 1u)) continue;
+          if (tkey[k] == key[k] || tkey[k] == kEmptyKey) { walk &= ~(1u << k); continue; }
+          const unsigned h = (table_home(t, key[k]) + probes) & t.cap_mask;
+          tkey[k] = __ldcg(&t.keys[h]);
+          trow[k] = __ldcg(&t.slots[h]);
+        }
       }
     }
 #pragma unroll
@@ -147,6 +196,7 @@ __device__ __forceinline__ void dedup_assign(const PullArgs& a, int n_ids, int t
           pos = b + __popc(peers & lanemask_lt());
         }
       }
+      bool missing = false;
       if (winner) {
         if (pos >= capo) {
           set_status(c.status, kOwnerSegOverflow, 1, owner);
@@ -154,7 +204,16 @@ __device__ __forceinline__ void dedup_assign(const PullArgs& a, int n_ids, int t
         } else {
           c.stage_ids[owner * capo + pos] = key[k];
           c.dd_vals[hw[k]] = owner * capo + pos;
+          if (kLocal) {
+            missing = tkey[k] != key[k] && !a.lookup_only;
+            c.req_row[pos] = tkey[k] == key[k] && trow[k] >= 0 ? trow[k] : kReqNone;
+          }
         }
+      }
+      if (kLocal) {
+        const unsigned mm = __ballot_sync(0xffffffffu, missing);
+        const int at = warp_alloc(c.ocount, mm);
+        if (missing) c.req_ou[at] = pos;
       }
       __syncwarp();
       const unsigned slot = __shfl_sync(0xffffffffu, hw[k], from[k]);
@@ -192,6 +251,23 @@ __device__ __forceinline__ void dedup_resolve(const PullArgs& a, int n_ids, int 
         const float y = a.label_mod > 0 ? a.labels[i % a.label_mod] : a.labels[i];
         if (y != 0.f) atomicAdd(rec + 1, y);
       }
+    }
+  }
+}
+
+// Show / click counts of a batch whose inverse map is complete.
+__device__ __forceinline__ void count_shows(const PullArgs& a, int n_ids, int tid, int nth) {
+  const int lane = threadIdx.x & 31;
+  for (int base = tid - lane; base < n_ids; base += nth) {
+    const int i = base + lane;
+    const int v = i < n_ids ? a.inverse[i] : -1;
+    const unsigned same = __match_any_sync(0xffffffffu, v >= 0 ? v : -2 - lane);
+    if (v < 0) continue;
+    float* rec = a.c.cnts + 2 * (size_t)v;
+    if (lane == __ffs(same) - 1) atomicAdd(rec, (float)__popc(same));
+    if (a.labels != nullptr) {
+      const float y = a.label_mod > 0 ? a.labels[i % a.label_mod] : a.labels[i];
+      if (y != 0.f) atomicAdd(rec + 1, y);
     }
   }
 }
@@ -323,27 +399,12 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_pull_fused_kernel(const __
   if (front_done) {
     // show / click counts of the batch into the gradient records (the front runs while the previous step's records
     // are still in use, so it leaves them alone)
-    if (a.training) {
-      for (int base = tid - lane; base < n_ids; base += nth) {
-        const int i = base + lane;
-        const bool valid = i < n_ids;
-        const int v = valid ? a.inverse[i] : -1;
-        const unsigned same = __match_any_sync(0xffffffffu, (valid && v >= 0) ? v : -2 - lane);
-        if (valid && v >= 0) {
-          float* rec = c.cnts + 2 * (size_t)v;
-          if (lane == __ffs(same) - 1) atomicAdd(rec, (float)__popc(same));
-          if (a.labels != nullptr) {
-            float y = a.label_mod > 0 ? a.labels[i % a.label_mod] : a.labels[i];
-            if (y != 0.f) atomicAdd(rec + 1, y);
-          }
-        }
-      }
-    }
+    if (a.training) count_shows(a, n_ids, tid, nth);
     prof_mark(c, 1);
     prof_mark(c, 2);
   } else {
   // ---- phase A: dedup; first occurrence of a sign allocates a slot in its owner's segment --------
-  dedup_assign(a, n_ids, tid, nth);
+  dedup_assign<false>(a, t, n_ids, tid, nth);
   if (!gs.sync(1, false)) goto done;
   prof_mark(c, 1);
 
@@ -641,7 +702,7 @@ __global__ void __launch_bounds__(kFrontThreads) pull_front_dedup_kernel(const _
   const int nth = gridDim.x * blockDim.x;
   const int n_ids = a.n_ids;
   if (c.prof != nullptr && tid == 0) c.prof[16] = globaltimer_ns();
-  dedup_assign(a, n_ids, tid, nth);
+  dedup_assign<false>(a, a.tbl, n_ids, tid, nth);
   if (c.prof != nullptr && threadIdx.x == 0) atomicMax(&c.prof[17], globaltimer_ns());      // last CTA's end
 }
 
@@ -679,6 +740,160 @@ __global__ void __launch_bounds__(kFrontThreads) pull_front_ship_kernel(const __
   }
   dedup_resolve(a, n_ids, tid, nth, false);
   if (c.prof != nullptr && threadIdx.x == 0) atomicMax(&c.prof[18], globaltimer_ns());      // last CTA's end
+}
+
+// =======================================================================================
+// One GPU: nothing is exchanged, so a pull is two ordinary kernels and leaves the rows where they are.  The first one
+// deduplicates the batch and looks every distinct sign up; the second one turns dedup slots into positions, counts shows
+// and clicks, gives signs that have no row yet their row and puts the scratch back.  Pooling then reads the table's rows
+// through req_row (RowSource), so no row is copied into a per-batch matrix and read from there again.  As one
+// cooperative kernel that writes the rows out, a pull cost a grid barrier per phase and the copy.  Bound by the latency of
+// dependent accesses, for large batches by random sectors.  Pull (and pooling) before and now, us: 10 K ids 33 (2.4) and
+// 8.0 + 4.7 (3.0); 64 K ids 31 (3.4) and 8.5 + 5.7 (3.7); 213 K ids 51 (9) and 24 + 6 (11); 2.1 M ids with rows of 128
+// floats 420 (312) and 126 + 40 (326).
+// Ahead of its step (pull_local_probe_kernel, pull_local_resolve_kernel on a second stream) the table's index is only
+// read; what the step itself still runs is the second kernel without its first part.
+// =======================================================================================
+constexpr int kLocalThreads = 256;
+
+__global__ void __launch_bounds__(kLocalThreads, 4) pull_local_probe_kernel(const __grid_constant__ PullArgs a) {
+  const TableView t = *a.tbl_dev;         // (changes between steps only: safe to read before the kernel ahead has finished)
+  pdl_sync();
+  const SparseCommView& c = a.c;
+  const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
+  const int n_ids = batch_ids(a);
+  if (c.prof != nullptr && tid == 0) c.prof[a.front_done ? 16 : 0] = globaltimer_ns();
+  if (ld_volatile_s32(c.status) != 0) {   // an earlier error has not been dealt with: no id has a row
+    for (int i = tid; i < n_ids; i += nth) a.inverse[i] = -1;
+    return;
+  }
+  dedup_assign<true>(a, t, n_ids, tid, nth);
+  if (c.prof != nullptr && threadIdx.x == 0) atomicMax(&c.prof[a.front_done ? 17 : 1], globaltimer_ns());      // last CTA's end
+}
+
+__device__ __forceinline__ void clear_dedup_keys(const SparseCommView& c, int tid, int nth) {
+  ulonglong2* kk = reinterpret_cast<ulonglong2*>(c.dd_keys);
+  const int n2 = (int)((c.dd_mask + 1u) >> 1);
+  for (int i = tid; i < n2; i += nth) kk[i] = make_ulonglong2(kEmptyKey, kEmptyKey);
+}
+
+// Second half of a front: positions, and the dedup keys (which only the first kernel reads) back to empty.
+__global__ void __launch_bounds__(kLocalThreads) pull_local_resolve_kernel(const __grid_constant__ PullArgs a) {
+  pdl_sync();
+  const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
+  dedup_resolve(a, batch_ids(a), tid, nth, false);
+  clear_dedup_keys(a.c, tid, nth);
+  if (a.c.prof != nullptr && threadIdx.x == 0) atomicMax(&a.c.prof[18], globaltimer_ns());
+}
+
+__global__ void __launch_bounds__(kLocalThreads) pull_local_finish_kernel(const __grid_constant__ PullArgs a) {
+  const TableView t = *a.tbl_dev;
+  pdl_sync();
+  const SparseCommView& c = a.c;
+  __shared__ int s_bad, s_new;
+  const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
+  const int lane = threadIdx.x & 31;
+  if (a.front_done) { prof_mark(c, 0); prof_mark(c, 1); }
+  prof_mark(c, 2);
+  if (threadIdx.x == 0) {
+    s_bad = ld_volatile_s32(c.status);
+    s_new = __ldcg(c.ocount);
+  }
+  __syncthreads();
+  const bool bad = s_bad != 0;            // (the state this CTA started in: what it sets itself comes later)
+  const int n_new = s_new;
+  if (threadIdx.x == 0) {
+    // the CTA that is the last to have read the counters leaves them ready for the next pull: no tail at the end
+    __threadfence();
+    if (atomicAdd(&c.bar[3], 1u) == gridDim.x - 1) {
+      c.cnt_saved[0] = bad ? 0 : min(__ldcg(&c.cnt[0]), c.capo);
+      c.cnt[0] = 0;
+      *c.ocount = 0;
+      c.bar[3] = 0;
+      *c.epoch = __ldcg(c.epoch) + 1ull;
+    }
+  }
+  if (!bad) {
+    const int n_ids = batch_ids(a);
+    if (!a.front_done) {
+      dedup_resolve(a, n_ids, tid, nth, a.training != 0);
+      clear_dedup_keys(c, tid, nth);
+    } else if (a.training) {
+      count_shows(a, n_ids, tid, nth);
+    }
+    // new rows, 32 to a warp: the keys are distinct and nobody else inserts, so a lane never meets its own key half done
+    const int G = a.lanes, gl = threadIdx.x % G, sub = lane / G, rpp = 32 / G;
+    for (int base = tid - lane; base < n_new; base += nth) {
+      const int m = base + lane;
+      int pos = -1, r = kReqNone;
+      unsigned long long key = kEmptyKey;
+      unsigned h = 0;
+      bool placed = m >= n_new, is_new = false;
+      if (!placed) {
+        pos = __ldcg(&c.req_ou[m]);
+        key = __ldcg(&c.stage_ids[pos]);
+        h = table_home(t, key);
+        for (unsigned probes = 0; probes <= t.cap_mask; ++probes) {
+          unsigned long long k = __ldcg(&t.keys[h]);
+          if (k == kEmptyKey) {
+            k = atomicCAS(&t.keys[h], kEmptyKey, key);
+            if (k == kEmptyKey) { is_new = placed = true; break; }
+          }
+          if (k == key) { r = ld_volatile_s32(&t.slots[h]); placed = true; break; }     // inserted since it was looked up
+          h = (h + 1) & t.cap_mask;
+        }
+        if (!placed) set_status(c.status, kTableFull, 3, 0);
+      }
+      __syncwarp();
+      const int r_new = warp_alloc(t.n_rows, __ballot_sync(0xffffffffu, is_new));
+      if (is_new) {
+        if (r_new >= t.row_cap) {
+          atomicSub(t.n_rows, 1);
+          set_status(c.status, kTableFull, 3, 0);
+          t.slots[h] = -3;
+          is_new = false;
+        } else {
+          t.row_keys[r_new] = key;
+          t.slots[h] = r_new;
+          r = r_new;
+        }
+      }
+      if (pos >= 0) c.req_row[pos] = r >= 0 ? r : kReqNone;
+      unsigned left = __ballot_sync(0xffffffffu, is_new);
+      while (left != 0) {                  // the warp's groups write one new row each
+        unsigned rest = left;
+        for (int k = 0; k < sub; ++k) rest &= rest - 1;
+        const int from = rest != 0 ? __ffs(rest) - 1 : 0;
+        const int r_s = __shfl_sync(0xffffffffu, r, from);
+        const unsigned long long key_s = __shfl_sync(0xffffffffu, key, from);
+        if (rest != 0) {
+          float* row = t.rows + (size_t)r_s * t.stride;
+          for (int ch = gl; ch < (t.stride >> 2); ch += G)
+            *reinterpret_cast<float4*>(row + 4 * ch) =
+                make_float4(new_row_elem(a.opt, key_s, 4 * ch, t.dim), new_row_elem(a.opt, key_s, 4 * ch + 1, t.dim),
+                            new_row_elem(a.opt, key_s, 4 * ch + 2, t.dim), new_row_elem(a.opt, key_s, 4 * ch + 3, t.dim));
+        }
+        for (int k = 0; k < rpp; ++k) left &= left - 1;
+      }
+    }
+  }
+  if (c.prof != nullptr && threadIdx.x == 0) {
+    const unsigned long long now = globaltimer_ns();
+    atomicMax(&c.prof[3], now); atomicMax(&c.prof[4], now); atomicMax(&c.prof[5], now);
+  }
+}
+
+// The rows of the distinct signs of the last pull into the per-batch matrix, for callers that ask for it.
+__global__ void __launch_bounds__(kLocalThreads) pull_local_rows_kernel(const __grid_constant__ PullArgs a) {
+  pdl_sync();
+  const SparseCommView& c = a.c;
+  __shared__ TableView s_tbl;
+  if (threadIdx.x == 0) s_tbl = *a.tbl_dev;
+  __syncthreads();
+  const int G = a.lanes, gl = threadIdx.x % G;
+  const int n = __ldcg(&c.cnt_saved[0]);
+  for (int j = (blockIdx.x * blockDim.x + threadIdx.x) / G; j < n; j += gridDim.x * blockDim.x / G)
+    pull_return_row(a, s_tbl, __ldcg(&c.req_row[j]), 0ull, c.U[0] + (size_t)j * c.ustride, gl, G);
 }
 
 // =======================================================================================
@@ -1175,6 +1390,31 @@ static int coop_grid(const void* fn, int device) {
   if (per_sm < 1) per_sm = 1;
   if (per_sm > 1) per_sm = 1;
   return per_sm * sms;
+}
+
+// A thread per id up to what the chip holds at once; kernels that also clear the dedup keys have a thread per 16 of them.
+static int local_grid(const PullArgs& args, bool clears) {
+  long long work = args.n_ids;
+  if (clears && ((long long)args.c.dd_mask + 1) / 16 > work) work = ((long long)args.c.dd_mask + 1) / 16;
+  const long long blocks = (work + kLocalThreads - 1) / kLocalThreads;
+  return blocks < 1 ? 1 : (int)(blocks > 148ll * 4 ? 148ll * 4 : blocks);
+}
+
+// One GPU, rows left in the table (see pull_local_probe_kernel).  `rows`: also written out to the per-batch matrix.
+cudaError_t launch_sparse_pull_local(const PullArgs& args, bool rows, cudaStream_t stream) {
+  const dim3 block(kLocalThreads);
+  cudaError_t e = cudaSuccess;
+  if (!args.front_done) e = launch_pdl(pull_local_probe_kernel, dim3(local_grid(args, false)), block, 0, stream, args);
+  if (e == cudaSuccess) e = launch_pdl(pull_local_finish_kernel, dim3(local_grid(args, !args.front_done)), block, 0, stream, args);
+  if (e != cudaSuccess || !rows) return e;
+  const long long want = ((long long)args.n_ids * args.lanes + kLocalThreads - 1) / kLocalThreads;
+  return launch_pdl(pull_local_rows_kernel, dim3(want > 148 * 8 ? 148 * 8 : want < 1 ? 1 : (int)want), block, 0, stream, args);
+}
+
+cudaError_t launch_sparse_pull_local_front(const PullArgs& args, cudaStream_t stream) {
+  const dim3 block(kLocalThreads);
+  const cudaError_t e = launch_pdl(pull_local_probe_kernel, dim3(local_grid(args, false)), block, 0, stream, args);
+  return e != cudaSuccess ? e : launch_pdl(pull_local_resolve_kernel, dim3(local_grid(args, true)), block, 0, stream, args);
 }
 
 cudaError_t launch_sparse_pull(const PullArgs& args, int work_items, cudaStream_t stream) {

@@ -7,12 +7,12 @@
 namespace tn {
 
 // pooling.cu
-void launch_pool_fwd(const float* U, int ustride, const int* inverse, const int* offsets, int B, int S, int pd,
-                     int combiner, float* out, int out_ld, cudaStream_t st);
+void launch_pool_fwd(const RowSource& src, const int* inverse, const int* offsets, int B, int S, int pd, int combiner, float* out,
+                     int out_ld, cudaStream_t st);
 void launch_pool_bwd(float* gU, int gstride, const int* inverse, const int* offsets, int B, int S, int pd, int dim,
                      int combiner, const float* gout, int gout_ld, cudaStream_t st);
-void launch_seq_fwd(const float* U, int ustride, const int* inverse, const int* offsets, int B, int T, int pd,
-                    float* out, int* lengths, cudaStream_t st);
+void launch_seq_fwd(const RowSource& src, const int* inverse, const int* offsets, int B, int T, int pd, float* out, int* lengths,
+                    cudaStream_t st);
 void launch_seq_bwd(float* gU, int gstride, const int* inverse, const int* offsets, int B, int T, int pd, int dim,
                     const float* gout, cudaStream_t st);
 void launch_expand_bag_labels(const float* y, const int* offsets, int B, int nbags, float* out, int room, cudaStream_t st);
@@ -80,10 +80,11 @@ void launch_cross_v2_bwd_sum(const CrossTerms& t, const void* g0, void* out, lon
 void launch_cross_v2_bwd_final(const float* gx0, const void* g, void* out, long long n, cudaStream_t st);
 
 // deepfm_fused.cu  (return nullptr or a static error string)
-const char* launch_deepfm_input_fwd(const float* U, int ustride, const int* inverse, int B, int S, int D, const float* dense, int Dd,
-                                    int ld_dense, void* X0, int ld, float* fm, int lin_col, float* Lout, cudaStream_t st);
-const char* launch_deepfm_input_bwd(const float* U, int ustride, const int* inverse, int B, int S, int D, const void* dX0, int ld,
-                                    const float* gfm, float* gU, int gstride, int lin_col, const float* dL, cudaStream_t st);
+// `E`: the rows as they were read, [B, S * D] fp32, which the backward pass takes
+const char* launch_deepfm_input_fwd(const RowSource& src, const int* inverse, int B, int S, int D, const float* dense, int Dd, int ld_dense,
+                                    void* X0, int ld, float* fm, int lin_col, float* Lout, float* E, cudaStream_t st);
+const char* launch_deepfm_input_bwd(const float* E, const int* inverse, int B, int S, int D, const void* dX0, int ld, const float* gfm,
+                                    float* gU, int gstride, int lin_col, const float* dL, cudaStream_t st);
 const char* launch_deepfm_head_loss(const void* H, int ldh, int NH, const float* L, int NL, const float* fm, const float* w,
                                     const float* label, int B, void* dH, float* dL, float* dfm, float* gw, float* sums, int nbins,
                                     float* pred, float* loss_out, float* scratch, cudaStream_t st);

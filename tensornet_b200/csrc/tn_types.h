@@ -81,6 +81,17 @@ struct PullArgs {
   int front_done;         // dedup, id dispatch and inverse map of this batch already ran (launch_sparse_pull_front)
 };
 
+// Where the pulled row of position v is: row v of the per-batch matrix `U`, or (`row_of` not null; one GPU) row row_of[v]
+// of the table itself, whose descriptor `tbl` lies in device memory so that recorded launches follow a shard that grows.
+struct RowSource {
+  const float* U;
+  int ustride;
+  const int* row_of;
+  const TableView* tbl;
+  int stride, dim;        // of the table's rows
+  int cvm;                // two columns behind the weights: 0 none, 1 show and ln(click + 1) - ln(show + 1), 2 zeros
+};
+
 struct PushArgs {
   SparseCommView c;
   TableView tbl;
@@ -163,6 +174,9 @@ cudaError_t launch_sparse_pull_front(const PullArgs& args, cudaStream_t stream);
 cudaError_t launch_dense_step(const DenseStepArgs& a, cudaStream_t st);
 int dense_step_ctas_per_sm();      // resident CTAs of the multi-GPU dense kernel per SM
 cudaError_t launch_sparse_pull(const PullArgs& args, int work_items, cudaStream_t stream);
+// One GPU: the pull as ordinary kernels, rows read in place (`rows`: also written out to U), and its part that can run ahead.
+cudaError_t launch_sparse_pull_local(const PullArgs& args, bool rows, cudaStream_t stream);
+cudaError_t launch_sparse_pull_local_front(const PullArgs& args, cudaStream_t stream);
 cudaError_t launch_sparse_push(const PushArgs& args, int work_items, int max_ctas, const DenseStepArgs* dense, cudaStream_t stream);
 
 }  // namespace tn

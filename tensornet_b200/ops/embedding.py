@@ -1,7 +1,7 @@
 """Pull + pool as one differentiable op, and the matching gradient path.
 
-Forward  : ids -> (fused dedup / all-to-all pull into the per-batch unique-row matrix ``U``)
-           -> bag pooling into ``[B, S * width]``.
+Forward  : ids -> (fused dedup / all-to-all pull into the per-batch unique-row matrix ``U``; on one GPU the rows
+           stay in the table) -> bag pooling into ``[B, S * width]``.
 Backward : scatter-add of the pooled gradient into the unique-gradient matrix ``gU`` that the
            fused push kernel later ships to the owning GPUs.
 
@@ -37,13 +37,13 @@ def _bag_scale(offsets, nbags, combiner, device):
 class _PullPool(torch.autograd.Function):
     @staticmethod
     def forward(ctx, anchor, table, ids, offsets, B, S, combiner, labels, label_mod, training, n_dev):
-        inverse = table.pull(ids, labels, label_mod, training) if n_dev is None else \
-            table.pull(ids, labels, label_mod, training, n_dev=n_dev)
         pd = table.pdim
         if ids.is_cuda:
+            inverse = table.pull_in_place(ids, labels, label_mod, training, n_dev)
             out = torch.empty((B, S * pd), dtype=torch.float32, device=ids.device)
-            _build.cuda_ext().pool_fwd(table.U, table.ustride, inverse, offsets, B, S, pd, combiner, out, S * pd)
+            table.ctx.pool_fwd(inverse, offsets, B, S, combiner, out, table.req)
         else:
+            inverse = table.pull(ids, labels, label_mod, training)
             nnz = ids.numel()
             inv = inverse.long()
             rows = table.U[inv.clamp(min=0), :pd] * (inv >= 0).unsqueeze(1)
@@ -100,13 +100,14 @@ class _PullSeq(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, anchor, table, ids, offsets, B, T, labels, training):
-        inverse = table.pull(ids, labels, 0, training)
         pd = table.pdim
         if ids.is_cuda:
+            inverse = table.pull_in_place(ids, labels, 0, training)
             out = torch.zeros((B, T, pd), dtype=torch.float32, device=ids.device)
             lengths = torch.zeros(B, dtype=torch.int32, device=ids.device)
-            _build.cuda_ext().seq_fwd(table.U, table.ustride, inverse, offsets, B, T, pd, out, lengths)
+            table.ctx.seq_fwd(inverse, offsets, B, T, out, lengths, table.req)
         else:
+            inverse = table.pull(ids, labels, 0, training)
             out = torch.zeros((B, T, pd), dtype=torch.float32)
             lens = (offsets[1:] - offsets[:-1]).long()
             lengths = lens.clamp(max=T).int()

@@ -517,15 +517,16 @@ def cross_v2(x0: torch.Tensor, weights: Sequence[torch.Tensor], dim: int) -> tor
 class _DeepFMInput(torch.autograd.Function):
     @staticmethod
     def forward(ctx, anchor, link, ids, B, S, dense, training, emb_dim, lin_col):
-        inverse = link.pull(ids, None, 0, training)
+        inverse = link.pull_in_place(ids, None, 0, training)
         D = emb_dim
         Dd = 0 if dense is None else int(dense.shape[1])
         ld = pad8(S * D + Dd + 1)
         x0 = torch.empty((B, ld), dtype=torch.bfloat16, device=ids.device)
         fm = torch.empty(B, dtype=torch.float32, device=ids.device)
         lin = torch.empty((B, S), dtype=torch.float32, device=ids.device) if lin_col >= 0 else None
-        _ext().deepfm_input_fwd(link.U, link.ustride, inverse, B, S, D, dense, x0, fm, lin_col, lin)
-        ctx.link, ctx.inverse, ctx.meta = link, inverse, (B, S, D, lin_col)
+        emb = torch.empty((B, S * D), dtype=torch.float32, device=ids.device)
+        link.ctx.deepfm_input_fwd(inverse, B, S, D, dense, x0, fm, lin_col, lin, emb, link.req)
+        ctx.link, ctx.inverse, ctx.emb, ctx.meta = link, inverse, emb, (B, S, D, lin_col)
         if lin is None:
             lin = torch.empty(0, device=ids.device)
             ctx.mark_non_differentiable(lin)
@@ -538,7 +539,7 @@ class _DeepFMInput(torch.autograd.Function):
         if gfm is None:
             gfm = torch.zeros(B, dtype=torch.float32, device=gx0.device)
         dl = glin.contiguous() if (lin_col >= 0 and glin is not None) else None
-        _ext().deepfm_input_bwd(link.U, link.ustride, ctx.inverse, B, S, D, gx0.contiguous(), gfm.contiguous().view(-1), link.gU,
+        _ext().deepfm_input_bwd(ctx.emb, ctx.inverse, B, S, D, gx0.contiguous(), gfm.contiguous().view(-1), link.gU,
                                 link.gstride, lin_col, dl)
         return (None,) * 9
 

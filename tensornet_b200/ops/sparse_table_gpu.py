@@ -108,7 +108,14 @@ class GpuSparseTable:
         rate = float(getattr(self.opt, "show_decay_rate", 1.0))
         self.ext.table_decay(self.table_dict(), self.kind, rate, int(delta_days))
 
+    def _drop_fronts(self):
+        """Rows move or go: on one GPU a pull that started ahead has already looked its signs up."""
+        for lk in self.links:
+            if lk._front is not None and lk.ctx.in_place():
+                lk.discard_front()
+
     def clear(self):
+        self._drop_fronts()
         self.keys.fill_(-1)
         self.slots.fill_(-1)
         self.row_tag.zero_()
@@ -238,6 +245,7 @@ class GpuSparseTable:
                 src, dst = movers[s:s + piece], holes[s:s + piece]
                 self.rows[dst] = self.rows[src]
                 self.row_keys[dst] = self.row_keys[src]
+            self._drop_fronts()
             self.row_tag[:n].zero_()
             self.n_rows_dev.fill_(n_keep)
             self.keys.fill_(-1)
@@ -264,9 +272,11 @@ class GpuSparseTable:
 def dedup_slots(max_unique: int, capo: int, world: int) -> int:
     """Slots of the dedup scratch.  One GPU: at most two thirds full with all the signs a segment holds.  It is probed at
     random and cleared every batch, so what counts is that it stays in L2 (4.1 M ids of 4.9 M that fit: 67 MB of keys
-    instead of 134, pull 627 -> 570 us).  Several GPUs: the segments of all owners together hold more than ``max_unique``
+    instead of 134, pull 627 -> 570 us).  Where that is no question, short probe chains count, since a warp waits for the
+    longest of 32: a quarter full at most up to 256 K signs (lookup of 10 K ids 13.0 -> 8.0 us, of 213 K 25.4 -> 23.6, but
+    of 2.1 M 126 -> 172).  Several GPUs: the segments of all owners together hold more than ``max_unique``
     signs, and a batch of up to twice that many is taken."""
-    return next_pow2(max(capo * 3 // 2, 32) if world == 1 else 2 * max_unique + 16)
+    return next_pow2(max(capo * 4 if capo <= 1 << 18 else capo * 3 // 2, 32) if world == 1 else 2 * max_unique + 16)
 
 
 _FRONT_STREAMS = {}
@@ -354,6 +364,8 @@ class GpuSparseLink:
         self.front_in_flight = False # a front was forked onto the side stream during this step (the model joins it)
         self.front_hits = 0          # pulls that found their front done (a model checks that its layers really pull)
         self._fork = torch.cuda.Event() if runtime().on_gpu else None
+        self.req = None              # rows of the batch at hand, when its pull started ahead on one GPU (else the link's own array)
+        self._front_req = {}
         self._front_inverse = {}     # inverse buffers of the fronts, one per id buffer (stable addresses for CUDA graphs)
         if multi:
             rt.barrier()
@@ -364,12 +376,21 @@ class GpuSparseLink:
         return ``inverse``: the row of ``self.U`` holding each id's embedding.  ``lookup_only`` (inference)
         never creates rows: signs no shard holds come back as zeros.  ``n_dev``: one int32 on the device, the number
         of ids that are there (``ids`` of a captured step has room for more)."""
+        return self._pull(ids, labels, label_mod, training, inverse, lookup_only, n_dev, True)
+
+    def pull_in_place(self, ids: torch.Tensor, labels: Optional[torch.Tensor] = None, label_mod: int = 0, training: bool = True,
+                      n_dev: Optional[torch.Tensor] = None, lookup_only: bool = False) -> torch.Tensor:
+        """:meth:`pull` for callers that read the rows at once and through ``self.ctx`` (``pool_fwd``, ``seq_fwd``,
+        ``deepfm_input_fwd``, given ``self.req``): on one GPU they stay in the table and ``self.U`` is not written."""
+        return self._pull(ids, labels, label_mod, training, None, lookup_only, n_dev, False)
+
+    def _pull(self, ids, labels, label_mod, training, inverse, lookup_only, n_dev, rows):
         n = ids.numel()
         front, self._front = self._front, None
-        front_done = False
+        front_done, self.req = False, None
         if front is not None:
             if front[0] == ids.data_ptr() and front[1] == n and training and not lookup_only and inverse is None:
-                inverse, front_done = front[2], True
+                inverse, self.req, front_done = front[2], front[3], True
                 self.front_hits += 1
             else:
                 self.discard_front()
@@ -377,7 +398,8 @@ class GpuSparseLink:
             inverse = torch.empty(n, dtype=torch.int32, device=self.dev)
         self._last_n_ids = n
         with phase("tn.sparse_pull"):
-            self.ctx.pull(ids.reshape(-1), inverse, labels, int(label_mod), bool(training), bool(lookup_only), front_done, n_dev)
+            self.ctx.pull(ids.reshape(-1), inverse, labels, int(label_mod), bool(training), bool(lookup_only), front_done, n_dev, rows,
+                          self.req)
         return inverse
 
     def fork_front(self):
@@ -395,20 +417,25 @@ class GpuSparseLink:
         self.front_in_flight = True
 
     def prefetch(self, ids: torch.Tensor):
-        """Run the front of the pull (dedup, id dispatch to the owners, inverse map) for the batch ``ids`` on the
-        current stream.  The next :meth:`pull` must be a training pull of this very tensor; it then only probes and
-        returns rows.  Anything else discards the front (:meth:`discard_front`).  ``ids`` must not live in the
+        """Run the front of the pull (dedup, id dispatch to the owners, inverse map; on one GPU also the lookup of the
+        signs) for the batch ``ids`` on the current stream.  The next :meth:`pull` must be a training pull of this very
+        tensor; it then only probes and returns rows (one GPU: creates those that are missing).  Anything else discards the front (:meth:`discard_front`).  ``ids`` must not live in the
         buffer of a batch whose backward pass is still to come: the inverse map of a front is kept per id buffer."""
         n = ids.numel()
         key = (ids.data_ptr(), n)
         inverse = self._front_inverse.get(key)
         if inverse is None:
             if len(self._front_inverse) >= 8:
-                self._front_inverse.pop(next(iter(self._front_inverse)))
+                oldest = next(iter(self._front_inverse))
+                self._front_inverse.pop(oldest)
+                self._front_req.pop(oldest, None)
             inverse = self._front_inverse[key] = torch.empty(n, dtype=torch.int32, device=self.dev)
+            if self.ctx.in_place():      # the front looks the signs up too, while the rows of the batch before are still to be pushed
+                self._front_req[key] = torch.empty(self.capo, dtype=torch.int32, device=self.dev)
+        req = self._front_req.get(key)
         with phase("tn.sparse_pull_front"):
-            self.ctx.front(ids.reshape(-1), inverse)
-        self._front = (ids.data_ptr(), n, inverse)
+            self.ctx.front(ids.reshape(-1), inverse, req)
+        self._front = (ids.data_ptr(), n, inverse, req)
 
     def discard_front(self):
         """Forget a front that ran for a batch which is not pulled next: the per-owner counters it built are
@@ -416,13 +443,15 @@ class GpuSparseLink:
         those of the pull that follows.  Every rank must do this at the same point (they do: same program)."""
         self._front = None
         self._loc["cnt"].zero_()
+        if self.ctx.in_place():
+            self._loc["ocount"].zero_()      # signs without a row
         self.table.epoch.add_(1)
 
     def push(self):
         """Apply the accumulated unique-row gradients (``self.gU``) on the owning GPUs."""
         rider, self.dense_rider = self.dense_rider, None
         with phase("tn.sparse_push+dense_step" if rider is not None else "tn.sparse_push"):
-            self.ctx.push(max(self._last_n_ids, 1), int(self.push_cta_cap), rider.ctx if rider is not None else None)
+            self.ctx.push(max(self._last_n_ids, 1), int(self.push_cta_cap), rider.ctx if rider is not None else None, self.req)
         if self.table.world > 1:
             runtime().peer_synced_pushes += 1      # this kernel waited for every peer's gradient records
 
@@ -437,13 +466,15 @@ class GpuSparseLink:
             l[k].zero_()
         for k in ("req_row", "req_ou", "ou_row"):
             l[k].fill_(-1)
+        self.req = None
         self.arena.tensor("sig").zero_()
         self._front = None           # a pull front that ran ahead is gone with the counters it built
 
     def pull_phase_us(self):
         """Durations (microseconds) of the last pull's phases as seen by CTA 0: dedup; id dispatch + inverse map;
         probe and row return of this GPU's own segment; wait for the other GPUs' ids, their probe and row return;
-        completion flags + scratch clear."""
+        completion flags + scratch clear.  One GPU: dedup and lookup; (launch of the second kernel); positions, counts
+        and new rows; 0; 0."""
         t = self.prof.tolist()
         return [(t[i + 1] - t[i]) / 1e3 for i in range(5)]
 

@@ -233,10 +233,9 @@ class ShardedInferenceEngine:
     def _forward(self, ids, offsets, B):
         ext = _build.cuda_ext()
         lk = self.link
-        inverse = lk.pull(ids, None, 0, training=False, lookup_only=True)
-        pd = lk.pdim
-        pooled = torch.empty((B, self.S * pd), dtype=torch.float32, device=ids.device)
-        ext.pool_fwd(lk.U, lk.ustride, inverse, offsets, B, self.S, pd, self.combiner, pooled, self.S * pd)
+        inverse = lk.pull_in_place(ids, None, 0, training=False, lookup_only=True)
+        pooled = torch.empty((B, self.S * lk.pdim), dtype=torch.float32, device=ids.device)
+        lk.ctx.pool_fwd(inverse, offsets, B, self.S, self.combiner, pooled, lk.req)
         x0 = F.concat_cast([pooled], ones=True)
         logit = self.head(self.mlp(x0)).view(-1)
         prob = torch.empty_like(logit)
