@@ -198,12 +198,17 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     // kEpiSubs warps share each TMEM lane quarter and take column chunks round-robin.
     const int q = warp & 3;                 // TMEM lane quarter this warp may read
     const int sub = (warp - 2) >> 2;        // which of the interleaved chunk sequences
-    bool ok = nk > 0;
-    if (ok && !mbar_wait(smem_u32(&s_accum), 0u, s_abort)) { *s_abort = 1; ok = false; }
-    tc_fence_after();
-    if (prof && warp == 2 && lane == 0) prof[10] = globaltimer_ns();
-    if (ok) {
-      // The accumulator barrier has fired: every TMA load has landed and every MMA has read its
+    bool waited = false;
+    auto ready = [&]() {
+      if (waited) return true;
+      if (!mbar_wait(smem_u32(&s_accum), 0u, s_abort)) { *s_abort = 1; return false; }
+      waited = true;
+      tc_fence_after();
+      if (prof && warp == 2 && lane == 0) prof[10] = globaltimer_ns();
+      return true;
+    };
+    if (nk > 0) {
+      // Once the accumulator barrier has fired every TMA load has landed and every MMA has read its
       // operands, so the stage ring is free.  Each epilogue warp takes 6 KiB of it as a transpose
       // buffer: TMEM gives a lane one ROW of the tile, global memory wants a warp on whole lines.
       // Blocks of 32 rows x 64 bytes go through shared memory (16-byte pieces, XOR-swizzled so both
@@ -215,7 +220,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
       for (int half = 0; half < halves; ++half) {
         const int row_base = m0 + half * kBM + q * 32;
         const uint32_t tm_lane = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(half * 256);
-        gemm_epi::store_rows(p, tm_lane, row_base, n0, BN, sub, kEpiSubs, lane, sm_out);
+        if (!gemm_epi::store_rows<true>(p, tm_lane, row_base, n0, BN, sub, kEpiSubs, lane, sm_out, ready)) break;
       }
     }
   }
