@@ -202,10 +202,9 @@ struct SparseCtx {
     TORCH_CHECK(n_dev->is_cuda() && n_dev->scalar_type() == at::kInt && n_dev->numel() == 1, "n_dev: one int32 on the device");
     return ptr_of<const int>(*n_dev);
   }
-  // `rows`: the pulled rows are wanted in the per-batch matrix (always the case where they are not read in place)
-  void pull(at::Tensor ids, at::Tensor inverse, c10::optional<at::Tensor> labels, int label_mod, bool training, bool lookup_only,
-            bool front_done, c10::optional<at::Tensor> n_dev, bool rows, c10::optional<at::Tensor> req) {
-    c10::cuda::CUDAGuard guard(ids.device());
+  tn::PullArgs batch_args(const at::Tensor& ids, const at::Tensor& inverse, const c10::optional<at::Tensor>& labels, int label_mod,
+                          bool training, bool lookup_only, bool front_done, const c10::optional<at::Tensor>& n_dev,
+                          const c10::optional<at::Tensor>& req) const {
     tn::PullArgs a = pull_args(ids, inverse, req);
     a.n_dev = count_ptr(n_dev);
     a.labels = labels.has_value() ? ptr_of<const float>(*labels) : nullptr;
@@ -214,9 +213,20 @@ struct SparseCtx {
     a.lookup_only = lookup_only ? 1 : 0;
     TORCH_CHECK(!(training && lookup_only), "a training pull creates rows; lookup_only is for inference");
     a.front_done = front_done ? 1 : 0;
+    return a;
+  }
+  // `rows`: the pulled rows are wanted in the per-batch matrix (always the case where they are not read in place)
+  void pull(at::Tensor ids, at::Tensor inverse, c10::optional<at::Tensor> labels, int label_mod, bool training, bool lookup_only,
+            bool front_done, c10::optional<at::Tensor> n_dev, bool rows, c10::optional<at::Tensor> req) {
+    c10::cuda::CUDAGuard guard(ids.device());
+    tn::PullArgs a = batch_args(ids, inverse, labels, label_mod, training, lookup_only, front_done, n_dev, req);
     if (in_place()) {
-      check(tn::launch_sparse_pull_local(a, rows, cur_stream()), "sparse_pull_local launch");
-      g_launches.fetch_add((front_done ? 0 : 1) + (rows ? 1 : 0), std::memory_order_relaxed);
+      tn::PullBatch batch{};
+      batch.n = 1;
+      batch.a[0] = a;
+      check(tn::launch_sparse_pull_local(batch, cur_stream()), "sparse_pull_local launch");
+      if (!front_done) g_launches.fetch_add(1, std::memory_order_relaxed);
+      if (rows) check(tn::launch_sparse_pull_local_rows(a, cur_stream()), "sparse_pull_local_rows launch");
       return;
     }
     a.tile_rows = tile_rows;
@@ -640,6 +650,24 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       }, py::arg("work_hint"), py::arg("max_ctas") = 0, py::arg("dense") = py::none(), py::arg("req") = py::none())
       .def("front", &SparseCtx::front, py::arg("ids"), py::arg("inverse"), py::arg("req") = py::none())
       .def("in_place", &SparseCtx::in_place)
+      // in-place pulls of different tables side by side: all of them behind a front (`front_done`) or none
+      .def_static("pull_many", [](std::vector<SparseCtx*> ctx, std::vector<at::Tensor> ids, std::vector<at::Tensor> inverse,
+                                  std::vector<c10::optional<at::Tensor>> labels, std::vector<int> label_mod, std::vector<bool> training,
+                                  bool front_done, std::vector<c10::optional<at::Tensor>> n_dev, std::vector<c10::optional<at::Tensor>> req) {
+        const size_t n = ctx.size();
+        TORCH_CHECK(n >= 1 && n <= (size_t)tn::kMaxPullBatch && ids.size() == n && inverse.size() == n && labels.size() == n &&
+                        label_mod.size() == n && training.size() == n && n_dev.size() == n && req.size() == n, "pull_many: one entry per pull");
+        c10::cuda::CUDAGuard guard(ids[0].device());
+        tn::PullBatch batch{};
+        batch.n = (int)n;
+        for (size_t k = 0; k < n; ++k) {
+          TORCH_CHECK(ctx[k]->in_place(), "pull_many: in-place pulls only");
+          for (size_t j = 0; j < k; ++j) TORCH_CHECK(ctx[j]->t.keys != ctx[k]->t.keys, "pull_many: different tables");
+          batch.a[k] = ctx[k]->batch_args(ids[k], inverse[k], labels[k], label_mod[k], training[k], false, front_done, n_dev[k], req[k]);
+        }
+        check(tn::launch_sparse_pull_local(batch, cur_stream()), "sparse_pull_local launch");
+        if (!front_done) g_launches.fetch_add(1, std::memory_order_relaxed);
+      })
       .def("pool_fwd", [](SparseCtx& self, at::Tensor inverse, c10::optional<at::Tensor> offsets, int B, int S, int combiner, at::Tensor out,
                           c10::optional<at::Tensor> req) {
         c10::cuda::CUDAGuard guard(out.device());

@@ -124,6 +124,10 @@ class EmbeddingFeatures(nn.Module):
         self._args_cache = (features, training, args)
         return args
 
+    def _n_dev(self, features, offsets):
+        """A captured step's buffers have room to spare: the last offset is the number of ids of this batch."""
+        return offsets[-1:] if offsets is not None and padded_columns(features, self._keys) else None
+
     def forward(self, features: Dict, training: Optional[bool] = None):
         if not isinstance(features, dict):
             raise ValueError("We expected a dictionary here. Instead we got: ", features)
@@ -131,8 +135,7 @@ class EmbeddingFeatures(nn.Module):
         self.table.set_training(training)
         ids, offsets, B, labels, label_mod, count = self._pull_args(features, training)
         S = len(self._keys)
-        # a captured step's buffers have room to spare: the last offset is the number of ids of this batch
-        n_dev = offsets[-1:] if offsets is not None and padded_columns(features, self._keys) else None
+        n_dev = self._n_dev(features, offsets)
         out = pull_pool(self._anchor, self.link, ids, offsets, B, S, self.combiner, labels, label_mod, count, n_dev)
         self._pending_push = count
         if self.is_concat:
@@ -145,8 +148,7 @@ class EmbeddingFeatures(nn.Module):
         Used by model-specific fused kernels that consume the pulled rows directly."""
         if self.use_cvm or self.dim % 4 != 0:
             return None
-        dev = core.runtime().device
-        ids, offsets, B = gather_columns(features, self._keys, dev)
+        ids, offsets, B = self.stash_pull_args(features, training)[:3]
         if offsets is not None:
             return None
         self.table.set_training(training)
@@ -183,3 +185,23 @@ class EmbeddingFeatures(nn.Module):
 
     def show_decay(self, delta_days: int = 0):
         return core.show_decay(self.sparse_table_handle, delta_days)
+
+
+def pull_together(layers: Sequence[EmbeddingFeatures], features: Dict, training: Optional[bool] = None):
+    """Run the pulls of several layers over one batch side by side (one GPU; their ids are all they need).  The
+    forward pass of every one of them has to follow; it then finds its pull done."""
+    rt = core.runtime()
+    if not rt.on_gpu or rt.world > 1 or not isinstance(features, dict) or not all(type(l) is EmbeddingFeatures for l in layers):
+        return
+    if training is None:
+        training = layers[0].training
+        if any(l.training != training for l in layers):
+            return
+    if len({id(l.table) for l in layers}) < len(layers) or not all(l.link.ctx.in_place() for l in layers):
+        return
+    calls = []
+    for l in layers:
+        l.table.set_training(training)
+        ids, offsets, _, labels, label_mod, count = l.stash_pull_args(features, training)
+        calls.append((l.link, ids, labels, label_mod, count, l._n_dev(features, offsets)))
+    layers[0].link.pull_many(calls)

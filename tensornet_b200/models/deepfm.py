@@ -14,6 +14,7 @@ from torch import nn
 
 from .. import core, feature_column as fc
 from ..layers import DenseHead, EmbeddingFeatures, MLP
+from ..layers.embedding_features import pull_together
 from ..model import Model
 from ..ops import functional as F
 
@@ -87,6 +88,9 @@ class DeepFM(Model):
         if got is None:
             return None
         ids, B = got
+        if not self.share_linear_table:
+            pull_together([self.linear_emb, self.deep_emb], features, True)
+        self.deep_emb._args_cache = None            # its forward pass does not follow
         dense = features[self.dense_key].to(ids.device, non_blocking=True) if self.dense_dim else None
         if self.share_linear_table:
             x0, fm, lin = F.deepfm_input(self.deep_emb._anchor, self.deep_emb.link, ids, B, len(self.deep_emb._keys), dense, True,
@@ -107,6 +111,8 @@ class DeepFM(Model):
             deep = both[:, :, : self.emb_dim].reshape(both.shape[0], -1)
             dense = features[self.dense_key].to(deep.device, non_blocking=True) if self.dense_dim else None
             return self.sub_model(lin, deep, dense)
+        if self.linear_emb is not None:
+            pull_together([self.linear_emb, self.deep_emb], features)
         lin = self.linear_emb(features) if self.linear_emb is not None else None
         deep = self.deep_emb(features)
         dense = None

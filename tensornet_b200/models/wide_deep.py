@@ -10,6 +10,7 @@ from torch import nn
 
 from .. import core, feature_column as fc
 from ..layers import DenseHead, EmbeddingFeatures, MLP, TNBatchNormalization
+from ..layers.embedding_features import pull_together
 from ..model import Model
 from ..ops import functional as F
 
@@ -51,6 +52,7 @@ class WideDeep(Model):
                                           dense_dim, dnn_hidden_units, use_bn)
 
     def forward(self, features):
+        pull_together([self.linear_emb, self.deep_emb], features)
         lin = self.linear_emb(features)
         deep = self.deep_emb(features)
         dense = features[self.dense_key].to(deep.device, non_blocking=True) if self.dense_dim else None

@@ -111,6 +111,7 @@ class GpuSparseTable:
     def _drop_fronts(self):
         """Rows move or go: on one GPU a pull that started ahead has already looked its signs up."""
         for lk in self.links:
+            lk._pulled = None
             if lk._front is not None and lk.ctx.in_place():
                 lk.discard_front()
 
@@ -364,6 +365,7 @@ class GpuSparseLink:
         self.front_in_flight = False # a front was forked onto the side stream during this step (the model joins it)
         self.front_hits = 0          # pulls that found their front done (a model checks that its layers really pull)
         self._fork = torch.cuda.Event() if runtime().on_gpu else None
+        self._pulled = None          # (ids, their version, training, inverse) of a pull that was run for the forward pass to come
         self.req = None              # rows of the batch at hand, when its pull started ahead on one GPU (else the link's own array)
         self._front_req = {}
         self._front_inverse = {}     # inverse buffers of the fronts, one per id buffer (stable addresses for CUDA graphs)
@@ -385,6 +387,18 @@ class GpuSparseLink:
         return self._pull(ids, labels, label_mod, training, None, lookup_only, n_dev, False)
 
     def _pull(self, ids, labels, label_mod, training, inverse, lookup_only, n_dev, rows):
+        n, done, self._pulled = ids.numel(), self._pulled, None
+        if (done is not None and not rows and not lookup_only and done[0].data_ptr() == ids.data_ptr() and done[0].numel() == n
+                and done[0]._version == done[1] and done[2] == bool(training)):
+            return done[3]
+        inverse, front_done = self._begin(ids, training, lookup_only, inverse)
+        with phase("tn.sparse_pull"):
+            self.ctx.pull(ids.reshape(-1), inverse, labels, int(label_mod), bool(training), bool(lookup_only), front_done, n_dev, rows,
+                          self.req)
+        return inverse
+
+    def _begin(self, ids, training, lookup_only=False, inverse=None):
+        """``(inverse, front_done)`` for a pull of ``ids``; a front that ran for another batch is discarded."""
         n = ids.numel()
         front, self._front = self._front, None
         front_done, self.req = False, None
@@ -397,10 +411,28 @@ class GpuSparseLink:
         if inverse is None:
             inverse = torch.empty(n, dtype=torch.int32, device=self.dev)
         self._last_n_ids = n
-        with phase("tn.sparse_pull"):
-            self.ctx.pull(ids.reshape(-1), inverse, labels, int(label_mod), bool(training), bool(lookup_only), front_done, n_dev, rows,
-                          self.req)
-        return inverse
+        return inverse, front_done
+
+    @staticmethod
+    def pull_many(calls):
+        """In-place pulls of different tables in one go.  ``calls``: ``(link, ids, labels, label_mod, training, n_dev)`` of
+        each; the :meth:`pull_in_place` of the same ids that follows on a link finds its pull done.  False (and nothing
+        done) where they do not go together."""
+        links = [c[0] for c in calls]
+        if not 2 <= len(calls) <= 4 or len({id(lk.table) for lk in links}) < len(links) or not all(lk.ctx.in_place() for lk in links) or \
+                any(c[1].is_inference() for c in calls):
+            return False
+        begun = [lk._begin(ids, training) for lk, ids, _, _, training, _ in calls]
+        # (a model runs every front ahead or none: a mixture is two calls of different batches, and goes one by one)
+        for done in sorted({b[1] for b in begun}):
+            at = [k for k, b in enumerate(begun) if b[1] == done]
+            with phase("tn.sparse_pull"):
+                links[0].table.ext.SparseCtx.pull_many(
+                    [links[k].ctx for k in at], [calls[k][1].reshape(-1) for k in at], [begun[k][0] for k in at], [calls[k][2] for k in at],
+                    [int(calls[k][3]) for k in at], [bool(calls[k][4]) for k in at], done, [calls[k][5] for k in at], [links[k].req for k in at])
+        for (lk, ids, _, _, training, _), (inverse, _) in zip(calls, begun):
+            lk._pulled = (ids, ids._version, bool(training), inverse)
+        return True
 
     def fork_front(self):
         """The batch of the following step is known (``next_ids``): run its dedup and id dispatch on the side stream
@@ -466,7 +498,7 @@ class GpuSparseLink:
             l[k].zero_()
         for k in ("req_row", "req_ou", "ou_row"):
             l[k].fill_(-1)
-        self.req = None
+        self.req = self._pulled = None
         self.arena.tensor("sig").zero_()
         self._front = None           # a pull front that ran ahead is gone with the counters it built
 

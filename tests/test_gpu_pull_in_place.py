@@ -33,7 +33,7 @@ def _batch(tn, g, slots, B, ragged, top, dev):
 @pytest.mark.parametrize("dim,kind,cvm", [(1, "adagrad", False), (1, "adagrad", True), (2, "adagrad", True), (3, "adam", False),
                                           (8, "adagrad", True), (10, "ftrl", False), (12, "adam", False), (38, "adagrad", True),
                                           (64, "ftrl", False), (128, "adagrad", False), (140, "adam", False)])
-@pytest.mark.parametrize("ragged,combiner,B", [(False, "sum", 1), (False, "mean", 700), (True, "mean", 333), (True, "sqrtn", 2050)])
+@pytest.mark.parametrize("ragged,combiner,B", [(False, "sum", 1), (False, "mean", 700), (True, "sum", 333), (True, "mean", 40), (True, "sqrtn", 2050)])
 def test_in_place_pull_matches_the_exchange_kernel(tn_gpu, status_ok, dim, kind, cvm, ragged, combiner, B):
     tn = tn_gpu
     dev = tn.core.runtime().device
@@ -60,10 +60,13 @@ def test_in_place_pull_matches_the_exchange_kernel(tn_gpu, status_ok, dim, kind,
             outs.append(layer.table.rows[rows][:, : dim + 3 if kind == "adagrad" else 3 * dim].clone())
         outs.append(torch.tensor(float(layer.table.n_rows)))
         got.append(outs)
-    for a, b in zip(*got):
-        # mean and sqrtn scale the terms of a sum, whose order is free: 64 terms of 2^-24 each at most, carried through the updates
-        assert a.shape == b.shape
-        assert bool(((a - b).abs() <= 2.0 ** -17 * (1 + a.abs())).all()), float((a - b).abs().max())
+    # single ids and plain sums: gradients are sums of quarters, exact in any order, and all is the same to the bit.  With a
+    # scale the sums of the gradients depend on their order, so only what comes before the first update is compared.
+    exact = not ragged or combiner == "sum"
+    assert len(got[0]) == len(got[1]) == 8
+    for a, b in list(zip(*got))[: None if exact else 1]:
+        assert torch.equal(a, b), float((a - b).abs().max())
+    assert float(got[0][-1]) == float(got[1][-1])
 
 
 @pytest.mark.parametrize("n", [1, 33, 5000, 151553, 460001])
@@ -135,3 +138,44 @@ def test_front_that_has_looked_its_signs_up_meets_a_changed_table(tn_gpu, status
     t.clear()
     shows.zero_()
     check(a)
+
+
+@pytest.mark.parametrize("ragged", [False, True])
+def test_pulls_of_two_layers_side_by_side(tn_gpu, status_ok, ragged):
+    """One launch for both tables against one pull after the other; with fronts ahead of both, of one and of none."""
+    from tensornet_b200.layers.embedding_features import pull_together
+
+    tn = tn_gpu
+    dev = tn.core.runtime().device
+    slots, B = ["a", "b"], 500
+    got = []
+    for together in (False, True):
+        layers = [_layer(tn, 1, "adagrad", True, "sum", slots, 6 * B + 8, False), _layer(tn, 12, "adam", False, "sum", slots, 6 * B + 8, False)]
+        g = torch.Generator().manual_seed(3)
+        outs = []
+        batches = [_batch(tn, g, slots, B, ragged, 300 * (k + 1), dev) for k in range(5)]
+        for k, (f, signs) in enumerate(batches):
+            if not ragged:
+                for layer in layers[: {3: 1, 4: 2}.get(k, 0)]:
+                    layer.link.prefetch(layer.ids_pulled_for(f))
+            if together:
+                pull_together(layers, f, k != 2)
+                assert all(layer.link._pulled is not None for layer in layers)
+            for layer in layers:
+                out = layer(f, training=k != 2)
+                assert layer.link._pulled is None
+                outs.append(out.detach().clone())
+                if k != 2:
+                    out.backward(((torch.arange(out.numel(), device=dev) % 13).float() - 6).view_as(out) / 4)
+            for layer in layers:
+                layer.backwards()
+                outs.append(layer.table.rows[layer.table.lookup_rows(signs).long()][:, : 4 if layer.dim == 1 else 36].clone())
+        got.append(outs)
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+    # a pull that was run ahead is for that batch only: other ids, or the same buffer with new contents, are pulled again
+    (f, _), (f2, s2) = batches[0], batches[1]
+    pull_together(layers, f, True)
+    for layer in layers:
+        out = layer(f2, training=False)
+        assert layer.link.unique_counts()[0] == s2.numel() and out.shape[0] == B
