@@ -356,15 +356,48 @@ struct BnCtx {
       has_sync = true;
     }
   }
-  // sums of one batch -> totals, increments and moments (two launches)
-  void push(at::Tensor x, bool centered) {
-    TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kFloat && x.dim() == 2 && x.size(1) == t.C && x.stride(1) == 1, "x must be fp32 [B, C]");
+  // [h (bf16, first nh columns) | x (fp32)], or x alone
+  tn::BnInput input(const c10::optional<at::Tensor>& h, int nh, const at::Tensor& x) const {
+    tn::BnInput in{};
+    TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kFloat && x.dim() == 2 && x.size(1) == t.C - nh && x.stride(1) == 1, "x must be fp32 [B, C]");
+    in.x = ptr_of<float>(x);
+    in.ldx = (int)x.stride(0);
+    if (h.has_value()) {
+      TORCH_CHECK(h->is_cuda() && h->scalar_type() == at::kBFloat16 && h->is_contiguous() && h->dim() == 2 && h->size(0) == x.size(0) && h->size(1) >= nh,
+                  "h must be contiguous bf16 [B, >= nh]");
+      in.h = h->data_ptr();
+      in.ldh = (int)h->size(1);
+      in.nh = nh;
+    }
+    return in;
+  }
+  // sums of one batch -> totals, increments (or none pending: `drop_inc`) and moments (two launches)
+  void push(at::Tensor x, bool centered, bool drop_inc, c10::optional<at::Tensor> h, int nh) {
+    const tn::BnInput in = input(h, h.has_value() ? nh : 0, x);
     c10::cuda::CUDAGuard guard(x.device());
-    tn::launch_bn_batch_stats(ptr_of<float>(x), (int)x.stride(0), (int)x.size(0), t.C, centered ? t.mean : nullptr, batch, cur_stream());
-    tn::launch_bn_table_append(t, batch, cur_stream());
+    tn::launch_bn_batch_stats(in, (int)x.size(0), t.C, centered ? t.mean : nullptr, batch, cur_stream());
+    tn::launch_bn_table_append(t, batch, drop_inc, cur_stream());
+  }
+  void join_fwd(at::Tensor h, int nh, at::Tensor x, c10::optional<at::Tensor> gamma, c10::optional<at::Tensor> beta, double eps, at::Tensor z,
+                at::Tensor moments) {
+    const tn::BnInput in = input(h, nh, x);
+    TORCH_CHECK(z.scalar_type() == at::kBFloat16 && z.is_contiguous() && z.size(1) % 2 == 0 && z.size(1) > t.C, "join: z");
+    c10::cuda::CUDAGuard guard(x.device());
+    tn::launch_bn_join_fwd(in, (int)x.size(0), t.C, t.mean, t.var, gamma ? ptr_of<float>(*gamma) : nullptr, beta ? ptr_of<float>(*beta) : nullptr,
+                           (float)eps, z.data_ptr(), (int)z.size(1), ptr_of<float>(moments), ptr_of<float>(moments) + t.C, cur_stream());
+  }
+  void join_bwd(at::Tensor dz, at::Tensor h, int nh, at::Tensor x, at::Tensor moments, c10::optional<at::Tensor> gamma, double eps, bool mask,
+                c10::optional<at::Tensor> gh, c10::optional<at::Tensor> gx, c10::optional<at::Tensor> gg, c10::optional<at::Tensor> gb) {
+    const tn::BnInput in = input(h, nh, x);
+    TORCH_CHECK(dz.scalar_type() == at::kBFloat16 && dz.is_contiguous() && dz.size(1) >= t.C, "join: dz");
+    c10::cuda::CUDAGuard guard(x.device());
+    tn::launch_bn_join_bwd(dz.data_ptr(), (int)dz.size(1), in, (int)x.size(0), t.C, ptr_of<float>(moments), ptr_of<float>(moments) + t.C,
+                           gamma ? ptr_of<float>(*gamma) : nullptr, (float)eps, mask ? 1 : 0, gh ? gh->data_ptr() : nullptr,
+                           gx ? ptr_of<float>(*gx) : nullptr, gx ? (int)gx->stride(0) : 0, gg ? ptr_of<float>(*gg) : nullptr,
+                           gb ? ptr_of<float>(*gb) : nullptr, cur_stream());
   }
   // fold a record the host has staged in `batch`
-  void append_staged() { tn::launch_bn_table_append(t, batch, cur_stream()); }
+  void append_staged() { tn::launch_bn_table_append(t, batch, false, cur_stream()); }
   void refresh() { tn::launch_bn_table_refresh(t, cur_stream()); }
   void sync() {
     if (has_sync) tn::launch_bn_table_sync(t, s, scratch, cur_stream());
@@ -698,11 +731,13 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("forward", &ServeCtx::forward);
   py::class_<BnCtx>(m, "BnCtx")
       .def(py::init<py::dict>())
-      .def("push", &BnCtx::push)
+      .def("push", &BnCtx::push, py::arg("x"), py::arg("centered"), py::arg("drop_inc") = false, py::arg("h") = py::none(), py::arg("nh") = 0)
       .def("append_staged", &BnCtx::append_staged)
       .def("refresh", &BnCtx::refresh)
       .def("sync", &BnCtx::sync)
       .def("apply_fwd", &BnCtx::apply_fwd)
+      .def("join_fwd", &BnCtx::join_fwd)
+      .def("join_bwd", &BnCtx::join_bwd)
       .def("apply_bwd", &BnCtx::apply_bwd);
   py::class_<DenseCtx>(m, "DenseCtx").def(py::init<py::dict>()).def("step", &DenseCtx::step, py::arg("skip_open") = false).def("set_gated", &DenseCtx::set_gated).def("set_max_ctas", &DenseCtx::set_max_ctas);
   m.def("dense_ctas_per_sm", [] { return tn::dense_step_ctas_per_sm(); });

@@ -11,9 +11,12 @@
 //   bn_batch_stats   per-feature sum and squared sum (optionally around a centre) in fp64
 //   bn_table_append  fold the batch into the totals, refresh the fp32 moments, re-zero the scratch
 //   bn_apply_fwd/bwd normalise with the moments (moments are constants for the backward pass)
+//   bn_join_fwd/bwd  the same for [h | x], where h is a tower's padded bf16 output and x fp32, straight into the padded bf16
+//                    operand of the next layer and back (the ReLU mask of the tower's output included)
 // and, when the layer is synchronised, every `sync_freq` steps
 //   bn_table_sync    cross-GPU exchange of the pending increments by peer loads, bracketed by
 //                    bounded flag handshakes.
+#include <cuda_bf16.h>
 #include "tn_device.cuh"
 #include "tn_ops.h"
 
@@ -23,10 +26,16 @@ namespace {
 
 constexpr int kBnCols = 32;    // columns per CTA
 constexpr int kBnRows = 8;     // row lanes per CTA (256 threads)
+constexpr int kBnMinRows = 64; // rows per CTA at least
 
-__global__ void __launch_bounds__(kBnCols * kBnRows) bn_batch_stats_kernel(const float* __restrict__ x, int ld, int B, int C,
-                                                                          const float* __restrict__ center, double* batch,
-                                                                          int rows_per_cta) {
+__device__ __forceinline__ float bn_at(const BnInput& in, int r, int c) {
+  if (c < in.nh) return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(in.h)[(size_t)r * in.ldh + c]);
+  return in.x[(size_t)r * in.ldx + (c - in.nh)];
+}
+
+__global__ void __launch_bounds__(kBnCols * kBnRows) bn_batch_stats_kernel(const BnInput in, int B, int C, const float* __restrict__ center,
+                                                                          double* batch, int rows_per_cta) {
+  pdl_sync();
   __shared__ double s_sum[kBnRows][kBnCols], s_sq[kBnRows][kBnCols];
   const int cl = threadIdx.x % kBnCols, rl = threadIdx.x / kBnCols;
   const int c = blockIdx.x * kBnCols + cl;
@@ -36,7 +45,7 @@ __global__ void __launch_bounds__(kBnCols * kBnRows) bn_batch_stats_kernel(const
   if (c < C) {
     const float ctr = center ? center[c] : 0.f;
     for (int r = r0 + rl; r < r1; r += kBnRows) {
-      const double v = (double)x[(size_t)r * ld + c];
+      const double v = (double)bn_at(in, r, c);
       const double d = v - (double)ctr;
       s += v;
       q += d * d;
@@ -102,7 +111,8 @@ __device__ __forceinline__ void bn_moments(const BnTableView& t, int c) {
 
 // `acc` = [3][C] sums to fold in.  Decides between plain accumulation and the moving window exactly as the
 // host table does: window mode once max(total_count) exceeds max_count, with ratio = max(acc_count) / max(total_count).
-__device__ void bn_append_block(const BnTableView& t, const double* acc, bool is_local, bool zero_acc) {
+// `drop_inc`: nobody is waiting for the pending increments, which go to zero instead.
+__device__ void bn_append_block(const BnTableView& t, const double* acc, bool is_local, bool zero_acc, bool drop_inc = false) {
   const int C = t.C;
   double cur = 0.0, am = 0.0;
   for (int c = threadIdx.x; c < C; c += blockDim.x) { cur = fmax(cur, t.total_count[c]); am = fmax(am, acc[2 * C + c]); }
@@ -112,15 +122,17 @@ __device__ void bn_append_block(const BnTableView& t, const double* acc, bool is
   const double k = window ? (1.0 - t.moment) * (am / cur) : -1.0;
   for (int c = threadIdx.x; c < C; c += blockDim.x) {
     const double as = acc[c], aq = acc[C + c], ac = acc[2 * C + c];
-    if (is_local) { t.inc[c] += as; t.inc[C + c] += aq; t.inc[2 * C + c] += ac; }
+    if (drop_inc) { t.inc[c] = 0.0; t.inc[C + c] = 0.0; t.inc[2 * C + c] = 0.0; }
+    else if (is_local) { t.inc[c] += as; t.inc[C + c] += aq; t.inc[2 * C + c] += ac; }
     bn_fold(t, c, as, aq, ac, k);
     bn_moments(t, c);
     if (zero_acc) { const_cast<double*>(acc)[c] = 0.0; const_cast<double*>(acc)[C + c] = 0.0; const_cast<double*>(acc)[2 * C + c] = 0.0; }
   }
 }
 
-__global__ void __launch_bounds__(1024) bn_table_append_kernel(const BnTableView t, double* batch) {
-  bn_append_block(t, batch, true, true);
+__global__ void __launch_bounds__(1024) bn_table_append_kernel(const BnTableView t, double* batch, int drop_inc) {
+  pdl_sync();
+  bn_append_block(t, batch, true, true, drop_inc != 0);
 }
 
 __global__ void __launch_bounds__(1024) bn_table_refresh_moments_kernel(const BnTableView t) {
@@ -171,6 +183,7 @@ __global__ void __launch_bounds__(1024) bn_table_sync_kernel(const BnTableView t
 __global__ void bn_apply_fwd_kernel(const float* __restrict__ x, int ldx, int B, int C, const float* __restrict__ mean,
                                     const float* __restrict__ var, const float* __restrict__ gamma, const float* __restrict__ beta,
                                     float eps, float* __restrict__ y, int ldy) {
+  pdl_sync();
   const long long n = (long long)B * C;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const int r = (int)(i / C), c = (int)(i - (long long)r * C);
@@ -187,6 +200,7 @@ __global__ void __launch_bounds__(kBnCols * kBnRows) bn_apply_bwd_kernel(const f
                                                                         const float* __restrict__ var, const float* __restrict__ gamma,
                                                                         float eps, float* __restrict__ dx, int ldo, float* gg, float* gb,
                                                                         int rows_per_cta) {
+  pdl_sync();
   __shared__ float s_g[kBnRows][kBnCols], s_b[kBnRows][kBnCols];
   const int cl = threadIdx.x % kBnCols, rl = threadIdx.x / kBnCols;
   const int c = blockIdx.x * kBnCols + cl;
@@ -212,23 +226,107 @@ __global__ void __launch_bounds__(kBnCols * kBnRows) bn_apply_bwd_kernel(const f
   }
 }
 
+// z = bf16([bn([h | x]) | 1 | 0]); one thread per pair of columns.  `mean_out` / `var_out` keep the moments it used for the
+// backward pass.  As separate kernels (h to fp32, concatenation, two copies of the moments, normalisation, operand assembly)
+// this took six launches of 1 to 4 us at 32 x 260, and their gradients nine: from the
+// tower to the loss 24 us and back 28; a step of 1024 x 36 by 133 to 108 us with these.
+__global__ void __launch_bounds__(256) bn_join_fwd_kernel(const BnInput in, int B, int C, const float* __restrict__ mean,
+                                                          const float* __restrict__ var, const float* __restrict__ gamma,
+                                                          const float* __restrict__ beta, float eps, __nv_bfloat16* __restrict__ z, int ldz,
+                                                          float* __restrict__ mean_out, float* __restrict__ var_out) {
+  pdl_sync();
+  const int half = ldz >> 1;
+  const long long n = (long long)B * half, first = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  for (long long i = first; i < C; i += (long long)gridDim.x * blockDim.x) { mean_out[i] = mean[i]; var_out[i] = var[i]; }
+  for (long long i = first; i < n; i += (long long)gridDim.x * blockDim.x) {
+    const int r = (int)(i / half), c0 = 2 * (int)(i - (long long)r * half);
+    float v[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int c = c0 + k;
+      v[k] = c == C ? 1.f : 0.f;
+      if (c < C) {
+        v[k] = (bn_at(in, r, c) - mean[c]) * rsqrtf(var[c] + eps);
+        if (gamma) v[k] *= gamma[c];
+        if (beta) v[k] += beta[c];
+      }
+    }
+    *reinterpret_cast<__nv_bfloat162*>(z + (size_t)r * ldz + c0) = __floats2bfloat162_rn(v[0], v[1]);
+  }
+}
+
+// Gradients of the same: gh (bf16, zero beyond its columns, and with `mask` where h is not above zero), gx (fp32), gamma, beta.
+__global__ void __launch_bounds__(kBnCols * kBnRows) bn_join_bwd_kernel(const __nv_bfloat16* __restrict__ dz, int ldz, const BnInput in, int B,
+                                                                        int C, const float* __restrict__ mean, const float* __restrict__ var,
+                                                                        const float* __restrict__ gamma, float eps, int mask,
+                                                                        __nv_bfloat16* __restrict__ gh, float* __restrict__ gx, int ldg,
+                                                                        float* gg, float* gb, int rows_per_cta) {
+  pdl_sync();
+  __shared__ float s_g[kBnRows][kBnCols], s_b[kBnRows][kBnCols];
+  const int cl = threadIdx.x % kBnCols, rl = threadIdx.x / kBnCols;
+  const int c = blockIdx.x * kBnCols + cl;
+  const int r0 = blockIdx.y * rows_per_cta, r1 = min(B, r0 + rows_per_cta);
+  float ag = 0.f, ab = 0.f;
+  if (c < C) {
+    const float rs = rsqrtf(var[c] + eps), m = mean[c], gm = gamma ? gamma[c] : 1.f;
+    for (int r = r0 + rl; r < r1; r += kBnRows) {
+      const float d = __bfloat162float(dz[(size_t)r * ldz + c]), x = bn_at(in, r, c);
+      ag += d * (x - m) * rs;
+      ab += d;
+      const float dx = d * gm * rs;
+      if (c < in.nh) {
+        if (gh) gh[(size_t)r * in.ldh + c] = __float2bfloat16(mask && !(x > 0.f) ? 0.f : dx);
+      } else if (gx) {
+        gx[(size_t)r * ldg + (c - in.nh)] = dx;
+      }
+    }
+  } else if (gh && c - C < in.ldh - in.nh) {               // the columns behind h's
+    for (int r = r0 + rl; r < r1; r += kBnRows) gh[(size_t)r * in.ldh + in.nh + (c - C)] = __float2bfloat16(0.f);
+  }
+  s_g[rl][cl] = ag;
+  s_b[rl][cl] = ab;
+  __syncthreads();
+  if (rl == 0 && c < C) {
+#pragma unroll
+    for (int k = 1; k < kBnRows; ++k) { ag += s_g[k][cl]; ab += s_b[k][cl]; }
+    if (gg) atomicAdd(&gg[c], ag);
+    if (gb) atomicAdd(&gb[c], ab);
+  }
+}
+
 inline int rows_per_cta_for(int B, int C) {
   const int col_tiles = (C + kBnCols - 1) / kBnCols;
   int want_y = (148 * 4 + col_tiles - 1) / col_tiles;       // enough CTAs to fill the GPU
   if (want_y < 1) want_y = 1;
   int rows = (B + want_y - 1) / want_y;
-  if (rows < 64) rows = 64;
+  if (rows < kBnMinRows) rows = kBnMinRows;
   return rows;
 }
 
 }  // namespace
 
-void launch_bn_batch_stats(const float* x, int ld, int B, int C, const float* center, double* batch, cudaStream_t st) {
+void launch_bn_batch_stats(const BnInput& in, int B, int C, const float* center, double* batch, cudaStream_t st) {
   const int rows = rows_per_cta_for(B, C);
   dim3 grid((C + kBnCols - 1) / kBnCols, (B + rows - 1) / rows);
-  bn_batch_stats_kernel<<<grid, kBnCols * kBnRows, 0, st>>>(x, ld, B, C, center, batch, rows);
+  launch_pdl(bn_batch_stats_kernel, grid, dim3(kBnCols * kBnRows), 0, st, in, B, C, center, batch, rows);
 }
-void launch_bn_table_append(const BnTableView& t, double* batch, cudaStream_t st) { bn_table_append_kernel<<<1, 1024, 0, st>>>(t, batch); }
+void launch_bn_table_append(const BnTableView& t, double* batch, bool drop_inc, cudaStream_t st) {
+  launch_pdl(bn_table_append_kernel, dim3(1), dim3(1024), 0, st, t, batch, drop_inc ? 1 : 0);
+}
+void launch_bn_join_fwd(const BnInput& in, int B, int C, const float* mean, const float* var, const float* gamma, const float* beta, float eps,
+                        void* z, int ldz, float* mean_out, float* var_out, cudaStream_t st) {
+  long long blocks = ((long long)B * (ldz >> 1) + 255) / 256;
+  if (blocks > 148 * 8) blocks = 148 * 8;
+  launch_pdl(bn_join_fwd_kernel, dim3(blocks < 1 ? 1 : (int)blocks), dim3(256), 0, st, in, B, C, mean, var, gamma, beta, eps,
+             reinterpret_cast<__nv_bfloat16*>(z), ldz, mean_out, var_out);
+}
+void launch_bn_join_bwd(const void* dz, int ldz, const BnInput& in, int B, int C, const float* mean, const float* var, const float* gamma,
+                        float eps, int mask, void* gh, float* gx, int ldg, float* gg, float* gb, cudaStream_t st) {
+  const int cols = C + (in.ldh - in.nh), rows = rows_per_cta_for(B, cols);
+  dim3 grid((cols + kBnCols - 1) / kBnCols, (B + rows - 1) / rows);
+  launch_pdl(bn_join_bwd_kernel, grid, dim3(kBnCols * kBnRows), 0, st, reinterpret_cast<const __nv_bfloat16*>(dz), ldz, in, B, C, mean, var,
+             gamma, eps, mask, reinterpret_cast<__nv_bfloat16*>(gh), gx, ldg, gg, gb, rows);
+}
 void launch_bn_table_refresh(const BnTableView& t, cudaStream_t st) { bn_table_refresh_moments_kernel<<<1, 1024, 0, st>>>(t); }
 void launch_bn_table_sync(const BnTableView& t, const BnSyncView& s, double* scratch, cudaStream_t st) {
   bn_table_sync_kernel<<<1, 1024, 0, st>>>(t, s, scratch);
@@ -239,13 +337,13 @@ void launch_bn_apply_fwd(const float* x, int ldx, int B, int C, const float* mea
   int blocks = (int)((n + 255) / 256);
   if (blocks > 148 * 8) blocks = 148 * 8;
   if (blocks < 1) blocks = 1;
-  bn_apply_fwd_kernel<<<blocks, 256, 0, st>>>(x, ldx, B, C, mean, var, gamma, beta, eps, y, ldy);
+  launch_pdl(bn_apply_fwd_kernel, dim3(blocks), dim3(256), 0, st, x, ldx, B, C, mean, var, gamma, beta, eps, y, ldy);
 }
 void launch_bn_apply_bwd(const float* dy, int ldd, const float* x, int ldx, int B, int C, const float* mean, const float* var,
                          const float* gamma, float eps, float* dx, int ldo, float* gg, float* gb, cudaStream_t st) {
   const int rows = rows_per_cta_for(B, C);
   dim3 grid((C + kBnCols - 1) / kBnCols, (B + rows - 1) / rows);
-  bn_apply_bwd_kernel<<<grid, kBnCols * kBnRows, 0, st>>>(dy, ldd, x, ldx, B, C, mean, var, gamma, eps, dx, ldo, gg, gb, rows);
+  launch_pdl(bn_apply_bwd_kernel, grid, dim3(kBnCols * kBnRows), 0, st, dy, ldd, x, ldx, B, C, mean, var, gamma, eps, dx, ldo, gg, gb, rows);
 }
 
 }  // namespace tn

@@ -95,8 +95,18 @@ void launch_unique_assign(const long long* ids, int n, const float* labels, unsi
                           int* count, int* status, cudaStream_t st);
 
 // bn.cu
-void launch_bn_batch_stats(const float* x, int ld, int B, int C, const float* center, double* batch, cudaStream_t st);
-void launch_bn_table_append(const BnTableView& t, double* batch, cudaStream_t st);
+struct BnInput {                 // columns [0, nh) of a bf16 matrix of rows ldh long, then those of an fp32 matrix
+  const void* h;
+  int ldh, nh;
+  const float* x;
+  int ldx;
+};
+void launch_bn_batch_stats(const BnInput& in, int B, int C, const float* center, double* batch, cudaStream_t st);
+void launch_bn_table_append(const BnTableView& t, double* batch, bool drop_inc, cudaStream_t st);
+void launch_bn_join_fwd(const BnInput& in, int B, int C, const float* mean, const float* var, const float* gamma, const float* beta, float eps,
+                        void* z, int ldz, float* mean_out, float* var_out, cudaStream_t st);
+void launch_bn_join_bwd(const void* dz, int ldz, const BnInput& in, int B, int C, const float* mean, const float* var, const float* gamma,
+                        float eps, int mask, void* gh, float* gx, int ldg, float* gg, float* gb, cudaStream_t st);
 void launch_bn_table_refresh(const BnTableView& t, cudaStream_t st);
 void launch_bn_table_sync(const BnTableView& t, const BnSyncView& s, double* scratch, cudaStream_t st);
 void launch_bn_apply_fwd(const float* x, int ldx, int B, int C, const float* mean, const float* var, const float* gamma,

@@ -13,6 +13,7 @@ import torch
 from torch import nn
 
 from .. import core
+from ..ops import functional as F
 
 
 class _BnApply(torch.autograd.Function):
@@ -37,6 +38,34 @@ class _BnApply(torch.autograd.Function):
         gb = torch.zeros(x.shape[1], dtype=torch.float32, device=x.device) if ctx.has_beta else None
         ctx.table.ctx.apply_bwd(dy, x, mean, var, gamma, ctx.eps, dx, gg, gb)
         return dx, gg, gb, None, None
+
+
+class _BnJoin(torch.autograd.Function):
+    """``z = bf16([bn([h[:, :n_h] | x]) | 1 | 0])`` with :class:`_BnApply`'s mathematics, in one kernel each way; ``masked``: the
+    gradient of ``h`` is zero where ``h`` is not above zero (the backward pass of the ReLU that made it)."""
+
+    @staticmethod
+    def forward(ctx, h, x, gamma, beta, table, eps, n_h, masked):
+        C = n_h + x.shape[1]
+        z = torch.empty((h.shape[0], F.pad8(C + 1)), dtype=torch.bfloat16, device=h.device)
+        moments = torch.empty(2 * C, dtype=torch.float32, device=h.device)       # the table moves on before the backward pass runs
+        table.ctx.join_fwd(h, n_h, x, gamma, beta, float(eps), z, moments)
+        ctx.save_for_backward(h, x, gamma, moments)
+        ctx.table, ctx.meta, ctx.has_beta = table, (float(eps), n_h, masked), beta is not None
+        return z
+
+    @staticmethod
+    def backward(ctx, dz):
+        h, x, gamma, moments = ctx.saved_tensors
+        eps, n_h, masked = ctx.meta
+        C = n_h + x.shape[1]
+        gh = torch.empty_like(h) if ctx.needs_input_grad[0] else None
+        gx = torch.empty((x.shape[0], x.shape[1]), dtype=torch.float32, device=x.device) if ctx.needs_input_grad[1] else None
+        sums = torch.zeros((2, C), dtype=torch.float32, device=h.device)
+        gg = sums[0] if gamma is not None else None
+        gb = sums[1] if ctx.has_beta else None
+        ctx.table.ctx.join_bwd(dz.contiguous(), h, n_h, x, moments, gamma, eps, masked, gh, gx, gg, gb)
+        return gh, gx, gg, gb, None, None, None, None
 
 
 class TNBatchNormalizationBase(nn.Module):
@@ -104,19 +133,18 @@ class TNBatchNormalizationBase(nn.Module):
         self.moving_variance.copy_(torch.from_numpy(var))
 
     # ---- device path: statistics, table update and normalisation without leaving the GPU ------
-    def _device_push(self, x2: torch.Tensor, centered: bool):
-        self.table.push_batch(x2, centered)
-        if self.synchronized:
-            if torch.cuda.is_current_stream_capturing():
-                # a captured step replays the same launches every time, so the exchange cannot run every
-                # sync_freq-th step only: inside a CUDA graph it runs every step (one small kernel)
+    def _device_push(self, x2: torch.Tensor, centered: bool, h=None, n_h: int = 0):
+        # a captured step replays the same launches every time, so the exchange cannot run every
+        # sync_freq-th step only: inside a CUDA graph it runs every step (one small kernel)
+        exchange = self.synchronized and (torch.cuda.is_current_stream_capturing() or self.batch_counter + 1 == self.sync_freq)
+        alone = core.runtime().world == 1          # nobody to exchange with: the increments are not kept
+        self.table.push_batch(x2, centered, exchange and alone, h, n_h)
+        if exchange:
+            if not alone:
                 self.table.sync_increments()
-                self.batch_counter = 0
-                return
+            self.batch_counter = 0
+        elif self.synchronized:
             self.batch_counter += 1
-            if self.batch_counter == self.sync_freq:
-                self.table.sync_increments()
-                self.batch_counter = 0
 
     def _device_forward(self, inputs: torch.Tensor, training: bool, centered: bool):
         x2 = inputs.reshape(-1, inputs.shape[-1])
@@ -128,6 +156,13 @@ class TNBatchNormalizationBase(nn.Module):
         if training and centered:
             self._device_push(x2.detach(), True)
         return y.view(*inputs.shape[:-1], inputs.shape[-1])
+
+    def join_operand(self, h: torch.Tensor, n_h: int, x: torch.Tensor, masked: bool = False) -> torch.Tensor:
+        """``concat_cast([self(cat([h[:, :n_h].float(), x], 1))], ones=True)`` without the steps in between (device tables
+        only): ``h`` is a tower's padded bf16 output.  ``masked``: see :class:`_BnJoin`."""
+        if self.training:
+            self._device_push(x.detach(), False, h.detach(), n_h)
+        return _BnJoin.apply(h, x, self.gamma, self.beta, self.table, self.epsilon, n_h, masked)
 
     def bn_statistics_pull(self):
         """Fold the other ranks' pending increments in (called by rank 0 before saving)."""

@@ -7,6 +7,7 @@ from typing import Optional, Sequence
 
 import torch
 from torch import nn
+from torch.nn.modules import module as torch_hooks
 
 from .. import core, feature_column as fc
 from ..layers import DenseHead, EmbeddingFeatures, MLP, TNBatchNormalization
@@ -24,8 +25,23 @@ class WideDeepSubModel(nn.Module):
         self.bn = TNBatchNormalization(width, synchronized=True, sync_freq=4, max_count=1000000, name="both_bn") if use_bn else None
         self.head = DenseHead(width)
 
+    def _joins(self, x0, linear_emb) -> bool:
+        """Whether the tower's output and the batch norm go through the joint kernels: the layers are the package's own and
+        nobody looks at what passes between them."""
+        bn, mlp = self.bn, self.mlp
+        return (type(bn) is TNBatchNormalization and type(mlp) is MLP and bn.bn_table_handle is not None and bn._on_device and mlp.relu_last
+                and x0.is_cuda and x0.shape[0] > 0 and linear_emb.dim() == 2 and linear_emb.dtype == torch.float32 and linear_emb.stride(1) == 1
+                and not (torch_hooks._global_forward_hooks or torch_hooks._global_forward_pre_hooks or torch_hooks._global_backward_hooks
+                         or torch_hooks._global_backward_pre_hooks)
+                and not any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or "forward" in m.__dict__
+                            for m in (bn, mlp)))
+
     def forward(self, linear_emb, deep_emb, dense=None):
         x0 = F.concat_cast([deep_emb] + ([dense.float()] if self.dense_dim else []), ones=True)
+        if self._joins(x0, linear_emb):
+            # normalisation straight from the tower's output to the head's operand; its gradient comes back masked
+            h = self.mlp(x0, grad_premasked=True)
+            return self.head(self.bn.join_operand(h, self.mlp.out_dim, linear_emb, masked=True))
         h = self.mlp(x0)
         if self.bn is None:
             z = F.concat_cast([h, linear_emb], ones=True, widths=[self.mlp.out_dim, None])

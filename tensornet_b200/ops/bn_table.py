@@ -150,10 +150,11 @@ class GpuBnTable:
         self.ctx.refresh()
 
     # ---- device-side step -------------------------------------------------------------------
-    def push_batch(self, x: torch.Tensor, centered: bool = False):
+    def push_batch(self, x: torch.Tensor, centered: bool = False, drop_increments: bool = False, h: torch.Tensor = None, n_h: int = 0):
         """Fold the per-feature sums of ``x`` ([B, C] fp32) into the table; ``centered`` squares deviations
-        from the table's current mean (the PCTR variant)."""
-        self.ctx.push(x, bool(centered))
+        from the table's current mean (the PCTR variant).  ``h``: its first ``n_h`` columns (bf16) come before those of
+        ``x``.  ``drop_increments``: the pending increments go to zero, as by :meth:`sync_increments` on one GPU."""
+        self.ctx.push(x, bool(centered), bool(drop_increments), h, int(n_h))
 
     def sync_increments(self):
         """All ranks call this at the same step; a no-op with one GPU apart from dropping the increments."""

@@ -92,3 +92,49 @@ def test_pctr_bn_accumulates_deviation_from_current_mean(tn_gpu, status_ok):
     mg, vg = bn.table.get_moments()
     mh, vh = h.get_moments()
     assert np.allclose(mg, mh, rtol=1e-6, atol=1e-6) and np.allclose(vg, vh, rtol=1e-5)
+
+
+@pytest.mark.parametrize("B,n_h,L", [(1, 5, 1), (33, 32, 3), (700, 250, 26), (129, 64, 40)])
+@pytest.mark.parametrize("training", [False, True])
+def test_join_matches_the_steps_in_between(tn_gpu, status_ok, B, n_h, L, training):
+    """``join_operand`` against normalising the concatenation and building the operand: the same operand, gradients and
+    table to the bit but for gamma's and beta's gradients, sums of B 32-bit terms."""
+    tn = tn_gpu
+    dev = tn.core.runtime().device
+    F = tn.ops.functional
+    g = torch.Generator().manual_seed(B)
+    ldh = F.pad8(n_h + 1)
+    h0 = torch.relu(torch.randn((B, ldh), generator=g)).to(dev).bfloat16()
+    h0[:, n_h:] = 0
+    h0[:, n_h] = 1
+    x0 = torch.randn((B, L), generator=g).to(dev)
+    C = n_h + L
+    gz = torch.randn((B, F.pad8(C + 1)), generator=g).to(dev).bfloat16()
+    got = []
+    for joined in (False, True):
+        bn = tn.layers.TNBatchNormalization(C, synchronized=True, sync_freq=4, max_count=1000000, name=f"join{joined}{B}{training}")
+        with torch.no_grad():
+            bn.gamma.copy_(torch.linspace(0.5, 1.5, C))
+            bn.beta.copy_(torch.linspace(-0.5, 0.5, C))
+        bn.table.push_batch(torch.randn((50, C), generator=torch.Generator().manual_seed(1)).to(dev) * 2 + 1)
+        bn.train(training)
+        h, x = h0.clone().requires_grad_(), x0.clone().requires_grad_()
+        for _ in range(5):                               # across an exchange of the increments
+            h.grad = x.grad = bn.gamma.grad = bn.beta.grad = None
+            if joined:
+                z = bn.join_operand(h, n_h, x, masked=True)
+            else:
+                z = F.concat_cast([bn(torch.cat([h[:, :n_h].float(), x], dim=1))], ones=True)
+            z.backward(gz)
+        gh = h.grad.clone()
+        if not joined:
+            gh[:, :n_h] = torch.where(h0[:, :n_h] > 0, gh[:, :n_h], torch.zeros_like(gh[:, :n_h]))
+        got.append((z.detach(), gh, x.grad, bn.table.inc.clone(), bn.table.total_sum.clone(), bn.gamma.grad, bn.beta.grad, bn.batch_counter))
+    a, b = got
+    assert a[-1] == b[-1]
+    for k in range(3):
+        assert torch.equal(a[k], b[k]), k
+    for k in (3, 4):                                     # 64-bit sums whose order is free
+        assert bool(((a[k] - b[k]).abs() <= 1e-12 * (1 + a[k].abs())).all())
+    for k in (5, 6):
+        assert bool(((a[k] - b[k]).abs() <= B * 2.0 ** -23 * 20 + 1e-6).all())
