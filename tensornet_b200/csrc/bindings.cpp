@@ -1088,6 +1088,42 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     TORCH_CHECK(g.numel() % 8 == 0 && g.numel() == y.numel(), "relu_mask: numel must be a multiple of 8");
     tn::launch_relu_mask(g.data_ptr(), y.data_ptr(), g.numel(), cur_stream());
   });
+  {
+    // ws, bs (and their gradients): fp32 vectors of the input's width, one per layer
+    auto net = [](const at::Tensor& x0, const std::vector<at::Tensor>& ws, const std::vector<at::Tensor>& bs) {
+      TORCH_CHECK(x0.is_cuda() && x0.scalar_type() == at::kFloat && x0.is_contiguous() && x0.dim() == 2 && x0.size(0) >= 1 &&
+                      x0.size(1) <= tn::kCrossNetColumns, "cross_v1_net: input must be fp32 [B, D], D at most 1024");
+      TORCH_CHECK(!ws.empty() && ws.size() <= (size_t)tn::kMaxCrossLayers && bs.size() == ws.size(), "cross_v1_net: one to eight layers");
+      tn::CrossNet n{};
+      n.layers = (int)ws.size();
+      for (size_t l = 0; l < ws.size(); ++l) {
+        for (const at::Tensor& v : {ws[l], bs[l]})
+          TORCH_CHECK(v.is_cuda() && v.scalar_type() == at::kFloat && v.is_contiguous() && v.numel() == x0.size(1), "cross_v1_net: layer vectors");
+        n.w[l] = ptr_of<float>(ws[l]);
+        n.b[l] = ptr_of<float>(bs[l]);
+      }
+      return n;
+    };
+    m.def("cross_v1_net_fwd", [net](at::Tensor x0, std::vector<at::Tensor> ws, std::vector<at::Tensor> bs, at::Tensor y, at::Tensor dots) {
+      c10::cuda::CUDAGuard guard(x0.device());
+      tn::launch_cross_v1_net_fwd(net(x0, ws, bs), ptr_of<float>(x0), (int)x0.size(0), (int)x0.size(1), ptr_of<float>(y), ptr_of<float>(dots),
+                                  cur_stream());
+    });
+    m.def("cross_v1_net_bwd", [net](at::Tensor x0, std::vector<at::Tensor> ws, std::vector<at::Tensor> bs, at::Tensor dots, at::Tensor gy,
+                                    at::Tensor gx0, at::Tensor gw, at::Tensor gb, at::Tensor t_row) {
+      c10::cuda::CUDAGuard guard(x0.device());
+      tn::CrossNet n = net(x0, ws, bs);
+      TORCH_CHECK(gy.is_contiguous() && gy.scalar_type() == at::kFloat && gw.is_contiguous() && gb.is_contiguous() &&
+                      gw.numel() == n.layers * x0.size(1) && gb.numel() == gw.numel(), "cross_v1_net: gradients");
+      for (int l = 0; l < n.layers; ++l) {
+        n.gw[l] = ptr_of<float>(gw) + l * x0.size(1);
+        n.gb[l] = ptr_of<float>(gb) + l * x0.size(1);
+      }
+      tn::launch_cross_v1_net_bwd(n, ptr_of<float>(x0), (int)x0.size(0), (int)x0.size(1), ptr_of<float>(dots), ptr_of<float>(gy),
+                                  ptr_of<float>(gx0), ptr_of<float>(t_row), cur_stream());
+      g_launches.fetch_add(1, std::memory_order_relaxed);
+    });
+  }
   m.def("cross_v1_fwd", [](at::Tensor x0, at::Tensor xl, at::Tensor w, at::Tensor bias, at::Tensor y, at::Tensor dot) {
     c10::cuda::CUDAGuard guard(x0.device());
     tn::launch_cross_v1_fwd(ptr_of<float>(x0), ptr_of<float>(xl), ptr_of<float>(w), ptr_of<float>(bias), (int)x0.size(0),

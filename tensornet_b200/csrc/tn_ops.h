@@ -75,6 +75,18 @@ struct CrossTerms {              // gradient of each layer's output and its u, l
   const void* u[kMaxCrossLayers];
   int n;
 };
+struct CrossNet {                // a DCN-v1 cross network of up to kMaxCrossLayers layers, every vector [D]
+  const float* w[kMaxCrossLayers];
+  const float* b[kMaxCrossLayers];
+  float* gw[kMaxCrossLayers];    // added to by the backward pass
+  float* gb[kMaxCrossLayers];
+  int layers;
+};
+constexpr int kCrossNetColumns = 1024;   // widest input
+// dots, t_row: [layers][B], each layer's x_l . w_l and (backward, scratch) its gradient . x0
+void launch_cross_v1_net_fwd(const CrossNet& n, const float* x0, int B, int D, float* y, float* dots, cudaStream_t st);
+void launch_cross_v1_net_bwd(const CrossNet& n, const float* x0, int B, int D, const float* dots, const float* gy, float* gx0, float* t_row,
+                             cudaStream_t st);
 void launch_cross_v2_du(const void* g, const void* x0, void* du, long long n, cudaStream_t st);
 void launch_cross_v2_bwd_sum(const CrossTerms& t, const void* g0, void* out, long long n, cudaStream_t st);
 void launch_cross_v2_bwd_final(const float* gx0, const void* g, void* out, long long n, cudaStream_t st);

@@ -97,7 +97,4 @@ class DeepCrossLayer(nn.Module):
         self.bias = nn.ParameterList([nn.Parameter(torch.zeros(input_dim)) for _ in range(num_layer)])
 
     def forward(self, inputs: torch.Tensor) -> torch.Tensor:
-        cross = inputs
-        for w, b in zip(self.W, self.bias):
-            cross = F.cross_v1(inputs, cross, w, b)
-        return cross
+        return F.cross_v1_net(inputs, list(self.W), list(self.bias))

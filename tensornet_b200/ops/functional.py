@@ -429,6 +429,45 @@ def cross_v1(x0, xl, w, b):
     return x0 * (xl @ w.view(-1, 1)) + b + xl
 
 
+class _CrossV1Net(torch.autograd.Function):
+    """All layers of a rank-1 cross network over one input (``csrc/elementwise.cu``, ``cross_v1_net_*``)."""
+
+    @staticmethod
+    def forward(ctx, x0, L, *params):
+        x0 = x0.contiguous()
+        B, D = x0.shape
+        ws, bs = [w.reshape(-1) for w in params[:L]], list(params[L:])
+        y = torch.empty_like(x0)
+        dots = torch.empty((L, B), dtype=torch.float32, device=x0.device)
+        _ext().cross_v1_net_fwd(x0, ws, bs, y, dots)
+        ctx.save_for_backward(x0, dots, *params)
+        ctx.L = L
+        return y
+
+    @staticmethod
+    def backward(ctx, gy):
+        x0, dots, *params = ctx.saved_tensors
+        L = ctx.L
+        B, D = x0.shape
+        gx0 = torch.empty_like(x0)
+        sums = torch.zeros((2, L, D), dtype=torch.float32, device=x0.device)
+        _ext().cross_v1_net_bwd(x0, [w.reshape(-1) for w in params[:L]], list(params[L:]), dots, gy.contiguous(), gx0, sums[0], sums[1],
+                                torch.empty_like(dots))
+        return (gx0, None, *[sums[0, l].view(params[l].shape) for l in range(L)], *[sums[1, l].view(params[L + l].shape) for l in range(L)])
+
+
+def cross_v1_net(x0, ws, bs):
+    """``x_{l+1} = x0 * (x_l . w_l) + b_l + x_l`` from ``x_0 = x0`` on, for all layers."""
+    D = x0.shape[-1]
+    if (x0.is_cuda and x0.dim() == 2 and x0.dtype == torch.float32 and x0.shape[0] > 0 and D <= 1024 and 1 <= len(ws) <= 8
+            and all(p.device == x0.device and p.dtype == torch.float32 and p.is_contiguous() and p.numel() == D for p in (*ws, *bs))):
+        return _CrossV1Net.apply(x0, len(ws), *ws, *bs)
+    cross = x0
+    for w, b in zip(ws, bs):
+        cross = cross_v1(x0, cross, w, b)
+    return cross
+
+
 # =========================================================================================
 # DCN-v2 cross network  x_{l+1} = x0 * (W_l x_l + b_l) + x_l   on padded bf16 operands
 # =========================================================================================
