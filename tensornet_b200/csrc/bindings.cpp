@@ -716,14 +716,16 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                            ptr_of<float>(out), ptr_of<int>(lengths), cur_stream());
       })
       .def("deepfm_input_fwd", [](SparseCtx& self, at::Tensor inverse, int B, int S, int D, c10::optional<at::Tensor> dense, at::Tensor X0,
-                                  at::Tensor fm, int lin_col, c10::optional<at::Tensor> Lout, at::Tensor E, c10::optional<at::Tensor> req) {
+                                  at::Tensor fm, int lin_col, c10::optional<at::Tensor> Lout, c10::optional<at::Tensor> E,
+                                  c10::optional<at::Tensor> req) {
         c10::cuda::CUDAGuard guard(X0.device());
         const int Dd = dense ? (int)dense->size(1) : 0;
-        TORCH_CHECK(E.scalar_type() == at::kFloat && E.is_contiguous() && E.numel() == (int64_t)B * S * D, "deepfm_input: E must be fp32 [B, S * D]");
+        TORCH_CHECK(!E || (E->scalar_type() == at::kFloat && E->is_contiguous() && E->numel() == (int64_t)B * S * D),
+                    "deepfm_input: E must be fp32 [B, S * D]");
         const char* err = tn::launch_deepfm_input_fwd(self.source(req), ptr_of<int>(inverse), B, S, D, dense ? ptr_of<float>(*dense) : nullptr,
                                                       Dd, dense ? (int)dense->stride(0) : 0, X0.data_ptr(), (int)X0.stride(0),
                                                       ptr_of<float>(fm), Lout ? lin_col : -1, Lout ? ptr_of<float>(*Lout) : nullptr,
-                                                      ptr_of<float>(E), cur_stream());
+                                                      E ? ptr_of<float>(*E) : nullptr, cur_stream());
         if (err) throw std::runtime_error(err);
       });
   py::class_<ServeCtx>(m, "ServeCtx")
@@ -1083,10 +1085,13 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     c10::cuda::CUDAGuard guard(g.device());
     tn::launch_cross_v2_bwd_final(ptr_of<float>(gx0), g.data_ptr(), out.data_ptr(), g.numel(), cur_stream());
   });
-  m.def("relu_mask", [](at::Tensor g, at::Tensor y) {
+  m.def("relu_mask", [](at::Tensor g, at::Tensor y, at::Tensor out) {
     c10::cuda::CUDAGuard guard(g.device());
-    TORCH_CHECK(g.numel() % 8 == 0 && g.numel() == y.numel(), "relu_mask: numel must be a multiple of 8");
-    tn::launch_relu_mask(g.data_ptr(), y.data_ptr(), g.numel(), cur_stream());
+    TORCH_CHECK(g.numel() % 8 == 0 && g.numel() == y.numel() && g.numel() == out.numel(), "relu_mask: numel must be a multiple of 8");
+    for (const at::Tensor& v : {g, y, out})
+      TORCH_CHECK(v.is_contiguous() && v.scalar_type() == at::kBFloat16 && reinterpret_cast<uintptr_t>(v.data_ptr()) % 16 == 0,
+                  "relu_mask: contiguous bf16 tensors on 16 bytes");
+    tn::launch_relu_mask(g.data_ptr(), y.data_ptr(), out.data_ptr(), g.numel(), cur_stream());
   });
   {
     // ws, bs (and their gradients): fp32 vectors of the input's width, one per layer

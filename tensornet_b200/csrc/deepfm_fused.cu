@@ -27,7 +27,7 @@ __device__ __forceinline__ float wsum(float v) {
 
 // D % 4 == 0, dq = D/4 a power of two <= 32.  One warp per example.  The rows it has read are left in `E` as they are: the
 // backward pass then reads them as one run per example instead of gathering them once more (and does not depend on
-// what happens to the pulled rows in between).
+// what happens to the pulled rows in between); null when there is none.
 template <bool kInPlace>
 __global__ void __launch_bounds__(256, 6) deepfm_input_fwd_kernel(const RowSource src, const int* __restrict__ inverse, int B, int S, int D,
                                         const float* __restrict__ dense, int Dd, int ld_dense, __nv_bfloat16* __restrict__ X0, int ld,
@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(256, 6) deepfm_input_fwd_kernel(const RowSourc
       for (int k = 0; k < 4; ++k) {
         const int c = c0 + 32 * k + lane;
         if (c >= nch) continue;
-        *reinterpret_cast<float4*>(E + (size_t)b * S * D + 4 * c) = x[k];
+        if (E != nullptr) *reinterpret_cast<float4*>(E + (size_t)b * S * D + 4 * c) = x[k];
         s.x += x[k].x; s.y += x[k].y; s.z += x[k].z; s.w += x[k].w;
         sq += x[k].x * x[k].x + x[k].y * x[k].y + x[k].z * x[k].z + x[k].w * x[k].w;
         __nv_bfloat162 lo = __floats2bfloat162_rn(x[k].x, x[k].y), hi = __floats2bfloat162_rn(x[k].z, x[k].w);

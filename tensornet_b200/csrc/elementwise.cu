@@ -625,8 +625,8 @@ __global__ void __launch_bounds__(256) cross_v1_net_bwd_cols_kernel(const __grid
   }
 }
 
-// g[i] = y[i] > 0 ? g[i] : 0   (bf16, 8 elements per thread)
-__global__ void relu_mask_kernel(uint4* __restrict__ g, const uint4* __restrict__ y, long long n8) {
+// out[i] = y[i] > 0 ? g[i] : 0   (bf16, 8 elements per thread; `out` may be `g`)
+__global__ void relu_mask_kernel(const uint4* g, const uint4* __restrict__ y, uint4* out, long long n8) {
   pdl_sync();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n8; i += (long long)gridDim.x * blockDim.x) {
     uint4 gv = g[i]; const uint4 yv = y[i];
@@ -634,7 +634,7 @@ __global__ void relu_mask_kernel(uint4* __restrict__ g, const uint4* __restrict_
     const __nv_bfloat16* yp = reinterpret_cast<const __nv_bfloat16*>(&yv);
 #pragma unroll
     for (int k = 0; k < 8; ++k) if (!(__bfloat162float(yp[k]) > 0.f)) gp[k] = __float2bfloat16(0.f);
-    g[i] = gv;
+    out[i] = gv;
   }
 }
 
@@ -793,8 +793,9 @@ void launch_bce(const float* logit, const float* label, int B, float* pred, floa
                 int nbins, cudaStream_t st) {
   launch_pdl(bce_kernel, dim3(blocks_for(B, 256)), dim3(256), 0, st, logit, label, B, pred, dlogit, grad_scale, sums, nbins);
 }
-void launch_relu_mask(void* g, const void* y, long long n, cudaStream_t st) {
-  launch_pdl(relu_mask_kernel, dim3(blocks_for(n / 8, 256)), dim3(256), 0, st, reinterpret_cast<uint4*>(g), reinterpret_cast<const uint4*>(y), n / 8);
+void launch_relu_mask(const void* g, const void* y, void* out, long long n, cudaStream_t st) {
+  launch_pdl(relu_mask_kernel, dim3(blocks_for(n / 8, 256)), dim3(256), 0, st, reinterpret_cast<const uint4*>(g),
+             reinterpret_cast<const uint4*>(y), reinterpret_cast<uint4*>(out), n / 8);
 }
 void launch_cross_v2_bwd_elem(const void* g, const void* u, const void* x0, float* gx0, void* du, long long n, int first, cudaStream_t st) {
   launch_pdl(cross_v2_bwd_elem_kernel, dim3(blocks_for(n / 8, 256)), dim3(256), 0, st, reinterpret_cast<const uint4*>(g),

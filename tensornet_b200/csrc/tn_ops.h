@@ -67,7 +67,7 @@ void launch_cross_v1_fwd(const float* x0, const float* xl, const float* w, const
 constexpr int kCrossV1OneTile = 1024;   // wider rows take `row_scratch`: fp32 [B]
 void launch_cross_v1_bwd(const float* x0, const float* xl, const float* w, const float* dot, const float* gy, int B, int D,
                          float* gx0, float* gxl, float* gw, float* gb, float* row_scratch, cudaStream_t st);
-void launch_relu_mask(void* g, const void* y, long long n, cudaStream_t st);
+void launch_relu_mask(const void* g, const void* y, void* out, long long n, cudaStream_t st);
 void launch_cross_v2_bwd_elem(const void* g, const void* u, const void* x0, float* gx0, void* du, long long n, int first, cudaStream_t st);
 constexpr int kMaxCrossLayers = 8;
 struct CrossTerms {              // gradient of each layer's output and its u, last layer first; bf16
@@ -92,7 +92,7 @@ void launch_cross_v2_bwd_sum(const CrossTerms& t, const void* g0, void* out, lon
 void launch_cross_v2_bwd_final(const float* gx0, const void* g, void* out, long long n, cudaStream_t st);
 
 // deepfm_fused.cu  (return nullptr or a static error string)
-// `E`: the rows as they were read, [B, S * D] fp32, which the backward pass takes
+// `E` (may be null): the rows as they were read, [B, S * D] fp32, which the backward pass takes
 const char* launch_deepfm_input_fwd(const RowSource& src, const int* inverse, int B, int S, int D, const float* dense, int Dd, int ld_dense,
                                     void* X0, int ld, float* fm, int lin_col, float* Lout, float* E, cudaStream_t st);
 const char* launch_deepfm_input_bwd(const float* E, const int* inverse, int B, int S, int D, const void* dX0, int ld, const float* gfm,

@@ -11,6 +11,7 @@ from typing import Optional, Sequence
 
 import torch
 from torch import nn
+from torch.nn.modules import module as torch_hooks
 
 from .. import core, feature_column as fc
 from ..layers import DenseHead, EmbeddingFeatures, MLP
@@ -78,32 +79,60 @@ class DeepFM(Model):
         """Training loss through the fused DeepFM kernels (gather + FM + operand build in one kernel; head, loss and
         head backward in one kernel).  Returns None when the inputs do not qualify (ragged slots, CVM columns,
         CPU); the caller then uses the generic path."""
-        if not core.runtime().on_gpu or (self.linear_emb is None and not self.share_linear_table):
-            return None
         mlp = self.sub_model.mlp
-        dq = self.emb_dim // 4
-        if self.emb_dim % 4 or dq & (dq - 1) or dq > 32 or F.pad8(mlp.out_dim + 1) > 512 or self.sub_model.n_linear > 32:
+        if F.pad8(mlp.out_dim + 1) > 512 or self.sub_model.n_linear > 32:
             return None
-        got = self.deep_emb.fused_single_hot_inputs(features, True)
+        got = self._fused_inputs(features, True)
+        if got is None:
+            return None
+        x0, fm, lin = got
+        h = mlp(x0, grad_premasked=True)
+        loss, _ = F.deepfm_head_loss(h, lin, fm, self.sub_model.head.weight, labels.to(x0.device, non_blocking=True), sums,
+                                     mlp.out_dim)
+        return loss
+
+    def _fused_inputs(self, features, training):
+        """``(x0, fm, lin)``: the first layer's operand, FM term and linear weights through the fused input kernel, or None
+        when the inputs do not qualify."""
+        dq = self.emb_dim // 4
+        if (not core.runtime().on_gpu or (self.linear_emb is None and not self.share_linear_table) or self.emb_dim % 4 or dq & (dq - 1)
+                or dq > 32):
+            return None
+        got = self.deep_emb.fused_single_hot_inputs(features, training)
         if got is None:
             return None
         ids, B = got
         if not self.share_linear_table:
-            pull_together([self.linear_emb, self.deep_emb], features, True)
+            pull_together([self.linear_emb, self.deep_emb], features, training)
         self.deep_emb._args_cache = None            # its forward pass does not follow
         dense = features[self.dense_key].to(ids.device, non_blocking=True) if self.dense_dim else None
+        args = (self.deep_emb._anchor, self.deep_emb.link, ids, B, len(self.deep_emb._keys), dense, training)
         if self.share_linear_table:
-            x0, fm, lin = F.deepfm_input(self.deep_emb._anchor, self.deep_emb.link, ids, B, len(self.deep_emb._keys), dense, True,
-                                         self.emb_dim, self.emb_dim)
-        else:
-            lin = self.linear_emb(features, training=True)
-            x0, fm, _ = F.deepfm_input(self.deep_emb._anchor, self.deep_emb.link, ids, B, len(self.deep_emb._keys), dense, True)
-        h = mlp(x0, grad_premasked=True)
-        loss, _ = F.deepfm_head_loss(h, lin, fm, self.sub_model.head.weight, labels.to(ids.device, non_blocking=True), sums,
-                                     mlp.out_dim)
-        return loss
+            return F.deepfm_input(*args, self.emb_dim, self.emb_dim)
+        lin = self.linear_emb(features, training=training)
+        x0, fm, _ = F.deepfm_input(*args)
+        return x0, fm, lin
+
+    def _scores(self, features):
+        """The logits by way of the fused input kernel (scoring: no gradients, layers in inference mode), or None when the
+        batch does not qualify or somebody looks at what passes between the layers."""
+        own = [self.deep_emb, self.sub_model] + ([self.linear_emb] if self.linear_emb is not None else [])
+        if (torch.is_grad_enabled() or not self.use_fused or type(self.sub_model) is not DeepFMSubModel or not isinstance(features, dict)
+                or any(m.training for m in own) or type(self.deep_emb) is not EmbeddingFeatures
+                or any(m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__ for m in own)
+                or torch_hooks._global_forward_hooks or torch_hooks._global_forward_pre_hooks):
+            return None
+        got = self._fused_inputs(features, False)
+        if got is None:
+            return None
+        x0, fm, lin = got
+        mlp = self.sub_model.mlp
+        return self.sub_model.head(F.concat_cast([mlp(x0), lin, fm], ones=True, widths=[mlp.out_dim, None, None]))
 
     def forward(self, features):
+        logits = self._scores(features)
+        if logits is not None:
+            return logits
         if self.share_linear_table:
             both = self.deep_emb(features)
             both = both.view(both.shape[0], -1, self.emb_dim + 4)

@@ -189,8 +189,9 @@ class _MLP(torch.autograd.Function):
         B = gy.shape[0]
         g = gy.contiguous()
         if ctx.relu_last and not ctx.premasked:
-            g = g.clone()
-            ext.relu_mask(g, acts[L])
+            src = g if g.data_ptr() % 16 == 0 else g.clone()
+            g = torch.empty_like(src)
+            ext.relu_mask(src, acts[L], g)
         # The weight gradients are off the critical path (only the optimizer needs them): they run on a side
         # stream next to the input-gradient chain and are joined before this function returns.
         main = torch.cuda.current_stream()
@@ -369,10 +370,13 @@ class _BCE(torch.autograd.Function):
         ctx.save_for_backward(dl)
         ctx.shape = logit.shape
         ctx.mark_non_differentiable(pred)
+        ctx.set_materialize_grads(False)        # (no zeros for the prediction's)
         return s[0] - loss_before, pred.view(logit.shape)
 
     @staticmethod
     def backward(ctx, gloss, _gpred):
+        if gloss is None:
+            return None, None, None
         (dl,) = ctx.saved_tensors
         return (dl * gloss).view(ctx.shape), None, None
 
@@ -555,7 +559,7 @@ def cross_v2(x0: torch.Tensor, weights: Sequence[torch.Tensor], dim: int) -> tor
 # =========================================================================================
 class _DeepFMInput(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, anchor, link, ids, B, S, dense, training, emb_dim, lin_col):
+    def forward(ctx, anchor, link, ids, B, S, dense, training, emb_dim, lin_col, keep):
         inverse = link.pull_in_place(ids, None, 0, training)
         D = emb_dim
         Dd = 0 if dense is None else int(dense.shape[1])
@@ -563,7 +567,7 @@ class _DeepFMInput(torch.autograd.Function):
         x0 = torch.empty((B, ld), dtype=torch.bfloat16, device=ids.device)
         fm = torch.empty(B, dtype=torch.float32, device=ids.device)
         lin = torch.empty((B, S), dtype=torch.float32, device=ids.device) if lin_col >= 0 else None
-        emb = torch.empty((B, S * D), dtype=torch.float32, device=ids.device)
+        emb = torch.empty((B, S * D), dtype=torch.float32, device=ids.device) if keep else None      # for the backward pass
         link.ctx.deepfm_input_fwd(inverse, B, S, D, dense, x0, fm, lin_col, lin, emb, link.req)
         ctx.link, ctx.inverse, ctx.emb, ctx.meta = link, inverse, emb, (B, S, D, lin_col)
         if lin is None:
@@ -580,7 +584,7 @@ class _DeepFMInput(torch.autograd.Function):
         dl = glin.contiguous() if (lin_col >= 0 and glin is not None) else None
         _ext().deepfm_input_bwd(ctx.emb, ctx.inverse, B, S, D, gx0.contiguous(), gfm.contiguous().view(-1), link.gU,
                                 link.gstride, lin_col, dl)
-        return (None,) * 9
+        return (None,) * 10
 
 
 def deepfm_input(anchor, link, ids, B, S, dense=None, training=True, emb_dim=None, lin_col=-1):
@@ -589,7 +593,7 @@ def deepfm_input(anchor, link, ids, B, S, dense=None, training=True, emb_dim=Non
     the slot's linear weight in column ``lin_col`` (``emb_dim`` < row width), also returns those weights ``[B, S]``."""
     if dense is not None:
         dense = dense.float().contiguous()
-    x0, fm, lin = _DeepFMInput.apply(anchor, link, ids, B, S, dense, training, emb_dim or link.dim, lin_col)
+    x0, fm, lin = _DeepFMInput.apply(anchor, link, ids, B, S, dense, training, emb_dim or link.dim, lin_col, torch.is_grad_enabled())
     return x0, fm, (lin if lin_col >= 0 else None)
 
 
@@ -621,6 +625,7 @@ class _DeepFMHeadLoss(torch.autograd.Function):
         ctx.save_for_backward(dh, dl if dl is not None else dfm, dfm)
         ctx.has_lin = lin is not None
         ctx.mark_non_differentiable(pred)
+        ctx.set_materialize_grads(False)        # (no zeros for the prediction's)
         return loss, pred
 
     @staticmethod
