@@ -221,10 +221,7 @@ struct SparseCtx {
     c10::cuda::CUDAGuard guard(ids.device());
     tn::PullArgs a = batch_args(ids, inverse, labels, label_mod, training, lookup_only, front_done, n_dev, req);
     if (in_place()) {
-      tn::PullBatch batch{};
-      batch.n = 1;
-      batch.a[0] = a;
-      check(tn::launch_sparse_pull_local(batch, cur_stream()), "sparse_pull_local launch");
+      check(tn::launch_sparse_pull_local(&a, 1, cur_stream()), "sparse_pull_local launch");
       if (!front_done) g_launches.fetch_add(1, std::memory_order_relaxed);
       if (rows) check(tn::launch_sparse_pull_local_rows(a, cur_stream()), "sparse_pull_local_rows launch");
       return;
@@ -691,14 +688,13 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         TORCH_CHECK(n >= 1 && n <= (size_t)tn::kMaxPullBatch && ids.size() == n && inverse.size() == n && labels.size() == n &&
                         label_mod.size() == n && training.size() == n && n_dev.size() == n && req.size() == n, "pull_many: one entry per pull");
         c10::cuda::CUDAGuard guard(ids[0].device());
-        tn::PullBatch batch{};
-        batch.n = (int)n;
+        tn::PullArgs batch[tn::kMaxPullBatch];
         for (size_t k = 0; k < n; ++k) {
           TORCH_CHECK(ctx[k]->in_place(), "pull_many: in-place pulls only");
           for (size_t j = 0; j < k; ++j) TORCH_CHECK(ctx[j]->t.keys != ctx[k]->t.keys, "pull_many: different tables");
-          batch.a[k] = ctx[k]->batch_args(ids[k], inverse[k], labels[k], label_mod[k], training[k], false, front_done, n_dev[k], req[k]);
+          batch[k] = ctx[k]->batch_args(ids[k], inverse[k], labels[k], label_mod[k], training[k], false, front_done, n_dev[k], req[k]);
         }
-        check(tn::launch_sparse_pull_local(batch, cur_stream()), "sparse_pull_local launch");
+        check(tn::launch_sparse_pull_local(batch, (int)n, cur_stream()), "sparse_pull_local launch");
         if (!front_done) g_launches.fetch_add(1, std::memory_order_relaxed);
       })
       .def("pool_fwd", [](SparseCtx& self, at::Tensor inverse, c10::optional<at::Tensor> offsets, int B, int S, int combiner, at::Tensor out,

@@ -759,8 +759,11 @@ constexpr int kLocalThreads = 256;
 // Both kernels take the pulls of several tables at once (blockIdx.y): a model's pulls need only the ids of the batch, and a
 // small one is all latency.  Two of 10 K ids, one after the other and
 // together: 26 and 14 us.
-__global__ void __launch_bounds__(kLocalThreads, 4) pull_local_probe_kernel(const __grid_constant__ PullBatch batch) {
-  const PullArgs& a = batch.a[blockIdx.y];
+// (Launches of one table carry one table's arguments: a parameter block of 3 KB costs the host more than a microsecond.)
+template <int N> struct PullArgsOf { PullArgs a[N]; };
+template <int N>
+__global__ void __launch_bounds__(kLocalThreads, 4) pull_local_probe_kernel(const __grid_constant__ PullArgsOf<N> batch) {
+  const PullArgs& a = batch.a[N == 1 ? 0 : blockIdx.y];
   const TableView t = *a.tbl_dev;         // (changes between steps only: safe to read before the kernel ahead has finished)
   pdl_sync();
   const SparseCommView& c = a.c;
@@ -790,8 +793,9 @@ __global__ void __launch_bounds__(kLocalThreads) pull_local_resolve_kernel(const
   if (a.c.prof != nullptr && threadIdx.x == 0) atomicMax(&a.c.prof[18], globaltimer_ns());
 }
 
-__global__ void __launch_bounds__(kLocalThreads) pull_local_finish_kernel(const __grid_constant__ PullBatch batch) {
-  const PullArgs& a = batch.a[blockIdx.y];
+template <int N>
+__global__ void __launch_bounds__(kLocalThreads, 4) pull_local_finish_kernel(const __grid_constant__ PullArgsOf<N> batch) {
+  const PullArgs& a = batch.a[N == 1 ? 0 : blockIdx.y];
   const TableView t = *a.tbl_dev;
   pdl_sync();
   const SparseCommView& c = a.c;
@@ -1472,19 +1476,26 @@ static int local_grid(const PullArgs& args, bool clears) {
   return blocks < 1 ? 1 : (int)(blocks > 148ll * 4 ? 148ll * 4 : blocks);
 }
 
-// One GPU, rows left in the table (see pull_local_probe_kernel).  The pulls of a batch are all behind a front or all not.
-cudaError_t launch_sparse_pull_local(const PullBatch& batch, cudaStream_t stream) {
+template <int N>
+static cudaError_t launch_pulls(const PullArgs* pulls, int n, cudaStream_t stream) {
+  PullArgsOf<N> batch;
   int probe = 1, finish = 1;
-  for (int k = 0; k < batch.n; ++k) {
-    const PullArgs& a = batch.a[k];
-    if (a.front_done != batch.a[0].front_done) return cudaErrorInvalidValue;
-    probe = max(probe, local_grid(a, false));
-    finish = max(finish, local_grid(a, !a.front_done));
+  for (int k = 0; k < n; ++k) {
+    batch.a[k] = pulls[k];
+    if (pulls[k].front_done != pulls[0].front_done) return cudaErrorInvalidValue;
+    probe = max(probe, local_grid(pulls[k], false));
+    finish = max(finish, local_grid(pulls[k], !pulls[k].front_done));
   }
   const dim3 block(kLocalThreads);
   cudaError_t e = cudaSuccess;
-  if (!batch.a[0].front_done) e = launch_pdl(pull_local_probe_kernel, dim3(probe, batch.n), block, 0, stream, batch);
-  return e == cudaSuccess ? launch_pdl(pull_local_finish_kernel, dim3(finish, batch.n), block, 0, stream, batch) : e;
+  if (!pulls[0].front_done) e = launch_pdl(pull_local_probe_kernel<N>, dim3(probe, n), block, 0, stream, batch);
+  return e == cudaSuccess ? launch_pdl(pull_local_finish_kernel<N>, dim3(finish, n), block, 0, stream, batch) : e;
+}
+// One GPU, rows left in the table (see pull_local_probe_kernel).  The `n` pulls are all behind a front or all not.
+cudaError_t launch_sparse_pull_local(const PullArgs* pulls, int n, cudaStream_t stream) {
+  static_assert(kMaxPullBatch == 4, "instances below");
+  if (n < 1 || n > kMaxPullBatch) return cudaErrorInvalidValue;
+  return n == 1 ? launch_pulls<1>(pulls, n, stream) : n == 2 ? launch_pulls<2>(pulls, n, stream) : launch_pulls<4>(pulls, n, stream);
 }
 
 // The pulled rows also into the per-batch matrix.
@@ -1494,11 +1505,10 @@ cudaError_t launch_sparse_pull_local_rows(const PullArgs& args, cudaStream_t str
 }
 
 cudaError_t launch_sparse_pull_local_front(const PullArgs& args, cudaStream_t stream) {
-  PullBatch batch{};
-  batch.n = 1;
+  PullArgsOf<1> batch;
   batch.a[0] = args;
   const dim3 block(kLocalThreads);
-  const cudaError_t e = launch_pdl(pull_local_probe_kernel, dim3(local_grid(args, false)), block, 0, stream, batch);
+  const cudaError_t e = launch_pdl(pull_local_probe_kernel<1>, dim3(local_grid(args, false)), block, 0, stream, batch);
   return e != cudaSuccess ? e : launch_pdl(pull_local_resolve_kernel, dim3(local_grid(args, true)), block, 0, stream, args);
 }
 

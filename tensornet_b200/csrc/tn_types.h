@@ -81,12 +81,7 @@ struct PullArgs {
   int front_done;         // dedup, id dispatch and inverse map of this batch already ran (launch_sparse_pull_front)
 };
 
-// Pulls of different tables in one launch (one GPU).
-constexpr int kMaxPullBatch = 4;
-struct PullBatch {
-  PullArgs a[kMaxPullBatch];
-  int n;
-};
+constexpr int kMaxPullBatch = 4;      // pulls of different tables in one launch (one GPU)
 
 // Where the pulled row of position v is: row v of the per-batch matrix `U`, or (`row_of` not null; one GPU) row row_of[v]
 // of the table itself, whose descriptor `tbl` lies in device memory so that recorded launches follow a shard that grows.
@@ -182,7 +177,7 @@ cudaError_t launch_dense_step(const DenseStepArgs& a, cudaStream_t st);
 int dense_step_ctas_per_sm();      // resident CTAs of the multi-GPU dense kernel per SM
 cudaError_t launch_sparse_pull(const PullArgs& args, int work_items, cudaStream_t stream);
 // One GPU: the pull as ordinary kernels, rows read in place (or also written out to U), and its part that can run ahead.
-cudaError_t launch_sparse_pull_local(const PullBatch& batch, cudaStream_t stream);
+cudaError_t launch_sparse_pull_local(const PullArgs* pulls, int n, cudaStream_t stream);
 cudaError_t launch_sparse_pull_local_rows(const PullArgs& args, cudaStream_t stream);
 cudaError_t launch_sparse_pull_local_front(const PullArgs& args, cudaStream_t stream);
 cudaError_t launch_sparse_push(const PushArgs& args, int work_items, int max_ctas, const DenseStepArgs* dense, cudaStream_t stream);
