@@ -12,6 +12,7 @@ embedding_features.py:288-295, core/ps/optimizer/ada_grad_kernel.cc:121-128).
 """
 from __future__ import annotations
 
+import contextlib
 from typing import Dict, Optional, Sequence
 
 import torch
@@ -21,6 +22,7 @@ from .. import core
 from ..data.features import PACKED_KEY, gather_columns, padded_columns
 from ..feature_column import EmbeddingColumn
 from ..ops.embedding import expand_bag_labels, pull_pool
+from ..utils.hooks import unobserved
 
 
 class EmbeddingFeatures(nn.Module):
@@ -150,6 +152,8 @@ class EmbeddingFeatures(nn.Module):
             return None
         ids, offsets, B = self.stash_pull_args(features, training)[:3]
         if offsets is not None:
+            if not unobserved(self):          # a hook may still change what `forward` finds in `features`
+                self._args_cache = None
             return None
         self.table.set_training(training)
         self._pending_push = training and self.trainable
@@ -187,21 +191,36 @@ class EmbeddingFeatures(nn.Module):
         return core.show_decay(self.sparse_table_handle, delta_days)
 
 
-def pull_together(layers: Sequence[EmbeddingFeatures], features: Dict, training: Optional[bool] = None):
+@contextlib.contextmanager
+def pulled_together(layers: Sequence[EmbeddingFeatures], features: Dict, training: Optional[bool] = None):
+    """:func:`pull_together` around the forward passes that use it: a pull that none of them took is undone at the end."""
+    pulled = pull_together(layers, features, training)
+    try:
+        yield
+    finally:
+        if pulled:
+            for l in layers:
+                l.link.drop_pulled()
+
+
+def pull_together(layers: Sequence[EmbeddingFeatures], features: Dict, training: Optional[bool] = None) -> bool:
     """Run the pulls of several layers over one batch side by side (one GPU; their ids are all they need).  The
-    forward pass of every one of them has to follow; it then finds its pull done."""
+    forward pass of every one of them has to follow; it then finds its pull done.  A training pull counts shows and clicks
+    and creates rows, so it is run for ``features`` only where that is what the layers will be given: not when a hook or a
+    ``forward`` set on an instance comes in between."""
     rt = core.runtime()
-    if not rt.on_gpu or rt.world > 1 or not isinstance(features, dict) or not all(type(l) is EmbeddingFeatures for l in layers):
-        return
+    if (not rt.on_gpu or rt.world > 1 or not isinstance(features, dict) or not all(type(l) is EmbeddingFeatures for l in layers)
+            or not unobserved(*layers)):
+        return False
     if training is None:
         training = layers[0].training
         if any(l.training != training for l in layers):
-            return
+            return False
     if len({id(l.table) for l in layers}) < len(layers) or not all(l.link.ctx.in_place() for l in layers):
-        return
+        return False
     calls = []
     for l in layers:
         l.table.set_training(training)
         ids, offsets, _, labels, label_mod, count = l.stash_pull_args(features, training)
         calls.append((l.link, ids, labels, label_mod, count, l._n_dev(features, offsets)))
-    layers[0].link.pull_many(calls)
+    return layers[0].link.pull_many(calls)

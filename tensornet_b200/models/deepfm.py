@@ -11,13 +11,13 @@ from typing import Optional, Sequence
 
 import torch
 from torch import nn
-from torch.nn.modules import module as torch_hooks
 
 from .. import core, feature_column as fc
 from ..layers import DenseHead, EmbeddingFeatures, MLP
-from ..layers.embedding_features import pull_together
+from ..layers.embedding_features import pulled_together
 from ..model import Model
 from ..ops import functional as F
+from ..utils.hooks import unobserved
 
 
 class DeepFMSubModel(nn.Module):
@@ -102,15 +102,15 @@ class DeepFM(Model):
         if got is None:
             return None
         ids, B = got
-        if not self.share_linear_table:
-            pull_together([self.linear_emb, self.deep_emb], features, training)
-        self.deep_emb._args_cache = None            # its forward pass does not follow
         dense = features[self.dense_key].to(ids.device, non_blocking=True) if self.dense_dim else None
         args = (self.deep_emb._anchor, self.deep_emb.link, ids, B, len(self.deep_emb._keys), dense, training)
         if self.share_linear_table:
+            self.deep_emb._args_cache = None        # its forward pass does not follow
             return F.deepfm_input(*args, self.emb_dim, self.emb_dim)
-        lin = self.linear_emb(features, training=training)
-        x0, fm, _ = F.deepfm_input(*args)
+        with pulled_together([self.linear_emb, self.deep_emb], features, training):
+            self.deep_emb._args_cache = None
+            lin = self.linear_emb(features, training=training)
+            x0, fm, _ = F.deepfm_input(*args)
         return x0, fm, lin
 
     def _scores(self, features):
@@ -119,8 +119,7 @@ class DeepFM(Model):
         own = [self.deep_emb, self.sub_model] + ([self.linear_emb] if self.linear_emb is not None else [])
         if (torch.is_grad_enabled() or not self.use_fused or type(self.sub_model) is not DeepFMSubModel or not isinstance(features, dict)
                 or any(m.training for m in own) or type(self.deep_emb) is not EmbeddingFeatures
-                or any(m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__ for m in own)
-                or torch_hooks._global_forward_hooks or torch_hooks._global_forward_pre_hooks):
+                or not unobserved(*own)):
             return None
         got = self._fused_inputs(features, False)
         if got is None:
@@ -141,9 +140,11 @@ class DeepFM(Model):
             dense = features[self.dense_key].to(deep.device, non_blocking=True) if self.dense_dim else None
             return self.sub_model(lin, deep, dense)
         if self.linear_emb is not None:
-            pull_together([self.linear_emb, self.deep_emb], features)
-        lin = self.linear_emb(features) if self.linear_emb is not None else None
-        deep = self.deep_emb(features)
+            with pulled_together([self.linear_emb, self.deep_emb], features):
+                lin = self.linear_emb(features)
+                deep = self.deep_emb(features)
+        else:
+            lin, deep = None, self.deep_emb(features)
         dense = None
         if self.dense_dim:
             dense = features[self.dense_key].to(deep.device, non_blocking=True)

@@ -7,13 +7,13 @@ from typing import Optional, Sequence
 
 import torch
 from torch import nn
-from torch.nn.modules import module as torch_hooks
 
 from .. import core, feature_column as fc
 from ..layers import DenseHead, EmbeddingFeatures, MLP, TNBatchNormalization
-from ..layers.embedding_features import pull_together
+from ..layers.embedding_features import pulled_together
 from ..model import Model
 from ..ops import functional as F
+from ..utils.hooks import unobserved
 
 
 class WideDeepSubModel(nn.Module):
@@ -31,10 +31,7 @@ class WideDeepSubModel(nn.Module):
         bn, mlp = self.bn, self.mlp
         return (type(bn) is TNBatchNormalization and type(mlp) is MLP and bn.bn_table_handle is not None and bn._on_device and mlp.relu_last
                 and x0.is_cuda and x0.shape[0] > 0 and linear_emb.dim() == 2 and linear_emb.dtype == torch.float32 and linear_emb.stride(1) == 1
-                and not (torch_hooks._global_forward_hooks or torch_hooks._global_forward_pre_hooks or torch_hooks._global_backward_hooks
-                         or torch_hooks._global_backward_pre_hooks)
-                and not any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or "forward" in m.__dict__
-                            for m in (bn, mlp)))
+                and unobserved(bn, mlp, backward=True))
 
     def forward(self, linear_emb, deep_emb, dense=None):
         x0 = F.concat_cast([deep_emb] + ([dense.float()] if self.dense_dim else []), ones=True)
@@ -68,8 +65,8 @@ class WideDeep(Model):
                                           dense_dim, dnn_hidden_units, use_bn)
 
     def forward(self, features):
-        pull_together([self.linear_emb, self.deep_emb], features)
-        lin = self.linear_emb(features)
-        deep = self.deep_emb(features)
+        with pulled_together([self.linear_emb, self.deep_emb], features):
+            lin = self.linear_emb(features)
+            deep = self.deep_emb(features)
         dense = features[self.dense_key].to(deep.device, non_blocking=True) if self.dense_dim else None
         return self.sub_model(lin, deep, dense)

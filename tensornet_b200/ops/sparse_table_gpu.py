@@ -11,7 +11,7 @@ from __future__ import annotations
 
 import math
 import weakref
-from typing import Optional, Tuple
+from typing import NamedTuple, Optional, Tuple
 
 import numpy as np
 import torch
@@ -111,7 +111,7 @@ class GpuSparseTable:
     def _drop_fronts(self):
         """Rows move or go: on one GPU a pull that started ahead has already looked its signs up."""
         for lk in self.links:
-            lk._pulled = None
+            lk.drop_pulled()
             if lk._front is not None and lk.ctx.in_place():
                 lk.discard_front()
 
@@ -292,6 +292,20 @@ def front_stream(device) -> "torch.cuda.Stream":
     return st
 
 
+class _Pulled(NamedTuple):
+    """A pull that was run ahead.  The tensors are held so that their addresses stay theirs."""
+    tensors: tuple
+    inputs: tuple
+    label_mod: int
+    training: bool
+    inverse: torch.Tensor
+
+
+def _marks(*tensors):
+    """What tells a pull's inputs from others: address, length and version of each."""
+    return tuple(None if t is None else (t.data_ptr(), t.numel(), None if t.is_inference() else t._version) for t in tensors)
+
+
 class GpuSparseLink:
     """Per-layer exchange state of a table: symmetric inboxes, the per-batch unique-row matrix
     ``U``, its gradient ``gU`` and the bookkeeping that ties one pull to the following push."""
@@ -365,7 +379,7 @@ class GpuSparseLink:
         self.front_in_flight = False # a front was forked onto the side stream during this step (the model joins it)
         self.front_hits = 0          # pulls that found their front done (a model checks that its layers really pull)
         self._fork = torch.cuda.Event() if runtime().on_gpu else None
-        self._pulled = None          # (ids, their version, training, inverse) of a pull that was run for the forward pass to come
+        self._pulled = None          # a pull that was run for the forward pass to come (see pull_many)
         self.req = None              # rows of the batch at hand, when its pull started ahead on one GPU (else the link's own array)
         self._front_req = {}
         self._front_inverse = {}     # inverse buffers of the fronts, one per id buffer (stable addresses for CUDA graphs)
@@ -387,10 +401,11 @@ class GpuSparseLink:
         return self._pull(ids, labels, label_mod, training, None, lookup_only, n_dev, False)
 
     def _pull(self, ids, labels, label_mod, training, inverse, lookup_only, n_dev, rows):
-        n, done, self._pulled = ids.numel(), self._pulled, None
-        if (done is not None and not rows and not lookup_only and done[0].data_ptr() == ids.data_ptr() and done[0].numel() == n
-                and done[0]._version == done[1] and done[2] == bool(training)):
-            return done[3]
+        done = self._pulled
+        if (done is not None and not rows and not lookup_only and done.training == bool(training) and done.label_mod == int(label_mod)
+                and done.inputs == _marks(ids, labels, n_dev)):
+            self._pulled = None
+            return done.inverse
         inverse, front_done = self._begin(ids, training, lookup_only, inverse)
         with phase("tn.sparse_pull"):
             self.ctx.pull(ids.reshape(-1), inverse, labels, int(label_mod), bool(training), bool(lookup_only), front_done, n_dev, rows,
@@ -399,6 +414,7 @@ class GpuSparseLink:
 
     def _begin(self, ids, training, lookup_only=False, inverse=None):
         """``(inverse, front_done)`` for a pull of ``ids``; a front that ran for another batch is discarded."""
+        self.drop_pulled()
         n = ids.numel()
         front, self._front = self._front, None
         front_done, self.req = False, None
@@ -413,6 +429,13 @@ class GpuSparseLink:
         self._last_n_ids = n
         return inverse, front_done
 
+    def drop_pulled(self):
+        """Undo a pull that was run ahead and that no forward pass has asked for: the shows and clicks it counted go (the
+        rows it created stay, as those of any batch that is pulled and not trained on)."""
+        done, self._pulled = self._pulled, None
+        if done is not None and done.training:
+            self.cnts.zero_()
+
     @staticmethod
     def pull_many(calls):
         """In-place pulls of different tables in one go.  ``calls``: ``(link, ids, labels, label_mod, training, n_dev)`` of
@@ -420,7 +443,7 @@ class GpuSparseLink:
         done) where they do not go together."""
         links = [c[0] for c in calls]
         if not 2 <= len(calls) <= 4 or len({id(lk.table) for lk in links}) < len(links) or not all(lk.ctx.in_place() for lk in links) or \
-                any(c[1].is_inference() for c in calls):
+                any(t is not None and t.is_inference() for _, ids, labels, _, _, n_dev in calls for t in (ids, labels, n_dev)):
             return False
         begun = [lk._begin(ids, training) for lk, ids, _, _, training, _ in calls]
         # (a model runs every front ahead or none: a mixture is two calls of different batches, and goes one by one)
@@ -430,8 +453,8 @@ class GpuSparseLink:
                 links[0].table.ext.SparseCtx.pull_many(
                     [links[k].ctx for k in at], [calls[k][1].reshape(-1) for k in at], [begun[k][0] for k in at], [calls[k][2] for k in at],
                     [int(calls[k][3]) for k in at], [bool(calls[k][4]) for k in at], done, [calls[k][5] for k in at], [links[k].req for k in at])
-        for (lk, ids, _, _, training, _), (inverse, _) in zip(calls, begun):
-            lk._pulled = (ids, ids._version, bool(training), inverse)
+        for (lk, ids, labels, label_mod, training, n_dev), (inverse, _) in zip(calls, begun):
+            lk._pulled = _Pulled((ids, labels, n_dev), _marks(ids, labels, n_dev), int(label_mod), bool(training), inverse)
         return True
 
     def fork_front(self):
