@@ -136,7 +136,8 @@ class Runtime:
     def raise_status(self, code: int, phase: int, aux: int):
         """A kernel reported ``code``.  Until :func:`tensornet_b200.core.recover` has run, every fused kernel skips
         its work (they all test the status word first), so nothing is half-applied behind the error; the runtime is
-        marked failed and says so in the exception."""
+        marked failed and says so in the exception.  On one GPU the step that met a full table runs to its end, as does a
+        pull that had started ahead of its step: signs that found no room have no row, all others are as ever."""
         self.failed = True
         raise DeviceError(code, phase, aux)
 

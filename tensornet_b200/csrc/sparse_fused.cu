@@ -61,6 +61,11 @@ __device__ __forceinline__ int warp_alloc(int* counter, unsigned mask) {
   return base + __popc(mask & lanemask_lt());
 }
 
+// One GPU: word of `bar` that is set when an error has been met by the time a batch's signs are looked up.  All CTAs of the
+// kernels behind go by this word: the status word may change while they run, by their own insertions or those of another
+// table in the same launch, and CTAs that start later would do otherwise than those that went before.
+constexpr int kLocalSkip = 5;
+
 // ---- dedup of a batch ------------------------------------------------------------------------------------------
 // A warp takes `per` x 32 ids at a time (a lane: ids base + lane, base + 32 + lane, ...).  What a batch costs here is the
 // latency of the dedup table, which is why a lane has several probes in flight, and the counter that hands out
@@ -138,6 +143,7 @@ __device__ __forceinline__ void dedup_assign(const PullArgs& a, const TableView&
       }
       if (todo != 0 && probes > c.dd_mask) {
         set_status(c.status, kDedupOverflow, 1, 0);
+        if (kLocal) c.bar[kLocalSkip] = 1;
 #pragma unroll
         for (int k = 0; k < kDedupIds; ++k) if ((todo >> k) & 1u) hw[k] = 0xffffffffu;
         break;
@@ -200,6 +206,7 @@ __device__ __forceinline__ void dedup_assign(const PullArgs& a, const TableView&
       if (winner) {
         if (pos >= capo) {
           set_status(c.status, kOwnerSegOverflow, 1, owner);
+          if (kLocal) c.bar[kLocalSkip] = 1;
           c.dd_vals[hw[k]] = -1;
         } else {
           c.stage_ids[owner * capo + pos] = key[k];
@@ -771,6 +778,7 @@ __global__ void __launch_bounds__(kLocalThreads, 4) pull_local_probe_kernel(cons
   const int n_ids = batch_ids(a);
   if (c.prof != nullptr && tid == 0) c.prof[a.front_done ? 16 : 0] = globaltimer_ns();
   if (ld_volatile_s32(c.status) != 0) {   // an earlier error has not been dealt with: no id has a row
+    if (threadIdx.x == 0) c.bar[kLocalSkip] = 1;
     for (int i = tid; i < n_ids; i += nth) a.inverse[i] = -1;
     return;
   }
@@ -805,11 +813,11 @@ __global__ void __launch_bounds__(kLocalThreads, 4) pull_local_finish_kernel(con
   if (a.front_done) { prof_mark(c, 0); prof_mark(c, 1); }
   prof_mark(c, 2);
   if (threadIdx.x == 0) {
-    s_bad = ld_volatile_s32(c.status);
+    s_bad = (int)__ldcg(&c.bar[kLocalSkip]);
     s_new = __ldcg(c.ocount);
   }
   __syncthreads();
-  const bool bad = s_bad != 0;            // (the state this CTA started in: what it sets itself comes later)
+  const bool bad = s_bad != 0;
   const int n_new = s_new;
   if (threadIdx.x == 0) {
     // the CTA that is the last to have read the counters leaves them ready for the next pull: no tail at the end
@@ -819,6 +827,7 @@ __global__ void __launch_bounds__(kLocalThreads, 4) pull_local_finish_kernel(con
       c.cnt[0] = 0;
       *c.ocount = 0;
       c.bar[3] = 0;
+      c.bar[kLocalSkip] = 0;
       *c.epoch = __ldcg(c.epoch) + 1ull;
     }
   }

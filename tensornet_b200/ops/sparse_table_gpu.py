@@ -500,6 +500,7 @@ class GpuSparseLink:
         self._loc["cnt"].zero_()
         if self.ctx.in_place():
             self._loc["ocount"].zero_()      # signs without a row
+            self._loc["bar"].zero_()         # (an error that the front met)
         self.table.epoch.add_(1)
 
     def push(self):
