@@ -59,7 +59,8 @@ __device__ __forceinline__ void tile_of(const PairTiles& g, int t, int* tile_m, 
 }
 
 // kNB: 256-column MMA blocks per tile (2 for BN = 512); kStages: operand ring depth; kEpiW: epilogue warps (a multiple of
-// four: warp w reads TMEM lane quarter w % 4; sixteen of them only where the epilogue has no auxiliary operands).  Threads: warp 0 TMA, warp 1 MMA + TMEM owner, then the epilogue warps.
+// four: warp w reads TMEM lane quarter w % 4; sixteen of them only where the epilogue has no auxiliary operands).
+// Threads: warp 0 TMA, warp 1 MMA + TMEM owner, then the epilogue warps.
 template <int kNB, int kStages, int kEpiW>
 __global__ void __launch_bounds__(32 * (2 + kEpiW), 1)
 gemm_bf16_2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p,
@@ -228,7 +229,7 @@ gemm_bf16_2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       const int row_base = tile_m * 2 * kBM + (int)rank * kBM + q * 32;
       if (kEpiW != 16) gemm_epi::prefetch_aux(p, row_base, tile_n * BN, BN, sub, kEpiW / 4, lane);
       const uint32_t tm_lane = tmem + ((uint32_t)(q * 32) << 16) + a * (uint32_t)BN;
-      if (!gemm_epi::store_rows<kEpiW != 16>(p, tm_lane, row_base, tile_n * BN, BN, sub, kEpiW / 4, lane, sm_out, ready)) { ok = false; break; }
+      if (!gemm_epi::store_rows<kEpiW != 16 ? gemm_epi::kAny : gemm_epi::kNoAux>(p, tm_lane, row_base, tile_n * BN, BN, sub, kEpiW / 4, lane, sm_out, ready)) { ok = false; break; }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_remote(acc_empty_even + a * (uint32_t)sizeof(uint64_t));

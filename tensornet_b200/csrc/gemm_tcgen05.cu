@@ -31,6 +31,8 @@
 namespace tn {
 
 using namespace tc;
+using gemm_epi::kAny;
+using gemm_epi::kBf16;
 
 namespace {
 
@@ -43,7 +45,7 @@ constexpr int kEpiWarps = 4 * kEpiSubs;
 constexpr int kGemmThreads = 32 * (2 + kEpiWarps);   // warp0 TMA, warp1 MMA + TMEM owner, the rest epilogue
 constexpr int kEpiBytesPerWarp = gemm_epi::kBytesPerWarp;
 
-template <int kStages, int kHalves>
+template <int kStages, int kHalves, gemm_epi::Kinds kKinds>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                          const GemmParams p) {
@@ -220,7 +222,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
       for (int half = 0; half < halves; ++half) {
         const int row_base = m0 + half * kBM + q * 32;
         const uint32_t tm_lane = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(half * 256);
-        if (!gemm_epi::store_rows<true>(p, tm_lane, row_base, n0, BN, sub, kEpiSubs, lane, sm_out, ready)) break;
+        if (!gemm_epi::store_rows<kKinds>(p, tm_lane, row_base, n0, BN, sub, kEpiSubs, lane, sm_out, ready)) break;
       }
     }
   }
@@ -444,10 +446,10 @@ const char* gemm_bf16(const GemmDesc& d, cudaStream_t stream) {
   if (smem < epi_bytes) smem = epi_bytes;
   static bool attr_set = false;
   if (!attr_set) {
-    cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<6, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<4, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<3, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+    for (auto* k : {gemm_bf16_tcgen05_kernel<8, 1, kBf16>, gemm_bf16_tcgen05_kernel<6, 1, kBf16>, gemm_bf16_tcgen05_kernel<4, 1, kBf16>,
+                    gemm_bf16_tcgen05_kernel<3, 2, kBf16>, gemm_bf16_tcgen05_kernel<8, 1, kAny>, gemm_bf16_tcgen05_kernel<6, 1, kAny>,
+                    gemm_bf16_tcgen05_kernel<4, 1, kAny>, gemm_bf16_tcgen05_kernel<3, 2, kAny>})
+      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
     attr_set = true;
   }
   // launched as a programmatic dependent of whatever precedes it in the stream (plain serialisation when the
@@ -462,13 +464,20 @@ const char* gemm_bf16(const GemmDesc& d, cudaStream_t stream) {
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = use_pdl ? 1 : 0;
+  // Plain bf16 outputs (forward products) have instances of their own.  With all epilogues in one kernel the plain one takes
+  // 0.2 to 0.7 us longer where its instructions are at hand (512 x 512 x 1025 8.9 -> 9.1, 8192 x 400 x 401 9.85 -> 10.35,
+  // launch to launch) and 2 us where the kernel runs once between others, as in a request of 512 examples (a pass 93.5 ->
+  // 97.6).  Everything else stays together: each further kernel of a short step is one more that starts without its
+  // instructions (1024 examples through 64-32: 1 560 us a pass; fp32 outputs beside the plain ones 1 630; all in one 1 620).
+  const bool plain = !d.out_f32 && !d.mask_aux && !d.had_x0 && !d.had_xl;
   cudaError_t e;
   if (smem > 220 * 1024) return "gemm_bf16: tile does not fit in shared memory";
   cfg.dynamicSmemBytes = smem;
-  if (halves == 2) e = cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_kernel<3, 2>, tmA, tmB, p);
-  else if (stages == 8) e = cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_kernel<8, 1>, tmA, tmB, p);
-  else if (stages == 6) e = cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_kernel<6, 1>, tmA, tmB, p);
-  else e = cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_kernel<4, 1>, tmA, tmB, p);
+  auto* kernel = halves == 2   ? (plain ? gemm_bf16_tcgen05_kernel<3, 2, kBf16> : gemm_bf16_tcgen05_kernel<3, 2, kAny>)
+                 : stages == 8 ? (plain ? gemm_bf16_tcgen05_kernel<8, 1, kBf16> : gemm_bf16_tcgen05_kernel<8, 1, kAny>)
+                 : stages == 6 ? (plain ? gemm_bf16_tcgen05_kernel<6, 1, kBf16> : gemm_bf16_tcgen05_kernel<6, 1, kAny>)
+                               : (plain ? gemm_bf16_tcgen05_kernel<4, 1, kBf16> : gemm_bf16_tcgen05_kernel<4, 1, kAny>);
+  e = cudaLaunchKernelEx(&cfg, kernel, tmA, tmB, p);
   if (e == cudaSuccess) e = cudaGetLastError();
   return e == cudaSuccess ? nullptr : cudaGetErrorString(e);
 }

@@ -228,6 +228,37 @@ def test_hadamard_epilogue_keeps_pre_activation_and_residual_mode(tn_gpu, status
     assert _rel_err(R, A.float() @ B.float().t() + xl.float()) < 2e-2
 
 
+@pytest.mark.parametrize("M,N,K,BN,halves", [(1, 16, 8, 0, 0), (200, 80, 200, 0, 0), (333, 256, 380, 64, 1), (512, 512, 1025, 128, 1),
+                                             (130, 100, 700, 256, 1), (300, 300, 450, 128, 2)])
+@pytest.mark.parametrize("b_mn", [False, True])
+def test_products_with_and_without_auxiliary_operands(tn_gpu, status_ok, M, N, K, BN, halves, b_mn):
+    """Every ring depth, one and two accumulators: a mask that keeps everything and a residual of zeros change nothing."""
+    dev = tn_gpu.core.runtime().device
+    p8 = lambda n: (n + 7) // 8 * 8
+    g = torch.Generator(device="cpu").manual_seed(M + N + K)
+    A = torch.zeros(M, p8(K)).bfloat16()
+    A[:, :K] = torch.randn(M, K, generator=g).bfloat16()
+    rows, cols = (K, N) if b_mn else (N, K)
+    B = torch.zeros(rows, p8(cols)).bfloat16()
+    B[:, :cols] = (torch.randn(rows, cols, generator=g) * 0.1).bfloat16()
+    A, B = A.to(dev), B.to(dev)
+    ld = p8(N + 1)
+    got = []
+    for aux in ("none", "mask", "residual"):
+        C = torch.full((M, ld), 7.0, dtype=torch.bfloat16, device=dev)
+        operand = torch.full((M, ld), 1.0 if aux == "mask" else 0.0, dtype=torch.bfloat16, device=dev)
+        _ext().gemm(A, B, C, M, N, K, p8(K), p8(cols), ld, False, b_mn, False, False, None, operand if aux == "mask" else None, None,
+                    operand if aux == "residual" else None, ld, N, ld, 1, BN, tn_gpu.core.runtime().status, m_halves=halves)
+        got.append(C)
+    a, b = A[:, :K].double(), B[:, :cols].double()
+    ref = a @ (b if b_mn else b.t())
+    # sums in 32 bits and one rounding to bf16
+    bound = 2.0 ** -8 * ref.abs() + 2.0 ** -23 * K * (a.abs() @ (b if b_mn else b.t()).abs())
+    assert bool(((got[0][:, :N].double() - ref).abs() <= bound).all())
+    assert bool((got[0][:, N] == 1).all()) and bool((got[0][:, N + 1:] == 0).all())
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+
+
 def test_cross_v2_backward_elementwise_kernels(tn_gpu, status_ok):
     dev = tn_gpu.core.runtime().device
     n = 256 * 136
