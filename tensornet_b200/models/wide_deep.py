@@ -33,9 +33,10 @@ class WideDeepSubModel(nn.Module):
                 and x0.is_cuda and x0.shape[0] > 0 and linear_emb.dim() == 2 and linear_emb.dtype == torch.float32 and linear_emb.stride(1) == 1
                 and unobserved(bn, mlp, backward=True))
 
-    def forward(self, linear_emb, deep_emb, dense=None):
+    def forward(self, linear_emb, deep_emb, dense=None, fused: bool = True):
+        """``fused``: the joint kernels may be used (a model's ``use_fused``)."""
         x0 = F.concat_cast([deep_emb] + ([dense.float()] if self.dense_dim else []), ones=True)
-        if self._joins(x0, linear_emb):
+        if fused and self._joins(x0, linear_emb):
             # normalisation straight from the tower's output to the head's operand; its gradient comes back masked
             h = self.mlp(x0, grad_premasked=True)
             return self.head(self.bn.join_operand(h, self.mlp.out_dim, linear_emb, masked=True))
@@ -69,4 +70,7 @@ class WideDeep(Model):
             lin = self.linear_emb(features)
             deep = self.deep_emb(features)
         dense = features[self.dense_key].to(deep.device, non_blocking=True) if self.dense_dim else None
-        return self.sub_model(lin, deep, dense)
+        sub = self.sub_model
+        if not self.use_fused and type(sub) is WideDeepSubModel and "forward" not in sub.__dict__:
+            return sub(lin, deep, dense, fused=False)
+        return sub(lin, deep, dense)

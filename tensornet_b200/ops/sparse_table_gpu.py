@@ -414,7 +414,8 @@ class GpuSparseLink:
 
     def _begin(self, ids, training, lookup_only=False, inverse=None):
         """``(inverse, front_done)`` for a pull of ``ids``; a front that ran for another batch is discarded."""
-        self.drop_pulled()
+        if self._pulled is not None:
+            self.drop_pulled()
         n = ids.numel()
         front, self._front = self._front, None
         front_done, self.req = False, None

@@ -138,3 +138,21 @@ def test_join_matches_the_steps_in_between(tn_gpu, status_ok, B, n_h, L, trainin
         assert bool(((a[k] - b[k]).abs() <= 1e-12 * (1 + a[k].abs())).all())
     for k in (5, 6):
         assert bool(((a[k] - b[k]).abs() <= B * 2.0 ** -23 * 20 + 1e-6).all())
+
+
+def test_use_fused_holds_for_the_joint_kernels(tn_gpu, status_ok):
+    """``use_fused = False`` keeps Wide&Deep's tower, batch norm and head apart, in training and in scoring."""
+    tn = tn_gpu
+    torch.manual_seed(1)
+    slots, B = ["a", "b"], 40
+    m = tn.models.WideDeep(slots, slots, dnn_hidden_units=(16, 8), embedding_dim=8, bucket_size=4 * B, table_rows=1 << 12)
+    m.compile(optimizer=tn.optimizer.Optimizer(tn.core.Adam(learning_rate=1e-3)), cuda_graph=False)
+    f = {tn.data.PACKED_KEY: tn.data.PackedFeatures(slots, ids=torch.arange(2 * B).view(2, B) % 50)}
+    y = (torch.arange(B) % 3 == 0).float()
+    joined, join = [], m.sub_model.bn.join_operand
+    m.sub_model.bn.join_operand = lambda *a, **k: joined.append(1) or join(*a, **k)
+    for fused, seen in ((True, 2), (False, 2), (True, 4)):
+        m.use_fused = fused
+        m.train_on_batch(f, y)
+        m.predict_step((f, y))
+        assert len(joined) == seen
