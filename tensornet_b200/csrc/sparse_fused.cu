@@ -763,9 +763,8 @@ __global__ void __launch_bounds__(kFrontThreads) pull_front_ship_kernel(const __
 // =======================================================================================
 constexpr int kLocalThreads = 256;
 
-// Both kernels take the pulls of several tables at once (blockIdx.y): a model's pulls need only the ids of the batch, and a
-// small one is all latency.  Two of 10 K ids, one after the other and
-// together: 26 and 14 us.
+// Both kernels take the pulls of two tables at once (blockIdx.y): a model's pulls need only the ids of the batch, and a small
+// one is all latency.  Two of 10 K ids, one after the other and together: 26 and 14 us.
 // (Launches of one table carry one table's arguments: a parameter block of 3 KB costs the host more than a microsecond.)
 template <int N> struct PullArgsOf { PullArgs a[N]; };
 template <int N>
@@ -1502,9 +1501,9 @@ static cudaError_t launch_pulls(const PullArgs* pulls, int n, cudaStream_t strea
 }
 // One GPU, rows left in the table (see pull_local_probe_kernel).  The `n` pulls are all behind a front or all not.
 cudaError_t launch_sparse_pull_local(const PullArgs* pulls, int n, cudaStream_t stream) {
-  static_assert(kMaxPullBatch == 4, "instances below");
+  static_assert(kMaxPullBatch == 2, "instances below");
   if (n < 1 || n > kMaxPullBatch) return cudaErrorInvalidValue;
-  return n == 1 ? launch_pulls<1>(pulls, n, stream) : n == 2 ? launch_pulls<2>(pulls, n, stream) : launch_pulls<4>(pulls, n, stream);
+  return n == 1 ? launch_pulls<1>(pulls, n, stream) : launch_pulls<2>(pulls, n, stream);
 }
 
 // The pulled rows also into the per-batch matrix.

@@ -81,7 +81,7 @@ struct PullArgs {
   int front_done;         // dedup, id dispatch and inverse map of this batch already ran (launch_sparse_pull_front)
 };
 
-constexpr int kMaxPullBatch = 4;      // pulls of different tables in one launch (one GPU)
+constexpr int kMaxPullBatch = 2;      // pulls of different tables in one launch (one GPU): a model's linear and deep layers
 
 // Where the pulled row of position v is: row v of the per-batch matrix `U`, or (`row_of` not null; one GPU) row row_of[v]
 // of the table itself, whose descriptor `tbl` lies in device memory so that recorded launches follow a shard that grows.

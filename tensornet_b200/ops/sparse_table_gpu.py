@@ -439,11 +439,11 @@ class GpuSparseLink:
 
     @staticmethod
     def pull_many(calls):
-        """In-place pulls of different tables in one go.  ``calls``: ``(link, ids, labels, label_mod, training, n_dev)`` of
+        """In-place pulls of two tables in one go.  ``calls``: ``(link, ids, labels, label_mod, training, n_dev)`` of
         each; the :meth:`pull_in_place` of the same ids that follows on a link finds its pull done.  False (and nothing
         done) where they do not go together."""
         links = [c[0] for c in calls]
-        if not 2 <= len(calls) <= 4 or len({id(lk.table) for lk in links}) < len(links) or not all(lk.ctx.in_place() for lk in links) or \
+        if len(calls) != 2 or len({id(lk.table) for lk in links}) < len(links) or not all(lk.ctx.in_place() for lk in links) or \
                 any(t is not None and t.is_inference() for _, ids, labels, _, _, n_dev in calls for t in (ids, labels, n_dev)):
             return False
         begun = [lk._begin(ids, training) for lk, ids, _, _, training, _ in calls]

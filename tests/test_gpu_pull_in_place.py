@@ -15,7 +15,7 @@ def _layer(tn, dim, kind, cvm, combiner, slots, bucket, staged, rows=1 << 14):
         layer = tn.layers.EmbeddingFeatures(cols, opt, name="e", is_concat=True, target_columns=["label"] if cvm else None, rows=rows)
     finally:
         tn.core.config.staged_row_return = old
-    assert not (layer.link.ctx.in_place() and staged) or layer.link.ustride > 40      # (wide rows have no staged return)
+    assert layer.link.ctx.in_place() == (not staged)
     return layer
 
 
@@ -173,7 +173,7 @@ def test_pulls_of_two_layers_side_by_side(tn_gpu, status_ok, ragged):
         got.append(outs)
     for a, b in zip(*got):
         assert torch.equal(a, b)
-    # a pull that was run ahead is for that batch only: other ids, or the same buffer with new contents, are pulled again
+    # a pull that was run ahead is for that batch only: other ids are pulled again
     (f, _), (f2, s2) = batches[0], batches[1]
     pull_together(layers, f, True)
     for layer in layers:
