@@ -228,8 +228,8 @@ __global__ void __launch_bounds__(kBnCols * kBnRows) bn_apply_bwd_kernel(const f
 
 // z = bf16([bn([h | x]) | 1 | 0]); one thread per pair of columns.  `mean_out` / `var_out` keep the moments it used for the
 // backward pass.  As separate kernels (h to fp32, concatenation, two copies of the moments, normalisation, operand assembly)
-// this took six launches of 1 to 4 us at 32 x 260, and their gradients nine: from the
-// tower to the loss 24 us and back 28; a step of 1024 x 36 by 133 to 108 us with these.
+// this took six launches of 1 to 4 us at 32 x 260, and their gradients nine: from the tower to the loss 24 us and back 28.  A
+// Wide&Deep step of 1024 examples and 42 columns went from 133 to 108 us with these.
 __global__ void __launch_bounds__(256) bn_join_fwd_kernel(const BnInput in, int B, int C, const float* __restrict__ mean,
                                                           const float* __restrict__ var, const float* __restrict__ gamma,
                                                           const float* __restrict__ beta, float eps, __nv_bfloat16* __restrict__ z, int ldz,

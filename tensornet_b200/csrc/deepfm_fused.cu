@@ -178,8 +178,8 @@ __global__ void deepfm_input_bwd_kernel(const float* __restrict__ E, const int* 
 // Bound by latency: 15 MB at 8192 x 408 take 3 us, a row's chain of load, dot product, loss and stores about as long.  So a
 // warp has kHeadRows rows on the way at once (packed as they are stored: 8 registers a row), their scalar mathematics run
 // side by side in one lane per row, and warps meet in shared memory with plain stores (a float add to shared memory is a
-// compare-and-swap loop) and add the sums of a block to memory
-// once.  8192 x 400: 21.2 us with a row at a time and adds to shared memory, 9.7 now.
+// compare-and-swap loop) and add the sums of a block to memory once.  8192 x 400: 21.2 us with a row at a time and adds to
+// shared memory, 9.5 now.
 constexpr int kHeadPairs = 8;
 constexpr int kHeadRows = 4;
 constexpr int kHeadParts = 16;            // partial copies of the weight gradient in the scratch area
@@ -366,8 +366,8 @@ const char* launch_deepfm_head_loss(const void* H, int ldh, int NH, const float*
   if (ldh > 64 * kHeadPairs || (ldh & 1)) return "deepfm_head: hidden width must be even and at most 512 columns";
   if (NL > 32) return "deepfm_head: at most 32 linear inputs";
   if (((NH + NL + 5) & ~3) > kHeadPartStride) return "deepfm_head: too many head inputs";
-  // two blocks per SM: measured 254 us per DeepFM step against 257 (three) and 264 (four), with scalar or 16-byte
-  // reductions of the per-block weight gradient alike
+  // two blocks per SM, which is what the registers of four rows a warp leave room for: 9.5 us at 8192 x 400, a DeepFM step
+  // 198.5 us; one block 11.3 and 201.3, three 13.5 and 201.9
   int blocks = (B + 7) / 8; if (blocks > 148 * 2) blocks = 148 * 2; if (blocks < 1) blocks = 1;
   cudaError_t e = launch_pdl(deepfm_head_loss_kernel, dim3(blocks), dim3(256), 8 * ((NH + NL + 5) & ~3) * sizeof(float), st,
                              reinterpret_cast<const __nv_bfloat16*>(H), ldh, NH, L, NL, fm, w, label, B,

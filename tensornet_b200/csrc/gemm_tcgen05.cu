@@ -465,10 +465,10 @@ const char* gemm_bf16(const GemmDesc& d, cudaStream_t stream) {
   cfg.attrs = attr;
   cfg.numAttrs = use_pdl ? 1 : 0;
   // Plain bf16 outputs (forward products) have instances of their own.  With all epilogues in one kernel the plain one takes
-  // 0.2 to 0.7 us longer where its instructions are at hand (512 x 512 x 1025 8.9 -> 9.1, 8192 x 400 x 401 9.85 -> 10.35,
+  // 0.2 to 0.5 us longer where its instructions are at hand (512 x 512 x 1025 8.9 -> 9.1, 8192 x 400 x 401 9.8 -> 10.3,
   // launch to launch) and 2 us where the kernel runs once between others, as in a request of 512 examples (a pass 93.5 ->
   // 97.6).  Everything else stays together: each further kernel of a short step is one more that starts without its
-  // instructions (1024 examples through 64-32: 1 560 us a pass; fp32 outputs beside the plain ones 1 630; all in one 1 620).
+  // instructions (sixteen steps of 1024 examples through 64-32: 1 570 us; fp32 outputs beside the plain ones 1 625; all in one 1 610).
   const bool plain = !d.out_f32 && !d.mask_aux && !d.had_x0 && !d.had_xl;
   cudaError_t e;
   if (smem > 220 * 1024) return "gemm_bf16: tile does not fit in shared memory";

@@ -757,7 +757,11 @@ __global__ void __launch_bounds__(kFrontThreads) pull_front_ship_kernel(const __
 // cooperative kernel that writes the rows out, a pull cost a grid barrier per phase and the copy.  Bound by the latency of
 // dependent accesses, for large batches by random sectors.  Pull (and pooling) before and now, us: 10 K ids 33 (2.4) and
 // 8.0 + 4.7 (3.0); 64 K ids 31 (3.4) and 8.5 + 5.7 (3.7); 213 K ids 51 (9) and 24 + 6 (11); 2.1 M ids with rows of 128
-// floats 420 (312) and 126 + 40 (326).
+// floats 420 (312) and 121 + 40 (329).
+// The price is paid by signs without a row, whose key and slot sectors are asked for twice, by the lookup and by the
+// insertion: 4.2 M new signs 2 280 us then and 560 + 1 840 now (Ftrl, dim 64), 1 190 and 570 + 770 (Adam, 20), 790 and 455 +
+// 490 (AdaGrad, 8).  What did not help: several insertions in flight per lane (490 -> 550), the arithmetic of the initial
+// values spread evenly over the lanes, rows cleared as one run before their weights are written.
 // Ahead of its step (pull_local_probe_kernel, pull_local_resolve_kernel on a second stream) the table's index is only
 // read; what the step itself still runs is the second kernel without its first part.
 // =======================================================================================
@@ -1187,6 +1191,8 @@ __global__ void __launch_bounds__(256, LocalPush<KIND>::kBlocks) sparse_push_loc
 // the middle of a 16-byte piece.  A row is whole pieces all the same, so a lane takes one of them, whatever it holds, the
 // accumulator is handed round the group, and the row costs one load and one store per lane.  Two rows at a time,
 // 84 K rows of ten columns and of one: 24.1 us a row at a time and element by element, 16.5 now.
+// (Adam and Ftrl keep three arrays of such a width, which start at three different places of their pieces: a column's three
+// values then lie with different lanes.  Those rows are left to sparse_push_local_rows_kernel.)
 constexpr int kOddRows = 2;
 __global__ void __launch_bounds__(256, 5) sparse_push_local_odd_kernel(const __grid_constant__ PushArgs a) {
   const float* const rows = a.tbl_dev->rows;        // (changes between steps only)

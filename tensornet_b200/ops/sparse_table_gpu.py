@@ -274,8 +274,9 @@ def dedup_slots(max_unique: int, capo: int, world: int) -> int:
     """Slots of the dedup scratch.  One GPU: at most two thirds full with all the signs a segment holds.  It is probed at
     random and cleared every batch, so what counts is that it stays in L2 (4.1 M ids of 4.9 M that fit: 67 MB of keys
     instead of 134, pull 627 -> 570 us).  Where that is no question, short probe chains count, since a warp waits for the
-    longest of 32: a quarter full at most up to 256 K signs (lookup of 10 K ids 13.0 -> 8.0 us, of 213 K 25.4 -> 23.6, but
-    of 2.1 M 126 -> 172).  Several GPUs: the segments of all owners together hold more than ``max_unique``
+    longest of 32: a quarter full at most up to 256 K signs.  Pulls of as many ids as fit, a quarter and two thirds full:
+    65 K 25.6 and 25.8 us, 262 K 39.9 and 42.0, 300 K 44.0 and 44.0, 524 K 68.6 and 64.5, 1 M 103 and 95, 2.1 M 183 and
+    142.  Several GPUs: the segments of all owners together hold more than ``max_unique``
     signs, and a batch of up to twice that many is taken."""
     return next_pow2(max(capo * 4 if capo <= 1 << 18 else capo * 3 // 2, 32) if world == 1 else 2 * max_unique + 16)
 
@@ -475,8 +476,10 @@ class GpuSparseLink:
     def prefetch(self, ids: torch.Tensor):
         """Run the front of the pull (dedup, id dispatch to the owners, inverse map; on one GPU also the lookup of the
         signs) for the batch ``ids`` on the current stream.  The next :meth:`pull` must be a training pull of this very
-        tensor; it then only probes and returns rows (one GPU: creates those that are missing).  Anything else discards the front (:meth:`discard_front`).  ``ids`` must not live in the
-        buffer of a batch whose backward pass is still to come: the inverse map of a front is kept per id buffer."""
+        tensor; it then only probes and returns rows (one GPU: creates those that are missing).  Anything else discards
+        the front (:meth:`discard_front`).  ``ids`` must not live in the buffer of a batch whose backward pass is still
+        to come: the inverse map of a front is kept per id buffer, for up to eight of them (4 bytes per id; on one GPU
+        the row numbers too, 4 bytes per sign that the segment holds)."""
         n = ids.numel()
         key = (ids.data_ptr(), n)
         inverse = self._front_inverse.get(key)
