@@ -229,7 +229,9 @@ gemm_bf16_2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       const int row_base = tile_m * 2 * kBM + (int)rank * kBM + q * 32;
       if (kEpiW != 16) gemm_epi::prefetch_aux(p, row_base, tile_n * BN, BN, sub, kEpiW / 4, lane);
       const uint32_t tm_lane = tmem + ((uint32_t)(q * 32) << 16) + a * (uint32_t)BN;
-      if (!gemm_epi::store_rows<kEpiW != 16 ? gemm_epi::kAny : gemm_epi::kNoAux>(p, tm_lane, row_base, tile_n * BN, BN, sub, kEpiW / 4, lane, sm_out, ready)) { ok = false; break; }
+      constexpr gemm_epi::Kinds kKinds = kEpiW != 16 ? gemm_epi::kAny : gemm_epi::kNoAux;
+      ok = gemm_epi::store_rows<kKinds>(p, tm_lane, row_base, tile_n * BN, BN, sub, kEpiW / 4, lane, sm_out, ready);
+      if (!ok) break;
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_remote(acc_empty_even + a * (uint32_t)sizeof(uint64_t));
