@@ -42,6 +42,7 @@ CUDA_SOURCES = [
     "mlp_fused.cu", "gemm_2sm.cu", "gemm_splitk.cu",
     "dense_fused.cu",
     "elementwise.cu",
+    "head.cu",
     "serving.cu",
     "bn.cu",
     "unique.cu",

@@ -1004,22 +1004,60 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                                                   dL ? ptr_of<float>(*dL) : nullptr, cur_stream());
     if (err) throw std::runtime_error(err);
   });
-  m.def("deepfm_head_loss", [](at::Tensor H, int NH, c10::optional<at::Tensor> L, at::Tensor fm, at::Tensor w, at::Tensor label,
-                               at::Tensor dH, c10::optional<at::Tensor> dL, at::Tensor dfm, at::Tensor gw, at::Tensor sums,
-                               c10::optional<at::Tensor> pred, at::Tensor loss_out, at::Tensor scratch) {
-    c10::cuda::CUDAGuard guard(H.device());
-    TORCH_CHECK(scratch.numel() >= 4 + 16 * 576 && scratch.scalar_type() == at::kFloat && (reinterpret_cast<uintptr_t>(scratch.data_ptr()) & 15) == 0,
-                "deepfm_head_loss: scratch must be fp32[4 + 16 * 576], 16-byte aligned, zero between calls");
-    const int NL = L ? (int)L->size(1) : 0;
-    TORCH_CHECK(w.numel() == NH + NL + 2, "deepfm_head_loss: weight must be [NH + NL + 2]");
-    const char* err = tn::launch_deepfm_head_loss(H.data_ptr(), (int)H.stride(0), NH, L ? ptr_of<float>(*L) : nullptr, NL,
-                                                  ptr_of<float>(fm), ptr_of<float>(w), ptr_of<float>(label), (int)H.size(0),
-                                                  dH.data_ptr(), dL ? ptr_of<float>(*dL) : nullptr, ptr_of<float>(dfm),
-                                                  ptr_of<float>(gw), ptr_of<float>(sums), hist_bins(sums),
-                                                  pred ? ptr_of<float>(*pred) : nullptr,
-                                                  ptr_of<float>(loss_out), ptr_of<float>(scratch), cur_stream());
-    if (err) throw std::runtime_error(err);
-  });
+  {
+    auto pieces_of = [](const std::vector<at::Tensor>& pieces, const std::vector<int>& widths, at::Tensor w) {
+      TORCH_CHECK(!pieces.empty() && pieces.size() <= tn::kMaxHeadPieces && widths.size() == pieces.size(), "head: number of pieces");
+      TORCH_CHECK(w.scalar_type() == at::kFloat && w.is_contiguous(), "head: weight must be contiguous fp32");
+      tn::HeadArgs a = {};
+      a.B = (int)pieces[0].size(0); a.n = (int)pieces.size(); a.K = (int)w.numel() - 1;
+      a.w = ptr_of<float>(w);
+      for (int p = 0; p < a.n; ++p) {
+        const at::Tensor& t = pieces[p];
+        TORCH_CHECK(t.is_cuda() && t.dim() == 2 && t.size(0) == a.B && (t.stride(1) == 1 || t.size(1) == 1) && widths[p] <= t.size(1) &&
+                        (t.scalar_type() == at::kBFloat16 || t.scalar_type() == at::kFloat), "head: piece ", p);
+        a.src[p] = t.data_ptr();
+        a.width[p] = widths[p];
+        a.ld[p] = a.gld[p] = (int)t.stride(0);
+        a.kind[p] = t.scalar_type() == at::kBFloat16 ? tn::kHeadBf16 : tn::kHeadF32;
+      }
+      return a;
+    };
+    m.attr("HEAD_MAX_SPAN") = tn::kMaxHeadSpan;
+    m.attr("HEAD_COPIES") = tn::kHeadCopies;
+    m.def("head_loss", [pieces_of](std::vector<at::Tensor> pieces, std::vector<int> widths, at::Tensor w, at::Tensor label,
+                                   std::vector<c10::optional<at::Tensor>> grads, bool relu_first, at::Tensor gw, at::Tensor sums,
+                                   at::Tensor loss_out, at::Tensor scratch, c10::optional<at::Tensor> pred) {
+      c10::cuda::CUDAGuard guard(w.device());
+      tn::HeadArgs a = pieces_of(pieces, widths, w);
+      TORCH_CHECK(grads.size() == pieces.size() && gw.is_contiguous() && gw.numel() == w.numel() && gw.scalar_type() == at::kFloat &&
+                      label.is_contiguous() && label.scalar_type() == at::kFloat && label.numel() == a.B, "head_loss: gradients or labels");
+      int64_t span = 0;
+      for (int p = 0; p < a.n; ++p) {
+        span += (widths[p] + 7) / 8 * 8;
+        if (!grads[p]) continue;
+        const at::Tensor& g = *grads[p];
+        TORCH_CHECK(g.dim() == 2 && g.size(0) == a.B && g.size(1) >= widths[p] && (g.stride(1) == 1 || g.size(1) == 1) &&
+                        g.scalar_type() == pieces[p].scalar_type(), "head_loss: gradient of piece ", p);
+        a.grad[p] = g.data_ptr();
+        a.gld[p] = (int)g.stride(0);
+      }
+      TORCH_CHECK(scratch.scalar_type() == at::kFloat && scratch.numel() >= 4 + tn::kHeadCopies * (span + 8) &&
+                      (reinterpret_cast<uintptr_t>(scratch.data_ptr()) & 15) == 0, "head_loss: scratch too small");
+      a.relu_first = relu_first;
+      a.label = ptr_of<float>(label); a.gw = ptr_of<float>(gw); a.sums = ptr_of<float>(sums); a.nbins = hist_bins(sums);
+      TORCH_CHECK(!pred || (pred->is_contiguous() && pred->numel() == a.B && pred->scalar_type() == at::kFloat), "head_loss: pred");
+      a.pred = pred ? ptr_of<float>(*pred) : nullptr;
+      a.loss_out = ptr_of<float>(loss_out); a.scratch = ptr_of<float>(scratch);
+      if (const char* err = tn::launch_head_loss(a, cur_stream())) throw std::runtime_error(err);
+    });
+    m.def("head_score", [pieces_of](std::vector<at::Tensor> pieces, std::vector<int> widths, at::Tensor w, at::Tensor logits) {
+      c10::cuda::CUDAGuard guard(w.device());
+      tn::HeadArgs a = pieces_of(pieces, widths, w);
+      TORCH_CHECK(logits.is_contiguous() && logits.numel() == a.B && logits.scalar_type() == at::kFloat, "head_score: logits");
+      a.pred = ptr_of<float>(logits);
+      if (const char* err = tn::launch_head_score(a, cur_stream())) throw std::runtime_error(err);
+    });
+  }
   m.def("unique_assign", [](at::Tensor ids, c10::optional<at::Tensor> labels, at::Tensor dd_keys, at::Tensor dd_vals, at::Tensor uniq,
                             at::Tensor inverse, c10::optional<at::Tensor> show, c10::optional<at::Tensor> click, at::Tensor count,
                             at::Tensor status) {

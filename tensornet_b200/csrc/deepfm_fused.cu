@@ -7,10 +7,6 @@
 //   deepfm_input_bwd : gradient of that operand (bf16, from the first layer's dgrad) plus the FM
 //                      gradient, scattered straight into the unique-gradient rows - replaces
 //                      split/cast + FM backward + add + pool backward.
-//   deepfm_head_loss : Dense(1) over [h | linear | fm | 1], sigmoid cross-entropy, CTR / PCTR sums
-//                      and the complete backward of the head (dH with the ReLU mask applied, dLinear,
-//                      dFM, weight gradient) in one kernel - the logit gradient depends on nothing
-//                      but the logit and the label, so forward and backward of the head are one pass.
 #include <cuda_bf16.h>
 #include "sparse_table.cuh"
 #include "tn_ops.h"
@@ -172,173 +168,6 @@ __global__ void deepfm_input_bwd_kernel(const float* __restrict__ E, const int* 
   }
 }
 
-// Head + loss + head backward.  w = [ wH (NH) | wL (NL) | wfm | bias ].  ldh <= 512, even.
-// sums: [0] += mean loss, [1] += sum(label), [2] += sum(pred), [3] += B; with nbins > 0 the words behind them are the
-// two prediction histograms (u32 counts; positives, then negatives) of a streaming AUC.
-// Bound by latency: 15 MB at 8192 x 408 take 3 us, a row's chain of load, dot product, loss and stores about as long.  So a
-// warp has kHeadRows rows on the way at once (packed as they are stored: 8 registers a row), their scalar mathematics run
-// side by side in one lane per row, and warps meet in shared memory with plain stores (a float add to shared memory is a
-// compare-and-swap loop) and add the sums of a block to memory once.  8192 x 400: 21.2 us with a row at a time and adds to
-// shared memory, 9.5 now.
-constexpr int kHeadPairs = 8;
-constexpr int kHeadRows = 4;
-constexpr int kHeadParts = 16;            // partial copies of the weight gradient in the scratch area
-constexpr int kHeadPartStride = 576;      // floats per copy: >= 64 * kHeadPairs + 32 + 2, multiple of 4
-__global__ void __launch_bounds__(256, 2) deepfm_head_loss_kernel(const __nv_bfloat16* __restrict__ H, int ldh, int NH,
-                                        const float* __restrict__ L, int NL,
-                                        const float* __restrict__ fm, const float* __restrict__ w, const float* __restrict__ label,
-                                        int B, __nv_bfloat16* __restrict__ dH, float* __restrict__ dL, float* __restrict__ dfm,
-                                        float* __restrict__ gw, float* __restrict__ sums, int nbins,
-                                        float* __restrict__ pred, float* __restrict__ loss_out, float* __restrict__ scratch) {
-  pdl_sync();
-  extern __shared__ __align__(16) float s_gw[];   // [warps of the block][NWp]
-  __shared__ float s_sum[3][8];
-  const int NW = NH + NL + 2, NWp = (NW + 3) & ~3;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  float2 wv[kHeadPairs], acc[kHeadPairs];
-#pragma unroll
-  for (int i = 0; i < kHeadPairs; ++i) {
-    const int c = 64 * i + 2 * lane;
-    wv[i].x = c < NH ? __ldg(w + c) : 0.f;
-    wv[i].y = c + 1 < NH ? __ldg(w + c + 1) : 0.f;
-    acc[i] = make_float2(0.f, 0.f);
-  }
-  const float wl = lane < NL ? __ldg(w + NH + lane) : 0.f;       // NL <= 32 linear weights, one per lane
-  const float wfm = __ldg(w + NH + NL), bias = __ldg(w + NH + NL + 1);
-  float accL = 0.f, accfm = 0.f, accb = 0.f, ls = 0.f, ys = 0.f, ps = 0.f;
-  const float invB = 1.f / (float)B;
-  for (int b0 = warp; b0 < B; b0 += kHeadRows * nwarps) {
-    __nv_bfloat162 z[kHeadRows][kHeadPairs];
-    float lv[kHeadRows], dot[kHeadRows];
-#pragma unroll
-    for (int q = 0; q < kHeadRows; ++q) {
-      const int b = b0 + q * nwarps;
-      const __nv_bfloat162* zr = reinterpret_cast<const __nv_bfloat162*>(H + (size_t)b * ldh);
-#pragma unroll
-      for (int i = 0; i < kHeadPairs; ++i) {
-        z[q][i] = b < B && 64 * i + 2 * lane < ldh ? zr[32 * i + lane] : __floats2bfloat162_rn(0.f, 0.f);
-      }
-      lv[q] = b < B && lane < NL ? L[(size_t)b * NL + lane] : 0.f;
-    }
-    const int mine = b0 + lane * nwarps;                          // lane q looks after row q
-    const bool own = lane < kHeadRows && mine < B;
-    const float f = own ? fm[mine] : 0.f, y = own ? label[mine] : 0.f;
-#pragma unroll
-    for (int q = 0; q < kHeadRows; ++q) {
-      dot[q] = lv[q] * wl;
-#pragma unroll
-      for (int i = 0; i < kHeadPairs; ++i) {
-        const float2 zz = __bfloat1622float2(z[q][i]);
-        dot[q] += zz.x * wv[i].x + zz.y * wv[i].y;
-      }
-    }
-    float sum = 0.f;
-#pragma unroll
-    for (int q = 0; q < kHeadRows; ++q) {
-      const float d = wsum(dot[q]);
-      if (lane == q) sum = d;
-    }
-    const float logit = sum + f * wfm + bias;
-    const float p = 1.f / (1.f + expf(-logit));
-    const float dl = (p - y) * invB;
-    if (own) {
-      ls += fmaxf(logit, 0.f) + log1pf(expf(-fabsf(logit))) - y * logit;
-      ys += y; ps += p;
-      if (pred) pred[mine] = p;
-      if (nbins > 0)
-        atomicAdd(reinterpret_cast<unsigned*>(sums + 4) + (y > 0.5f ? 0 : nbins) + min(nbins - 1, (int)(p * (float)nbins)), 1u);
-      dfm[mine] = dl * wfm;
-      accfm += dl * f;
-      accb += dl;
-    }
-#pragma unroll
-    for (int q = 0; q < kHeadRows; ++q) {
-      const int b = b0 + q * nwarps;
-      const float d = __shfl_sync(0xffffffffu, dl, q);
-      if (b >= B) continue;
-      if (lane < NL) { dL[(size_t)b * NL + lane] = d * wl; accL += d * lv[q]; }
-      __nv_bfloat162* dz = reinterpret_cast<__nv_bfloat162*>(dH + (size_t)b * ldh);
-#pragma unroll
-      for (int i = 0; i < kHeadPairs; ++i) {
-        const int c = 64 * i + 2 * lane;
-        if (c >= ldh) continue;
-        const float2 zz = __bfloat1622float2(z[q][i]);
-        // gradient w.r.t. the ReLU output h, already masked by h > 0 (columns >= NH are the ones / pad columns)
-        const float gx = (c < NH && zz.x > 0.f) ? d * wv[i].x : 0.f;
-        const float gy = (c + 1 < NH && zz.y > 0.f) ? d * wv[i].y : 0.f;
-        dz[32 * i + lane] = __floats2bfloat162_rn(gx, gy);
-        acc[i].x += d * zz.x;
-        acc[i].y += d * zz.y;
-      }
-    }
-  }
-  float* my_gw = s_gw + wib * NWp;
-#pragma unroll
-  for (int i = 0; i < kHeadPairs; ++i) {
-    const int c = 64 * i + 2 * lane;
-    if (c < NH) my_gw[c] = acc[i].x;
-    if (c + 1 < NH) my_gw[c + 1] = acc[i].y;
-  }
-  if (lane < NL) my_gw[NH + lane] = accL;
-  accfm = wsum(accfm); accb = wsum(accb); ls = wsum(ls); ys = wsum(ys); ps = wsum(ps);
-  if (lane == 0) {
-    my_gw[NH + NL] = accfm;
-    my_gw[NH + NL + 1] = accb;
-    for (int k = NW; k < NWp; ++k) my_gw[k] = 0.f;
-    s_sum[0][wib] = ls * invB; s_sum[1][wib] = ys; s_sum[2][wib] = ps;
-  }
-  __syncthreads();
-  if (threadIdx.x < 3) {
-    float v = 0.f;
-    for (int k = 0; k < 8; ++k) v += s_sum[threadIdx.x][k];
-    atomicAdd(&sums[threadIdx.x], v);
-    if (threadIdx.x == 0) atomicAdd(&scratch[0], v);
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 3) atomicAdd(&sums[3], (float)B);
-  // The per-block weight gradients are summed in two steps.  Hundreds of blocks adding to the same few hundred words of
-  // `gw` at the same moment queue up behind one another in L2 (that tail used to be most of the kernel); instead a block
-  // adds into one of kHeadParts partial copies in the scratch area (a sixteenth of the blocks per copy), and the last
-  // block to finish folds the copies into `gw` and leaves them at zero for the next launch.
-  float* parts = scratch + 4;                              // [kHeadParts][kHeadPartStride]
-  for (int k = 4 * threadIdx.x; k < NWp; k += 4 * blockDim.x) {
-    float4 v = *reinterpret_cast<const float4*>(s_gw + k);
-#pragma unroll
-    for (int q = 1; q < 8; ++q) {
-      const float4 x = *reinterpret_cast<const float4*>(s_gw + q * NWp + k);
-      v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
-    }
-    red_add_f32x4(parts + (size_t)(blockIdx.x % kHeadParts) * kHeadPartStride + k, v);
-  }
-  // The loss is summed in a persistent scratch word that is zero between launches; the last block to finish
-  // moves the total into `loss_out` and re-arms the scratch, so the caller never has to clear anything.
-  __shared__ int s_last;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    const unsigned prev = atomicAdd(reinterpret_cast<unsigned*>(scratch) + 1, 1u);
-    s_last = prev == gridDim.x - 1;
-    if (s_last) {
-      __threadfence();
-      *loss_out = atomicExch(&scratch[0], 0.f);
-      reinterpret_cast<unsigned*>(scratch)[1] = 0u;
-    }
-  }
-  __syncthreads();
-  if (s_last) {
-    for (int k = threadIdx.x; k < NW; k += blockDim.x) {
-      float sum = 0.f;
-#pragma unroll
-      for (int q = 0; q < kHeadParts; ++q) {
-        float* pq = parts + (size_t)q * kHeadPartStride + k;
-        sum += __ldcg(pq);
-        *pq = 0.f;
-      }
-      gw[k] += sum;          // nobody else touches the head's gradient while this kernel runs
-    }
-  }
-}
-
 }  // namespace
 
 const char* launch_deepfm_input_fwd(const RowSource& src, const int* inverse, int B, int S, int D, const float* dense, int Dd, int ld_dense,
@@ -358,20 +187,6 @@ const char* launch_deepfm_input_bwd(const float* E, const int* inverse, int B, i
   int blocks = (B + 7) / 8; if (blocks > 148 * 8) blocks = 148 * 8; if (blocks < 1) blocks = 1;
   cudaError_t e = launch_pdl(deepfm_input_bwd_kernel, dim3(blocks), dim3(256), 0, st, E, inverse, B, S, D,
                              reinterpret_cast<const __nv_bfloat16*>(dX0), ld, gfm, gU, gstride, lin_col, dL);
-  return e == cudaSuccess ? nullptr : cudaGetErrorString(e);
-}
-const char* launch_deepfm_head_loss(const void* H, int ldh, int NH, const float* L, int NL, const float* fm, const float* w,
-                                    const float* label, int B, void* dH, float* dL, float* dfm, float* gw, float* sums, int nbins,
-                                    float* pred, float* loss_out, float* scratch, cudaStream_t st) {
-  if (ldh > 64 * kHeadPairs || (ldh & 1)) return "deepfm_head: hidden width must be even and at most 512 columns";
-  if (NL > 32) return "deepfm_head: at most 32 linear inputs";
-  if (((NH + NL + 5) & ~3) > kHeadPartStride) return "deepfm_head: too many head inputs";
-  // two blocks per SM, which is what the registers of four rows a warp leave room for: 9.5 us at 8192 x 400, a DeepFM step
-  // 198.5 us; one block 11.3 and 201.3, three 13.5 and 201.9
-  int blocks = (B + 7) / 8; if (blocks > 148 * 2) blocks = 148 * 2; if (blocks < 1) blocks = 1;
-  cudaError_t e = launch_pdl(deepfm_head_loss_kernel, dim3(blocks), dim3(256), 8 * ((NH + NL + 5) & ~3) * sizeof(float), st,
-                             reinterpret_cast<const __nv_bfloat16*>(H), ldh, NH, L, NL, fm, w, label, B,
-                             reinterpret_cast<__nv_bfloat16*>(dH), dL, dfm, gw, sums, nbins, pred, loss_out, scratch);
   return e == cudaSuccess ? nullptr : cudaGetErrorString(e);
 }
 

@@ -91,15 +91,36 @@ void launch_cross_v2_du(const void* g, const void* x0, void* du, long long n, cu
 void launch_cross_v2_bwd_sum(const CrossTerms& t, const void* g0, void* out, long long n, cudaStream_t st);
 void launch_cross_v2_bwd_final(const float* gx0, const void* g, void* out, long long n, cudaStream_t st);
 
+// head.cu  (return nullptr or a static error string)
+constexpr int kMaxHeadPieces = 4;
+constexpr int kMaxHeadSpan = 4096;      // weights that fit, every piece's rounded up to eight
+constexpr int kHeadCopies = 16;         // partial copies of the weight gradient in the scratch
+enum HeadKind { kHeadBf16, kHeadF32, kHeadF32x4 };
+struct HeadArgs {
+  int B, n, K;                          // rows, pieces, weights without the bias (w[K])
+  const void* src[kMaxHeadPieces];      // piece p: [B, width[p]] with row stride ld[p]
+  void* grad[kMaxHeadPieces];           // its gradient, row stride gld[p] (bf16: zeros behind width[p]); null: not wanted
+  int width[kMaxHeadPieces], ld[kMaxHeadPieces], gld[kMaxHeadPieces], kind[kMaxHeadPieces];
+  int relu_first;                       // piece 0 is a ReLU's output: its gradient comes masked
+  const float* w;
+  const float* label;
+  float* gw;                            // added to
+  float* sums;                          // [0] += mean loss, [1] += sum(label), [2] += sum(pred), [3] += B, then the histograms
+  int nbins;
+  float* pred;                          // head_loss: probabilities (may be null); head_score: logits
+  float* loss_out;
+  float* scratch;                       // 4 + kHeadCopies * (span + 8) floats, zero between calls
+  int at[kMaxHeadPieces], first[kMaxHeadPieces], units[kMaxHeadPieces], span, groups, copies;      // filled in by the launch
+};
+const char* launch_head_loss(HeadArgs a, cudaStream_t st);
+const char* launch_head_score(HeadArgs a, cudaStream_t st);
+
 // deepfm_fused.cu  (return nullptr or a static error string)
 // `E` (may be null): the rows as they were read, [B, S * D] fp32, which the backward pass takes
 const char* launch_deepfm_input_fwd(const RowSource& src, const int* inverse, int B, int S, int D, const float* dense, int Dd, int ld_dense,
                                     void* X0, int ld, float* fm, int lin_col, float* Lout, float* E, cudaStream_t st);
 const char* launch_deepfm_input_bwd(const float* E, const int* inverse, int B, int S, int D, const void* dX0, int ld, const float* gfm,
                                     float* gU, int gstride, int lin_col, const float* dL, cudaStream_t st);
-const char* launch_deepfm_head_loss(const void* H, int ldh, int NH, const float* L, int NL, const float* fm, const float* w,
-                                    const float* label, int B, void* dH, float* dL, float* dfm, float* gw, float* sums, int nbins,
-                                    float* pred, float* loss_out, float* scratch, cudaStream_t st);
 
 // unique.cu
 void launch_unique_assign(const long long* ids, int n, const float* labels, unsigned long long* dd_keys, int* dd_vals,

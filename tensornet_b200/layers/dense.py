@@ -8,12 +8,14 @@ the constant 1, so every layer is one GEMM with the bias folded into the weight 
 from __future__ import annotations
 
 import math
-from typing import Sequence
+from typing import Optional, Sequence
 
 import torch
 from torch import nn
 
+from .. import _build
 from ..ops import functional as F
+from ..utils.hooks import unobserved
 
 
 def _glorot_aug(n_out: int, n_in: int) -> torch.Tensor:
@@ -65,9 +67,53 @@ class DenseHead(nn.Module):
         limit = math.sqrt(6.0 / (in_dim + 1))
         w[:in_dim].uniform_(-limit, limit)
         self.weight = nn.Parameter(w)
+        self._scratch = None
 
     def forward(self, z: torch.Tensor) -> torch.Tensor:
         return F.head(z, self.weight)
+
+    # ---- straight from the pieces of the operand, without assembling it (GPU) -------------------------------------
+    def fits(self, widths: Sequence[int], rows: int) -> bool:
+        """Whether the head kernels take pieces of these widths."""
+        w = self.weight
+        return (type(self) is DenseHead and w.is_cuda and w.dtype == torch.float32 and w.is_contiguous() and sum(widths) == w.numel() - 1
+                and 0 < len(widths) <= 4 and min(widths) > 0 and rows > 0 and F.head_span(widths) <= _build.cuda_ext().HEAD_MAX_SPAN)
+
+    def on_pieces(self, pieces, widths: Sequence[Optional[int]]) -> torch.Tensor:
+        """The logits of ``[piece[:, :width] ...]``; scoring does without the operand where nobody looks at it."""
+        widths = [int(p.shape[1]) if k is None else int(k) for p, k in zip(pieces, widths)]
+        if not torch.is_grad_enabled() and pieces[0].is_cuda and unobserved(self) and self.fits(widths, pieces[0].shape[0]):
+            return F.head_score([_head_piece(p, k) for p, k in zip(pieces, widths)], widths, self.weight)
+        return self(F.concat_cast(pieces, ones=True, widths=widths))
+
+    def loss(self, pieces, widths: Sequence[int], label: torch.Tensor, sums: torch.Tensor, relu_first: bool) -> torch.Tensor:
+        """Mean sigmoid cross-entropy of the logits, see :func:`tensornet_b200.ops.functional.head_loss`; for pieces that fit."""
+        key = (F.head_span(widths), self.weight.device)
+        if self._scratch is None or self._scratch[0] != key:      # one per layer: two models may train side by side
+            self._scratch = (key, F.head_scratch(widths, self.weight.device))
+        s = self._scratch[1]
+        label = label.to(self.weight.device, non_blocking=True).contiguous().view(-1).float()
+        return F.head_loss([_head_piece(p, k) for p, k in zip(pieces, widths)], widths, self.weight, label, sums, s, relu_first)
+
+
+def _head_piece(p: torch.Tensor, width: int) -> torch.Tensor:
+    """``p`` in a form that the head kernels read: padded bf16 rows of whole 16-byte pieces, or fp32 of exactly its width."""
+    p = p if p.dim() == 2 else p.reshape(p.shape[0], -1)
+    if p.dtype == torch.bfloat16 and p.shape[1] % 8 == 0 and p.is_contiguous() and p.data_ptr() % 16 == 0:
+        return p
+    return (p if p.shape[1] == width else p[:, :width]).float().contiguous()
+
+
+def tower_loss(head: DenseHead, mlp: MLP, widths: Sequence[int], pieces, labels: torch.Tensor, sums: torch.Tensor) -> torch.Tensor:
+    """A training step's loss for a head over ``[mlp output | ...]``, with the head's backward pass in the same kernel where
+    that takes it.  ``pieces(**kw)`` runs the layers before it and returns the pieces; ``kw`` are for ``mlp``."""
+    B = int(labels.numel())
+    masked = type(mlp) is MLP and mlp.relu_last and unobserved(mlp, backward=True)      # the kernel masks the gradient of the last ReLU
+    if head.weight.requires_grad and head.fits(widths, B):
+        got = pieces(grad_premasked=True) if masked else pieces()
+        assert got[0].shape[0] == B, "as many labels as examples"
+        return head.loss(got, widths, labels, sums, masked)
+    return F.bce_with_logits(head(F.concat_cast(pieces(), ones=True, widths=widths)), labels, sums)[0]
 
 
 class FMLayer(nn.Module):

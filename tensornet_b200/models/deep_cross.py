@@ -14,8 +14,10 @@ from torch import nn
 
 from .. import core, feature_column as fc
 from ..layers import DeepCrossLayer, DenseHead, EmbeddingFeatures, MLP
+from ..layers.dense import tower_loss
 from ..model import Model
 from ..ops import functional as F
+from ..utils.hooks import own_step
 
 
 class DeepCrossSubModel(nn.Module):
@@ -26,11 +28,16 @@ class DeepCrossSubModel(nn.Module):
         self.mlp = MLP(in_dim, hidden_units)
         self.head = DenseHead(self.mlp.out_dim + in_dim)
 
-    def forward(self, x: torch.Tensor):
+    def _head_pieces(self, x: torch.Tensor, **kw):
         cross = self.cross(x)
-        h = self.mlp(F.concat_cast([x], ones=True))
-        z = F.concat_cast([h, cross], ones=True, widths=[self.mlp.out_dim, None])
-        return self.head(z)
+        h = self.mlp(F.concat_cast([x], ones=True), **kw)
+        return [h, cross], [self.mlp.out_dim, None]
+
+    def forward(self, x: torch.Tensor):
+        return self.head.on_pieces(*self._head_pieces(x))
+
+    def train_loss(self, x, labels, sums):
+        return tower_loss(self.head, self.mlp, [self.mlp.out_dim, x.shape[1]], lambda **kw: self._head_pieces(x, **kw)[0], labels, sums)
 
 
 class CrossV2(nn.Module):
@@ -58,13 +65,18 @@ class DCNv2SubModel(nn.Module):
         self.mlp = MLP(in_dim, hidden_units)
         self.head = DenseHead(self.mlp.out_dim)
 
+    def _head_pieces(self, x, **kw):
+        x0 = F.concat_cast(list(x) if isinstance(x, (list, tuple)) else [x], ones=True)
+        xc = self.cross(x0)          # stacked structure: cross network feeds the deep network
+        return [self.mlp(xc, **kw)], [self.mlp.out_dim]
+
     def forward(self, x):
         """``x``: the input matrix, or its column blocks (embeddings, dense features): the blocks go straight into
         the padded bf16 operand, without an fp32 concatenation in between (a 210 MB copy each way at width 6413)."""
-        x0 = F.concat_cast(list(x) if isinstance(x, (list, tuple)) else [x], ones=True)
-        xc = self.cross(x0)          # stacked structure: cross network feeds the deep network
-        h = self.mlp(xc)
-        return self.head(h)
+        return self.head(self._head_pieces(x)[0][0])
+
+    def train_loss(self, x, labels, sums):
+        return tower_loss(self.head, self.mlp, [self.mlp.out_dim], lambda **kw: self._head_pieces(x, **kw)[0], labels, sums)
 
 
 class _CrossModel(Model):
@@ -78,14 +90,25 @@ class _CrossModel(Model):
                                           rows=table_rows)
         self.sub_model = sub_cls(len(features) * self.deep_emb.out_dim + dense_dim, dnn_hidden_units, num_cross)
 
-    def forward(self, features):
+    def _inputs(self, features):
         x = self.deep_emb(features)
         if self.dense_dim:
             dense = features[self.dense_key].to(x.device, non_blocking=True).float()
             if x.is_cuda and isinstance(self.sub_model, DCNv2SubModel):
-                return self.sub_model([x, dense])
+                return [x, dense]
             x = torch.cat([x, dense], dim=1)
-        return self.sub_model(x)
+        return x
+
+    def fused_train_loss(self, features, labels, sums):
+        """Training loss with the head, its loss and its backward pass in one kernel; None where somebody looks at what
+        passes in between."""
+        sub = self.sub_model
+        if type(sub) not in (DeepCrossSubModel, DCNv2SubModel) or not own_step(self, _CrossModel, sub, type(sub)):
+            return None
+        return sub.train_loss(self._inputs(features), labels, sums)
+
+    def forward(self, features):
+        return self.sub_model(self._inputs(features))
 
 
 class DeepCross(_CrossModel):

@@ -14,10 +14,11 @@ from torch import nn
 
 from .. import core, feature_column as fc
 from ..layers import DenseHead, EmbeddingFeatures, MLP
+from ..layers.dense import tower_loss
 from ..layers.embedding_features import pulled_together
 from ..model import Model
 from ..ops import functional as F
-from ..utils.hooks import unobserved
+from ..utils.hooks import own_step, unobserved
 
 
 class DeepFMSubModel(nn.Module):
@@ -29,14 +30,21 @@ class DeepFMSubModel(nn.Module):
         self.mlp = MLP(n_fields * emb_dim + dense_dim, hidden_units)
         self.head = DenseHead(self.mlp.out_dim + n_linear + 1)
 
-    def forward(self, linear_emb: Optional[torch.Tensor], deep_emb: torch.Tensor, dense: Optional[torch.Tensor] = None):
+    def _head_pieces(self, linear_emb, deep_emb, dense, **kw):
         fm = F.fm(deep_emb, self.n_fields, self.emb_dim)
         pieces = [deep_emb] + ([dense.float()] if self.dense_dim else [])
-        x0 = F.concat_cast(pieces, ones=True)
-        h = self.mlp(x0)
-        tail = [h] + ([linear_emb] if self.n_linear else []) + [fm]
-        z = F.concat_cast(tail, ones=True, widths=[self.mlp.out_dim] + [None] * (len(tail) - 1))
-        return self.head(z)
+        h = self.mlp(F.concat_cast(pieces, ones=True), **kw)
+        return [h] + ([linear_emb] if self.n_linear else []) + [fm]
+
+    def _head_widths(self):
+        return [self.mlp.out_dim] + ([self.n_linear] if self.n_linear else []) + [1]
+
+    def forward(self, linear_emb: Optional[torch.Tensor], deep_emb: torch.Tensor, dense: Optional[torch.Tensor] = None):
+        return self.head.on_pieces(self._head_pieces(linear_emb, deep_emb, dense), self._head_widths())
+
+    def train_loss(self, linear_emb, deep_emb, dense, labels, sums):
+        return tower_loss(self.head, self.mlp, self._head_widths(), lambda **kw: self._head_pieces(linear_emb, deep_emb, dense, **kw),
+                          labels, sums)
 
 
 class DeepFM(Model):
@@ -76,20 +84,19 @@ class DeepFM(Model):
         return self.sub_model.mlp
 
     def fused_train_loss(self, features, labels, sums):
-        """Training loss through the fused DeepFM kernels (gather + FM + operand build in one kernel; head, loss and
-        head backward in one kernel).  Returns None when the inputs do not qualify (ragged slots, CVM columns,
-        CPU); the caller then uses the generic path."""
-        mlp = self.sub_model.mlp
-        if F.pad8(mlp.out_dim + 1) > 512 or self.sub_model.n_linear > 32:
+        """Training loss through the fused kernels: gather + FM + operand build in one kernel where the inputs qualify (no
+        ragged slots, no CVM columns); head, loss and head backward in one kernel.  None: the caller uses the generic path."""
+        sub = self.sub_model
+        if not own_step(self, DeepFM, sub, DeepFMSubModel):
             return None
-        got = self._fused_inputs(features, True)
+        emb = [self.deep_emb] + ([self.linear_emb] if self.linear_emb is not None else [])
+        got = None
+        if all(type(e) is EmbeddingFeatures for e in emb) and unobserved(*emb, backward=True):
+            got = self._fused_inputs(features, True)
         if got is None:
-            return None
+            return sub.train_loss(*self._inputs(features), labels, sums)
         x0, fm, lin = got
-        h = mlp(x0, grad_premasked=True)
-        loss, _ = F.deepfm_head_loss(h, lin, fm, self.sub_model.head.weight, labels.to(x0.device, non_blocking=True), sums,
-                                     mlp.out_dim)
-        return loss
+        return tower_loss(sub.head, sub.mlp, sub._head_widths(), lambda **kw: [sub.mlp(x0, **kw), lin, fm], labels, sums)
 
     def _fused_inputs(self, features, training):
         """``(x0, fm, lin)``: the first layer's operand, FM term and linear weights through the fused input kernel, or None
@@ -125,20 +132,17 @@ class DeepFM(Model):
         if got is None:
             return None
         x0, fm, lin = got
-        mlp = self.sub_model.mlp
-        return self.sub_model.head(F.concat_cast([mlp(x0), lin, fm], ones=True, widths=[mlp.out_dim, None, None]))
+        return self.sub_model.head.on_pieces([self.sub_model.mlp(x0), lin, fm], self.sub_model._head_widths())
 
-    def forward(self, features):
-        logits = self._scores(features)
-        if logits is not None:
-            return logits
+    def _inputs(self, features):
+        """The dense part's inputs through the layers one by one."""
         if self.share_linear_table:
             both = self.deep_emb(features)
             both = both.view(both.shape[0], -1, self.emb_dim + 4)
             lin = both[:, :, self.emb_dim].contiguous()
             deep = both[:, :, : self.emb_dim].reshape(both.shape[0], -1)
             dense = features[self.dense_key].to(deep.device, non_blocking=True) if self.dense_dim else None
-            return self.sub_model(lin, deep, dense)
+            return lin, deep, dense
         if self.linear_emb is not None:
             with pulled_together([self.linear_emb, self.deep_emb], features):
                 lin = self.linear_emb(features)
@@ -148,4 +152,10 @@ class DeepFM(Model):
         dense = None
         if self.dense_dim:
             dense = features[self.dense_key].to(deep.device, non_blocking=True)
-        return self.sub_model(lin, deep, dense)
+        return lin, deep, dense
+
+    def forward(self, features):
+        logits = self._scores(features)
+        if logits is not None:
+            return logits
+        return self.sub_model(*self._inputs(features))

@@ -13,7 +13,7 @@ from ..layers import DenseHead, EmbeddingFeatures, MLP, TNBatchNormalization
 from ..layers.embedding_features import pulled_together
 from ..model import Model
 from ..ops import functional as F
-from ..utils.hooks import unobserved
+from ..utils.hooks import own_step, unobserved
 
 
 class WideDeepSubModel(nn.Module):
@@ -33,20 +33,29 @@ class WideDeepSubModel(nn.Module):
                 and x0.is_cuda and x0.shape[0] > 0 and linear_emb.dim() == 2 and linear_emb.dtype == torch.float32 and linear_emb.stride(1) == 1
                 and unobserved(bn, mlp, backward=True))
 
-    def forward(self, linear_emb, deep_emb, dense=None, fused: bool = True):
-        """``fused``: the joint kernels may be used (a model's ``use_fused``)."""
+    def _head_operand(self, linear_emb, deep_emb, dense, fused: bool):
+        """Padded bf16 operand of the head."""
         x0 = F.concat_cast([deep_emb] + ([dense.float()] if self.dense_dim else []), ones=True)
         if fused and self._joins(x0, linear_emb):
             # normalisation straight from the tower's output to the head's operand; its gradient comes back masked
             h = self.mlp(x0, grad_premasked=True)
-            return self.head(self.bn.join_operand(h, self.mlp.out_dim, linear_emb, masked=True))
+            return self.bn.join_operand(h, self.mlp.out_dim, linear_emb, masked=True)
         h = self.mlp(x0)
         if self.bn is None:
-            z = F.concat_cast([h, linear_emb], ones=True, widths=[self.mlp.out_dim, None])
-        else:
-            both = torch.cat([h[:, : self.mlp.out_dim].float(), linear_emb], dim=1)
-            z = F.concat_cast([self.bn(both)], ones=True)
-        return self.head(z)
+            return F.concat_cast([h, linear_emb], ones=True, widths=[self.mlp.out_dim, None])
+        both = torch.cat([h[:, : self.mlp.out_dim].float(), linear_emb], dim=1)
+        return F.concat_cast([self.bn(both)], ones=True)
+
+    def forward(self, linear_emb, deep_emb, dense=None, fused: bool = True):
+        """``fused``: the joint kernels may be used (a model's ``use_fused``)."""
+        return self.head(self._head_operand(linear_emb, deep_emb, dense, fused))
+
+    def train_loss(self, linear_emb, deep_emb, dense, labels, sums):
+        """Loss of a step's logits with the head's backward pass in the same kernel."""
+        z = self._head_operand(linear_emb, deep_emb, dense, True)
+        if self.head.weight.requires_grad and labels.numel() == z.shape[0] and self.head.fits([self.head.in_dim], z.shape[0]):
+            return self.head.loss([z], [self.head.in_dim], labels, sums, relu_first=False)
+        return F.bce_with_logits(self.head(z), labels, sums)[0]
 
 
 class WideDeep(Model):
@@ -65,11 +74,21 @@ class WideDeep(Model):
         self.sub_model = WideDeepSubModel(len(linear_features) * self.linear_emb.out_dim, len(dnn_features) * self.deep_emb.out_dim,
                                           dense_dim, dnn_hidden_units, use_bn)
 
-    def forward(self, features):
+    def _inputs(self, features):
         with pulled_together([self.linear_emb, self.deep_emb], features):
             lin = self.linear_emb(features)
             deep = self.deep_emb(features)
-        dense = features[self.dense_key].to(deep.device, non_blocking=True) if self.dense_dim else None
+        return lin, deep, features[self.dense_key].to(deep.device, non_blocking=True) if self.dense_dim else None
+
+    def fused_train_loss(self, features, labels, sums):
+        """Training loss with the head, its loss and its backward pass in one kernel; None where somebody looks at what
+        passes in between."""
+        if not own_step(self, WideDeep, self.sub_model, WideDeepSubModel):
+            return None
+        return self.sub_model.train_loss(*self._inputs(features), labels, sums)
+
+    def forward(self, features):
+        lin, deep, dense = self._inputs(features)
         sub = self.sub_model
         if not self.use_fused and type(sub) is WideDeepSubModel and "forward" not in sub.__dict__:
             return sub(lin, deep, dense, fused=False)

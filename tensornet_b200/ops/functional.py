@@ -597,47 +597,54 @@ def deepfm_input(anchor, link, ids, B, S, dense=None, training=True, emb_dim=Non
     return x0, fm, (lin if lin_col >= 0 else None)
 
 
-_HEAD_SCRATCH = {}
-
-
-def _head_scratch(dev) -> torch.Tensor:
-    """Persistent scratch per device that the head kernel leaves at zero: partial loss, finished-block count and
-    sixteen partial copies of the head's weight gradient."""
-    key = (dev.type, dev.index)
-    if key not in _HEAD_SCRATCH:
-        _HEAD_SCRATCH[key] = torch.zeros(4 + 16 * 576, dtype=torch.float32, device=dev)
-    return _HEAD_SCRATCH[key]
-
-
-class _DeepFMHeadLoss(torch.autograd.Function):
+class _HeadLoss(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, h, lin, fm, w, label, sums, n_hidden):
-        B = h.shape[0]
-        dev = h.device
-        dh = torch.empty_like(h)
-        dl = torch.empty_like(lin) if lin is not None else None
-        dfm = torch.empty(B, dtype=torch.float32, device=dev)
-        loss = torch.empty((), dtype=torch.float32, device=dev)     # written (not accumulated) by the last block
-        pred = torch.empty(B, dtype=torch.float32, device=dev)
-        _ext().deepfm_head_loss(h, n_hidden, None if lin is None else lin.contiguous(), fm.contiguous().view(-1), w,
-                                label.contiguous().view(-1).float(), dh, dl, dfm, _grad_buffer(w), sums, pred, loss,
-                                _head_scratch(dev))
-        ctx.save_for_backward(dh, dl if dl is not None else dfm, dfm)
-        ctx.has_lin = lin is not None
-        ctx.mark_non_differentiable(pred)
-        ctx.set_materialize_grads(False)        # (no zeros for the prediction's)
-        return loss, pred
+    def forward(ctx, w, label, sums, scratch, relu_first, widths, pred, *pieces):
+        needs = ctx.needs_input_grad[7:]
+        # (a bf16 piece's gradient has its padding too, zeros there)
+        grads = [torch.empty(p.shape, dtype=p.dtype, device=p.device) if need else None for p, need in zip(pieces, needs)]
+        loss = torch.empty((), dtype=torch.float32, device=w.device)
+        _ext().head_loss(list(pieces), list(widths), w, label, grads, relu_first, _grad_buffer(w), sums, loss, scratch, pred)
+        ctx.save_for_backward(*[g for g in grads if g is not None])
+        ctx.there = [g is not None for g in grads]
+        return loss
 
     @staticmethod
-    def backward(ctx, gloss, _gpred):
-        # The head's gradients were produced by the forward pass for d(loss) = 1, which is what
-        # ``loss.backward()`` supplies; a caller that scales the loss must use the unfused head.
-        dh, dl, dfm = ctx.saved_tensors
-        return dh, (dl if ctx.has_lin else None), dfm.view(-1, 1), None, None, None, None
+    def backward(ctx, gloss):
+        # The gradients were produced by the forward pass for d(loss) = 1, which is what a model's own step supplies.
+        it = iter(ctx.saved_tensors)
+        return (None,) * 7 + tuple(next(it) if there else None for there in ctx.there)
+
+
+def head_span(widths: Sequence[int]) -> int:
+    """Weights of a head over pieces of these widths as the head kernels lay them out."""
+    return sum(pad8(k) for k in widths)
+
+
+def head_scratch(widths: Sequence[int], device) -> torch.Tensor:
+    """What :func:`head_loss` keeps between calls: zeros, which the kernel leaves as zeros."""
+    return torch.zeros(4 + _ext().HEAD_COPIES * (head_span(widths) + 8), dtype=torch.float32, device=device)
+
+
+def head_loss(pieces, widths, w, label, sums, scratch, relu_first: bool = True, pred: Optional[torch.Tensor] = None):
+    """``Dense(1)`` over ``[piece[:, :width] ... | 1]``, mean sigmoid cross-entropy and the whole backward pass of the head in one
+    kernel (GPU).  Pieces are bf16 matrices in the padded layout of the towers or fp32 ones of exactly their width.
+    ``relu_first``: the first piece is a ReLU's output, its gradient comes masked.  The weight's gradient is added to
+    ``w.grad`` right away, and the loss has to be back-propagated with a unit gradient.  ``scratch``: see
+    :func:`head_scratch`; ``pred`` (fp32 ``[B]``) receives the probabilities."""
+    return _HeadLoss.apply(w, label, sums, scratch, relu_first, tuple(widths), pred, *pieces)
+
+
+def head_score(pieces, widths, w) -> torch.Tensor:
+    """The logits ``[B, 1]`` of the same head, without gradients (GPU)."""
+    out = torch.empty((pieces[0].shape[0], 1), dtype=torch.float32, device=w.device)
+    _ext().head_score([p.detach() for p in pieces], list(widths), w.detach(), out)
+    return out
 
 
 def deepfm_head_loss(h, lin, fm, w, label, sums, n_hidden):
-    """``Dense(1)`` over ``[h[:, :n_hidden] | lin | fm | 1]`` + mean sigmoid cross-entropy, with the whole backward of
-    the head computed in the same kernel.  The weight gradient is accumulated into ``w.grad`` right away and the
-    returned loss must be back-propagated with a unit gradient.  Returns ``(loss, prediction)``."""
-    return _DeepFMHeadLoss.apply(h, lin, fm, w, label, sums, n_hidden)
+    """:func:`head_loss` over ``[h[:, :n_hidden] | lin | fm]`` as ``(loss, prediction)``."""
+    pieces = [h] + ([lin.contiguous()] if lin is not None else []) + [fm.reshape(-1, 1)]
+    widths = [n_hidden] + [int(p.shape[1]) for p in pieces[1:]]
+    pred = torch.empty(h.shape[0], dtype=torch.float32, device=h.device)
+    return head_loss(pieces, widths, w, label.contiguous().view(-1).float(), sums, head_scratch(widths, h.device), True, pred), pred

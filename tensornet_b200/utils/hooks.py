@@ -13,3 +13,17 @@ def unobserved(*modules, backward: bool = False) -> bool:
         return False
     return not any(m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__
                    or (backward and (m._backward_hooks or m._backward_pre_hooks)) for m in modules)
+
+
+def own_step(model, model_cls, sub_model, sub_cls) -> bool:
+    """Whether a training step of ``model`` may pass by the calls of the model, of its dense part and of its ``Dense(1)`` head: they
+    are the package's own (a subclass of the user's may add methods, not replace the ones passed by), on a GPU, with nobody looking on."""
+    from ..core.runtime import runtime
+    from ..layers.dense import DenseHead
+
+    cls = type(model)
+    if not runtime().on_gpu or type(sub_model) is not sub_cls or type(sub_model.head) is not DenseHead:
+        return False
+    if any(getattr(cls, k) is not getattr(model_cls, k) or k in model.__dict__ for k in ("forward", "__call__", "_loss")):
+        return False
+    return unobserved(model, sub_model, sub_model.head, backward=True)
