@@ -249,13 +249,13 @@ __device__ __forceinline__ void prefetch_aux(const GemmParams& p, int row_base, 
 }
 
 // What a kernel's epilogue has to be ready for.
-enum Kinds { kBf16, kNoAux, kAny };          // a plain bf16 output; no auxiliary operands; everything
+enum Kinds { kBf16, kNoAux, kGrad, kAny };   // a plain bf16 output; no auxiliary operands; fp32 or masked; everything
 template <Kinds kKinds, class Ready>
 __device__ __forceinline__ bool store_rows(const GemmParams& p, uint32_t tm_lane, int row_base, int n0, int BN, int sub, int nsubs,
                                            int lane, uint8_t* sm_out, Ready&& ready) {
   if (kKinds != kBf16 && p.out_f32) return store_f32(p, tm_lane, row_base, n0, BN, sub, nsubs, lane, sm_out, ready);
-  if (kKinds != kAny) return store_bf16<kPlain>(p, tm_lane, row_base, n0, BN, sub, nsubs, lane, sm_out, ready);
-  if (p.mask_aux != nullptr) return store_bf16<kMask>(p, tm_lane, row_base, n0, BN, sub, nsubs, lane, sm_out, ready);
+  if (kKinds == kBf16 || kKinds == kNoAux) return store_bf16<kPlain>(p, tm_lane, row_base, n0, BN, sub, nsubs, lane, sm_out, ready);
+  if (kKinds == kGrad || p.mask_aux != nullptr) return store_bf16<kMask>(p, tm_lane, row_base, n0, BN, sub, nsubs, lane, sm_out, ready);
   if (p.had_xl != nullptr) return store_bf16<kResidual>(p, tm_lane, row_base, n0, BN, sub, nsubs, lane, sm_out, ready);
   return store_bf16<kPlain>(p, tm_lane, row_base, n0, BN, sub, nsubs, lane, sm_out, ready);
 }

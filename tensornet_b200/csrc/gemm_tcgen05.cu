@@ -33,6 +33,7 @@ namespace tn {
 using namespace tc;
 using gemm_epi::kAny;
 using gemm_epi::kBf16;
+using gemm_epi::kGrad;
 
 namespace {
 
@@ -45,8 +46,11 @@ constexpr int kEpiWarps = 4 * kEpiSubs;
 constexpr int kGemmThreads = 32 * (2 + kEpiWarps);   // warp0 TMA, warp1 MMA + TMEM owner, the rest epilogue
 constexpr int kEpiBytesPerWarp = gemm_epi::kBytesPerWarp;
 
+// 64 registers for what a training step runs: an SM's four register files take five warps of this kernel and then have room for
+// three of another one, so that a block of 128 threads (the lookup of the next batch) can run beside it.  At 72, for none of 256
+// threads, at 96 for none.  Nothing is spilled; kernel times are the same.
 template <int kStages, int kHalves, gemm_epi::Kinds kKinds>
-__global__ void __launch_bounds__(kGemmThreads, 1)
+__global__ void __maxnreg__(kKinds == kAny || kHalves == 2 ? 96 : 64)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                          const GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -312,6 +316,11 @@ const char* gemm_bf16_pair(const GemmDesc& d, const GemmParams& p, int raster_gr
 double gemm_splitk_plan(const GemmDesc& d, int* best_bn, int* best_s);
 const char* gemm_bf16_splitk(const GemmDesc& d, GemmParams p, int BN, int S, cudaStream_t stream);
 
+static int highest_priority() {
+  static const int p = []() { int lo = 0, hi = 0; return cudaDeviceGetStreamPriorityRange(&lo, &hi) == cudaSuccess ? hi : 0; }();
+  return p;
+}
+
 const char* gemm_bf16(const GemmDesc& d, cudaStream_t stream) {
   if (d.M <= 0 || d.N <= 0 || d.K <= 0) return "gemm_bf16: empty problem";
   if ((reinterpret_cast<uintptr_t>(d.A) & 15) || (reinterpret_cast<uintptr_t>(d.B) & 15)) return "gemm_bf16: operands must be 16-byte aligned";
@@ -447,7 +456,8 @@ const char* gemm_bf16(const GemmDesc& d, cudaStream_t stream) {
   static bool attr_set = false;
   if (!attr_set) {
     for (auto* k : {gemm_bf16_tcgen05_kernel<8, 1, kBf16>, gemm_bf16_tcgen05_kernel<6, 1, kBf16>, gemm_bf16_tcgen05_kernel<4, 1, kBf16>,
-                    gemm_bf16_tcgen05_kernel<3, 2, kBf16>, gemm_bf16_tcgen05_kernel<8, 1, kAny>, gemm_bf16_tcgen05_kernel<6, 1, kAny>,
+                    gemm_bf16_tcgen05_kernel<3, 2, kBf16>, gemm_bf16_tcgen05_kernel<8, 1, kGrad>, gemm_bf16_tcgen05_kernel<6, 1, kGrad>,
+                    gemm_bf16_tcgen05_kernel<4, 1, kGrad>, gemm_bf16_tcgen05_kernel<8, 1, kAny>, gemm_bf16_tcgen05_kernel<6, 1, kAny>,
                     gemm_bf16_tcgen05_kernel<4, 1, kAny>, gemm_bf16_tcgen05_kernel<3, 2, kAny>})
       cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
     attr_set = true;
@@ -459,24 +469,29 @@ const char* gemm_bf16(const GemmDesc& d, cudaStream_t stream) {
   cfg.gridDim = grid;
   cfg.blockDim = dim3(kGemmThreads);
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[2];
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  attr[0].id = cudaLaunchAttributePriority;            // before what runs beside them, such as the next batch's lookup
+  attr[0].val.priority = highest_priority();
   cfg.attrs = attr;
-  cfg.numAttrs = use_pdl ? 1 : 0;
+  cfg.numAttrs = use_pdl ? 2 : 1;
   // Plain bf16 outputs (forward products) have instances of their own.  With all epilogues in one kernel the plain one takes
   // 0.2 to 0.5 us longer where its instructions are at hand (512 x 512 x 1025 8.9 -> 9.1, 8192 x 400 x 401 9.8 -> 10.3,
   // launch to launch) and 2 us where the kernel runs once between others, as in a request of 512 examples (a pass 93.5 ->
-  // 97.6).  Everything else stays together: each further kernel of a short step is one more that starts without its
-  // instructions (sixteen steps of 1024 examples through 64-32: 1 570 us; fp32 outputs beside the plain ones 1 625; all in one 1 610).
+  // 97.6).  Weight gradients and masked products
+  // share another set, without the residual epilogue, whose registers it would take (sixteen steps of 1024 examples through
+  // 64-32: 1 580 -> 1 525 us, 32 steps of 32: 3 050 -> 2 920).  Each further kernel of a short step is one more that starts without
+  // its instructions: with fp32 and masked outputs apart the former took 3 % longer.
   const bool plain = !d.out_f32 && !d.mask_aux && !d.had_x0 && !d.had_xl;
   cudaError_t e;
   if (smem > 220 * 1024) return "gemm_bf16: tile does not fit in shared memory";
   cfg.dynamicSmemBytes = smem;
+  const bool grad = !plain && !d.had_x0 && !d.had_xl;
+#define TN_GEMM(st) (plain ? gemm_bf16_tcgen05_kernel<st, 1, kBf16> : grad ? gemm_bf16_tcgen05_kernel<st, 1, kGrad> : gemm_bf16_tcgen05_kernel<st, 1, kAny>)
   auto* kernel = halves == 2   ? (plain ? gemm_bf16_tcgen05_kernel<3, 2, kBf16> : gemm_bf16_tcgen05_kernel<3, 2, kAny>)
-                 : stages == 8 ? (plain ? gemm_bf16_tcgen05_kernel<8, 1, kBf16> : gemm_bf16_tcgen05_kernel<8, 1, kAny>)
-                 : stages == 6 ? (plain ? gemm_bf16_tcgen05_kernel<6, 1, kBf16> : gemm_bf16_tcgen05_kernel<6, 1, kAny>)
-                               : (plain ? gemm_bf16_tcgen05_kernel<4, 1, kBf16> : gemm_bf16_tcgen05_kernel<4, 1, kAny>);
+                 : stages == 8 ? TN_GEMM(8) : stages == 6 ? TN_GEMM(6) : TN_GEMM(4);
+#undef TN_GEMM
   e = cudaLaunchKernelEx(&cfg, kernel, tmA, tmB, p);
   if (e == cudaSuccess) e = cudaGetLastError();
   return e == cudaSuccess ? nullptr : cudaGetErrorString(e);
