@@ -46,7 +46,7 @@ CUDA_SOURCES = [
     "serving.cu",
     "bn.cu",
     "unique.cu",
-    "deepfm_fused.cu",
+    "embed_input.cu",
     "no_alloc.cu",
 ]
 CPU_SOURCES = ["cpu_ref.cpp", "tfrecord.cpp"]

@@ -711,18 +711,27 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         tn::launch_seq_fwd(self.source(req), ptr_of<int>(inverse), ptr_of<int>(offsets), B, T, self.t.dim + 2 * self.t.use_cvm,
                            ptr_of<float>(out), ptr_of<int>(lengths), cur_stream());
       })
-      .def("deepfm_input_fwd", [](SparseCtx& self, at::Tensor inverse, int B, int S, int D, c10::optional<at::Tensor> dense, at::Tensor X0,
-                                  at::Tensor fm, int lin_col, c10::optional<at::Tensor> Lout, c10::optional<at::Tensor> E,
-                                  c10::optional<at::Tensor> req) {
+      .def("embed_input_fwd", [](SparseCtx& self, at::Tensor inverse, c10::optional<at::Tensor> offsets, int B, int S, int D, int combiner,
+                                 c10::optional<at::Tensor> dense, at::Tensor X0, c10::optional<at::Tensor> E, c10::optional<at::Tensor> fm,
+                                 c10::optional<at::Tensor> fsum, int lin_col, c10::optional<at::Tensor> Lout, c10::optional<at::Tensor> req) {
         c10::cuda::CUDAGuard guard(X0.device());
-        const int Dd = dense ? (int)dense->size(1) : 0;
-        TORCH_CHECK(!E || (E->scalar_type() == at::kFloat && E->is_contiguous() && E->numel() == (int64_t)B * S * D),
-                    "deepfm_input: E must be fp32 [B, S * D]");
-        const char* err = tn::launch_deepfm_input_fwd(self.source(req), ptr_of<int>(inverse), B, S, D, dense ? ptr_of<float>(*dense) : nullptr,
-                                                      Dd, dense ? (int)dense->stride(0) : 0, X0.data_ptr(), (int)X0.stride(0),
-                                                      ptr_of<float>(fm), Lout ? lin_col : -1, Lout ? ptr_of<float>(*Lout) : nullptr,
-                                                      E ? ptr_of<float>(*E) : nullptr, cur_stream());
-        if (err) throw std::runtime_error(err);
+        auto f32 = [](const c10::optional<at::Tensor>& t, int64_t n) { return !t || (t->scalar_type() == at::kFloat && t->is_contiguous() && t->numel() >= n); };
+        const int pd = self.t.dim + 2 * self.t.use_cvm;
+        TORCH_CHECK(D >= 1 && D <= pd && lin_col < self.t.dim && (!offsets || offsets->numel() >= (int64_t)B * S + 1) &&
+                        (offsets || inverse.numel() >= (int64_t)B * S), "embed_input: slots");
+        TORCH_CHECK(X0.scalar_type() == at::kBFloat16 && X0.dim() == 2 && X0.stride(1) == 1 && X0.size(0) == B && (!E || (f32(E, 0) && E->dim() == 2 && E->size(0) == B)) &&
+                        f32(fm, B) && f32(fsum, (int64_t)B * ((D + 3) / 4 * 4)) && f32(Lout, (int64_t)B * S) &&
+                        (!dense || (dense->scalar_type() == at::kFloat && dense->dim() == 2 && dense->stride(1) == 1 && dense->size(0) == B)),
+                    "embed_input: outputs or dense features");
+        tn::EmbedInput a = {};
+        a.inverse = ptr_of<int>(inverse); a.offsets = offsets ? ptr_of<int>(*offsets) : nullptr;
+        a.B = B; a.S = S; a.D = D; a.combiner = combiner;
+        a.dense = dense ? ptr_of<float>(*dense) : nullptr;
+        a.Dd = dense ? (int)dense->size(1) : 0; a.ld_dense = dense ? (int)dense->stride(0) : 0;
+        a.X0 = X0.data_ptr(); a.ld = (int)X0.stride(0);
+        a.E = E ? ptr_of<float>(*E) : nullptr; a.ldE = E ? (int)E->size(1) : 0; a.fm = fm ? ptr_of<float>(*fm) : nullptr; a.fsum = fsum ? ptr_of<float>(*fsum) : nullptr;
+        a.Lout = Lout ? ptr_of<float>(*Lout) : nullptr; a.lin_col = Lout ? lin_col : -1;
+        if (const char* err = tn::launch_embed_input_fwd(self.source(req), a, cur_stream())) throw std::runtime_error(err);
       });
   py::class_<ServeCtx>(m, "ServeCtx")
       .def(py::init<py::dict, int, int, std::vector<int>, bool>())
@@ -996,13 +1005,24 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     tn::launch_bce(ptr_of<float>(logit), ptr_of<float>(label), (int)logit.numel(), pred ? ptr_of<float>(*pred) : nullptr,
                    dlogit ? ptr_of<float>(*dlogit) : nullptr, grad_scale, ptr_of<float>(sums), hist_bins(sums), cur_stream());
   });
-  m.def("deepfm_input_bwd", [](at::Tensor E, at::Tensor inverse, int B, int S, int D, at::Tensor dX0, at::Tensor gfm,
-                               at::Tensor gU, int gstride, int lin_col, c10::optional<at::Tensor> dL) {
-    c10::cuda::CUDAGuard guard(E.device());
-    const char* err = tn::launch_deepfm_input_bwd(ptr_of<float>(E), ptr_of<int>(inverse), B, S, D, dX0.data_ptr(),
-                                                  (int)dX0.stride(0), ptr_of<float>(gfm), ptr_of<float>(gU), gstride, dL ? lin_col : -1,
-                                                  dL ? ptr_of<float>(*dL) : nullptr, cur_stream());
-    if (err) throw std::runtime_error(err);
+  m.attr("EMBED_INPUT_COLUMNS") = tn::kEmbedInputColumns;
+  m.def("embed_input_bwd", [](at::Tensor inverse, c10::optional<at::Tensor> offsets, int B, int S, int D, int dim, int combiner, at::Tensor dX0,
+                              c10::optional<at::Tensor> E, c10::optional<at::Tensor> fsum, c10::optional<at::Tensor> gfm,
+                              c10::optional<at::Tensor> gE, c10::optional<at::Tensor> dL, int lin_col, at::Tensor gU, int gstride) {
+    c10::cuda::CUDAGuard guard(dX0.device());
+    auto f32 = [](const c10::optional<at::Tensor>& t, int64_t n) { return !t || (t->scalar_type() == at::kFloat && t->is_contiguous() && t->numel() >= n); };
+    auto cols = [&](const c10::optional<at::Tensor>& t) { return !t || (f32(t, 0) && t->dim() == 2 && t->size(0) == B && t->size(1) >= (int64_t)S * D); };
+    TORCH_CHECK(dX0.scalar_type() == at::kBFloat16 && dX0.dim() == 2 && dX0.stride(1) == 1 && dX0.size(0) == B && dX0.size(1) >= (int64_t)S * D &&
+                    cols(E) && cols(gE) && (!E || !gE || E->size(1) == gE->size(1)) && f32(fsum, (int64_t)B * ((D + 3) / 4 * 4)) && f32(gfm, B) &&
+                    f32(dL, (int64_t)B * S) && (!gfm || (E && fsum)), "embed_input_bwd: gradients");
+    tn::EmbedGrad a = {};
+    a.inverse = ptr_of<int>(inverse); a.offsets = offsets ? ptr_of<int>(*offsets) : nullptr;
+    a.B = B; a.S = S; a.D = D; a.dim = dim; a.combiner = combiner;
+    a.dX0 = dX0.data_ptr(); a.ld = (int)dX0.stride(0);
+    a.E = E ? ptr_of<float>(*E) : nullptr; a.fsum = fsum ? ptr_of<float>(*fsum) : nullptr; a.gfm = gfm ? ptr_of<float>(*gfm) : nullptr;
+    a.gE = gE ? ptr_of<float>(*gE) : nullptr; a.ldE = E ? (int)E->size(1) : gE ? (int)gE->size(1) : 0; a.dL = dL ? ptr_of<float>(*dL) : nullptr; a.lin_col = lin_col;
+    a.gU = ptr_of<float>(gU); a.gstride = gstride;
+    if (const char* err = tn::launch_embed_input_bwd(a, cur_stream())) throw std::runtime_error(err);
   });
   {
     auto pieces_of = [](const std::vector<at::Tensor>& pieces, const std::vector<int>& widths, at::Tensor w) {

@@ -115,12 +115,41 @@ struct HeadArgs {
 const char* launch_head_loss(HeadArgs a, cudaStream_t st);
 const char* launch_head_score(HeadArgs a, cudaStream_t st);
 
-// deepfm_fused.cu  (return nullptr or a static error string)
-// `E` (may be null): the rows as they were read, [B, S * D] fp32, which the backward pass takes
-const char* launch_deepfm_input_fwd(const RowSource& src, const int* inverse, int B, int S, int D, const float* dense, int Dd, int ld_dense,
-                                    void* X0, int ld, float* fm, int lin_col, float* Lout, float* E, cudaStream_t st);
-const char* launch_deepfm_input_bwd(const float* E, const int* inverse, int B, int S, int D, const void* dX0, int ld, const float* gfm,
-                                    float* gU, int gstride, int lin_col, const float* dL, cudaStream_t st);
+// embed_input.cu  (return nullptr or a static error string)
+constexpr int kEmbedInputColumns = 128;
+struct EmbedInput {
+  const int* inverse;
+  const int* offsets;        // as in pool_fwd; null: one id a bag
+  int B, S, D, combiner;     // columns of a pooled slot
+  const float* dense;        // [B, Dd], row stride ld_dense
+  int Dd, ld_dense;
+  void* X0;                  // bf16 [B, ld]
+  int ld;
+  float* E;                  // pooled columns [B, S * D] in fp32, or with the dense features behind them; may be null
+  int ldE;                   // S * D or S * D + Dd
+  float* fm;                 // [B]; may be null
+  float* fsum;               // [B, 4 * ceil(D / 4)], the field sums of the FM term for the backward pass; may be null
+  float* Lout;               // [B, S]: column lin_col of the rows; lin_col < 0: not wanted
+  int lin_col;
+};
+struct EmbedGrad {
+  const int* inverse;
+  const int* offsets;
+  int B, S, D, dim, combiner;      // the first `dim` columns of a slot have a gradient
+  const void* dX0;                 // bf16 [B, ld]
+  int ld;
+  const float* E;                  // with gfm: what the forward pass has left
+  const float* fsum;
+  const float* gfm;                // [B], or null
+  const float* gE;                 // gradient of the pooled columns, or null
+  int ldE;                         // row stride of E and gE
+  const float* dL;                 // [B, S], or null
+  int lin_col;
+  float* gU;
+  int gstride;
+};
+const char* launch_embed_input_fwd(const RowSource& src, const EmbedInput& a, cudaStream_t st);
+const char* launch_embed_input_bwd(const EmbedGrad& a, cudaStream_t st);
 
 // unique.cu
 void launch_unique_assign(const long long* ids, int n, const float* labels, unsigned long long* dd_keys, int* dd_vals,

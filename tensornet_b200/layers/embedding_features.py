@@ -21,7 +21,8 @@ from torch import nn
 from .. import core
 from ..data.features import PACKED_KEY, gather_columns, padded_columns
 from ..feature_column import EmbeddingColumn
-from ..ops.embedding import expand_bag_labels, pull_pool
+from ..ops import functional as F
+from ..ops.embedding import COMBINERS, expand_bag_labels, pull_pool
 from ..utils.hooks import unobserved
 
 
@@ -145,19 +146,22 @@ class EmbeddingFeatures(nn.Module):
         pd = self.out_dim
         return [out[:, s * pd:(s + 1) * pd] for s in range(S)]
 
-    def fused_single_hot_inputs(self, features: Dict, training: bool):
-        """(ids, B) when this layer's slots are all single-hot and carry no CVM columns, else None.
-        Used by model-specific fused kernels that consume the pulled rows directly."""
-        if self.use_cvm or self.dim % 4 != 0:
-            return None
-        ids, offsets, B = self.stash_pull_args(features, training)[:3]
-        if offsets is not None:
-            if not unobserved(self):          # a hook may still change what `forward` finds in `features`
-                self._args_cache = None
-            return None
+    def gives_operand(self, width: Optional[int] = None) -> bool:
+        """Whether :meth:`operand` may stand in for a call of this layer: on a GPU, with nobody looking on."""
+        return (core.runtime().on_gpu and type(self) is EmbeddingFeatures and self.is_concat and (width or self.out_dim) <= 128
+                and unobserved(self, backward=True))
+
+    def operand(self, features: Dict, training: bool, dense: Optional[torch.Tensor] = None, fm: bool = False, width: Optional[int] = None,
+                lin_col: int = -1, pooled: bool = False):
+        """``(x0, fm, lin, pooled)`` of :func:`tensornet_b200.ops.functional.embed_input` for a batch, in place of pooling its
+        slots and assembling the dense part's operand from them.  ``width``: only the first columns of a slot."""
         self.table.set_training(training)
-        self._pending_push = training and self.trainable
-        return ids, B
+        ids, offsets, B, labels, label_mod, count = self._pull_args(features, training)
+        if dense is not None:
+            dense = dense.to(ids.device, non_blocking=True).float().contiguous()
+        self._pending_push = count
+        return F.embed_input(self._anchor, self.link, ids, offsets, B, len(self._keys), width or self.out_dim, COMBINERS[self.combiner],
+                             labels, label_mod, count, self._n_dev(features, offsets), dense, fm, lin_col, pooled)
 
     def ids_pulled_for(self, features: Dict):
         """The id tensor this layer's next training pull will receive for ``features``, when that is known ahead

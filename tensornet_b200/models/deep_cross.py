@@ -28,16 +28,16 @@ class DeepCrossSubModel(nn.Module):
         self.mlp = MLP(in_dim, hidden_units)
         self.head = DenseHead(self.mlp.out_dim + in_dim)
 
-    def _head_pieces(self, x: torch.Tensor, **kw):
+    def _head_pieces(self, x: torch.Tensor, x0=None, **kw):
+        """``x0``: ``x`` as the tower's operand, where that is there already."""
         cross = self.cross(x)
-        h = self.mlp(F.concat_cast([x], ones=True), **kw)
-        return [h, cross], [self.mlp.out_dim, None]
+        return [self.mlp(F.concat_cast([x], ones=True) if x0 is None else x0, **kw), cross]
 
-    def forward(self, x: torch.Tensor):
-        return self.head.on_pieces(*self._head_pieces(x))
+    def forward(self, x: torch.Tensor, x0=None):
+        return self.head.on_pieces(self._head_pieces(x, x0), [self.mlp.out_dim, None])
 
-    def train_loss(self, x, labels, sums):
-        return tower_loss(self.head, self.mlp, [self.mlp.out_dim, x.shape[1]], lambda **kw: self._head_pieces(x, **kw)[0], labels, sums)
+    def train_loss(self, x, x0, labels, sums):
+        return tower_loss(self.head, self.mlp, [self.mlp.out_dim, x.shape[1]], lambda **kw: self._head_pieces(x, x0, **kw), labels, sums)
 
 
 class CrossV2(nn.Module):
@@ -65,18 +65,19 @@ class DCNv2SubModel(nn.Module):
         self.mlp = MLP(in_dim, hidden_units)
         self.head = DenseHead(self.mlp.out_dim)
 
-    def _head_pieces(self, x, **kw):
-        x0 = F.concat_cast(list(x) if isinstance(x, (list, tuple)) else [x], ones=True)
-        xc = self.cross(x0)          # stacked structure: cross network feeds the deep network
-        return [self.mlp(xc, **kw)], [self.mlp.out_dim]
+    def _tower(self, x, x0=None, **kw):
+        if x0 is None:
+            x0 = F.concat_cast(list(x) if isinstance(x, (list, tuple)) else [x], ones=True)
+        return self.mlp(self.cross(x0), **kw)          # stacked structure: cross network feeds the deep network
 
-    def forward(self, x):
+    def forward(self, x, x0=None):
         """``x``: the input matrix, or its column blocks (embeddings, dense features): the blocks go straight into
-        the padded bf16 operand, without an fp32 concatenation in between (a 210 MB copy each way at width 6413)."""
-        return self.head(self._head_pieces(x)[0][0])
+        the padded bf16 operand, without an fp32 concatenation in between (a 210 MB copy each way at width 6413).  ``x0``: that
+        operand, where it is there already."""
+        return self.head(self._tower(x, x0))
 
-    def train_loss(self, x, labels, sums):
-        return tower_loss(self.head, self.mlp, [self.mlp.out_dim], lambda **kw: self._head_pieces(x, **kw)[0], labels, sums)
+    def train_loss(self, x, x0, labels, sums):
+        return tower_loss(self.head, self.mlp, [self.mlp.out_dim], lambda **kw: [self._tower(x, x0, **kw)], labels, sums)
 
 
 class _CrossModel(Model):
@@ -99,15 +100,25 @@ class _CrossModel(Model):
             x = torch.cat([x, dense], dim=1)
         return x
 
+    def _own(self) -> bool:
+        return type(self.sub_model) in (DeepCrossSubModel, DCNv2SubModel) and own_step(self, _CrossModel, self.sub_model, type(self.sub_model))
+
+    def _operands(self, features):
+        """``(x, x0)``: the input matrix and the same as the tower's operand; for DCN-v2 the operand alone."""
+        dense = features[self.dense_key] if self.dense_dim else None
+        if not self.deep_emb.gives_operand() or (dense is not None and (dense.requires_grad or dense.dim() != 2)):
+            return self._inputs(features), None
+        x0, _, _, x = self.deep_emb.operand(features, self.deep_emb.training, dense, pooled=type(self.sub_model) is DeepCrossSubModel)
+        return x, x0
+
     def fused_train_loss(self, features, labels, sums):
-        """Training loss with the head, its loss and its backward pass in one kernel; None where somebody looks at what
-        passes in between."""
-        sub = self.sub_model
-        if type(sub) not in (DeepCrossSubModel, DCNv2SubModel) or not own_step(self, _CrossModel, sub, type(sub)):
-            return None
-        return sub.train_loss(self._inputs(features), labels, sums)
+        """Training loss with the operand straight from the rows, and the head, its loss and its backward pass in one kernel; None
+        where somebody looks at what passes in between."""
+        return self.sub_model.train_loss(*self._operands(features), labels, sums) if self._own() else None
 
     def forward(self, features):
+        if not torch.is_grad_enabled() and self.use_fused and self._own():
+            return self.sub_model(*self._operands(features))
         return self.sub_model(self._inputs(features))
 
 

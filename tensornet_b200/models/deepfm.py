@@ -89,50 +89,47 @@ class DeepFM(Model):
         sub = self.sub_model
         if not own_step(self, DeepFM, sub, DeepFMSubModel):
             return None
-        emb = [self.deep_emb] + ([self.linear_emb] if self.linear_emb is not None else [])
-        got = None
-        if all(type(e) is EmbeddingFeatures for e in emb) and unobserved(*emb, backward=True):
-            got = self._fused_inputs(features, True)
+        got = self._fused_inputs(features, True)
         if got is None:
             return sub.train_loss(*self._inputs(features), labels, sums)
-        x0, fm, lin = got
-        return tower_loss(sub.head, sub.mlp, sub._head_widths(), lambda **kw: [sub.mlp(x0, **kw), lin, fm], labels, sums)
+        x0, rest = got
+        return tower_loss(sub.head, sub.mlp, sub._head_widths(), lambda **kw: [sub.mlp(x0, **kw), *rest], labels, sums)
 
     def _fused_inputs(self, features, training):
-        """``(x0, fm, lin)``: the first layer's operand, FM term and linear weights through the fused input kernel, or None
-        when the inputs do not qualify."""
-        dq = self.emb_dim // 4
-        if (not core.runtime().on_gpu or (self.linear_emb is None and not self.share_linear_table) or self.emb_dim % 4 or dq & (dq - 1)
-                or dq > 32):
+        """``(x0, [linear weights, FM term])``: the first layer's operand and what goes to the head beside the tower's output,
+        through the fused input kernel; None when the layers are not the package's own or somebody looks on."""
+        emb = [self.deep_emb] + ([self.linear_emb] if self.linear_emb is not None else [])
+        dense = features[self.dense_key] if self.dense_dim else None
+        if (not isinstance(features, dict) or not all(type(e) is EmbeddingFeatures and unobserved(e, backward=True) for e in emb)
+                or not self.deep_emb.gives_operand(self.emb_dim if self.share_linear_table else None)
+                or (dense is not None and (dense.requires_grad or dense.dim() != 2))):
             return None
-        got = self.deep_emb.fused_single_hot_inputs(features, training)
-        if got is None:
-            return None
-        ids, B = got
-        dense = features[self.dense_key].to(ids.device, non_blocking=True) if self.dense_dim else None
-        args = (self.deep_emb._anchor, self.deep_emb.link, ids, B, len(self.deep_emb._keys), dense, training)
         if self.share_linear_table:
-            self.deep_emb._args_cache = None        # its forward pass does not follow
-            return F.deepfm_input(*args, self.emb_dim, self.emb_dim)
+            x0, fm, lin, _ = self.deep_emb.operand(features, training, dense, True, self.emb_dim, self.emb_dim)
+            return x0, [lin, fm]
+        if self.linear_emb is None:
+            x0, fm, _, _ = self.deep_emb.operand(features, training, dense, True)
+            return x0, [fm]
         with pulled_together([self.linear_emb, self.deep_emb], features, training):
-            self.deep_emb._args_cache = None
             lin = self.linear_emb(features, training=training)
-            x0, fm, _ = F.deepfm_input(*args)
-        return x0, fm, lin
+            x0, fm, _, _ = self.deep_emb.operand(features, training, dense, True)
+        return x0, [lin, fm]
 
-    def _scores(self, features):
+    def _scores(self, features, ragged: bool = False):
         """The logits by way of the fused input kernel (scoring: no gradients, layers in inference mode), or None when the
-        batch does not qualify or somebody looks at what passes between the layers."""
+        batch does not qualify or somebody looks at what passes between the layers.  ``ragged``: bags of ids qualify too."""
         own = [self.deep_emb, self.sub_model] + ([self.linear_emb] if self.linear_emb is not None else [])
         if (torch.is_grad_enabled() or not self.use_fused or type(self.sub_model) is not DeepFMSubModel or not isinstance(features, dict)
-                or any(m.training for m in own) or type(self.deep_emb) is not EmbeddingFeatures
-                or not unobserved(*own)):
+                or any(m.training for m in own) or not unobserved(*own)):
+            return None
+        if not ragged and self.deep_emb.stash_pull_args(features, False)[1] is not None:
+            self.deep_emb._args_cache = None
             return None
         got = self._fused_inputs(features, False)
         if got is None:
             return None
-        x0, fm, lin = got
-        return self.sub_model.head.on_pieces([self.sub_model.mlp(x0), lin, fm], self.sub_model._head_widths())
+        x0, rest = got
+        return self.sub_model.head.on_pieces([self.sub_model.mlp(x0), *rest], self.sub_model._head_widths())
 
     def _inputs(self, features):
         """The dense part's inputs through the layers one by one."""
@@ -155,7 +152,7 @@ class DeepFM(Model):
         return lin, deep, dense
 
     def forward(self, features):
-        logits = self._scores(features)
+        logits = self._scores(features, ragged=True)
         if logits is not None:
             return logits
         return self.sub_model(*self._inputs(features))

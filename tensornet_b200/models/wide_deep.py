@@ -33,9 +33,11 @@ class WideDeepSubModel(nn.Module):
                 and x0.is_cuda and x0.shape[0] > 0 and linear_emb.dim() == 2 and linear_emb.dtype == torch.float32 and linear_emb.stride(1) == 1
                 and unobserved(bn, mlp, backward=True))
 
-    def _head_operand(self, linear_emb, deep_emb, dense, fused: bool):
-        """Padded bf16 operand of the head."""
-        x0 = F.concat_cast([deep_emb] + ([dense.float()] if self.dense_dim else []), ones=True)
+    def _operand(self, deep_emb, dense):
+        return F.concat_cast([deep_emb] + ([dense.float()] if self.dense_dim else []), ones=True)
+
+    def _head_operand(self, linear_emb, x0, fused: bool):
+        """Padded bf16 operand of the head; ``x0``: of the tower."""
         if fused and self._joins(x0, linear_emb):
             # normalisation straight from the tower's output to the head's operand; its gradient comes back masked
             h = self.mlp(x0, grad_premasked=True)
@@ -48,11 +50,11 @@ class WideDeepSubModel(nn.Module):
 
     def forward(self, linear_emb, deep_emb, dense=None, fused: bool = True):
         """``fused``: the joint kernels may be used (a model's ``use_fused``)."""
-        return self.head(self._head_operand(linear_emb, deep_emb, dense, fused))
+        return self.head(self._head_operand(linear_emb, self._operand(deep_emb, dense), fused))
 
-    def train_loss(self, linear_emb, deep_emb, dense, labels, sums):
+    def train_loss(self, linear_emb, x0, labels, sums):
         """Loss of a step's logits with the head's backward pass in the same kernel."""
-        z = self._head_operand(linear_emb, deep_emb, dense, True)
+        z = self._head_operand(linear_emb, x0, True)
         if self.head.weight.requires_grad and labels.numel() == z.shape[0] and self.head.fits([self.head.in_dim], z.shape[0]):
             return self.head.loss([z], [self.head.in_dim], labels, sums, relu_first=False)
         return F.bce_with_logits(self.head(z), labels, sums)[0]
@@ -80,16 +82,28 @@ class WideDeep(Model):
             deep = self.deep_emb(features)
         return lin, deep, features[self.dense_key].to(deep.device, non_blocking=True) if self.dense_dim else None
 
+    def _operands(self, features):
+        """``(linear embeddings, operand of the tower)``."""
+        dense = features[self.dense_key] if self.dense_dim else None
+        if not self.deep_emb.gives_operand() or (dense is not None and (dense.requires_grad or dense.dim() != 2)):
+            lin, deep, dense = self._inputs(features)
+            return lin, self.sub_model._operand(deep, dense)
+        with pulled_together([self.linear_emb, self.deep_emb], features):
+            lin = self.linear_emb(features)
+            return lin, self.deep_emb.operand(features, self.deep_emb.training, dense)[0]
+
     def fused_train_loss(self, features, labels, sums):
-        """Training loss with the head, its loss and its backward pass in one kernel; None where somebody looks at what
-        passes in between."""
+        """Training loss with the tower's operand straight from the rows, and the head, its loss and its backward pass in one
+        kernel; None where somebody looks at what passes in between."""
         if not own_step(self, WideDeep, self.sub_model, WideDeepSubModel):
             return None
-        return self.sub_model.train_loss(*self._inputs(features), labels, sums)
+        return self.sub_model.train_loss(*self._operands(features), labels, sums)
 
     def forward(self, features):
-        lin, deep, dense = self._inputs(features)
         sub = self.sub_model
+        if not torch.is_grad_enabled() and self.use_fused and own_step(self, WideDeep, sub, WideDeepSubModel):
+            return sub.head(sub._head_operand(*self._operands(features), True))
+        lin, deep, dense = self._inputs(features)
         if not self.use_fused and type(sub) is WideDeepSubModel and "forward" not in sub.__dict__:
             return sub(lin, deep, dense, fused=False)
         return sub(lin, deep, dense)

@@ -555,48 +555,56 @@ def cross_v2(x0: torch.Tensor, weights: Sequence[torch.Tensor], dim: int) -> tor
 
 
 # =========================================================================================
-# DeepFM fusions (GPU only): embedding gather + FM + operand build; head + loss + head backward
+# the dense part's input straight from the pulled rows (GPU only)
 # =========================================================================================
-class _DeepFMInput(torch.autograd.Function):
+class _EmbedInput(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, anchor, link, ids, B, S, dense, training, emb_dim, lin_col, keep):
-        inverse = link.pull_in_place(ids, None, 0, training)
-        D = emb_dim
+    def forward(ctx, anchor, link, ids, offsets, B, S, D, combiner, labels, label_mod, training, n_dev, dense, fm, lin_col, pooled, keep):
+        inverse = link.pull_in_place(ids, labels, label_mod, training, n_dev)
+        dev = ids.device
         Dd = 0 if dense is None else int(dense.shape[1])
-        ld = pad8(S * D + Dd + 1)
-        x0 = torch.empty((B, ld), dtype=torch.bfloat16, device=ids.device)
-        fm = torch.empty(B, dtype=torch.float32, device=ids.device)
-        lin = torch.empty((B, S), dtype=torch.float32, device=ids.device) if lin_col >= 0 else None
-        emb = torch.empty((B, S * D), dtype=torch.float32, device=ids.device) if keep else None      # for the backward pass
-        link.ctx.deepfm_input_fwd(inverse, B, S, D, dense, x0, fm, lin_col, lin, emb, link.req)
-        ctx.link, ctx.inverse, ctx.emb, ctx.meta = link, inverse, emb, (B, S, D, lin_col)
-        if lin is None:
-            lin = torch.empty(0, device=ids.device)
-            ctx.mark_non_differentiable(lin)
-        return x0, fm.view(B, 1), lin
+
+        def f32(*shape):
+            return torch.empty(shape, dtype=torch.float32, device=dev)
+
+        x0 = torch.empty((B, pad8(S * D + Dd + 1)), dtype=torch.bfloat16, device=dev)
+        term = f32(B) if fm else None
+        lin = f32(B, S) if lin_col >= 0 else None
+        # the FM term's backward pass needs the pooled columns and their sums over the slots
+        emb = f32(B, S * D + Dd) if pooled else f32(B, S * D) if fm and keep else None
+        fsum = f32(B, (D + 3) // 4 * 4) if fm and keep else None
+        link.ctx.embed_input_fwd(inverse, offsets, B, S, D, combiner, dense, x0, emb, term, fsum, lin_col, lin, link.req)
+        ctx.link, ctx.inverse, ctx.offsets, ctx.meta = link, inverse, offsets, (B, S, D, combiner, lin_col)
+        ctx.emb, ctx.fsum = (emb, fsum) if fm else (None, None)
+        ctx.set_materialize_grads(False)
+        return x0, term.view(B, 1) if fm else None, lin, emb if pooled else None
 
     @staticmethod
-    def backward(ctx, gx0, gfm, glin):
+    def backward(ctx, gx0, gfm, glin, gpooled):
         link = ctx.link
-        B, S, D, lin_col = ctx.meta
-        if gfm is None:
-            gfm = torch.zeros(B, dtype=torch.float32, device=gx0.device)
-        dl = glin.contiguous() if (lin_col >= 0 and glin is not None) else None
-        _ext().deepfm_input_bwd(ctx.emb, ctx.inverse, B, S, D, gx0.contiguous(), gfm.contiguous().view(-1), link.gU,
-                                link.gstride, lin_col, dl)
-        return (None,) * 10
+        B, S, D, combiner, lin_col = ctx.meta
+        if gx0 is None:
+            gx0 = torch.zeros((B, pad8(S * D)), dtype=torch.bfloat16, device=link.dev)
+        _ext().embed_input_bwd(ctx.inverse, ctx.offsets, B, S, D, link.dim, combiner, gx0.contiguous(), ctx.emb if gfm is not None else None,
+                               ctx.fsum, None if gfm is None else gfm.contiguous().view(-1),
+                               None if gpooled is None else gpooled.contiguous(), None if glin is None else glin.contiguous(), lin_col,
+                               link.gU, link.gstride)
+        return (None,) * 17
 
 
-def deepfm_input(anchor, link, ids, B, S, dense=None, training=True, emb_dim=None, lin_col=-1):
-    """Pull the S single-hot slots of ``ids`` ([S*B], slot after slot) and build in one pass the padded bf16 operand
-    ``[emb | dense | 1 | 0]`` of the first MLP layer plus the second-order FM term ``[B, 1]``.  When the table rows carry
-    the slot's linear weight in column ``lin_col`` (``emb_dim`` < row width), also returns those weights ``[B, S]``."""
-    if dense is not None:
-        dense = dense.float().contiguous()
-    x0, fm, lin = _DeepFMInput.apply(anchor, link, ids, B, S, dense, training, emb_dim or link.dim, lin_col, torch.is_grad_enabled())
-    return x0, fm, (lin if lin_col >= 0 else None)
+def embed_input(anchor, link, ids, offsets, B, S, D, combiner, labels=None, label_mod=0, training=True, n_dev=None, dense=None, fm=False,
+                lin_col=-1, pooled=False):
+    """Pull the S slots of ``ids`` (as :func:`tensornet_b200.ops.embedding.pull_pool` does) and build in one pass ``(x0, fm, lin,
+    pooled)``: the padded bf16 operand ``[emb | dense | 1 | 0]`` of the first layer, with ``fm`` the second-order FM term of the
+    slots' first ``D`` columns ``[B, 1]``, where the rows carry the slot's linear weight in column ``lin_col`` those weights
+    ``[B, S]``, and with ``pooled`` the fp32 columns ``[emb | dense]``.  What is not asked for is None."""
+    return _EmbedInput.apply(anchor, link, ids, offsets, B, S, D, combiner, labels, label_mod, training, n_dev, dense, fm, lin_col, pooled,
+                             torch.is_grad_enabled())
 
 
+# =========================================================================================
+# head + loss + head backward (GPU only)
+# =========================================================================================
 class _HeadLoss(torch.autograd.Function):
     @staticmethod
     def forward(ctx, w, label, sums, scratch, relu_first, widths, pred, *pieces):

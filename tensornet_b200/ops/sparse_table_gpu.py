@@ -398,7 +398,7 @@ class GpuSparseLink:
     def pull_in_place(self, ids: torch.Tensor, labels: Optional[torch.Tensor] = None, label_mod: int = 0, training: bool = True,
                       n_dev: Optional[torch.Tensor] = None, lookup_only: bool = False) -> torch.Tensor:
         """:meth:`pull` for callers that read the rows at once and through ``self.ctx`` (``pool_fwd``, ``seq_fwd``,
-        ``deepfm_input_fwd``, given ``self.req``): on one GPU they stay in the table and ``self.U`` is not written."""
+        ``embed_input_fwd``, given ``self.req``): on one GPU they stay in the table and ``self.U`` is not written."""
         return self._pull(ids, labels, label_mod, training, None, lookup_only, n_dev, False)
 
     def _pull(self, ids, labels, label_mod, training, inverse, lookup_only, n_dev, rows):
