@@ -1169,14 +1169,15 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                                   cur_stream());
     });
     m.def("cross_v1_net_bwd", [net](at::Tensor x0, std::vector<at::Tensor> ws, std::vector<at::Tensor> bs, at::Tensor dots, at::Tensor gy,
-                                    at::Tensor gx0, at::Tensor gw, at::Tensor gb, at::Tensor t_row) {
+                                    at::Tensor gx0, std::vector<at::Tensor> gws, std::vector<at::Tensor> gbs, at::Tensor t_row) {
       c10::cuda::CUDAGuard guard(x0.device());
       tn::CrossNet n = net(x0, ws, bs);
-      TORCH_CHECK(gy.is_contiguous() && gy.scalar_type() == at::kFloat && gw.is_contiguous() && gb.is_contiguous() &&
-                      gw.numel() == n.layers * x0.size(1) && gb.numel() == gw.numel(), "cross_v1_net: gradients");
+      TORCH_CHECK(gy.is_contiguous() && gy.scalar_type() == at::kFloat && (int)gws.size() == n.layers && (int)gbs.size() == n.layers, "cross_v1_net: gradients");
       for (int l = 0; l < n.layers; ++l) {
-        n.gw[l] = ptr_of<float>(gw) + l * x0.size(1);
-        n.gb[l] = ptr_of<float>(gb) + l * x0.size(1);
+        for (const at::Tensor& g : {gws[l], gbs[l]})
+          TORCH_CHECK(g.is_cuda() && g.is_contiguous() && g.scalar_type() == at::kFloat && g.numel() == x0.size(1), "cross_v1_net: gradients");
+        n.gw[l] = ptr_of<float>(gws[l]);
+        n.gb[l] = ptr_of<float>(gbs[l]);
       }
       tn::launch_cross_v1_net_bwd(n, ptr_of<float>(x0), (int)x0.size(0), (int)x0.size(1), ptr_of<float>(dots), ptr_of<float>(gy),
                                   ptr_of<float>(gx0), ptr_of<float>(t_row), cur_stream());

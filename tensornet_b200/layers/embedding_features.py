@@ -222,9 +222,14 @@ def pull_together(layers: Sequence[EmbeddingFeatures], features: Dict, training:
             return False
     if len({id(l.table) for l in layers}) < len(layers) or not all(l.link.ctx.in_place() for l in layers):
         return False
-    calls = []
+    calls, first = [], layers[0]
     for l in layers:
         l.table.set_training(training)
-        ids, offsets, _, labels, label_mod, count = l.stash_pull_args(features, training)
+        if l is not first and l._keys == first._keys and l._target_columns == first._target_columns:
+            # the same slots: gathered once (columns of a batch are packed by a kernel)
+            l._args_cache = (features, training, (*first._args_cache[2][:5], training and l.trainable))
+            ids, offsets, _, labels, label_mod, count = l._args_cache[2]
+        else:
+            ids, offsets, _, labels, label_mod, count = l.stash_pull_args(features, training)
         calls.append((l.link, ids, labels, label_mod, count, l._n_dev(features, offsets)))
     return layers[0].link.pull_many(calls)

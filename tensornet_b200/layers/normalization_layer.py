@@ -45,13 +45,14 @@ class _BnJoin(torch.autograd.Function):
     gradient of ``h`` is zero where ``h`` is not above zero (the backward pass of the ReLU that made it)."""
 
     @staticmethod
-    def forward(ctx, h, x, gamma, beta, table, eps, n_h, masked):
+    def forward(ctx, h, x, gamma, beta, table, eps, n_h, masked, into):
         C = n_h + x.shape[1]
         z = torch.empty((h.shape[0], F.pad8(C + 1)), dtype=torch.bfloat16, device=h.device)
         moments = torch.empty(2 * C, dtype=torch.float32, device=h.device)       # the table moves on before the backward pass runs
         table.ctx.join_fwd(h, n_h, x, gamma, beta, float(eps), z, moments)
         ctx.save_for_backward(h, x, gamma, moments)
         ctx.table, ctx.meta, ctx.has_beta = table, (float(eps), n_h, masked), beta is not None
+        ctx.into = (gamma, beta) if into and F.adds_to_grad(gamma, beta) else None
         return z
 
     @staticmethod
@@ -61,11 +62,16 @@ class _BnJoin(torch.autograd.Function):
         C = n_h + x.shape[1]
         gh = torch.empty_like(h) if ctx.needs_input_grad[0] else None
         gx = torch.empty((x.shape[0], x.shape[1]), dtype=torch.float32, device=x.device) if ctx.needs_input_grad[1] else None
-        sums = torch.zeros((2, C), dtype=torch.float32, device=h.device)
-        gg = sums[0] if gamma is not None else None
-        gb = sums[1] if ctx.has_beta else None
+        if ctx.into is not None:
+            gg, gb = [None if p is None else p.grad for p in ctx.into]
+        else:
+            sums = torch.zeros((2, C), dtype=torch.float32, device=h.device)
+            gg = sums[0] if gamma is not None else None
+            gb = sums[1] if ctx.has_beta else None
         ctx.table.ctx.join_bwd(dz.contiguous(), h, n_h, x, moments, gamma, eps, masked, gh, gx, gg, gb)
-        return gh, gx, gg, gb, None, None, None, None
+        if ctx.into is not None:
+            gg = gb = None
+        return gh, gx, gg, gb, None, None, None, None, None
 
 
 class TNBatchNormalizationBase(nn.Module):
@@ -157,12 +163,13 @@ class TNBatchNormalizationBase(nn.Module):
             self._device_push(x2.detach(), True)
         return y.view(*inputs.shape[:-1], inputs.shape[-1])
 
-    def join_operand(self, h: torch.Tensor, n_h: int, x: torch.Tensor, masked: bool = False) -> torch.Tensor:
+    def join_operand(self, h: torch.Tensor, n_h: int, x: torch.Tensor, masked: bool = False, into_grads: bool = False) -> torch.Tensor:
         """``concat_cast([self(cat([h[:, :n_h].float(), x], 1))], ones=True)`` without the steps in between (device tables
-        only): ``h`` is a tower's padded bf16 output.  ``masked``: see :class:`_BnJoin`."""
+        only): ``h`` is a tower's padded bf16 output.  ``masked``: see :class:`_BnJoin`.  ``into_grads``: the backward pass is a model's
+        own and may add to the parameters' ``.grad`` itself."""
         if self.training:
             self._device_push(x.detach(), False, h.detach(), n_h)
-        return _BnJoin.apply(h, x, self.gamma, self.beta, self.table, self.epsilon, n_h, masked)
+        return _BnJoin.apply(h, x, self.gamma, self.beta, self.table, self.epsilon, n_h, masked, into_grads)
 
     def bn_statistics_pull(self):
         """Fold the other ranks' pending increments in (called by rank 0 before saving)."""

@@ -17,7 +17,7 @@ from ..layers import DeepCrossLayer, DenseHead, EmbeddingFeatures, MLP
 from ..layers.dense import tower_loss
 from ..model import Model
 from ..ops import functional as F
-from ..utils.hooks import own_step
+from ..utils.hooks import own_step, unobserved
 
 
 class DeepCrossSubModel(nn.Module):
@@ -28,16 +28,20 @@ class DeepCrossSubModel(nn.Module):
         self.mlp = MLP(in_dim, hidden_units)
         self.head = DenseHead(self.mlp.out_dim + in_dim)
 
-    def _head_pieces(self, x: torch.Tensor, x0=None, **kw):
-        """``x0``: ``x`` as the tower's operand, where that is there already."""
-        cross = self.cross(x)
+    def _head_pieces(self, x: torch.Tensor, x0=None, own: bool = False, **kw):
+        """``x0``: ``x`` as the tower's operand, where that is there already.  ``own``: for the backward pass of a model's own step."""
+        net = self.cross
+        if own and type(net) is DeepCrossLayer and unobserved(net, backward=True):
+            cross = F.cross_v1_net(x, list(net.W), list(net.bias), into_grads=True)
+        else:
+            cross = net(x)
         return [self.mlp(F.concat_cast([x], ones=True) if x0 is None else x0, **kw), cross]
 
     def forward(self, x: torch.Tensor, x0=None):
         return self.head.on_pieces(self._head_pieces(x, x0), [self.mlp.out_dim, None])
 
     def train_loss(self, x, x0, labels, sums):
-        return tower_loss(self.head, self.mlp, [self.mlp.out_dim, x.shape[1]], lambda **kw: self._head_pieces(x, x0, **kw), labels, sums)
+        return tower_loss(self.head, self.mlp, [self.mlp.out_dim, x.shape[1]], lambda **kw: self._head_pieces(x, x0, True, **kw), labels, sums)
 
 
 class CrossV2(nn.Module):

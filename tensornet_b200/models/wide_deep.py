@@ -36,12 +36,12 @@ class WideDeepSubModel(nn.Module):
     def _operand(self, deep_emb, dense):
         return F.concat_cast([deep_emb] + ([dense.float()] if self.dense_dim else []), ones=True)
 
-    def _head_operand(self, linear_emb, x0, fused: bool):
-        """Padded bf16 operand of the head; ``x0``: of the tower."""
+    def _head_operand(self, linear_emb, x0, fused: bool, own_step: bool = False):
+        """Padded bf16 operand of the head; ``x0``: of the tower.  ``own_step``: for the backward pass of a model's own step."""
         if fused and self._joins(x0, linear_emb):
             # normalisation straight from the tower's output to the head's operand; its gradient comes back masked
             h = self.mlp(x0, grad_premasked=True)
-            return self.bn.join_operand(h, self.mlp.out_dim, linear_emb, masked=True)
+            return self.bn.join_operand(h, self.mlp.out_dim, linear_emb, masked=True, into_grads=own_step)
         h = self.mlp(x0)
         if self.bn is None:
             return F.concat_cast([h, linear_emb], ones=True, widths=[self.mlp.out_dim, None])
@@ -54,7 +54,7 @@ class WideDeepSubModel(nn.Module):
 
     def train_loss(self, linear_emb, x0, labels, sums):
         """Loss of a step's logits with the head's backward pass in the same kernel."""
-        z = self._head_operand(linear_emb, x0, True)
+        z = self._head_operand(linear_emb, x0, True, own_step=True)
         if self.head.weight.requires_grad and labels.numel() == z.shape[0] and self.head.fits([self.head.in_dim], z.shape[0]):
             return self.head.loss([z], [self.head.in_dim], labels, sums, relu_first=False)
         return F.bce_with_logits(self.head(z), labels, sums)[0]

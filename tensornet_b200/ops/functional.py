@@ -64,6 +64,14 @@ def _grad_buffer(p: torch.Tensor) -> torch.Tensor:
     return p.grad
 
 
+def adds_to_grad(*params) -> bool:
+    """Whether a backward pass of a model's own step may add the gradients of these parameters (None: left out) to ``.grad`` itself:
+    they are leaves whose gradient is there, and no hook is to see it on the way."""
+    return all(p is None or (p.requires_grad and p.is_leaf and p.grad is not None and p.grad.is_contiguous() and p.grad.dtype == torch.float32
+                             and p.grad.device == p.device and not p._backward_hooks and not getattr(p, "_post_accumulate_grad_hooks", None))
+               for p in params)
+
+
 # =========================================================================================
 # concat + cast to the padded bf16 operand
 # =========================================================================================
@@ -437,7 +445,7 @@ class _CrossV1Net(torch.autograd.Function):
     """All layers of a rank-1 cross network over one input (``csrc/elementwise.cu``, ``cross_v1_net_*``)."""
 
     @staticmethod
-    def forward(ctx, x0, L, *params):
+    def forward(ctx, x0, L, into, *params):
         x0 = x0.contiguous()
         B, D = x0.shape
         ws, bs = [w.reshape(-1) for w in params[:L]], list(params[L:])
@@ -446,6 +454,7 @@ class _CrossV1Net(torch.autograd.Function):
         _ext().cross_v1_net_fwd(x0, ws, bs, y, dots)
         ctx.save_for_backward(x0, dots, *params)
         ctx.L = L
+        ctx.into = params if into and adds_to_grad(*params) else None
         return y
 
     @staticmethod
@@ -454,18 +463,22 @@ class _CrossV1Net(torch.autograd.Function):
         L = ctx.L
         B, D = x0.shape
         gx0 = torch.empty_like(x0)
-        sums = torch.zeros((2, L, D), dtype=torch.float32, device=x0.device)
-        _ext().cross_v1_net_bwd(x0, [w.reshape(-1) for w in params[:L]], list(params[L:]), dots, gy.contiguous(), gx0, sums[0], sums[1],
+        if ctx.into is not None:
+            grads = [p.grad for p in ctx.into]
+        else:
+            grads = [g.view(p.shape) for g, p in zip(torch.zeros((2 * L, D), dtype=torch.float32, device=x0.device), params)]
+        _ext().cross_v1_net_bwd(x0, [w.reshape(-1) for w in params[:L]], list(params[L:]), dots, gy.contiguous(), gx0, grads[:L], grads[L:],
                                 torch.empty_like(dots))
-        return (gx0, None, *[sums[0, l].view(params[l].shape) for l in range(L)], *[sums[1, l].view(params[L + l].shape) for l in range(L)])
+        return (gx0, None, None, *([None] * (2 * L) if ctx.into is not None else grads))
 
 
-def cross_v1_net(x0, ws, bs):
-    """``x_{l+1} = x0 * (x_l . w_l) + b_l + x_l`` from ``x_0 = x0`` on, for all layers."""
+def cross_v1_net(x0, ws, bs, into_grads: bool = False):
+    """``x_{l+1} = x0 * (x_l . w_l) + b_l + x_l`` from ``x_0 = x0`` on, for all layers.  ``into_grads``: the backward pass is a
+    model's own and may add the parameters' gradients to ``.grad`` itself (:func:`adds_to_grad`)."""
     D = x0.shape[-1]
     if (x0.is_cuda and x0.dim() == 2 and x0.dtype == torch.float32 and x0.shape[0] > 0 and D <= 1024 and 1 <= len(ws) <= 8
             and all(p.device == x0.device and p.dtype == torch.float32 and p.is_contiguous() and p.numel() == D for p in (*ws, *bs))):
-        return _CrossV1Net.apply(x0, len(ws), *ws, *bs)
+        return _CrossV1Net.apply(x0, len(ws), into_grads, *ws, *bs)
     cross = x0
     for w, b in zip(ws, bs):
         cross = cross_v1(x0, cross, w, b)

@@ -181,3 +181,23 @@ def test_models_with_the_head_in_one_kernel(kind, S, dim, hidden, bags, cvm):
     m.train_on_batch(f, y)
     assert seen
     hook.remove()
+
+
+@pytest.mark.parametrize("kind", ["wide_deep", "deep_cross"])
+def test_own_steps_add_to_the_gradients_and_hooks_still_see_them(kind):
+    """A model's own step adds the gradients of the cross network and of the batch norm to ``.grad`` in the kernels; a hook on one
+    of those parameters gets the gradient as before, and the steps are the same."""
+    tn.core.init()
+    B, seen, runs = 64, [], []
+    for hooked in (False, True):
+        m, slots = _model(kind, 5, 8, (32, 16), B, 1, False)
+        p = m.sub_model.bn.gamma if kind == "wide_deep" else m.sub_model.cross.W[1]
+        if hooked:
+            p.register_hook(lambda g: seen.append(g.clone()))
+        g = torch.Generator().manual_seed(2)
+        for _ in range(3):
+            f = {tn.data.PACKED_KEY: tn.data.PackedFeatures(slots, ids=torch.randint(0, 300, (5, B), generator=g)), "dense": torch.randn(B, 3, generator=g)}
+            m.train_on_batch(f, (torch.rand(B, generator=g) < 0.3).float())
+        runs.append(m.optimizer.table.W.clone())
+    assert len(seen) == 3 and all(bool(g.abs().sum() > 0) for g in seen)
+    assert float((runs[0] - runs[1]).norm()) <= 1e-3 * float(runs[1].norm())
