@@ -43,6 +43,7 @@ CUDA_SOURCES = [
     "dense_fused.cu",
     "elementwise.cu",
     "head.cu",
+    "stage.cu",
     "serving.cu",
     "bn.cu",
     "unique.cu",

@@ -792,10 +792,19 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("stage_inputs", [](std::vector<at::Tensor> dsts, std::vector<at::Tensor> srcs, int64_t copy_stream, int64_t main_stream,
                            int64_t done_event, int64_t copied_event, int64_t read_event) {
     TORCH_CHECK(dsts.size() == srcs.size(), "stage_inputs: one source per destination");
+    if (dsts.empty()) return;
+    c10::cuda::CUDAGuard guard(dsts[0].device());
     cudaStream_t cs = reinterpret_cast<cudaStream_t>(copy_stream), ms = reinterpret_cast<cudaStream_t>(main_stream);
     if (done_event) check(cudaStreamWaitEvent(cs, reinterpret_cast<cudaEvent_t>(done_event), 0), "cudaStreamWaitEvent");
     // the loss of the step that last used this buffer set has been read back (it lives in the same captured memory)
     if (read_event) check(cudaStreamWaitEvent(cs, reinterpret_cast<cudaEvent_t>(read_event), 0), "cudaStreamWaitEvent");
+    // Small leaves in page-locked memory go together, read by a kernel; larger ones, for which the copy engine is the faster reader,
+    // one copy each.  (A kernel for one leaf saves nothing; up to 256 KB its 22 to 30 GB/s are no slower than a copy's rate with
+    // its 2 us to the next one.)
+    constexpr int64_t kSmall = 256 * 1024;
+    tn::StagePieces pieces;
+    std::vector<size_t> small;
+    std::vector<const void*> seen;
     for (size_t i = 0; i < dsts.size(); ++i) {
       const at::Tensor& d = dsts[i];
       const at::Tensor& h = srcs[i];
@@ -803,13 +812,40 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       TORCH_CHECK(d.is_cuda() && !h.is_cuda() && d.is_contiguous() && h.is_contiguous() && d.scalar_type() == h.scalar_type() &&
                       (d.nbytes() == h.nbytes() || (d.dim() == 1 && h.dim() == 1 && h.nbytes() <= d.nbytes())),
                   "stage_inputs: leaf ", i, " must be a contiguous host tensor of the static buffer's type and size");
+      const void* p = (int64_t)h.nbytes() <= kSmall ? mapped_host_ptr(h) : nullptr;
+      if (p == nullptr) continue;
+      small.push_back(i);
+      seen.push_back(p);
+    }
+    if (small.size() < 2) { small.clear(); seen.clear(); }
+    size_t next = 0;
+    for (size_t i = 0; i < dsts.size(); ++i) {
+      const at::Tensor& d = dsts[i];
+      const at::Tensor& h = srcs[i];
       if (h.nbytes() == 0) continue;
+      if (next < small.size() && small[next] == i) { ++next; continue; }
       check(cudaMemcpyAsync(d.data_ptr(), h.data_ptr(), h.nbytes(), cudaMemcpyHostToDevice, cs), "cudaMemcpyAsync");
-      // a page-locked source from torch's host allocator must not be handed out again before the copy has run
-      // (what Tensor.copy_(non_blocking=True) does behind the scenes); a no-op for other host memory
-      if (h.is_pinned())
+    }
+    for (size_t at = 0; at < small.size(); at += tn::kStagePieces) {
+      pieces.n = 0;
+      for (size_t k = at; k < small.size() && k < at + tn::kStagePieces; ++k) {
+        pieces.src[pieces.n] = seen[k];
+        pieces.dst[pieces.n] = dsts[small[k]].data_ptr();
+        pieces.bytes[pieces.n++] = (int)srcs[small[k]].nbytes();
+      }
+      check(tn::launch_stage_inputs(pieces, cs), "stage_inputs launch");
+      g_launches.fetch_add(1, std::memory_order_relaxed);
+    }
+    // a page-locked source from torch's host allocator must not be handed out again before it has been read
+    // (what Tensor.copy_(non_blocking=True) does behind the scenes); a no-op for other host memory
+    next = 0;
+    for (size_t i = 0; i < dsts.size(); ++i) {
+      const bool in_kernel = next < small.size() && small[next] == i;
+      if (in_kernel) ++next;
+      const at::Tensor& h = srcs[i];
+      if (h.nbytes() != 0 && (in_kernel || h.is_pinned()))
         at::getHostAllocator(at::kCUDA)->record_event(const_cast<void*>(h.storage().data()), h.storage().data_ptr().get_context(),
-                                                      c10::cuda::getStreamFromExternal(cs, d.device().index()).unwrap());
+                                                      c10::cuda::getStreamFromExternal(cs, dsts[i].device().index()).unwrap());
     }
     check(cudaEventRecord(reinterpret_cast<cudaEvent_t>(copied_event), cs), "cudaEventRecord");
     check(cudaStreamWaitEvent(ms, reinterpret_cast<cudaEvent_t>(copied_event), 0), "cudaStreamWaitEvent");

@@ -151,6 +151,18 @@ struct EmbedGrad {
 const char* launch_embed_input_fwd(const RowSource& src, const EmbedInput& a, cudaStream_t st);
 const char* launch_embed_input_bwd(const EmbedGrad& a, cudaStream_t st);
 
+// stage.cu
+constexpr int kStagePieces = 96;
+constexpr int kStageBlockBytes = 8192;
+struct StagePieces {
+  int n;
+  const void* src[kStagePieces];       // page-locked host memory as the device sees it
+  void* dst[kStagePieces];
+  int bytes[kStagePieces];             // above zero
+  int first[kStagePieces];             // filled in by the launch
+};
+cudaError_t launch_stage_inputs(StagePieces& a, cudaStream_t st);
+
 // unique.cu
 void launch_unique_assign(const long long* ids, int n, const float* labels, unsigned long long* dd_keys, int* dd_vals,
                           unsigned scratch_cap, unsigned long long* uniq, int cap, int* inverse, float* show, float* click,

@@ -101,6 +101,19 @@ def batch_size_of(feature) -> int:
     return int(feature.shape[0])
 
 
+def adjacent_columns(cols) -> Optional[torch.Tensor]:
+    """Columns of int64 ids, one each per example, that lie one behind the other in one piece of memory, as a view of it; else
+    None.  (A captured step's static columns do: they need no concatenation.)"""
+    first = cols[0]
+    if not all(torch.is_tensor(c) and c.dtype == torch.int64 and c.is_contiguous() and c.dim() in (1, 2) and c.device == first.device for c in cols):
+        return None
+    n, at, base = first.numel(), first.data_ptr(), first.untyped_storage().data_ptr()
+    for k, c in enumerate(cols):
+        if c.numel() != n or (c.dim() == 2 and c.shape[1] != 1) or c.data_ptr() != at + 8 * n * k or c.untyped_storage().data_ptr() != base:
+            return None
+    return first.as_strided((n * len(cols),), (1,), first.storage_offset())
+
+
 def gather_columns(features: Dict, keys: List[str], device) -> Tuple[torch.Tensor, Optional[torch.Tensor], int]:
     """Collect the slots ``keys`` as ``(ids, offsets, B)`` in the column-after-column layout the
     pull kernel expects; ``offsets`` is None when every bag holds exactly one id."""
@@ -120,6 +133,10 @@ def gather_columns(features: Dict, keys: List[str], device) -> Tuple[torch.Tenso
     single = all(torch.is_tensor(c) and (c.dim() == 1 or (c.dim() == 2 and c.shape[1] == 1)) for c in cols)
     B = batch_size_of(cols[0])
     if single:
+        if cols[0].is_cuda and B > 0:
+            ids = adjacent_columns(cols)
+            if ids is not None:
+                return ids, None, B
         ids = torch.stack([c.reshape(-1).to(device, non_blocking=True).long() for c in cols]).reshape(-1)
         return ids, None, B
     if any(isinstance(c, PaddedRagged) for c in cols):

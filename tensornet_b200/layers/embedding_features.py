@@ -19,7 +19,7 @@ import torch
 from torch import nn
 
 from .. import core
-from ..data.features import PACKED_KEY, gather_columns, padded_columns
+from ..data.features import PACKED_KEY, adjacent_columns, gather_columns, padded_columns
 from ..feature_column import EmbeddingColumn
 from ..ops import functional as F
 from ..ops.embedding import COMBINERS, expand_bag_labels, pull_pool
@@ -165,16 +165,19 @@ class EmbeddingFeatures(nn.Module):
 
     def ids_pulled_for(self, features: Dict):
         """The id tensor this layer's next training pull will receive for ``features``, when that is known ahead
-        without any work: the packed single-hot ids of exactly this layer's slots, already on the device (the
-        tensor the pull gets is then a view of it, same address).  None otherwise, and for layers whose table
-        serves several links (their pulls share one step counter)."""
+        without any work: the packed single-hot ids of exactly this layer's slots, or its columns one behind the other, already
+        on the device (the tensor the pull gets is then a view of them, same address).  None otherwise, and for layers
+        whose table serves several links (their pulls share one step counter)."""
         rt = core.runtime()
         if not (rt.on_gpu and self.trainable and isinstance(features, dict)) or not hasattr(self.link, "prefetch"):
             return None
         if len(getattr(self.table, "links", ())) != 1:
             return None
         packed = features.get(PACKED_KEY)
-        if packed is None or list(packed.keys) != list(self._keys) or packed.ids is None or not packed.ids.is_cuda:
+        if packed is None:
+            cols = [features.get(k) for k in self._keys]
+            return adjacent_columns(cols) if torch.is_tensor(cols[0]) and cols[0].is_cuda and cols[0].numel() > 0 else None
+        if list(packed.keys) != list(self._keys) or packed.ids is None or not packed.ids.is_cuda:
             return None
         return packed.ids.reshape(-1)
 

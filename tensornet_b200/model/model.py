@@ -171,6 +171,29 @@ def _is_static(spec) -> bool:
     return True
 
 
+def _static_leaves(leaves: List[torch.Tensor], dev, rooms=None) -> List[torch.Tensor]:
+    """The buffers a captured step reads its inputs from.  ``rooms``: length of the buffer of every ragged leaf (zeros at first).
+    Neighbouring id columns of one length are slices of one buffer: a layer that reads them all takes them as they lie."""
+    out: List[torch.Tensor] = []
+    i = 0
+    while i < len(leaves):
+        t = leaves[i]
+        if rooms is not None and i in rooms:
+            out.append(torch.zeros((rooms[i],), dtype=t.dtype, device=dev))
+            i += 1
+            continue
+        j = i + 1
+        if t.dtype == torch.int64 and t.dim() == 1 and t.numel() > 0:
+            while j < len(leaves) and (rooms is None or j not in rooms) and leaves[j].dtype == torch.int64 and leaves[j].shape == t.shape:
+                j += 1
+        if j - i > 1:
+            out.extend(torch.empty((j - i, *t.shape), dtype=t.dtype, device=dev))
+        else:
+            out.append(torch.empty(t.shape, dtype=t.dtype, device=dev))
+        i = j
+    return out
+
+
 _LOSS_RING = 32     # pinned slots for per-step losses on their way to the host: how far the host may run ahead
 
 
@@ -985,7 +1008,7 @@ class Model(nn.Module):
         ring = _GraphRing()
         for i in range(ring.SETS):
             src = nleaves if i == 1 else leaves
-            st = [torch.empty(t.shape, dtype=t.dtype, device=dev) for t in src]
+            st = _static_leaves(src, dev)
             for d, h in zip(st, src):
                 d.copy_(h, non_blocking=True)
             ring.leaves.append(st)
@@ -1055,8 +1078,7 @@ class Model(nn.Module):
         loss_steps0 = self._loss_steps
         pool = None
         for p in range(2):
-            static_leaves = [torch.empty(t.shape, dtype=t.dtype, device=dev) if rooms is None or i not in rooms else
-                             torch.zeros((rooms[i],), dtype=t.dtype, device=dev) for i, t in enumerate(leaves)]
+            static_leaves = _static_leaves(leaves, dev, rooms)
             for dst, src in zip(static_leaves, leaves):
                 (dst if dst.shape == src.shape else dst[: src.numel()]).copy_(src, non_blocking=True)
             f, y = _unflatten(spec, iter(static_leaves), padded=rooms is not None)
@@ -1209,8 +1231,7 @@ class Model(nn.Module):
                 lk.discard_front()
         sets, pool = _PredictSets(), None
         for _ in range(2):
-            static = [torch.empty(t.shape, dtype=t.dtype, device=dev) if rooms is None or i not in rooms else
-                      torch.zeros((rooms[i],), dtype=t.dtype, device=dev) for i, t in enumerate(leaves)]
+            static = _static_leaves(leaves, dev, rooms)
             f = _unflatten(spec, iter(static), padded=rooms is not None)
             torch.cuda.synchronize()
             g = torch.cuda.CUDAGraph()
