@@ -417,10 +417,10 @@ struct BnCtx {
 
 // Device address of a host tensor that kernels may read in place (page-locked and mapped), else null.
 const void* mapped_host_ptr(const at::Tensor& t) {
-  if (t.is_cuda() || t.numel() == 0 || !t.is_contiguous() || !t.is_pinned()) return nullptr;
-  void* p = nullptr;
-  if (cudaHostGetDevicePointer(&p, t.data_ptr(), 0) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-  return p;
+  if (t.is_cuda() || t.numel() == 0 || !t.is_contiguous()) return nullptr;
+  cudaPointerAttributes at;          // one question to the driver, whether it is page-locked and where a kernel finds it
+  if (cudaPointerGetAttributes(&at, t.data_ptr()) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+  return at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr;
 }
 
 // InferenceEngine's request path: lookup + pooling, the layers of the tower, head and sigmoid, launched from one call.
@@ -839,13 +839,15 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     // a page-locked source from torch's host allocator must not be handed out again before it has been read
     // (what Tensor.copy_(non_blocking=True) does behind the scenes); a no-op for other host memory
     next = 0;
+    auto* hosts = at::getHostAllocator(at::kCUDA);
+    const c10::Stream on = c10::cuda::getStreamFromExternal(cs, dsts[0].device().index()).unwrap();
     for (size_t i = 0; i < dsts.size(); ++i) {
       const bool in_kernel = next < small.size() && small[next] == i;
       if (in_kernel) ++next;
       const at::Tensor& h = srcs[i];
-      if (h.nbytes() != 0 && (in_kernel || h.is_pinned()))
-        at::getHostAllocator(at::kCUDA)->record_event(const_cast<void*>(h.storage().data()), h.storage().data_ptr().get_context(),
-                                                      c10::cuda::getStreamFromExternal(cs, dsts[i].device().index()).unwrap());
+      if (h.nbytes() == 0 || !(in_kernel || h.is_pinned())) continue;
+      const at::DataPtr& mem = h.storage().data_ptr();
+      hosts->record_event(const_cast<void*>(mem.get()), mem.get_context(), on);
     }
     check(cudaEventRecord(reinterpret_cast<cudaEvent_t>(copied_event), cs), "cudaEventRecord");
     check(cudaStreamWaitEvent(ms, reinterpret_cast<cudaEvent_t>(copied_event), 0), "cudaStreamWaitEvent");

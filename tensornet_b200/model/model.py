@@ -79,11 +79,23 @@ def apply_mask(y_p, sw, mask):
 
 
 # ----------------------------------------------------------------------------------------------
+_TENSOR = ("t",)
+
+
 def _flatten(obj, out: List[torch.Tensor]):
     """Structure-preserving flatten of (nested) batch containers into a list of tensors."""
-    if torch.is_tensor(obj):
+    if isinstance(obj, torch.Tensor):
         out.append(obj)
-        return ("t",)
+        return _TENSOR
+    if isinstance(obj, dict):
+        items = []
+        for k, v in obj.items():
+            if isinstance(v, torch.Tensor):      # (the usual case, without a call per column)
+                out.append(v)
+                items.append((k, _TENSOR))
+            else:
+                items.append((k, _flatten(v, out)))
+        return ("dict", tuple(items))
     if isinstance(obj, PackedFeatures):
         spec = []
         for name in ("ids", "values", "offsets"):
@@ -92,10 +104,8 @@ def _flatten(obj, out: List[torch.Tensor]):
         return ("packed", tuple(obj.keys), obj.batch_size, tuple(spec))
     if isinstance(obj, Ragged):
         return ("ragged", (_flatten(obj.values, out), _flatten(obj.offsets, out)))
-    if isinstance(obj, dict):
-        return ("dict", tuple((k, _flatten(v, out)) for k, v in obj.items()))
     if isinstance(obj, (list, tuple)):
-        return ("list", tuple(_flatten(v, out) for v in obj))
+        return ("list", tuple([_flatten(v, out) for v in obj]))
     return ("const", obj)
 
 
@@ -165,9 +175,9 @@ def _is_static(spec) -> bool:
     if kind == "packed":
         return spec[3][0] is not None
     if kind == "dict":
-        return all(_is_static(s) for _, s in spec[1])
+        return all([s is _TENSOR or _is_static(s) for _, s in spec[1]])
     if kind == "list":
-        return all(_is_static(s) for s in spec[1])
+        return all([_is_static(s) for s in spec[1]])
     return True
 
 
@@ -746,7 +756,7 @@ class Model(nn.Module):
     def _padded_lengths(self, spec, leaves):
         """``(positions, lengths)`` of the ragged leaves of a batch in host memory that could run in a padded captured
         step, else None.  One GPU only: with several, every rank would have to capture at the same step."""
-        if self._padded_off or core.runtime().world > 1 or any(t.is_cuda for t in leaves):
+        if self._padded_off or core.runtime().world > 1 or any([t.is_cuda for t in leaves]):
             return None
         ragged = _ragged_leaves(spec)
         if not ragged:
@@ -766,7 +776,7 @@ class Model(nn.Module):
             return None
         ragged, n = got
         at = set(ragged)
-        base = (spec, tuple((None if i in at else t.shape, t.dtype) for i, t in enumerate(leaves)))
+        base = (spec, tuple([(None if i in at else t.shape, t.dtype) for i, t in enumerate(leaves)]))
         kind = _Kind.of(kinds, base)
         if not kind.sets and kind.held_off():
             return kind, None, None
@@ -817,8 +827,10 @@ class Model(nn.Module):
         ``next_data``: the batch that will be passed as ``data`` at the next call (same tensors, unchanged).  On the
         captured path its sparse ids are deduplicated and sent to their owners on a second stream while this step
         runs, so the next step's pull only probes and returns rows.  ``fit`` passes it by itself."""
+        flat = None
         if next_data is not None and self._use_graph and self._front_ahead_on():
-            loss = self._ring_step(data, next_data)
+            flat = self._flat(data)
+            loss = self._ring_step(flat, next_data)
             if loss is not None:
                 return loss
         features, labels = data
@@ -829,19 +841,25 @@ class Model(nn.Module):
         if not self._use_graph:
             return self._eager_step(features, labels)
         rt = core.runtime()
-        leaves: List[torch.Tensor] = []
-        spec = _flatten((features, labels), leaves)
-        key, rooms, kind = (spec, tuple((t.shape, t.dtype) for t in leaves)), None, None
+        if flat is None or type(data) is not tuple:
+            leaves: List[torch.Tensor] = []
+            spec = _flatten((features, labels), leaves)
+        else:
+            spec, leaves = flat[0], list(flat[1])
+        key, rooms, kind = None, None, None
         static = _is_static(spec)
         held = len(self._graphs) + len(self._rings)
         if not static:
             plan = self._padded_plan(spec, leaves, self._padded_kinds, held >= self._max_graphs)
             if plan is not None:
                 kind, key, rooms = plan
+        if kind is None:
+            key = (spec, tuple([(t.shape, t.dtype) for t in leaves]))
         what = "eager" if key is None else graph_decision(rt.world, key in self._graphs, static, held, self._max_graphs,
                                                           self._eager_steps, self._graph_warmup)
+        d = self.__dict__                            # plain attributes: nn.Module's bookkeeping costs microseconds per write
         if kind is not None and not kind.hold:       # (a kind held off captures is not to be captured at its exact lengths either)
-            self._uncaptured = self._uncaptured + 1 if key is None else 0
+            d["_uncaptured"] = self._uncaptured + 1 if key is None else 0
         if what == "eager":
             self._eager_steps += 1
             loss = self._eager_step(features, labels)
@@ -871,12 +889,12 @@ class Model(nn.Module):
         if rooms is not None:
             leaves = [t if t.is_contiguous() else t.contiguous() for t in leaves]
         read = gp.read[p]                        # the set's last loss must have left before its memory is written again
-        if any(t.is_cuda for t in leaves):
+        if any([t.is_cuda for t in leaves]):
             if read is not None:
                 main.wait_event(read)
             # inputs produced on the device come with the stream order of whatever produced them
             torch._foreach_copy_(gp.leaves[p], [t if t.is_cuda else t.to(rt.device, non_blocking=True) for t in leaves])
-        elif core.config.native_step_path and all(t.is_contiguous() for t in leaves):
+        elif core.config.native_step_path and all([t.is_contiguous() for t in leaves]):
             # one native call: copy stream waits for the replay that last read this input set, the leaves go host ->
             # device, their arrival is recorded and the compute stream waits for it
             self._ext.stage_inputs(gp.leaves[p], leaves, self._copy_stream.cuda_stream, main.cuda_stream,
@@ -897,25 +915,25 @@ class Model(nn.Module):
         gp.graphs[p].replay()
         gp.done[p].record(main)
         gp.done_recorded[p] = True
-        self._last_done = gp.done[p]
-        self._last_set, gp.read[p] = (gp, p), None
+        gp.read[p] = None
         if self.optimizer is not None:
             self.optimizer.iterations += 1
             self.optimizer.table.step_count += 1
-        self._loss_steps += self._graph_loss_steps
-        self._graph, self._graph_key, self._static_leaves, self._static_loss = gp.graphs[p], key, gp.leaves[p], gp.loss[p]
+        d["_last_done"], d["_last_set"] = gp.done[p], (gp, p)
+        d["_loss_steps"] = self._loss_steps + self._graph_loss_steps
+        d["_graph"], d["_graph_key"], d["_static_leaves"], d["_static_loss"] = gp.graphs[p], key, gp.leaves[p], gp.loss[p]
         return gp.loss[p]
 
     # ---- captured steps with the next batch's pull front run ahead -------------------------------------------
     @staticmethod
     def _sig(leaves):
-        return tuple((t.data_ptr(), tuple(t.shape)) for t in leaves)
+        return tuple([(t.data_ptr(), t.shape) for t in leaves])
 
     def _stage(self, ring, i, leaves, sig, main):
         """Inputs ``leaves`` into static set i of the ring (host leaves: native staged copy on the copy stream; device
         leaves: one foreach copy in stream order)."""
         read, ring.read[i] = ring.read[i], None
-        if any(t.is_cuda for t in leaves):
+        if any([t.is_cuda for t in leaves]):
             if read is not None:
                 main.wait_event(read)
             dev = core.runtime().device
@@ -935,19 +953,22 @@ class Model(nn.Module):
             return c[1]
         leaves: List[torch.Tensor] = []
         spec = _flatten(batch, leaves)
-        return spec, leaves, tuple((t.shape, t.dtype) for t in leaves), self._sig(leaves)
-
-    def _ring_step(self, data, next_data):
-        """The step through the three-set ring, or None when this batch does not take that path."""
-        setattr_ = object.__setattr__          # plain attributes: nn.Module's bookkeeping costs microseconds per write
-        spec, leaves, shapes, sig = self._flat(data)
         if not _is_static(spec):
+            return spec, leaves, None, None
+        return spec, leaves, tuple([(t.shape, t.dtype) for t in leaves]), self._sig(leaves)
+
+    def _ring_step(self, flat, next_data):
+        """The step through the three-set ring, or None when this batch does not take that path.  ``flat``: the batch
+        as :meth:`_flat` gives it."""
+        spec, leaves, shapes, sig = flat
+        if shapes is None:       # ragged
             return None
         nflat = self._flat(next_data)
         nspec, nleaves, nshapes, nsig = nflat
         if nspec != spec or nshapes != shapes:
             return None          # the following batch has another shape (a shorter last batch): no run-ahead for it
-        setattr_(self, "_flat_cache", (next_data, nflat))
+        d = self.__dict__        # plain attributes: nn.Module's bookkeeping costs microseconds per write
+        d["_flat_cache"] = (next_data, nflat)
         key = (spec, shapes)
         ring = self._rings.get(key)
         if ring is None:
@@ -989,13 +1010,9 @@ class Model(nn.Module):
             opt.iterations += 1
             opt.table.step_count += 1
         loss = ring.loss[cur] if warm else ring.cold_loss
-        setattr_(self, "_loss_steps", self._loss_steps + self._graph_loss_steps)
-        setattr_(self, "_graph", graph)
-        setattr_(self, "_graph_key", key)
-        setattr_(self, "_static_leaves", ring.leaves[cur])
-        setattr_(self, "_static_loss", loss)
-        setattr_(self, "_last_done", ring.done[cur])
-        setattr_(self, "_last_set", (ring, cur))
+        d["_loss_steps"] = self._loss_steps + self._graph_loss_steps
+        d["_graph"], d["_graph_key"], d["_static_leaves"], d["_static_loss"] = graph, key, ring.leaves[cur], loss
+        d["_last_done"], d["_last_set"] = ring.done[cur], (ring, cur)
         return loss
 
     def _capture_ring(self, spec, leaves, nleaves, key):
@@ -1433,6 +1450,7 @@ class Model(nn.Module):
                     if getattr(self, "_read_stream", None) is None:
                         self._read_stream = torch.cuda.Stream(device=rt.device)
                 pinned = self._pinned_loss
+                arrived = pinned.numpy()             # the same memory, read without a tensor per value
                 events = self._loss_events
             for cb in callbacks:
                 cb.set_model(self)
@@ -1474,9 +1492,13 @@ class Model(nn.Module):
                                 events[slot].record()
                             issued += 1
                             # read back what has arrived; wait only when the ring is about to wrap
-                            while collected < issued and (issued - collected >= _LOSS_RING or events[collected % _LOSS_RING].query()):
-                                events[collected % _LOSS_RING].synchronize()
-                                history["step_loss"].append(float(pinned[collected % _LOSS_RING]))
+                            while collected < issued:
+                                slot = collected % _LOSS_RING
+                                if issued - collected >= _LOSS_RING:
+                                    events[slot].synchronize()
+                                elif not events[slot].query():
+                                    break
+                                history["step_loss"].append(float(arrived[slot]))
                                 collected += 1
                     for cb in batch_cbs:
                         cb.on_train_batch_end(i, {"batch": int(batch[1].shape[0]) if torch.is_tensor(batch[1]) else 0})
@@ -1486,7 +1508,7 @@ class Model(nn.Module):
                         break
                 while pinned is not None and collected < issued:
                     events[collected % _LOSS_RING].synchronize()
-                    history["step_loss"].append(float(pinned[collected % _LOSS_RING]))
+                    history["step_loss"].append(float(arrived[collected % _LOSS_RING]))
                     collected += 1
                 core.runtime().check_status()
                 if core.config.verify_guards_each_pass:
