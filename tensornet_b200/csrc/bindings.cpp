@@ -233,12 +233,14 @@ struct SparseCtx {
   }
 
   // The rows of the last pull as the pooling kernels are to read them.
-  tn::RowSource source(const c10::optional<at::Tensor>& req) const {
+  // `direct`: positions are rows (lookup_many).
+  tn::RowSource source(const c10::optional<at::Tensor>& req, bool direct) const {
     tn::RowSource s{};
     s.U = c.U[c.rank];
     s.ustride = c.ustride;
+    TORCH_CHECK(!direct || in_place(), "direct rows: one GPU");
     if (in_place()) {
-      s.row_of = req_ptr(req);
+      s.row_of = direct ? nullptr : req_ptr(req);
       s.tbl = reinterpret_cast<const tn::TableView*>(tbl_dev.data_ptr());
     }
     s.stride = t.stride;
@@ -697,23 +699,39 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         check(tn::launch_sparse_pull_local(batch, (int)n, cur_stream()), "sparse_pull_local launch");
         if (!front_done) g_launches.fetch_add(1, std::memory_order_relaxed);
       })
+      // the rows of the ids of up to two tables (one GPU); nothing is counted
+      .def_static("lookup_many", [](std::vector<SparseCtx*> ctx, std::vector<at::Tensor> ids, std::vector<at::Tensor> rows,
+                                    std::vector<c10::optional<at::Tensor>> n_dev, bool lookup_only) {
+        const size_t n = ctx.size();
+        TORCH_CHECK(n >= 1 && n <= (size_t)tn::kMaxPullBatch && ids.size() == n && rows.size() == n && n_dev.size() == n, "lookup_many: one entry per lookup");
+        c10::cuda::CUDAGuard guard(ids[0].device());
+        tn::PullArgs batch[tn::kMaxPullBatch];
+        for (size_t k = 0; k < n; ++k) {
+          TORCH_CHECK(ctx[k]->in_place(), "lookup_many: one GPU only");
+          for (size_t j = 0; j < k; ++j) TORCH_CHECK(ctx[j]->t.keys != ctx[k]->t.keys, "lookup_many: different tables");
+          batch[k] = ctx[k]->batch_args(ids[k], rows[k], c10::nullopt, 0, false, lookup_only, false, n_dev[k], c10::nullopt);
+        }
+        check(tn::launch_sparse_lookup(batch, (int)n, cur_stream()), "sparse_lookup launch");
+        if (!lookup_only) g_launches.fetch_add(2, std::memory_order_relaxed);
+      })
       .def("pool_fwd", [](SparseCtx& self, at::Tensor inverse, c10::optional<at::Tensor> offsets, int B, int S, int combiner, at::Tensor out,
-                          c10::optional<at::Tensor> req) {
+                          c10::optional<at::Tensor> req, bool direct) {
         c10::cuda::CUDAGuard guard(out.device());
         const int pd = self.t.dim + 2 * self.t.use_cvm;
         TORCH_CHECK(out.scalar_type() == at::kFloat && out.is_contiguous() && out.numel() == (int64_t)B * S * pd, "pool_fwd: out must be fp32 [B, S * width]");
-        tn::launch_pool_fwd(self.source(req), ptr_of<int>(inverse), offsets ? ptr_of<int>(*offsets) : nullptr, B, S, pd, combiner,
+        tn::launch_pool_fwd(self.source(req, direct), ptr_of<int>(inverse), offsets ? ptr_of<int>(*offsets) : nullptr, B, S, pd, combiner,
                             ptr_of<float>(out), S * pd, cur_stream());
-      })
+      }, py::arg("inverse"), py::arg("offsets"), py::arg("B"), py::arg("S"), py::arg("combiner"), py::arg("out"), py::arg("req"),
+         py::arg("direct") = false)
       .def("seq_fwd", [](SparseCtx& self, at::Tensor inverse, at::Tensor offsets, int B, int T, at::Tensor out, at::Tensor lengths,
                          c10::optional<at::Tensor> req) {
         c10::cuda::CUDAGuard guard(out.device());
-        tn::launch_seq_fwd(self.source(req), ptr_of<int>(inverse), ptr_of<int>(offsets), B, T, self.t.dim + 2 * self.t.use_cvm,
+        tn::launch_seq_fwd(self.source(req, false), ptr_of<int>(inverse), ptr_of<int>(offsets), B, T, self.t.dim + 2 * self.t.use_cvm,
                            ptr_of<float>(out), ptr_of<int>(lengths), cur_stream());
       })
       .def("embed_input_fwd", [](SparseCtx& self, at::Tensor inverse, c10::optional<at::Tensor> offsets, int B, int S, int D, int combiner,
                                  c10::optional<at::Tensor> dense, at::Tensor X0, c10::optional<at::Tensor> E, c10::optional<at::Tensor> fm,
-                                 c10::optional<at::Tensor> fsum, int lin_col, c10::optional<at::Tensor> Lout, c10::optional<at::Tensor> req) {
+                                 c10::optional<at::Tensor> fsum, int lin_col, c10::optional<at::Tensor> Lout, c10::optional<at::Tensor> req, bool direct) {
         c10::cuda::CUDAGuard guard(X0.device());
         auto f32 = [](const c10::optional<at::Tensor>& t, int64_t n) { return !t || (t->scalar_type() == at::kFloat && t->is_contiguous() && t->numel() >= n); };
         const int pd = self.t.dim + 2 * self.t.use_cvm;
@@ -731,7 +749,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         a.X0 = X0.data_ptr(); a.ld = (int)X0.stride(0);
         a.E = E ? ptr_of<float>(*E) : nullptr; a.ldE = E ? (int)E->size(1) : 0; a.fm = fm ? ptr_of<float>(*fm) : nullptr; a.fsum = fsum ? ptr_of<float>(*fsum) : nullptr;
         a.Lout = Lout ? ptr_of<float>(*Lout) : nullptr; a.lin_col = Lout ? lin_col : -1;
-        if (const char* err = tn::launch_embed_input_fwd(self.source(req), a, cur_stream())) throw std::runtime_error(err);
+        if (const char* err = tn::launch_embed_input_fwd(self.source(req, direct), a, cur_stream())) throw std::runtime_error(err);
       });
   py::class_<ServeCtx>(m, "ServeCtx")
       .def(py::init<py::dict, int, int, std::vector<int>, bool>())
@@ -799,8 +817,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     // the loss of the step that last used this buffer set has been read back (it lives in the same captured memory)
     if (read_event) check(cudaStreamWaitEvent(cs, reinterpret_cast<cudaEvent_t>(read_event), 0), "cudaStreamWaitEvent");
     // Small leaves in page-locked memory go together, read by a kernel; larger ones, for which the copy engine is the faster reader,
-    // one copy each.  (A kernel for one leaf saves nothing; up to 256 KB its 22 to 30 GB/s are no slower than a copy's rate with
-    // its 2 us to the next one.)
+    // one copy each.  (Up to 256 KB a kernel's 22 to 30 GB/s are no slower than a copy's rate with its 2 us to the next one.  One or
+    // two leaves stay copies: a kernel then saves at most one of them, and it takes turns with those of the step: with two leaves
+    // of 16 KB beside 2 MB of ids a Deep&Cross step took 252 us in place of 246.)
     constexpr int64_t kSmall = 256 * 1024;
     tn::StagePieces pieces;
     std::vector<size_t> small;
@@ -817,7 +836,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       small.push_back(i);
       seen.push_back(p);
     }
-    if (small.size() < 2) { small.clear(); seen.clear(); }
+    if (small.size() < 3) { small.clear(); seen.clear(); }
     size_t next = 0;
     for (size_t i = 0; i < dsts.size(); ++i) {
       const at::Tensor& d = dsts[i];

@@ -310,7 +310,7 @@ const char* launch_embed_input_fwd(const RowSource& src, const EmbedInput& a, cu
   int blocks = (a.B + epb - 1) / epb;
   if (blocks > 148 * 8) blocks = 148 * 8;
   const int sv = cols_at_once(a.D, a.ld, a.ldE, a.X0, a.E, nullptr);
-  const bool in_place = src.row_of != nullptr;
+  const bool in_place = src.tbl != nullptr;
   // Turns of a warp's groups on the way at once: eight groups or four move enough with two (213 K rows of 16: 17.8 us, with four
   // 18.7), wider rows and bags take four (8192 x 100 bags of five ids and 64 columns: 330 us, with two 440).
   auto* k = a.offsets != nullptr ? (in_place ? fwd_kernel<true, true, 4>(sv) : fwd_kernel<false, true, 4>(sv))

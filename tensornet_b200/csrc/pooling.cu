@@ -295,7 +295,7 @@ static void pool_fwd(const RowSource& src, const int* inverse, const int* offset
 }
 void launch_pool_fwd(const RowSource& src, const int* inverse, const int* offsets, int B, int S, int pd, int combiner, float* out,
                      int out_ld, cudaStream_t st) {
-  const bool in_place = src.row_of != nullptr;
+  const bool in_place = src.tbl != nullptr;
   switch (cols_at_once(pd, out_ld, out)) {
     case 4: (in_place ? pool_fwd<true, 4> : pool_fwd<false, 4>)(src, inverse, offsets, B, S, pd, combiner, out, out_ld, st); break;
     case 2: (in_place ? pool_fwd<true, 2> : pool_fwd<false, 2>)(src, inverse, offsets, B, S, pd, combiner, out, out_ld, st); break;
@@ -326,7 +326,7 @@ void launch_pool_bwd(float* gU, int gstride, const int* inverse, const int* offs
 void launch_seq_fwd(const RowSource& src, const int* inverse, const int* offsets, int B, int T, int pd, float* out, int* lengths,
                     cudaStream_t st) {
   const int G = lanes_for_width(pd);
-  launch_pdl(src.row_of != nullptr ? seq_fwd_kernel<true> : seq_fwd_kernel<false>, dim3(grid_for((long long)B * T, G, 256)), dim3(256), 0, st,
+  launch_pdl(src.tbl != nullptr ? seq_fwd_kernel<true> : seq_fwd_kernel<false>, dim3(grid_for((long long)B * T, G, 256)), dim3(256), 0, st,
              src, inverse, offsets, B, T, pd, out, lengths, G);
 }
 void launch_seq_bwd(float* gU, int gstride, const int* inverse, const int* offsets, int B, int T, int pd, int dim,

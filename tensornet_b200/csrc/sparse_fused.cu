@@ -804,6 +804,73 @@ __global__ void __launch_bounds__(kLocalThreads) pull_local_resolve_kernel(const
   if (a.c.prof != nullptr && threadIdx.x == 0) atomicMax(&a.c.prof[18], globaltimer_ns());
 }
 
+// ---- One GPU, nobody asks for gradients (scoring, evaluation): the row of every id, straight from the table's index ------------
+// No dedup: nothing is summed per sign, and the second occurrence of a sign finds its sectors in L2.  A chain is then home slot
+// (key and row number together), with a quarter of the ids one slot more, instead of dedup slot, home slot, position, row
+// number.  Signs without a row are marked and counted; two more kernels give them one (whoever places the key creates
+// the row) and look them up again, and have nothing to do where there are none.
+// 213 K ids, 20 M rows: 14.1 us and 2 + 1.5 for the other two, where the pull takes 22.3 + 5.9 (and the gather behind it 1 us more,
+// for the positions).  Four slots of the index at a time (a sector of keys, sixteen bytes of rows): 16.7.
+constexpr int kLookupMissing = 6, kLookupLeft = 7;      // words of `bar`: ids without a row; blocks that are through with them
+constexpr int kNoRowYet = -2;                           // in a.inverse, until the last kernel has run
+
+__device__ __forceinline__ void write_new_row(const PullArgs& a, const TableView& t, int r, unsigned long long key, int first, int step) {
+  float* row = t.rows + (size_t)r * t.stride;
+  for (int ch = first; ch < (t.stride >> 2); ch += step)
+    *reinterpret_cast<float4*>(row + 4 * ch) = make_float4(new_row_elem(a.opt, key, 4 * ch, t.dim), new_row_elem(a.opt, key, 4 * ch + 1, t.dim),
+                                                           new_row_elem(a.opt, key, 4 * ch + 2, t.dim), new_row_elem(a.opt, key, 4 * ch + 3, t.dim));
+}
+// The row of a new key that this lane may have to create, for all lanes of a warp; lanes without `want` only help.  The key is
+// placed with one compare-and-swap, the rows of the warp's winners come from one addition to the row counter and are written by
+// its groups of G lanes.  Returns the row, or kReqNone when somebody else is placing the key or the table is full.
+__device__ __forceinline__ int insert_new(const PullArgs& a, const TableView& t, bool want, unsigned long long key) {
+  const SparseCommView& c = a.c;
+  const int lane = threadIdx.x & 31;
+  int r = kReqNone;
+  unsigned h = 0;
+  bool is_new = false;
+  if (want) {
+    bool placed = false;
+    h = table_home(t, key);
+    for (unsigned probes = 0; probes <= t.cap_mask; ++probes) {
+      unsigned long long k = __ldcg(&t.keys[h]);
+      if (k == kEmptyKey) {
+        k = atomicCAS(&t.keys[h], kEmptyKey, key);
+        if (k == kEmptyKey) { is_new = placed = true; break; }
+      }
+      if (k == key) { r = ld_volatile_s32(&t.slots[h]); placed = true; break; }     // inserted since it was looked up
+      h = (h + 1) & t.cap_mask;
+    }
+    if (!placed) set_status(c.status, kTableFull, 3, 0);
+  }
+  __syncwarp();
+  const int r_new = warp_alloc(t.n_rows, __ballot_sync(0xffffffffu, is_new));
+  if (is_new) {
+    if (r_new >= t.row_cap) {
+      atomicSub(t.n_rows, 1);
+      set_status(c.status, kTableFull, 3, 0);
+      t.slots[h] = -3;
+      is_new = false;
+    } else {
+      t.row_keys[r_new] = key;
+      t.slots[h] = r_new;
+      r = r_new;
+    }
+  }
+  const int G = a.lanes, gl = threadIdx.x % G, sub = lane / G, rpp = 32 / G;
+  unsigned left = __ballot_sync(0xffffffffu, is_new);
+  while (left != 0) {                  // the warp's groups write one new row each
+    unsigned rest = left;
+    for (int k = 0; k < sub; ++k) rest &= rest - 1;
+    const int from = rest != 0 ? __ffs(rest) - 1 : 0;
+    const int r_s = __shfl_sync(0xffffffffu, r, from);
+    const unsigned long long key_s = __shfl_sync(0xffffffffu, key, from);
+    if (rest != 0) write_new_row(a, t, r_s, key_s, gl, G);
+    for (int k = 0; k < rpp; ++k) left &= left - 1;
+  }
+  return r >= 0 ? r : kReqNone;
+}
+
 template <int N>
 __global__ void __launch_bounds__(kLocalThreads, 4) pull_local_finish_kernel(const __grid_constant__ PullArgsOf<N> batch) {
   const PullArgs& a = batch.a[N == 1 ? 0 : blockIdx.y];
@@ -843,64 +910,83 @@ __global__ void __launch_bounds__(kLocalThreads, 4) pull_local_finish_kernel(con
       count_shows(a, n_ids, tid, nth);
     }
     // new rows, 32 to a warp: the keys are distinct and nobody else inserts, so a lane never meets its own key half done
-    const int G = a.lanes, gl = threadIdx.x % G, sub = lane / G, rpp = 32 / G;
     for (int base = tid - lane; base < n_new; base += nth) {
-      const int m = base + lane;
-      int pos = -1, r = kReqNone;
-      unsigned long long key = kEmptyKey;
-      unsigned h = 0;
-      bool placed = m >= n_new, is_new = false;
-      if (!placed) {
-        pos = __ldcg(&c.req_ou[m]);
-        key = __ldcg(&c.stage_ids[pos]);
-        h = table_home(t, key);
-        for (unsigned probes = 0; probes <= t.cap_mask; ++probes) {
-          unsigned long long k = __ldcg(&t.keys[h]);
-          if (k == kEmptyKey) {
-            k = atomicCAS(&t.keys[h], kEmptyKey, key);
-            if (k == kEmptyKey) { is_new = placed = true; break; }
-          }
-          if (k == key) { r = ld_volatile_s32(&t.slots[h]); placed = true; break; }     // inserted since it was looked up
-          h = (h + 1) & t.cap_mask;
-        }
-        if (!placed) set_status(c.status, kTableFull, 3, 0);
-      }
-      __syncwarp();
-      const int r_new = warp_alloc(t.n_rows, __ballot_sync(0xffffffffu, is_new));
-      if (is_new) {
-        if (r_new >= t.row_cap) {
-          atomicSub(t.n_rows, 1);
-          set_status(c.status, kTableFull, 3, 0);
-          t.slots[h] = -3;
-          is_new = false;
-        } else {
-          t.row_keys[r_new] = key;
-          t.slots[h] = r_new;
-          r = r_new;
-        }
-      }
-      if (pos >= 0) c.req_row[pos] = r >= 0 ? r : kReqNone;
-      unsigned left = __ballot_sync(0xffffffffu, is_new);
-      while (left != 0) {                  // the warp's groups write one new row each
-        unsigned rest = left;
-        for (int k = 0; k < sub; ++k) rest &= rest - 1;
-        const int from = rest != 0 ? __ffs(rest) - 1 : 0;
-        const int r_s = __shfl_sync(0xffffffffu, r, from);
-        const unsigned long long key_s = __shfl_sync(0xffffffffu, key, from);
-        if (rest != 0) {
-          float* row = t.rows + (size_t)r_s * t.stride;
-          for (int ch = gl; ch < (t.stride >> 2); ch += G)
-            *reinterpret_cast<float4*>(row + 4 * ch) =
-                make_float4(new_row_elem(a.opt, key_s, 4 * ch, t.dim), new_row_elem(a.opt, key_s, 4 * ch + 1, t.dim),
-                            new_row_elem(a.opt, key_s, 4 * ch + 2, t.dim), new_row_elem(a.opt, key_s, 4 * ch + 3, t.dim));
-        }
-        for (int k = 0; k < rpp; ++k) left &= left - 1;
-      }
+      const int m = base + lane, pos = m < n_new ? __ldcg(&c.req_ou[m]) : -1;
+      const int r = insert_new(a, t, pos >= 0, pos >= 0 ? __ldcg(&c.stage_ids[pos]) : kEmptyKey);
+      if (pos >= 0) c.req_row[pos] = r;
     }
   }
   if (c.prof != nullptr && threadIdx.x == 0) {
     const unsigned long long now = globaltimer_ns();
     atomicMax(&c.prof[3], now); atomicMax(&c.prof[4], now); atomicMax(&c.prof[5], now);
+  }
+}
+
+template <int N>
+__global__ void __launch_bounds__(kLocalThreads, 8) lookup_rows_kernel(const __grid_constant__ PullArgsOf<N> batch) {
+  const PullArgs& a = batch.a[N == 1 ? 0 : blockIdx.y];
+  const TableView t = *a.tbl_dev;         // (as in pull_local_probe_kernel)
+  pdl_sync();
+  const SparseCommView& c = a.c;
+  const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x, lane = threadIdx.x & 31;
+  const int n_ids = batch_ids(a);
+  const bool bad = ld_volatile_s32(c.status) != 0;      // an earlier error has not been dealt with: no id has a row
+  for (int base = tid - lane; base < n_ids; base += nth) {
+    const int i = base + lane;
+    int r = kReqNone;
+    bool missing = false;
+    if (i < n_ids && !bad) {
+      const unsigned long long key = canon_key((unsigned long long)a.ids[i]);
+      unsigned h = table_home(t, key);
+      for (unsigned probes = 0; probes <= t.cap_mask; ++probes) {
+        const unsigned long long k = __ldcg(&t.keys[h]);
+        const int row = __ldcg(&t.slots[h]);
+        if (k == key) { r = row >= 0 ? row : kReqNone; break; }
+        if (k == kEmptyKey) { missing = !a.lookup_only; break; }
+        h = (h + 1) & t.cap_mask;
+      }
+    }
+    const unsigned mm = __ballot_sync(0xffffffffu, missing);
+    if (i < n_ids) a.inverse[i] = missing ? kNoRowYet : r;
+    if (mm != 0 && lane == 0) atomicAdd(&c.bar[kLookupMissing], (unsigned)__popc(mm));
+  }
+}
+template <int N>
+__global__ void __launch_bounds__(kLocalThreads, 4) lookup_insert_kernel(const __grid_constant__ PullArgsOf<N> batch) {
+  const PullArgs& a = batch.a[N == 1 ? 0 : blockIdx.y];
+  const TableView t = *a.tbl_dev;
+  pdl_sync();
+  if (__ldcg(&a.c.bar[kLookupMissing]) == 0) return;
+  const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x, lane = threadIdx.x & 31;
+  const int n_ids = batch_ids(a);
+  for (int base = tid - lane; base < n_ids; base += nth) {
+    const int i = base + lane;
+    const bool want = i < n_ids && a.inverse[i] == kNoRowYet;
+    const unsigned long long key = want ? canon_key((unsigned long long)a.ids[i]) : kEmptyKey;
+    const unsigned same = __match_any_sync(0xffffffffu, key);            // (every lane of the warp takes part)
+    if (__ballot_sync(0xffffffffu, want) != 0) insert_new(a, t, want && __ffs(same) - 1 == lane, key);
+  }
+}
+// (whose rows are all there now, but for those the table had no room for)
+template <int N>
+__global__ void __launch_bounds__(kLocalThreads, 8) lookup_again_kernel(const __grid_constant__ PullArgsOf<N> batch) {
+  const PullArgs& a = batch.a[N == 1 ? 0 : blockIdx.y];
+  const TableView t = *a.tbl_dev;
+  pdl_sync();
+  unsigned* bar = a.c.bar;
+  __shared__ int s_any;
+  if (threadIdx.x == 0) s_any = (int)__ldcg(&bar[kLookupMissing]);
+  __syncthreads();
+  if (s_any == 0) return;
+  if (threadIdx.x == 0) {              // the block that is the last to have read the count clears it
+    __threadfence();
+    if (atomicAdd(&bar[kLookupLeft], 1u) == gridDim.x - 1) { bar[kLookupMissing] = 0; bar[kLookupLeft] = 0; }
+  }
+  const int n_ids = batch_ids(a);
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_ids; i += gridDim.x * blockDim.x) {
+    if (a.inverse[i] != kNoRowYet) continue;
+    const int r = table_find(t, canon_key((unsigned long long)a.ids[i]));
+    a.inverse[i] = r >= 0 ? r : kReqNone;
   }
 }
 
@@ -1510,6 +1596,26 @@ cudaError_t launch_sparse_pull_local(const PullArgs* pulls, int n, cudaStream_t 
   static_assert(kMaxPullBatch == 2, "instances below");
   if (n < 1 || n > kMaxPullBatch) return cudaErrorInvalidValue;
   return n == 1 ? launch_pulls<1>(pulls, n, stream) : launch_pulls<2>(pulls, n, stream);
+}
+
+// The rows of a batch's ids (see lookup_rows_kernel).
+template <int N>
+static cudaError_t launch_lookups(const PullArgs* pulls, int n, cudaStream_t stream) {
+  PullArgsOf<N> batch;
+  int most = 1;
+  for (int k = 0; k < n; ++k) { batch.a[k] = pulls[k]; most = max(most, pulls[k].n_ids); }
+  const long long blocks = ((long long)most + kLocalThreads - 1) / kLocalThreads;
+  const dim3 block(kLocalThreads), all((unsigned)min(blocks, 148ll * 8), n), half((unsigned)min(blocks, 148ll * 4), n);
+  cudaError_t e = launch_pdl(lookup_rows_kernel<N>, all, block, 0, stream, batch);
+  if (e == cudaSuccess && !pulls[0].lookup_only) {
+    e = launch_pdl(lookup_insert_kernel<N>, half, block, 0, stream, batch);
+    if (e == cudaSuccess) e = launch_pdl(lookup_again_kernel<N>, half, block, 0, stream, batch);
+  }
+  return e;
+}
+cudaError_t launch_sparse_lookup(const PullArgs* pulls, int n, cudaStream_t stream) {
+  if (n < 1 || n > kMaxPullBatch) return cudaErrorInvalidValue;
+  return n == 1 ? launch_lookups<1>(pulls, n, stream) : launch_lookups<2>(pulls, n, stream);
 }
 
 // The pulled rows also into the per-batch matrix.

@@ -48,7 +48,7 @@ template <bool kInPlace> struct PulledRows {
       : base(kInPlace ? reinterpret_cast<const float*>(__ldg(reinterpret_cast<const unsigned long long*>(&s.tbl->rows))) : s.U),
         stride(kInPlace ? s.stride : s.ustride), row_of(s.row_of), dim(s.dim), cvm(s.cvm) {}
   // index of the row of position v (negative: none)
-  __device__ __forceinline__ int row(int v) const { return kInPlace && v >= 0 ? __ldg(row_of + v) : v; }
+  __device__ __forceinline__ int row(int v) const { return kInPlace && row_of != nullptr && v >= 0 ? __ldg(row_of + v) : v; }
   // Four columns of it from d on, a multiple of four.  A row is a whole number of 16-byte pieces and longer than its pulled
   // columns (the optimizer's state follows), so this never leaves it; what lies beyond the pulled columns is not to be used.
   __device__ __forceinline__ float4 load4(int r, int d) const {

@@ -83,8 +83,9 @@ struct PullArgs {
 
 constexpr int kMaxPullBatch = 2;      // pulls of different tables in one launch (one GPU): a model's linear and deep layers
 
-// Where the pulled row of position v is: row v of the per-batch matrix `U`, or (`row_of` not null; one GPU) row row_of[v]
-// of the table itself, whose descriptor `tbl` lies in device memory so that recorded launches follow a shard that grows.
+// Where the pulled row of position v is: row v of the per-batch matrix `U`, or (`tbl` not null; one GPU) row row_of[v]
+// of the table itself, row v where there is no `row_of` (positions are rows then, launch_sparse_lookup).  The table's
+// descriptor lies in device memory so that recorded launches follow a shard that grows.
 struct RowSource {
   const float* U;
   int ustride;
@@ -178,6 +179,8 @@ int dense_step_ctas_per_sm();      // resident CTAs of the multi-GPU dense kerne
 cudaError_t launch_sparse_pull(const PullArgs& args, int work_items, cudaStream_t stream);
 // One GPU: the pull as ordinary kernels, rows read in place (or also written out to U), and its part that can run ahead.
 cudaError_t launch_sparse_pull_local(const PullArgs* pulls, int n, cudaStream_t stream);
+// Row of every id into PullArgs::inverse, created on miss unless lookup_only; one GPU, nothing is counted.
+cudaError_t launch_sparse_lookup(const PullArgs* pulls, int n, cudaStream_t stream);
 cudaError_t launch_sparse_pull_local_rows(const PullArgs& args, cudaStream_t stream);
 cudaError_t launch_sparse_pull_local_front(const PullArgs& args, cudaStream_t stream);
 cudaError_t launch_sparse_push(const PushArgs& args, int work_items, int max_ctas, const DenseStepArgs* dense, cudaStream_t stream);

@@ -36,12 +36,12 @@ def _bag_scale(offsets, nbags, combiner, device):
 
 class _PullPool(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, anchor, table, ids, offsets, B, S, combiner, labels, label_mod, training, n_dev):
+    def forward(ctx, anchor, table, ids, offsets, B, S, combiner, labels, label_mod, training, n_dev, direct):
         pd = table.pdim
         if ids.is_cuda:
-            inverse = table.pull_in_place(ids, labels, label_mod, training, n_dev)
+            inverse = table.lookup_in_place(ids, n_dev) if direct else table.pull_in_place(ids, labels, label_mod, training, n_dev)
             out = torch.empty((B, S * pd), dtype=torch.float32, device=ids.device)
-            table.ctx.pool_fwd(inverse, offsets, B, S, combiner, out, table.req)
+            table.ctx.pool_fwd(inverse, offsets, B, S, combiner, out, None if direct else table.req, direct)
         else:
             inverse = table.pull(ids, labels, label_mod, training)
             nnz = ids.numel()
@@ -77,15 +77,16 @@ class _PullPool(torch.autograd.Function):
             inv = inverse.long()
             ok = inv >= 0
             table.gU[:, :dim].index_add_(0, inv[ok], gb[bag][ok])
-        return (None,) * 11
+        return (None,) * 12
 
 
 def pull_pool(anchor, table, ids, offsets, B, S, combiner="sum", labels=None, label_mod=0, training=True, n_dev=None):
     """``ids``: all ids of the layer's S columns, column after column (bag ``s*B + b``).
     ``offsets``: int32 ``[S*B + 1]`` bag boundaries, or None when every bag holds exactly one id.  ``n_dev`` (GPU): one
     int32 on the device saying how many of ``ids`` are there."""
+    direct = ids.is_cuda and table.looks_up(ids, training)
     return _PullPool.apply(anchor, table, ids, offsets, B, S, COMBINERS[combiner] if isinstance(combiner, str) else combiner,
-                           labels, label_mod, training, n_dev)
+                           labels, label_mod, training, n_dev, direct)
 
 
 def expand_bag_labels(y: torch.Tensor, offsets: torch.Tensor, S: int, n_ids: int) -> torch.Tensor:

@@ -573,7 +573,8 @@ def cross_v2(x0: torch.Tensor, weights: Sequence[torch.Tensor], dim: int) -> tor
 class _EmbedInput(torch.autograd.Function):
     @staticmethod
     def forward(ctx, anchor, link, ids, offsets, B, S, D, combiner, labels, label_mod, training, n_dev, dense, fm, lin_col, pooled, keep):
-        inverse = link.pull_in_place(ids, labels, label_mod, training, n_dev)
+        direct = not keep and link.looks_up(ids, training)
+        inverse = link.lookup_in_place(ids, n_dev) if direct else link.pull_in_place(ids, labels, label_mod, training, n_dev)
         dev = ids.device
         Dd = 0 if dense is None else int(dense.shape[1])
 
@@ -586,7 +587,8 @@ class _EmbedInput(torch.autograd.Function):
         # the FM term's backward pass needs the pooled columns and their sums over the slots
         emb = f32(B, S * D + Dd) if pooled else f32(B, S * D) if fm and keep else None
         fsum = f32(B, (D + 3) // 4 * 4) if fm and keep else None
-        link.ctx.embed_input_fwd(inverse, offsets, B, S, D, combiner, dense, x0, emb, term, fsum, lin_col, lin, link.req)
+        link.ctx.embed_input_fwd(inverse, offsets, B, S, D, combiner, dense, x0, emb, term, fsum, lin_col, lin,
+                                 None if direct else link.req, direct)
         ctx.link, ctx.inverse, ctx.offsets, ctx.meta = link, inverse, offsets, (B, S, D, combiner, lin_col)
         ctx.emb, ctx.fsum = (emb, fsum) if fm else (None, None)
         ctx.set_materialize_grads(False)

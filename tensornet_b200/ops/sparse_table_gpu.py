@@ -300,6 +300,7 @@ class _Pulled(NamedTuple):
     label_mod: int
     training: bool
     inverse: torch.Tensor
+    direct: bool = False         # a lookup: ``inverse`` holds rows of the table
 
 
 def _marks(*tensors):
@@ -403,7 +404,7 @@ class GpuSparseLink:
 
     def _pull(self, ids, labels, label_mod, training, inverse, lookup_only, n_dev, rows):
         done = self._pulled
-        if (done is not None and not rows and not lookup_only and done.training == bool(training) and done.label_mod == int(label_mod)
+        if (done is not None and not rows and not lookup_only and not done.direct and done.training == bool(training) and done.label_mod == int(label_mod)
                 and done.inputs == _marks(ids, labels, n_dev)):
             self._pulled = None
             return done.inverse
@@ -412,6 +413,25 @@ class GpuSparseLink:
             self.ctx.pull(ids.reshape(-1), inverse, labels, int(label_mod), bool(training), bool(lookup_only), front_done, n_dev, rows,
                           self.req)
         return inverse
+
+    def looks_up(self, ids: torch.Tensor, training: bool) -> bool:
+        """Whether a pull of ``ids`` that counts nothing and that no backward pass follows is a lookup of their rows.  (One of
+        more ids than a segment holds goes the way of a pull, which tells when it has too many signs.)"""
+        return not training and not torch.is_grad_enabled() and ids.is_cuda and self.ctx.in_place() and ids.numel() <= self.capo
+
+    def lookup_in_place(self, ids: torch.Tensor, n_dev: Optional[torch.Tensor] = None, lookup_only: bool = False) -> torch.Tensor:
+        """Rows of the table (created on miss unless ``lookup_only``) of every id, for ``self.ctx`` called with ``direct``.  A front
+        that waits for its step stays as it is."""
+        done, self._pulled = self._pulled, None
+        if done is not None:
+            if done.direct and not lookup_only and done.inputs == _marks(ids, None, n_dev):
+                return done.inverse
+            self._pulled = done
+            self.drop_pulled()
+        rows = torch.empty(ids.numel(), dtype=torch.int32, device=self.dev)
+        with phase("tn.sparse_lookup"):
+            self.ctx.lookup_many([self.ctx], [ids.reshape(-1)], [rows], [n_dev], bool(lookup_only))
+        return rows
 
     def _begin(self, ids, training, lookup_only=False, inverse=None):
         """``(inverse, front_done)`` for a pull of ``ids``; a front that ran for another batch is discarded."""
@@ -447,6 +467,16 @@ class GpuSparseLink:
         if len(calls) != 2 or len({id(lk.table) for lk in links}) < len(links) or not all(lk.ctx.in_place() for lk in links) or \
                 any(t is not None and t.is_inference() for _, ids, labels, _, _, n_dev in calls for t in (ids, labels, n_dev)):
             return False
+        if all(lk.looks_up(ids, training) for lk, ids, _, _, training, _ in calls):
+            for lk in links:
+                if lk._pulled is not None:
+                    lk.drop_pulled()
+            rows = [torch.empty(c[1].numel(), dtype=torch.int32, device=links[0].dev) for c in calls]
+            with phase("tn.sparse_lookup"):
+                links[0].ctx.lookup_many([lk.ctx for lk in links], [c[1].reshape(-1) for c in calls], rows, [c[5] for c in calls], False)
+            for (lk, ids, labels, _, _, n_dev), r in zip(calls, rows):
+                lk._pulled = _Pulled((ids, labels, n_dev), _marks(ids, None, n_dev), 0, False, r, True)
+            return True
         begun = [lk._begin(ids, training) for lk, ids, _, _, training, _ in calls]
         # (a model runs every front ahead or none: a mixture is two calls of different batches, and goes one by one)
         for done in sorted({b[1] for b in begun}):

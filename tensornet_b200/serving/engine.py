@@ -233,9 +233,10 @@ class ShardedInferenceEngine:
     def _forward(self, ids, offsets, B):
         ext = _build.cuda_ext()
         lk = self.link
-        inverse = lk.pull_in_place(ids, None, 0, training=False, lookup_only=True)
+        direct = lk.looks_up(ids, False)
+        inverse = lk.lookup_in_place(ids, lookup_only=True) if direct else lk.pull_in_place(ids, None, 0, training=False, lookup_only=True)
         pooled = torch.empty((B, self.S * lk.pdim), dtype=torch.float32, device=ids.device)
-        lk.ctx.pool_fwd(inverse, offsets, B, self.S, self.combiner, pooled, lk.req)
+        lk.ctx.pool_fwd(inverse, offsets, B, self.S, self.combiner, pooled, None if direct else lk.req, direct)
         x0 = F.concat_cast([pooled], ones=True)
         logit = self.head(self.mlp(x0)).view(-1)
         prob = torch.empty_like(logit)
