@@ -74,8 +74,8 @@ gemm_bf16_2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
   __shared__ int s_abort_i;
   volatile int* s_abort = &s_abort_i;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t rank = cluster_ctarank();          // 0: issues the MMAs
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;      // (known to be one per warp)
+  const uint32_t rank = __shfl_sync(0xffffffffu, cluster_ctarank(), 0);          // 0: issues the MMAs
   const int BN = p.BN, BNh = BN >> 1;
   const uint32_t b_bytes = (uint32_t)BNh * kBK * 2;
   const uint32_t stage_bytes = (uint32_t)kABytes + b_bytes;
@@ -111,7 +111,9 @@ gemm_bf16_2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
 
   if (warp == 0) {
     // ------------------------------- TMA producer (both CTAs) ----------------------------
-    if (lane == 0) {
+    // (whole warps with one elected lane that issues, as in gemm_tcgen05.cu)
+    {
+      const bool lead = elect_one();
       uint32_t it = 0;
       bool ok = true;
       for (int t = cid; t < n_tiles && ok; t += ncl) {
@@ -122,8 +124,9 @@ gemm_bf16_2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         for (int i = 0; i < nk; ++i, ++it) {
           const int s = (int)(it % kStages);
           const uint32_t ph = (it / kStages) & 1u;
-          if (!mbar_wait(smem_u32(&s_empty[s]), ph ^ 1u, s_abort)) { *s_abort = 1; ok = false; break; }
-          const uint32_t full_even = map_to_cta(smem_u32(&s_full[s]), 0);
+          if (!mbar_wait_warp(smem_u32(&s_empty[s]), ph ^ 1u, s_abort)) { *s_abort = 1; ok = false; break; }
+          const uint32_t full_even = __shfl_sync(0xffffffffu, map_to_cta(smem_u32(&s_full[s]), 0), 0);
+          if (!lead) continue;
           if (rank == 0) mbar_expect_tx(smem_u32(&s_full[s]), 2u * stage_bytes);
           const int kc = i * kBK;
           const uint32_t a_dst = base + s * stage_bytes;
@@ -154,12 +157,15 @@ gemm_bf16_2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             }
           }
         }
+        __syncwarp();
       }
     }
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------- MMA issuer (even CTA) -------------------------------
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
+      const bool lead = elect_one();
+      const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
       // instruction descriptor: D=f32, A=B=bf16, majors, N>>3, M>>4 with M = 256 over the pair
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.a_mn ? 1 : 0) << 15) |
                              ((uint32_t)(p.b_mn ? 1 : 0) << 16) | ((uint32_t)((kNB == 1 ? BN : 256) >> 3) << 17) | ((uint32_t)((2 * kBM) >> 4) << 24);
@@ -169,39 +175,43 @@ gemm_bf16_2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       bool ok = true;
       // optional diagnosis by cluster 0: [0] start, [1] end of the tile loop, [2] ns spent waiting for operand stages,
       // [3] ns spent waiting for a free accumulator stage, [4] tiles walked, [5] contraction steps per tile
-      unsigned long long* prof = (p.prof != nullptr && cid == 0) ? p.prof : nullptr;
+      unsigned long long* prof = (p.prof != nullptr && cid == 0 && lane == 0) ? p.prof : nullptr;
       unsigned long long w_full = 0, w_acc = 0, t_mark = 0;
       if (prof) prof[0] = globaltimer_ns();
       for (int t = cid; t < n_tiles && ok; t += ncl, ++lt) {
         const uint32_t a = lt % kAcc, aph = (lt / kAcc) & 1u;
         if (prof) t_mark = globaltimer_ns();
-        if (!mbar_wait_cluster(smem_u32(&s_acc_empty[a]), aph ^ 1u, s_abort)) { *s_abort = 1; ok = false; break; }
+        if (!__all_sync(0xffffffffu, mbar_wait_cluster(smem_u32(&s_acc_empty[a]), aph ^ 1u, s_abort))) { *s_abort = 1; ok = false; break; }
         if (prof) w_acc += globaltimer_ns() - t_mark;
         tc_fence_after();
-        const uint32_t d_tmem = tmem + a * (uint32_t)BN;
+        const uint32_t d_tmem = tm + a * (uint32_t)BN;
         for (int i = 0; i < nk; ++i, ++it) {
           const int s = (int)(it % kStages);
           const uint32_t ph = (it / kStages) & 1u;
           if (prof) t_mark = globaltimer_ns();
-          if (!mbar_wait(smem_u32(&s_full[s]), ph, s_abort)) { *s_abort = 1; ok = false; break; }
+          if (!mbar_wait_warp(smem_u32(&s_full[s]), ph, s_abort)) { *s_abort = 1; ok = false; break; }
           if (prof) w_full += globaltimer_ns() - t_mark;
           tc_fence_after();
           const uint32_t a_base = base + s * stage_bytes;
           const uint32_t b_base = a_base + kABytes;
+          const uint32_t empty_odd = __shfl_sync(0xffffffffu, map_to_cta(smem_u32(&s_empty[s]), 1), 0);
+          if (lead) {
 #pragma unroll
-          for (int k = 0; k < kBK / kUmmaK; ++k) {
-            const uint64_t ad = make_smem_desc(a_base + k * a_kstep, a_lbo, 1024u);
+            for (int k = 0; k < kBK / kUmmaK; ++k) {
+              const uint64_t ad = make_smem_desc(a_base + k * a_kstep, a_lbo, 1024u);
 #pragma unroll
-            for (int j = 0; j < kNB; ++j) {
-              const uint64_t bd = make_smem_desc(b_base + j * kNBlockBytes + k * b_kstep, b_lbo, 1024u);
-              umma_f16_2sm(d_tmem + (uint32_t)(256 * j), ad, bd, idesc, (i > 0 || k > 0) ? 1u : 0u);
+              for (int j = 0; j < kNB; ++j) {
+                const uint64_t bd = make_smem_desc(b_base + j * kNBlockBytes + k * b_kstep, b_lbo, 1024u);
+                umma_f16_2sm(d_tmem + (uint32_t)(256 * j), ad, bd, idesc, (i > 0 || k > 0) ? 1u : 0u);
+              }
             }
+            // frees the stage in both CTAs once the MMAs have read it
+            umma_commit_2sm(smem_u32(&s_empty[s]));
+            umma_commit_2sm(empty_odd);
           }
-          // frees the stage in both CTAs once the MMAs have read it
-          umma_commit_2sm(smem_u32(&s_empty[s]));
-          umma_commit_2sm(map_to_cta(smem_u32(&s_empty[s]), 1));
+          __syncwarp();
         }
-        if (ok) {
+        if (ok && lead) {
           umma_commit_2sm(smem_u32(&s_acc_full[a]));
           umma_commit_2sm(map_to_cta(smem_u32(&s_acc_full[a]), 1));
         }

@@ -53,12 +53,12 @@ gemm_bf16_splitk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
   __shared__ int s_abort_i;
   volatile int* s_abort = &s_abort_i;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;      // (known to be one per warp)
   const int BN = p.BN;
   const uint32_t b_bytes = (uint32_t)BN * kBK * 2;
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t a_smem = base, b_smem = base + kStages * kABytes;
-  const int rank = (int)cluster_ctarank();
+  const int rank = (int)__shfl_sync(0xffffffffu, cluster_ctarank(), 0);
   const int n0 = ((int)blockIdx.x / S) * BN, m0 = (int)blockIdx.y * kBM;
   const int kt_total = (p.K + kBK - 1) / kBK;
   const int kt0 = rank * p.k_tiles_per_split;
@@ -86,16 +86,18 @@ gemm_bf16_splitk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
+  // (whole warps with one elected lane that issues, as in gemm_tcgen05.cu)
   if (warp == 0) {
-    if (lane == 0) {
-      int s = 0;
-      uint32_t ph = 1u;
-      for (int i = 0; i < nk; ++i) {
-        if (!mbar_wait(smem_u32(&s_empty[s]), ph, s_abort)) { *s_abort = 1; break; }
-        const uint32_t full = smem_u32(&s_full[s]);
+    const bool lead = elect_one();
+    int s = 0;
+    uint32_t ph = 1u;
+    for (int i = 0; i < nk; ++i) {
+      if (i >= kStages && !mbar_wait_warp(smem_u32(&s_empty[s]), ph, s_abort)) { *s_abort = 1; break; }
+      const uint32_t full = smem_u32(&s_full[s]);
+      const int kc = (kt0 + i) * kBK;
+      const uint32_t a_dst = a_smem + s * kABytes, b_dst = b_smem + s * b_bytes;
+      if (lead) {
         mbar_expect_tx(full, kABytes + b_bytes);
-        const int kc = (kt0 + i) * kBK;
-        const uint32_t a_dst = a_smem + s * kABytes, b_dst = b_smem + s * b_bytes;
         if (!p.a_mn) {
           tma_load_2d(a_dst, &tmA, kc, m0, full);
         } else {
@@ -107,33 +109,36 @@ gemm_bf16_splitk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
         } else {
           for (int c = 0; c < BN / 64; ++c) tma_load_2d(b_dst + c * 8192, &tmB, n0 + 64 * c, kc, full);
         }
-        if (++s == kStages) { s = 0; ph ^= 1u; }
       }
+      __syncwarp();
+      if (++s == kStages) { s = 0; ph ^= 1u; }
     }
-    __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.a_mn ? 1 : 0) << 15) |
-                             ((uint32_t)(p.b_mn ? 1 : 0) << 16) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
-      const uint32_t a_lbo = p.a_mn ? 8192u : 16u, b_lbo = p.b_mn ? 8192u : 16u;
-      const uint32_t a_kstep = p.a_mn ? 2048u : 32u, b_kstep = p.b_mn ? 2048u : 32u;
-      bool ok = true;
-      int s = 0;
-      uint32_t ph = 0u;
-      for (int i = 0; i < nk && ok; ++i) {
-        if (!mbar_wait(smem_u32(&s_full[s]), ph, s_abort)) { *s_abort = 1; ok = false; break; }
-        tc_fence_after();
+    const bool lead = elect_one();
+    const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.a_mn ? 1 : 0) << 15) |
+                           ((uint32_t)(p.b_mn ? 1 : 0) << 16) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+    const uint32_t a_lbo = p.a_mn ? 8192u : 16u, b_lbo = p.b_mn ? 8192u : 16u;
+    const uint32_t a_kstep = p.a_mn ? 2048u : 32u, b_kstep = p.b_mn ? 2048u : 32u;
+    bool ok = true;
+    int s = 0;
+    uint32_t ph = 0u;
+    for (int i = 0; i < nk; ++i) {
+      if (!mbar_wait_warp(smem_u32(&s_full[s]), ph, s_abort)) { *s_abort = 1; ok = false; break; }
+      tc_fence_after();
+      if (lead) {
 #pragma unroll
         for (int k = 0; k < kBK / kUmmaK; ++k) {
           const uint64_t ad = make_smem_desc(a_smem + s * kABytes + k * a_kstep, a_lbo, 1024u);
           const uint64_t bd = make_smem_desc(b_smem + s * b_bytes + k * b_kstep, b_lbo, 1024u);
-          umma_f16(tmem, ad, bd, idesc, (i > 0 || k > 0) ? 1u : 0u);
+          umma_f16(tm, ad, bd, idesc, (i > 0 || k > 0) ? 1u : 0u);
         }
-        umma_commit(smem_u32(&s_empty[s]));
-        if (++s == kStages) { s = 0; ph ^= 1u; }
+        if (i + kStages < nk) umma_commit(smem_u32(&s_empty[s]));
       }
-      if (ok) umma_commit(smem_u32(&s_accum));
+      __syncwarp();
+      if (++s == kStages) { s = 0; ph ^= 1u; }
     }
+    if (ok && lead) umma_commit(smem_u32(&s_accum));
     __syncwarp();
   }
 

@@ -61,7 +61,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   __shared__ int s_abort_i;
   volatile int* s_abort = &s_abort_i;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;      // (known to be one per warp)
   const int BN = p.BN;
   const uint32_t b_bytes = (uint32_t)BN * kBK * 2;
   // A CTA owns one or two 128-row accumulators that share every B tile: with two, the operand bytes per FLOP drop
@@ -118,22 +118,35 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   // Programmatic dependent launch: everything above (barrier init, TMEM allocation, descriptor prefetch) touches
   // no tensor data and may overlap the tail of the kernel launched before this one; from here on the previous
   // kernel's results are needed.  The kernel launched after this one may start its own set-up right away.
+  // The first turn of the ring needs no wait for an empty stage, and its barriers are told the bytes to come up here, before the
+  // kernel ahead has finished.
+  const int first_turn = min(nk, kStages);
+  if (warp == 0 && lane == 0)
+    for (int s = 0; s < first_turn; ++s) mbar_expect_tx(smem_u32(&s_full[s]), a_stage + b_bytes);
+  __syncwarp();
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (prof && threadIdx.x == 0) prof[1] = globaltimer_ns();
 
+  // The producer and the MMA warp run their loops as whole warps; one elected lane issues.  A loop that only one lane is in has its
+  // addresses and descriptors in registers of that lane, from which each TMA or MMA instruction has to collect them: 0.1 us per
+  // tile load and 0.07 per MMA, so that a k-block took 0.31 us however narrow the tile; it takes 0.19 now, up to 128 columns, and
+  // what an SM can take in beyond.  Launch to launch, us: 32 x 256 x 513 5.7 -> 4.3, 512 x 512 x 1025 8.5 -> 6.3, 2999 x 300 x 396
+  // 5.6 -> 4.75, 8192 x 400 x 401 8.45 -> 7.95, 400 x 430 x 8192 (gradient) 10.3 -> 9.3, 8192 x 1024 x 6414 156 -> 141, and in
+  // gemm_splitk.cu 512 x 1024 x 6401 15.1 -> 12.8.  Sixteen epilogue warps that wait at a barrier in hardware in place of polling, and
+  // MMAs in turn into two accumulators, made no difference.
   if (warp == 0) {
     // ------------------------------- TMA producer ---------------------------------------
-    if (lane == 0) {
-      bool gate_ok = true;
-      if (p.gate_flags != nullptr) {
+    int gate_ok = 1;
+    if (p.gate_flags != nullptr) {
+      if (lane == 0) {
         // every owner's chunk of the weight array has landed in this GPU's replica
         const unsigned long long want = __ldcg(p.gate_epoch);
         for (int q = 0; q < p.gate_world && gate_ok; ++q) {
           const unsigned long long t0 = globaltimer_ns();
           unsigned spins = 0;
           while ((ld_acquire_sys_u64(p.gate_flags + q) >> 32) < want) {
-            if (((++spins) & 63u) == 0 && globaltimer_ns() - t0 > p.gate_wait_ns) { gate_ok = false; break; }
+            if (((++spins) & 63u) == 0 && globaltimer_ns() - t0 > p.gate_wait_ns) { gate_ok = 0; break; }
             __nanosleep(64);
           }
           if (!gate_ok) set_status(p.status, kPeerWaitTimeout, 70, q);
@@ -141,14 +154,20 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
         asm volatile("fence.proxy.async;" ::: "memory");
         if (!gate_ok) *s_abort = 1;
       }
-      for (int i = 0; i < nk && gate_ok; ++i) {
-        const int s = i % kStages;
+      gate_ok = __shfl_sync(0xffffffffu, gate_ok, 0);
+    }
+    const bool lead = elect_one();
+    for (int i = 0; i < nk && gate_ok; ++i) {
+      const int s = i % kStages;
+      const uint32_t full = smem_u32(&s_full[s]);
+      if (i >= kStages) {
         const uint32_t ph = (uint32_t)(i / kStages) & 1u;
-        if (!mbar_wait(smem_u32(&s_empty[s]), ph ^ 1u, s_abort)) { *s_abort = 1; break; }
-        const uint32_t full = smem_u32(&s_full[s]);
-        mbar_expect_tx(full, a_stage + b_bytes);
-        const int kc = (kt0 + i) * kBK;
-        const uint32_t b_dst = b_smem + s * b_bytes;
+        if (!mbar_wait_warp(smem_u32(&s_empty[s]), ph ^ 1u, s_abort)) { *s_abort = 1; break; }
+        if (lead) mbar_expect_tx(full, a_stage + b_bytes);
+      }
+      const int kc = (kt0 + i) * kBK;
+      const uint32_t b_dst = b_smem + s * b_bytes;
+      if (lead) {
 #pragma unroll
         for (int h = 0; h < halves; ++h) {
           const uint32_t a_dst = a_smem + s * a_stage + h * kABytes;
@@ -166,38 +185,41 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
           for (int c = 0; c < BN / 64; ++c) tma_load_2d(b_dst + c * 8192, &tmB, n0 + 64 * c, kc, full);
         }
       }
+      __syncwarp();
     }
-    __syncwarp();
   } else if (warp == 1) {
     // ------------------------------- MMA issuer -----------------------------------------
-    if (lane == 0) {
-      // instruction descriptor: D=f32, A=B=bf16, majors, N>>3, M>>4
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.a_mn ? 1 : 0) << 15) |
-                             ((uint32_t)(p.b_mn ? 1 : 0) << 16) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
-      const uint32_t a_lbo = p.a_mn ? 8192u : 16u, b_lbo = p.b_mn ? 8192u : 16u;
-      const uint32_t a_kstep = p.a_mn ? 2048u : 32u, b_kstep = p.b_mn ? 2048u : 32u;
-      bool ok = true;
-      for (int i = 0; i < nk && ok; ++i) {
-        const int s = i % kStages;
-        const uint32_t ph = (uint32_t)(i / kStages) & 1u;
-        if (!mbar_wait(smem_u32(&s_full[s]), ph, s_abort)) { *s_abort = 1; ok = false; break; }
-        tc_fence_after();
-        if (prof && i < 8) prof[2 + i] = globaltimer_ns();
-        const uint32_t a_base = a_smem + s * a_stage;
-        const uint32_t b_base = b_smem + s * b_bytes;
+    const bool lead = elect_one();
+    const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+    // instruction descriptor: D=f32, A=B=bf16, majors, N>>3, M>>4
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.a_mn ? 1 : 0) << 15) |
+                           ((uint32_t)(p.b_mn ? 1 : 0) << 16) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+    const uint32_t a_lbo = p.a_mn ? 8192u : 16u, b_lbo = p.b_mn ? 8192u : 16u;
+    const uint32_t a_kstep = p.a_mn ? 2048u : 32u, b_kstep = p.b_mn ? 2048u : 32u;
+    bool ok = true;
+    for (int i = 0; i < nk; ++i) {
+      const int s = i % kStages;
+      const uint32_t ph = (uint32_t)(i / kStages) & 1u;
+      if (!mbar_wait_warp(smem_u32(&s_full[s]), ph, s_abort)) { *s_abort = 1; ok = false; break; }
+      tc_fence_after();
+      if (prof && i < 8 && lane == 0) prof[2 + i] = globaltimer_ns();
+      const uint32_t a_base = a_smem + s * a_stage;
+      const uint32_t b_base = b_smem + s * b_bytes;
+      if (lead) {
 #pragma unroll
         for (int k = 0; k < kBK / kUmmaK; ++k) {
           const uint64_t bd = make_smem_desc(b_base + k * b_kstep, b_lbo, 1024u);
 #pragma unroll
           for (int h = 0; h < halves; ++h) {
             const uint64_t ad = make_smem_desc(a_base + h * kABytes + k * a_kstep, a_lbo, 1024u);
-            umma_f16(tmem + (uint32_t)(h * 256), ad, bd, idesc, (i > 0 || k > 0) ? 1u : 0u);
+            umma_f16(tm + (uint32_t)(h * 256), ad, bd, idesc, (i > 0 || k > 0) ? 1u : 0u);
           }
         }
-        umma_commit(smem_u32(&s_empty[s]));   // frees the stage once the MMAs have read it
+        if (i + kStages < nk) umma_commit(smem_u32(&s_empty[s]));   // frees the stage, once the MMAs have read it, for a later k-block
       }
-      if (ok) umma_commit(smem_u32(&s_accum));
+      __syncwarp();
     }
+    if (ok && lead) umma_commit(smem_u32(&s_accum));
     __syncwarp();
   } else {
     // ------------------------------- epilogue (warps 2..) --------------------------------
