@@ -385,6 +385,19 @@ struct BnCtx {
     tn::launch_bn_join_fwd(in, (int)x.size(0), t.C, t.mean, t.var, gamma ? ptr_of<float>(*gamma) : nullptr, beta ? ptr_of<float>(*beta) : nullptr,
                            (float)eps, z.data_ptr(), (int)z.size(1), ptr_of<float>(moments), ptr_of<float>(moments) + t.C, cur_stream());
   }
+  // push and join_fwd of one batch, in one launch where it fits
+  void join_train(at::Tensor h, int nh, at::Tensor x, c10::optional<at::Tensor> gamma, c10::optional<at::Tensor> beta, double eps, bool drop_inc,
+                  at::Tensor z, at::Tensor moments) {
+    if (!tn::bn_join_train_fits((int)x.size(0), t.C, (int)z.size(1))) {
+      push(x, false, drop_inc, h, nh);
+      return join_fwd(h, nh, x, gamma, beta, eps, z, moments);
+    }
+    const tn::BnInput in = input(h, nh, x);
+    TORCH_CHECK(z.scalar_type() == at::kBFloat16 && z.is_contiguous() && z.size(0) == x.size(0) && z.size(1) > t.C, "join: z");
+    c10::cuda::CUDAGuard guard(x.device());
+    tn::launch_bn_join_train(t, in, (int)x.size(0), gamma ? ptr_of<float>(*gamma) : nullptr, beta ? ptr_of<float>(*beta) : nullptr, (float)eps,
+                             drop_inc, z.data_ptr(), (int)z.size(1), ptr_of<float>(moments), ptr_of<float>(moments) + t.C, batch, cur_stream());
+  }
   void join_bwd(at::Tensor dz, at::Tensor h, int nh, at::Tensor x, at::Tensor moments, c10::optional<at::Tensor> gamma, double eps, bool mask,
                 c10::optional<at::Tensor> gh, c10::optional<at::Tensor> gx, c10::optional<at::Tensor> gg, c10::optional<at::Tensor> gb) {
     const tn::BnInput in = input(h, nh, x);
@@ -761,6 +774,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("refresh", &BnCtx::refresh)
       .def("sync", &BnCtx::sync)
       .def("apply_fwd", &BnCtx::apply_fwd)
+      .def("join_train", &BnCtx::join_train)
       .def("join_fwd", &BnCtx::join_fwd)
       .def("join_bwd", &BnCtx::join_bwd)
       .def("apply_bwd", &BnCtx::apply_bwd);

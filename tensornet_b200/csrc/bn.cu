@@ -13,6 +13,7 @@
 //   bn_apply_fwd/bwd normalise with the moments (moments are constants for the backward pass)
 //   bn_join_fwd/bwd  the same for [h | x], where h is a tower's padded bf16 output and x fp32, straight into the padded bf16
 //                    operand of the next layer and back (the ReLU mask of the tower's output included)
+//   bn_join_train    bn_batch_stats, bn_table_append and bn_join_fwd of up to kTrainRows examples in one launch
 // and, when the layer is synchronised, every `sync_freq` steps
 //   bn_table_sync    cross-GPU exchange of the pending increments by peer loads, bracketed by
 //                    bounded flag handshakes.
@@ -80,32 +81,38 @@ __device__ __forceinline__ double block_max(double v) {
   return r;
 }
 
-// One Kahan-compensated table update of feature c with (as, aq, ac); `decay_k` < 0 selects the plain path.
-__device__ __forceinline__ void bn_fold(const BnTableView& t, int c, double as, double aq, double ac, double decay_k) {
-  double ts = t.total_sum[c], te = t.total_sum_err[c], tq = t.total_sq[c], tqe = t.total_sq_err[c];
-  if (decay_k >= 0.0) {
-    ts *= (1.0 - decay_k); as *= decay_k;
-    tq *= (1.0 - decay_k); aq *= decay_k;
-  } else {
-    t.total_count[c] += ac;
-  }
-  double y = as - te, u = ts + y;
-  te = (u - ts) - y; ts = u;
-  y = aq - tqe; u = tq + y;
-  tqe = (u - tq) - y; tq = u;
-  t.total_sum[c] = ts; t.total_sum_err[c] = te; t.total_sq[c] = tq; t.total_sq_err[c] = tqe;
+struct BnTotals { double sum, sum_err, sq, sq_err, count; };
+__device__ __forceinline__ BnTotals bn_totals(const BnTableView& t, int c) {
+  return {t.total_sum[c], t.total_sum_err[c], t.total_sq[c], t.total_sq_err[c], t.total_count[c]};
+}
+__device__ __forceinline__ void bn_keep_sums(const BnTableView& t, int c, const BnTotals& a) {
+  t.total_sum[c] = a.sum; t.total_sum_err[c] = a.sum_err; t.total_sq[c] = a.sq; t.total_sq_err[c] = a.sq_err;
 }
 
-__device__ __forceinline__ void bn_moments(const BnTableView& t, int c) {
-  const double n = t.total_count[c];
-  const bool ok = n != 0.0 && n == n;
-  const double mean = ok ? t.total_sum[c] / n : 0.0;
-  t.mean[c] = (float)mean;
-  if (t.pctr) {
-    t.var[c] = (float)t.total_sq[c];
+// One Kahan-compensated update of a feature's totals with (as, aq, ac); `decay_k` < 0 selects the plain path.
+__device__ __forceinline__ void bn_fold(BnTotals& a, double as, double aq, double ac, double decay_k) {
+  if (decay_k >= 0.0) {
+    a.sum *= (1.0 - decay_k); as *= decay_k;
+    a.sq *= (1.0 - decay_k); aq *= decay_k;
   } else {
-    const float m = (float)mean, sm = ok ? (float)(t.total_sq[c] / n) : 0.f;
-    t.var[c] = ok ? fmaxf(sm - m * m, 0.f) : 1.f;     // no record yet: identity scale, the layer's initial moving variance
+    a.count += ac;
+  }
+  double y = as - a.sum_err, u = a.sum + y;
+  a.sum_err = (u - a.sum) - y; a.sum = u;
+  y = aq - a.sq_err; u = a.sq + y;
+  a.sq_err = (u - a.sq) - y; a.sq = u;
+}
+
+__device__ __forceinline__ void bn_moments(const BnTableView& t, const BnTotals& a, float* mean_out, float* var_out) {
+  const double n = a.count;
+  const bool ok = n != 0.0 && n == n;
+  const double mean = ok ? a.sum / n : 0.0;
+  *mean_out = (float)mean;
+  if (t.pctr) {
+    *var_out = (float)a.sq;
+  } else {
+    const float m = (float)mean, sm = ok ? (float)(a.sq / n) : 0.f;
+    *var_out = ok ? fmaxf(sm - m * m, 0.f) : 1.f;     // no record yet: identity scale, the layer's initial moving variance
   }
 }
 
@@ -124,8 +131,11 @@ __device__ void bn_append_block(const BnTableView& t, const double* acc, bool is
     const double as = acc[c], aq = acc[C + c], ac = acc[2 * C + c];
     if (drop_inc) { t.inc[c] = 0.0; t.inc[C + c] = 0.0; t.inc[2 * C + c] = 0.0; }
     else if (is_local) { t.inc[c] += as; t.inc[C + c] += aq; t.inc[2 * C + c] += ac; }
-    bn_fold(t, c, as, aq, ac, k);
-    bn_moments(t, c);
+    BnTotals a = bn_totals(t, c);
+    bn_fold(a, as, aq, ac, k);
+    bn_keep_sums(t, c, a);
+    if (!window) t.total_count[c] = a.count;
+    bn_moments(t, a, t.mean + c, t.var + c);
     if (zero_acc) { const_cast<double*>(acc)[c] = 0.0; const_cast<double*>(acc)[C + c] = 0.0; const_cast<double*>(acc)[2 * C + c] = 0.0; }
   }
 }
@@ -136,7 +146,7 @@ __global__ void __launch_bounds__(1024) bn_table_append_kernel(const BnTableView
 }
 
 __global__ void __launch_bounds__(1024) bn_table_refresh_moments_kernel(const BnTableView t) {
-  for (int c = threadIdx.x; c < t.C; c += blockDim.x) bn_moments(t, c);
+  for (int c = threadIdx.x; c < t.C; c += blockDim.x) bn_moments(t, bn_totals(t, c), t.mean + c, t.var + c);
 }
 
 // Cross-GPU exchange.  One CTA per GPU: (1) tell every peer "my increments are final" and wait for theirs,
@@ -255,6 +265,140 @@ __global__ void __launch_bounds__(256) bn_join_fwd_kernel(const BnInput in, int 
   }
 }
 
+// A training step's forward pass over the layer: sums of the batch, table and normalised operand.  A block has all rows of eight
+// columns, of which a thread holds a pair in kR rows in registers, so the batch is read once and no block waits for another: each
+// works its columns' moments out of the table and its own sums.  What they share is the count that decides between accumulation
+// and window, taken over all columns; every block reads it before it draws a ticket, and the last to draw writes the counts back.
+// `ticket` is a word of the batch scratch, which is zero between launches.
+// A chain of loads, barriers and 64-bit arithmetic: at 32 x 260 4.0 us from the tower's end to the head's start, as three
+// launches 6.5, at 1024 x 81 5.0 and 7.5.  (With the totals read after the barrier and a last block found out in front of the
+// arithmetic, 4.9.)  Beyond kTrainRows a thread's registers would not hold its rows.
+constexpr int kTrainPairs = 4;
+constexpr int kTrainMaxLanes = 256;                       // of rows, in a block
+constexpr int kTrainMaxFlight = 8;
+constexpr int kTrainRows = kTrainMaxLanes * kTrainMaxFlight;
+
+template <int kR>
+__global__ void __launch_bounds__(kTrainPairs * kTrainMaxLanes) bn_join_train_kernel(const BnTableView t, const BnInput in, int B,
+                                                                                     const float* __restrict__ gamma,
+                                                                                     const float* __restrict__ beta, float eps, int drop_inc,
+                                                                                     __nv_bfloat16* __restrict__ z, int ldz,
+                                                                                     float* __restrict__ mean_out,
+                                                                                     float* __restrict__ var_out, unsigned* ticket) {
+  constexpr int kCols = 2 * kTrainPairs;
+  __shared__ double s_part[kTrainPairs * kTrainMaxLanes / 32][kCols][2];
+  __shared__ double s_count[32];
+  __shared__ float s_mean[kCols], s_rs[kCols];
+  pdl_sync();
+  const int C = t.C, lanes = blockDim.x / kTrainPairs, pair = threadIdx.x % kTrainPairs, rl = threadIdx.x / kTrainPairs;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const int c0 = 2 * (blockIdx.x * kTrainPairs + pair);
+  float v[kR][2];
+#pragma unroll
+  for (int i = 0; i < kR; ++i) {
+    const int r = rl + i * lanes;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) v[i][k] = r < B && c0 + k < C ? bn_at(in, r, c0 + k) : 0.f;
+  }
+  double cur = 0.0;
+  for (int c = threadIdx.x; c < C; c += blockDim.x) cur = fmax(cur, t.total_count[c]);
+  // the first warp's lanes take a column each, four lanes to a column, of which the first keeps the table
+  const int own = blockIdx.x * kCols + lane % kCols;
+  const bool owner = warp == 0 && lane < kCols && own < C;
+  BnTotals total = {};
+  if (owner) total = bn_totals(t, own);
+  float g[2] = {1.f, 1.f}, b[2] = {0.f, 0.f};
+#pragma unroll
+  for (int k = 0; k < 2; ++k)
+    if (c0 + k < C) {
+      if (gamma) g[k] = gamma[c0 + k];
+      if (beta) b[k] = beta[c0 + k];
+    }
+  double s[2] = {0.0, 0.0}, q[2] = {0.0, 0.0};
+#pragma unroll
+  for (int i = 0; i < kR; ++i)
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const double d = (double)v[i][k];
+      s[k] += d;
+      q[k] += d * d;
+    }
+#pragma unroll
+  for (int k = 0; k < 2; ++k)
+    for (int off = kTrainPairs; off < 32; off <<= 1) {
+      s[k] += __shfl_xor_sync(0xffffffffu, s[k], off);
+      q[k] += __shfl_xor_sync(0xffffffffu, q[k], off);
+    }
+  for (int off = 16; off > 0; off >>= 1) cur = fmax(cur, __shfl_xor_sync(0xffffffffu, cur, off));
+  if (lane < kTrainPairs) {
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      s_part[warp][2 * pair + k][0] = s[k];
+      s_part[warp][2 * pair + k][1] = q[k];
+    }
+  }
+  if (lane == 0) s_count[warp] = cur;
+  __syncthreads();
+  bool window = false, last = false;
+  if (warp == 0 || warp == warps - 1) {
+    cur = lane < warps ? s_count[lane] : 0.0;
+    for (int off = 16; off > 0; off >>= 1) cur = fmax(cur, __shfl_xor_sync(0xffffffffu, cur, off));
+    cur = floor(cur);
+    window = t.max_count > 0 && cur > (double)t.max_count;
+  }
+  if (warp == warps - 1 && lane == 0) {                   // (never the first warp: a block has at least four)
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  if (warp == 0) {
+    double as = 0.0, aq = 0.0;
+    for (int w = lane / kCols; w < warps; w += 32 / kCols) { as += s_part[w][lane % kCols][0]; aq += s_part[w][lane % kCols][1]; }
+    for (int off = kCols; off < 32; off <<= 1) {
+      as += __shfl_xor_sync(0xffffffffu, as, off);
+      aq += __shfl_xor_sync(0xffffffffu, aq, off);
+    }
+    if (owner) {
+      bn_fold(total, as, aq, (double)B, window ? (1.0 - t.moment) * ((double)B / cur) : -1.0);
+      float mean, var;
+      bn_moments(t, total, &mean, &var);
+      s_mean[lane] = mean;
+      s_rs[lane] = rsqrtf(var + eps);
+      t.mean[own] = mean_out[own] = mean;
+      t.var[own] = var_out[own] = var;
+      if (drop_inc) { t.inc[own] = 0.0; t.inc[C + own] = 0.0; t.inc[2 * C + own] = 0.0; }
+      else { t.inc[own] += as; t.inc[C + own] += aq; t.inc[2 * C + own] += (double)B; }
+      bn_keep_sums(t, own, total);
+    }
+  }
+  __syncthreads();
+  float m[2], rs[2];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    m[k] = c0 + k < C ? s_mean[2 * pair + k] : 0.f;
+    rs[k] = c0 + k < C ? s_rs[2 * pair + k] : 0.f;
+  }
+#pragma unroll
+  for (int i = 0; i < kR; ++i) {
+    const int r = rl + i * lanes;
+    if (r >= B) break;
+    float o[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      o[k] = c0 + k == C ? 1.f : 0.f;
+      if (c0 + k < C) {
+        o[k] = (v[i][k] - m[k]) * rs[k];
+        if (gamma || beta) o[k] = __fmaf_rn(o[k], g[k], b[k]);
+      }
+    }
+    *reinterpret_cast<__nv_bfloat162*>(z + (size_t)r * ldz + c0) = __floats2bfloat162_rn(o[0], o[1]);
+  }
+  if (warp == warps - 1 && __shfl_sync(0xffffffffu, (int)last, 0)) {
+    if (!window)
+      for (int c = lane; c < C; c += 32) t.total_count[c] += (double)B;
+    if (lane == 0) *ticket = 0u;
+  }
+}
+
 // Gradients of the same: gh (bf16, zero beyond its columns, and with `mask` where h is not above zero), gx (fp32), gamma, beta.
 __global__ void __launch_bounds__(kBnCols * kBnRows) bn_join_bwd_kernel(const __nv_bfloat16* __restrict__ dz, int ldz, const BnInput in, int B,
                                                                         int C, const float* __restrict__ mean, const float* __restrict__ var,
@@ -319,6 +463,22 @@ void launch_bn_join_fwd(const BnInput& in, int B, int C, const float* mean, cons
   if (blocks > 148 * 8) blocks = 148 * 8;
   launch_pdl(bn_join_fwd_kernel, dim3(blocks < 1 ? 1 : (int)blocks), dim3(256), 0, st, in, B, C, mean, var, gamma, beta, eps,
              reinterpret_cast<__nv_bfloat16*>(z), ldz, mean_out, var_out);
+}
+bool bn_join_train_fits(int B, int C, int ldz) { return B >= 1 && B <= kTrainRows && C >= 1 && ldz % (2 * kTrainPairs) == 0; }
+void launch_bn_join_train(const BnTableView& t, const BnInput& in, int B, const float* gamma, const float* beta, float eps, bool drop_inc,
+                          void* z, int ldz, float* mean_out, float* var_out, double* batch, cudaStream_t st) {
+  int lanes = 32;
+  while (lanes < B && lanes < kTrainMaxLanes) lanes <<= 1;
+  const dim3 grid(ldz / (2 * kTrainPairs)), block(kTrainPairs * lanes);
+  auto go = [&](auto kernel) {
+    launch_pdl(kernel, grid, block, 0, st, t, in, B, gamma, beta, eps, drop_inc ? 1 : 0, reinterpret_cast<__nv_bfloat16*>(z), ldz, mean_out,
+               var_out, reinterpret_cast<unsigned*>(batch));
+  };
+  const int rows = (B + lanes - 1) / lanes;
+  if (rows <= 1) go(bn_join_train_kernel<1>);
+  else if (rows <= 2) go(bn_join_train_kernel<2>);
+  else if (rows <= 4) go(bn_join_train_kernel<4>);
+  else go(bn_join_train_kernel<kTrainMaxFlight>);
 }
 void launch_bn_join_bwd(const void* dz, int ldz, const BnInput& in, int B, int C, const float* mean, const float* var, const float* gamma,
                         float eps, int mask, void* gh, float* gx, int ldg, float* gg, float* gb, cudaStream_t st) {

@@ -179,6 +179,10 @@ void launch_bn_batch_stats(const BnInput& in, int B, int C, const float* center,
 void launch_bn_table_append(const BnTableView& t, double* batch, bool drop_inc, cudaStream_t st);
 void launch_bn_join_fwd(const BnInput& in, int B, int C, const float* mean, const float* var, const float* gamma, const float* beta, float eps,
                         void* z, int ldz, float* mean_out, float* var_out, cudaStream_t st);
+// the three above for a batch of up to a few thousand rows, whole rows of z written; `batch` (zeroed) is left so
+bool bn_join_train_fits(int B, int C, int ldz);
+void launch_bn_join_train(const BnTableView& t, const BnInput& in, int B, const float* gamma, const float* beta, float eps, bool drop_inc,
+                          void* z, int ldz, float* mean_out, float* var_out, double* batch, cudaStream_t st);
 void launch_bn_join_bwd(const void* dz, int ldz, const BnInput& in, int B, int C, const float* mean, const float* var, const float* gamma,
                         float eps, int mask, void* gh, float* gx, int ldg, float* gg, float* gb, cudaStream_t st);
 void launch_bn_table_refresh(const BnTableView& t, cudaStream_t st);

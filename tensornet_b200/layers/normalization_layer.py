@@ -42,14 +42,18 @@ class _BnApply(torch.autograd.Function):
 
 class _BnJoin(torch.autograd.Function):
     """``z = bf16([bn([h[:, :n_h] | x]) | 1 | 0])`` with :class:`_BnApply`'s mathematics, in one kernel each way; ``masked``: the
-    gradient of ``h`` is zero where ``h`` is not above zero (the backward pass of the ReLU that made it)."""
+    gradient of ``h`` is zero where ``h`` is not above zero (the backward pass of the ReLU that made it).  ``drop``: not None
+    for a batch that the table takes in first, and whether the pending increments are dropped with it."""
 
     @staticmethod
-    def forward(ctx, h, x, gamma, beta, table, eps, n_h, masked, into):
+    def forward(ctx, h, x, gamma, beta, table, eps, n_h, masked, into, drop):
         C = n_h + x.shape[1]
         z = torch.empty((h.shape[0], F.pad8(C + 1)), dtype=torch.bfloat16, device=h.device)
         moments = torch.empty(2 * C, dtype=torch.float32, device=h.device)       # the table moves on before the backward pass runs
-        table.ctx.join_fwd(h, n_h, x, gamma, beta, float(eps), z, moments)
+        if drop is None:
+            table.ctx.join_fwd(h, n_h, x, gamma, beta, float(eps), z, moments)
+        else:
+            table.ctx.join_train(h, n_h, x, gamma, beta, float(eps), drop, z, moments)
         ctx.save_for_backward(h, x, gamma, moments)
         ctx.table, ctx.meta, ctx.has_beta = table, (float(eps), n_h, masked), beta is not None
         ctx.into = (gamma, beta) if into and F.adds_to_grad(gamma, beta) else None
@@ -71,7 +75,7 @@ class _BnJoin(torch.autograd.Function):
         ctx.table.ctx.join_bwd(dz.contiguous(), h, n_h, x, moments, gamma, eps, masked, gh, gx, gg, gb)
         if ctx.into is not None:
             gg = gb = None
-        return gh, gx, gg, gb, None, None, None, None, None
+        return gh, gx, gg, gb, None, None, None, None, None, None
 
 
 class TNBatchNormalizationBase(nn.Module):
@@ -139,18 +143,25 @@ class TNBatchNormalizationBase(nn.Module):
         self.moving_variance.copy_(torch.from_numpy(var))
 
     # ---- device path: statistics, table update and normalisation without leaving the GPU ------
-    def _device_push(self, x2: torch.Tensor, centered: bool, h=None, n_h: int = 0):
+    def _exchanges(self):
+        """``(whether this batch is followed by an exchange of increments, whether there is nobody to exchange with)``"""
         # a captured step replays the same launches every time, so the exchange cannot run every
         # sync_freq-th step only: inside a CUDA graph it runs every step (one small kernel)
         exchange = self.synchronized and (torch.cuda.is_current_stream_capturing() or self.batch_counter + 1 == self.sync_freq)
-        alone = core.runtime().world == 1          # nobody to exchange with: the increments are not kept
-        self.table.push_batch(x2, centered, exchange and alone, h, n_h)
+        return exchange, core.runtime().world == 1
+
+    def _counted(self, exchange: bool):
         if exchange:
-            if not alone:
-                self.table.sync_increments()
             self.batch_counter = 0
         elif self.synchronized:
             self.batch_counter += 1
+
+    def _device_push(self, x2: torch.Tensor, centered: bool, h=None, n_h: int = 0):
+        exchange, alone = self._exchanges()        # alone: the increments are not kept
+        self.table.push_batch(x2, centered, exchange and alone, h, n_h)
+        if exchange and not alone:
+            self.table.sync_increments()
+        self._counted(exchange)
 
     def _device_forward(self, inputs: torch.Tensor, training: bool, centered: bool):
         x2 = inputs.reshape(-1, inputs.shape[-1])
@@ -167,9 +178,17 @@ class TNBatchNormalizationBase(nn.Module):
         """``concat_cast([self(cat([h[:, :n_h].float(), x], 1))], ones=True)`` without the steps in between (device tables
         only): ``h`` is a tower's padded bf16 output.  ``masked``: see :class:`_BnJoin`.  ``into_grads``: the backward pass is a model's
         own and may add to the parameters' ``.grad`` itself."""
+        drop = None
         if self.training:
-            self._device_push(x.detach(), False, h.detach(), n_h)
-        return _BnJoin.apply(h, x, self.gamma, self.beta, self.table, self.epsilon, n_h, masked, into_grads)
+            exchange, alone = self._exchanges()
+            if exchange and not alone:             # the peers' increments come between the batch's and the moments
+                self._device_push(x.detach(), False, h.detach(), n_h)
+            else:
+                drop = exchange
+        z = _BnJoin.apply(h, x, self.gamma, self.beta, self.table, self.epsilon, n_h, masked, into_grads, drop)
+        if drop is not None:
+            self._counted(exchange)
+        return z
 
     def bn_statistics_pull(self):
         """Fold the other ranks' pending increments in (called by rank 0 before saving)."""
