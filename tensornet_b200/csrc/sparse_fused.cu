@@ -1694,8 +1694,16 @@ static cudaError_t launch_sparse_push_local(PushArgs args, long long rows, int m
   }
   long long blocks = (rows * args.lanes + 256ll * rows_per_group - 1) / (256ll * rows_per_group);
   if (blocks < 1) blocks = 1;
+  // Blocks that come while those of the kernel ahead drain are spread unevenly over the SMs, and these stay to the end: the rows of
+  // 8192 examples of DCN-v2 (4 M ids, width 64, Ftrl) 1 240 us, and 940 when launched behind it.  A push of a few passes is over before that tells, and an early start
+  // is 1 to 2 us less (sixteen steps of Wide&Deep at 1024: 1 165 -> 1 135 us).
+  const bool many = blocks > 8 * 148ll * per_sm;
   if (blocks > 148ll * per_sm) blocks = 148ll * per_sm;
   if (max_ctas > 0 && blocks > (long long)max_ctas * per_sm) blocks = (long long)max_ctas * per_sm;
+  if (many) {
+    kernel<<<dim3((unsigned)blocks), dim3(256), 0, stream>>>(args);
+    return cudaGetLastError();
+  }
   return launch_pdl(kernel, dim3((unsigned)blocks), dim3(256), 0, stream, args);
 }
 

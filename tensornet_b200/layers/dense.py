@@ -45,8 +45,8 @@ class MLP(nn.Module):
     def out_dim(self) -> int:
         return self.hidden_units[-1]
 
-    def forward(self, x: torch.Tensor, grad_premasked: bool = False) -> torch.Tensor:
-        return F.mlp(x, list(self.weights), self.in_dim, self.relu_last, grad_premasked, gate=self.weight_gate)
+    def forward(self, x: torch.Tensor, grad_premasked: bool = False, late: Optional[F.LateGrads] = None) -> torch.Tensor:
+        return F.mlp(x, list(self.weights), self.in_dim, self.relu_last, grad_premasked, gate=self.weight_gate, late=late)
 
     def weight(self, i: int) -> torch.Tensor:
         dims = [self.in_dim] + self.hidden_units
@@ -104,13 +104,15 @@ def _head_piece(p: torch.Tensor, width: int) -> torch.Tensor:
     return (p if p.shape[1] == width else p[:, :width]).float().contiguous()
 
 
-def tower_loss(head: DenseHead, mlp: MLP, widths: Sequence[int], pieces, labels: torch.Tensor, sums: torch.Tensor) -> torch.Tensor:
+def tower_loss(head: DenseHead, mlp: MLP, widths: Sequence[int], pieces, labels: torch.Tensor, sums: torch.Tensor,
+               late: Optional[F.LateGrads] = None) -> torch.Tensor:
     """A training step's loss for a head over ``[mlp output | ...]``, with the head's backward pass in the same kernel where
-    that takes it.  ``pieces(**kw)`` runs the layers before it and returns the pieces; ``kw`` are for ``mlp``."""
+    that takes it.  ``pieces(**kw)`` runs the layers before it and returns the pieces; ``kw`` are for ``mlp``.
+    ``late``: of the model whose own step this is."""
     B = int(labels.numel())
     masked = type(mlp) is MLP and mlp.relu_last and unobserved(mlp, backward=True)      # the kernel masks the gradient of the last ReLU
     if head.weight.requires_grad and head.fits(widths, B):
-        got = pieces(grad_premasked=True) if masked else pieces()
+        got = pieces(grad_premasked=True, late=late) if masked else pieces()
         assert got[0].shape[0] == B, "as many labels as examples"
         return head.loss(got, widths, labels, sums, masked)
     return F.bce_with_logits(head(F.concat_cast(pieces(), ones=True, widths=widths)), labels, sums)[0]

@@ -27,6 +27,7 @@ from .. import core, metric as _metric
 from .._opentelemetry import phase, start_as_current_span
 from ..data.features import NeedsExactLengths, PackedFeatures, PaddedPacked, PaddedRagged, Ragged
 from ..ops import functional as F
+from ..optimizer.optimizer import Optimizer
 from ..parallel.symm import verify_all_arenas
 from ..utils.capture import capture
 
@@ -476,6 +477,7 @@ class Model(nn.Module):
         self._fronts_now = ()                        # (layer, next ids) of the step being issued
         self._loss_out = None                        # where the step being captured leaves its loss
         self._loss_stream = None                     # the stream that copies it there
+        self._late_grads = None                      # weight gradients that a step of its own joins itself
         self._last_done = None                       # event behind the last replayed step (None after an eager one)
         self._last_set = None                        # (captured sets, index) of the last replayed step
         self._padded_kinds: Dict[Any, _Kind] = {}    # ragged batches, by structure and fixed shapes
@@ -652,7 +654,16 @@ class Model(nn.Module):
         for layer, ids in fronts:
             layer.link.next_ids = ids
         object.__setattr__(self, "_fronts_now", fronts)
-        loss = self._step_body(features, labels)
+        late = None
+        if core.runtime().on_gpu and core.runtime().world == 1 and self.optimizer is not None:
+            late = F.LateGrads()
+        object.__setattr__(self, "_late_grads", late)
+        try:
+            loss = self._step_body(features, labels)
+        finally:
+            object.__setattr__(self, "_late_grads", None)
+            if late is not None:
+                late.join()
         if self._loss_stream is not None:      # the loss was copied out beside the backward pass
             torch.cuda.current_stream().wait_stream(self._loss_stream)
             object.__setattr__(self, "_loss_stream", None)
@@ -698,14 +709,23 @@ class Model(nn.Module):
                 loss.backward()
         if rt.on_gpu and rt.world == 1 and self.optimizer is not None:
             # one GPU: the sparse push and the dense update touch disjoint state and neither waits on other
-            # CTAs, so they run side by side
+            # CTAs, so they run side by side; the update where the weight gradients are, the push, which takes longer, behind
+            # the kernel that its gradients come from
             main = torch.cuda.current_stream()
             side = F._side_stream(rt.device)
+            opt = self.optimizer
             side.wait_stream(main)
-            with torch.cuda.stream(side):
+            if opt.table.initialized and type(opt).step is Optimizer.step and "step" not in vars(opt):
+                with torch.cuda.stream(side):
+                    opt.step()
                 self.backwards()
-            self.optimizer.step()
+            else:                                   # a step of the user's stays on the caller's stream
+                self._late_grads.join()
+                with torch.cuda.stream(side):
+                    self.backwards()
+                opt.step()
             main.wait_stream(side)
+            self._late_grads.joined()
         elif rt.on_gpu and self.optimizer is not None and getattr(self, "_overlap_dense", False):
             main = torch.cuda.current_stream()
             side = F._side_stream(rt.device)

@@ -40,8 +40,9 @@ class DeepCrossSubModel(nn.Module):
     def forward(self, x: torch.Tensor, x0=None):
         return self.head.on_pieces(self._head_pieces(x, x0), [self.mlp.out_dim, None])
 
-    def train_loss(self, x, x0, labels, sums):
-        return tower_loss(self.head, self.mlp, [self.mlp.out_dim, x.shape[1]], lambda **kw: self._head_pieces(x, x0, True, **kw), labels, sums)
+    def train_loss(self, x, x0, labels, sums, late=None):
+        return tower_loss(self.head, self.mlp, [self.mlp.out_dim, x.shape[1]], lambda **kw: self._head_pieces(x, x0, True, **kw), labels, sums,
+                          late)
 
 
 class CrossV2(nn.Module):
@@ -80,8 +81,8 @@ class DCNv2SubModel(nn.Module):
         operand, where it is there already."""
         return self.head(self._tower(x, x0))
 
-    def train_loss(self, x, x0, labels, sums):
-        return tower_loss(self.head, self.mlp, [self.mlp.out_dim], lambda **kw: [self._tower(x, x0, **kw)], labels, sums)
+    def train_loss(self, x, x0, labels, sums, late=None):
+        return tower_loss(self.head, self.mlp, [self.mlp.out_dim], lambda **kw: [self._tower(x, x0, **kw)], labels, sums, late)
 
 
 class _CrossModel(Model):
@@ -118,7 +119,7 @@ class _CrossModel(Model):
     def fused_train_loss(self, features, labels, sums):
         """Training loss with the operand straight from the rows, and the head, its loss and its backward pass in one kernel; None
         where somebody looks at what passes in between."""
-        return self.sub_model.train_loss(*self._operands(features), labels, sums) if self._own() else None
+        return self.sub_model.train_loss(*self._operands(features), labels, sums, self._late_grads) if self._own() else None
 
     def forward(self, features):
         if not torch.is_grad_enabled() and self.use_fused and self._own():

@@ -42,9 +42,9 @@ class DeepFMSubModel(nn.Module):
     def forward(self, linear_emb: Optional[torch.Tensor], deep_emb: torch.Tensor, dense: Optional[torch.Tensor] = None):
         return self.head.on_pieces(self._head_pieces(linear_emb, deep_emb, dense), self._head_widths())
 
-    def train_loss(self, linear_emb, deep_emb, dense, labels, sums):
+    def train_loss(self, linear_emb, deep_emb, dense, labels, sums, late=None):
         return tower_loss(self.head, self.mlp, self._head_widths(), lambda **kw: self._head_pieces(linear_emb, deep_emb, dense, **kw),
-                          labels, sums)
+                          labels, sums, late)
 
 
 class DeepFM(Model):
@@ -91,9 +91,10 @@ class DeepFM(Model):
             return None
         got = self._fused_inputs(features, True)
         if got is None:
-            return sub.train_loss(*self._inputs(features), labels, sums)
+            return sub.train_loss(*self._inputs(features), labels, sums, self._late_grads)
         x0, rest = got
-        return tower_loss(sub.head, sub.mlp, sub._head_widths(), lambda **kw: [sub.mlp(x0, **kw), *rest], labels, sums)
+        return tower_loss(sub.head, sub.mlp, sub._head_widths(), lambda **kw: [sub.mlp(x0, **kw), *rest], labels, sums,
+                          self._late_grads)
 
     def _fused_inputs(self, features, training):
         """``(x0, [linear weights, FM term])``: the first layer's operand and what goes to the head beside the tower's output,

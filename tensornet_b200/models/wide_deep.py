@@ -36,11 +36,12 @@ class WideDeepSubModel(nn.Module):
     def _operand(self, deep_emb, dense):
         return F.concat_cast([deep_emb] + ([dense.float()] if self.dense_dim else []), ones=True)
 
-    def _head_operand(self, linear_emb, x0, fused: bool, own_step: bool = False):
-        """Padded bf16 operand of the head; ``x0``: of the tower.  ``own_step``: for the backward pass of a model's own step."""
+    def _head_operand(self, linear_emb, x0, fused: bool, own_step: bool = False, late=None):
+        """Padded bf16 operand of the head; ``x0``: of the tower.  ``own_step``: for the backward pass of a model's own step, which
+        may see to ``late`` weight gradients."""
         if fused and self._joins(x0, linear_emb):
             # normalisation straight from the tower's output to the head's operand; its gradient comes back masked
-            h = self.mlp(x0, grad_premasked=True)
+            h = self.mlp(x0, grad_premasked=True, late=late)
             return self.bn.join_operand(h, self.mlp.out_dim, linear_emb, masked=True, into_grads=own_step)
         h = self.mlp(x0)
         if self.bn is None:
@@ -52,9 +53,9 @@ class WideDeepSubModel(nn.Module):
         """``fused``: the joint kernels may be used (a model's ``use_fused``)."""
         return self.head(self._head_operand(linear_emb, self._operand(deep_emb, dense), fused))
 
-    def train_loss(self, linear_emb, x0, labels, sums):
+    def train_loss(self, linear_emb, x0, labels, sums, late=None):
         """Loss of a step's logits with the head's backward pass in the same kernel."""
-        z = self._head_operand(linear_emb, x0, True, own_step=True)
+        z = self._head_operand(linear_emb, x0, True, own_step=True, late=late)
         if self.head.weight.requires_grad and labels.numel() == z.shape[0] and self.head.fits([self.head.in_dim], z.shape[0]):
             return self.head.loss([z], [self.head.in_dim], labels, sums, relu_first=False)
         return F.bce_with_logits(self.head(z), labels, sums)[0]
@@ -97,7 +98,7 @@ class WideDeep(Model):
         kernel; None where somebody looks at what passes in between."""
         if not own_step(self, WideDeep, self.sub_model, WideDeepSubModel):
             return None
-        return self.sub_model.train_loss(*self._operands(features), labels, sums)
+        return self.sub_model.train_loss(*self._operands(features), labels, sums, self._late_grads)
 
     def forward(self, features):
         sub = self.sub_model
