@@ -270,9 +270,10 @@ __global__ void __launch_bounds__(256) bn_join_fwd_kernel(const BnInput in, int 
 // works its columns' moments out of the table and its own sums.  What they share is the count that decides between accumulation
 // and window, taken over all columns; every block reads it before it draws a ticket, and the last to draw writes the counts back.
 // `ticket` is a word of the batch scratch, which is zero between launches.
-// A chain of loads, barriers and 64-bit arithmetic: at 32 x 260 4.0 us from the tower's end to the head's start, as three
-// launches 6.5, at 1024 x 81 5.0 and 7.5.  (With the totals read after the barrier and a last block found out in front of the
-// arithmetic, 4.9.)  Beyond kTrainRows a thread's registers would not hold its rows.
+// A chain of loads, barriers and 64-bit arithmetic: 32 x 260 4.2 us where the three launches take 8.1, 1024 x 42 6.3 for 9; in a
+// captured step, where launches overlap, 4.0 us for 6.5 from the tower's end to the head's start.  (With the totals read after
+// the barrier and a last block found out in front of the arithmetic, 4.9.)  Beyond kTrainRows a thread's registers would not
+// hold its rows.
 constexpr int kTrainPairs = 4;
 constexpr int kTrainMaxLanes = 256;                       // of rows, in a block
 constexpr int kTrainMaxFlight = 8;
