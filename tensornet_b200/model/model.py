@@ -660,10 +660,12 @@ class Model(nn.Module):
         object.__setattr__(self, "_late_grads", late)
         try:
             loss = self._step_body(features, labels)
+        except BaseException:
+            if late is not None:
+                late.abandon()
+            raise
         finally:
             object.__setattr__(self, "_late_grads", None)
-            if late is not None:
-                late.join()
         if self._loss_stream is not None:      # the loss was copied out beside the backward pass
             torch.cuda.current_stream().wait_stream(self._loss_stream)
             object.__setattr__(self, "_loss_stream", None)

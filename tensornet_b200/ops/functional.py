@@ -82,6 +82,13 @@ class LateGrads:
     def joined(self):
         self._held.clear()
 
+    def abandon(self):
+        """Of a step that failed: joined where that can still be done, as it cannot in a capture that came to an end with it."""
+        try:
+            self.join()
+        except RuntimeError:
+            self.joined()
+
 
 def adds_to_grad(*params) -> bool:
     """Whether a backward pass of a model's own step may add the gradients of these parameters (None: left out) to ``.grad`` itself:

@@ -56,7 +56,9 @@ class _Never:
         return Joined()
 
 
-def test_a_failed_step_leaves_nothing_behind(tn_gpu, status_ok):
+@pytest.mark.parametrize("joins", [True, False])
+def test_a_failed_step_leaves_nothing_behind(tn_gpu, status_ok, monkeypatch, joins):
+    """Its own error comes through, also where the streams cannot be joined any more."""
     tn = tn_gpu
     m = _model(tn, "DeepFM")
     f, y = _batch(tn, 33)
@@ -66,10 +68,15 @@ def test_a_failed_step_leaves_nothing_behind(tn_gpu, status_ok):
     def fails(*a):
         raise ValueError("on purpose")
     layer.backwards = fails
+    if not joins:
+        def cannot(self):
+            raise RuntimeError("capture has ended")
+        monkeypatch.setattr(tn.ops.functional.LateGrads, "join", cannot)
     with pytest.raises(ValueError):
         m.train_on_batch(f, y)
     assert m._late_grads is None
     layer.backwards = real
+    torch.cuda.synchronize()
     assert torch.isfinite(torch.as_tensor(m.train_on_batch(f, y))).all()
 
 
