@@ -35,7 +35,9 @@ cudaStream_t cur_stream() {
 }
 
 void check(cudaError_t e, const char* what) {
-  if (e != cudaSuccess) throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(e));
+  if (e == cudaSuccess) return;
+  cudaGetLastError();      // told here: the next check of a launch is not to find it again
+  throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(e));
 }
 
 tn::SparseOptParams opt_from_dict(const py::dict& d) {
@@ -433,9 +435,17 @@ struct BnCtx {
 // Device address of a host tensor that kernels may read in place (page-locked and mapped), else null.
 const void* mapped_host_ptr(const at::Tensor& t) {
   if (t.is_cuda() || t.numel() == 0 || !t.is_contiguous()) return nullptr;
+  const char* p = static_cast<const char*>(t.data_ptr());
   cudaPointerAttributes at;          // one question to the driver, whether it is page-locked and where a kernel finds it
-  if (cudaPointerGetAttributes(&at, t.data_ptr()) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-  return at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+  const char* d = static_cast<const char*>(at.devicePointer);
+  if (at.type != cudaMemoryTypeHost || d == nullptr) return nullptr;
+  // Memory that was registered by somebody, not allocated page-locked: its last byte too.  No more than the pages that it begins
+  // in may be known to the driver, and a kernel would read on behind them.
+  static const c10::DeleterFnPtr allocated = at::getHostAllocator(at::kCUDA)->allocate(1).get_deleter();
+  if (t.storage().data_ptr().get_deleter() == allocated) return d;
+  if (cudaPointerGetAttributes(&at, p + t.nbytes() - 1) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+  return at.type == cudaMemoryTypeHost && at.devicePointer == d + t.nbytes() - 1 ? d : nullptr;
 }
 
 // InferenceEngine's request path: lookup + pooling, the layers of the tower, head and sigmoid, launched from one call.

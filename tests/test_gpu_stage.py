@@ -30,6 +30,34 @@ def test_staged_inputs_arrive_whole(pinned, shift):
         assert torch.equal(d[: s.numel()].cpu(), s) and bool((d[s.numel():] == 9).all())
 
 
+def test_memory_that_is_page_locked_in_part_is_not_read_by_a_kernel():
+    """A leaf of which only the first page is registered: copied, or refused by the copy; and the context is as before."""
+    tn.core.init()
+    ext = _build.cuda_ext()
+    page = 4096
+    room = torch.arange(6 * page, dtype=torch.int64).to(torch.uint8)
+    at = -room.data_ptr() % page
+    part = room[at: at + 2 * page + 8]
+    srcs = [torch.full((100,), k, dtype=torch.uint8).pin_memory() for k in range(4)] + [part]
+    dsts = [torch.zeros(s.numel(), dtype=torch.uint8, device="cuda") for s in srcs]
+    rt = torch.cuda.cudart()
+    assert int(rt.cudaHostRegister(part.data_ptr(), page, 0)) == 0
+    try:
+        copy, done = torch.cuda.Stream(), torch.cuda.Event()
+        done.record()
+        try:
+            ext.stage_inputs(dsts, srcs, copy.cuda_stream, torch.cuda.current_stream().cuda_stream, 0, done.cuda_event, 0)
+        except RuntimeError as e:
+            assert "cudaMemcpyAsync" in str(e)
+        else:
+            torch.cuda.synchronize()
+            assert all(torch.equal(d.cpu(), s) for d, s in zip(dsts, srcs))
+        torch.cuda.synchronize()
+    finally:
+        rt.cudaHostUnregister(part.data_ptr())
+    assert float(torch.ones(4, device="cuda").sum()) == 4.0
+
+
 def test_columns_next_to_each_other_are_taken_as_they_lie():
     tn.core.init()
     ids = torch.randint(0, 100, (4, 10), device="cuda")
