@@ -137,27 +137,29 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   // MMAs in turn into two accumulators, made no difference.
   if (warp == 0) {
     // ------------------------------- TMA producer ---------------------------------------
-    const bool lead = elect_one();
-    bool gate_ok = true;
+    int gate_ok = 1;
     if (p.gate_flags != nullptr) {
-      if (lead) {
-        // Every owner's chunk of the weight array has landed in this GPU's replica.  The lane that loads the tiles is the one that
-        // has seen the flags and orders its asynchronous reads behind them: neither holds for another lane of the warp.
+      if (lane == 0) {
+        // every owner's chunk of the weight array has landed in this GPU's replica
         const unsigned long long want = __ldcg(p.gate_epoch);
         for (int q = 0; q < p.gate_world && gate_ok; ++q) {
           const unsigned long long t0 = globaltimer_ns();
           unsigned spins = 0;
           while ((ld_acquire_sys_u64(p.gate_flags + q) >> 32) < want) {
-            if (((++spins) & 63u) == 0 && globaltimer_ns() - t0 > p.gate_wait_ns) { gate_ok = false; break; }
+            if (((++spins) & 63u) == 0 && globaltimer_ns() - t0 > p.gate_wait_ns) { gate_ok = 0; break; }
             __nanosleep(64);
           }
           if (!gate_ok) set_status(p.status, kPeerWaitTimeout, 70, q);
         }
-        asm volatile("fence.proxy.async;" ::: "memory");
         if (!gate_ok) *s_abort = 1;
       }
-      gate_ok = __all_sync(0xffffffffu, gate_ok) != 0;
+      // What lane 0 has acquired holds for the whole warp behind this (a shuffle orders no memory), and whichever lane loads
+      // the tiles orders its own asynchronous reads behind it.  (Electing that lane in front of the poll costs every GEMM 0.1 us.)
+      __syncwarp();
+      asm volatile("fence.proxy.async;" ::: "memory");
+      gate_ok = __shfl_sync(0xffffffffu, gate_ok, 0);
     }
+    const bool lead = elect_one();
     for (int i = 0; i < nk && gate_ok; ++i) {
       const int s = i % kStages;
       const uint32_t full = smem_u32(&s_full[s]);

@@ -5,13 +5,14 @@ import re
 import tensornet_b200
 
 
-def test_the_lane_that_loads_is_the_lane_that_has_seen_the_flags():
+def test_the_lane_that_loads_is_ordered_behind_the_flags():
+    """One lane polls; a barrier of the warp, which orders memory as a shuffle does not, and the proxy fence of every lane follow
+    before any lane may load a tile."""
     path = os.path.join(os.path.dirname(tensornet_b200.__file__), "csrc", "gemm_tcgen05.cu")
     with open(path) as f:
-        src = f.read()
-    producer = src[src.index("TMA producer"):src.index("MMA issuer")]
-    elected = producer.index("lead = elect_one()")
-    gate = re.search(r"if \(p\.gate_flags != nullptr\) \{\s*if \((\w+)\) \{(.*?)fence\.proxy\.async", producer, re.S)
-    assert elected < gate.start() and gate[1] == "lead" and "ld_acquire_sys_u64(p.gate_flags" in gate[2]
-    loads = producer.index("tma_load_2d", gate.end())
-    assert "if (lead) {" in producer[gate.end():loads]
+        src = re.sub(r"//.*", "", f.read())
+    producer = src[src.index("const int first_turn"):src.index("tma_load_2d(")]
+    gate = producer[producer.index("if (p.gate_flags != nullptr) {"):producer.index("elect_one()")]
+    poll, behind = gate.split("__syncwarp();")
+    assert "ld_acquire_sys_u64(p.gate_flags" in poll and "fence.proxy.async" in behind
+    assert poll.count("{") - poll.count("}") == 1                     # the barrier is for all lanes, not in the branch of the polling one
