@@ -30,6 +30,10 @@ __device__ __forceinline__ void unpack8(const uint4& x, float* v) {
   }
 }
 
+// Bits of the pair of bf16 columns of which the first `n` count.  What lies behind a piece's columns is left out, not multiplied by
+// a zero weight: it need not be a number.
+__device__ __forceinline__ uint32_t pair_mask(int n) { return n >= 2 ? 0xffffffffu : n == 1 ? 0x0000ffffu : 0u; }
+
 // The loss is summed in a word of the scratch that is zero between launches; the last block to finish moves it into
 // `loss_out` and re-arms the scratch, so the caller never has to clear anything.  One thread per block, after its own add.
 __device__ __forceinline__ bool publish_loss(const HeadArgs& a) {
@@ -72,9 +76,12 @@ __device__ __forceinline__ void row_dots(const HeadArgs& a, const float* s_w, in
                          : make_uint4(0u, 0u, 0u, 0u);
         }
         const float4 w0 = *reinterpret_cast<const float4*>(sw + c), w1 = *reinterpret_cast<const float4*>(sw + c + 4);
+        const int n = width - c;
+        const uint32_t m0 = pair_mask(n), m1 = pair_mask(n - 2), m2 = pair_mask(n - 4), m3 = pair_mask(n - 6);
 #pragma unroll
         for (int q = 0; q < kRows; ++q) {
           float v[8];
+          z[q].x &= m0; z[q].y &= m1; z[q].z &= m2; z[q].w &= m3;
           unpack8(z[q], v);
           dot[q] += v[0] * w0.x + v[1] * w0.y + v[2] * w0.z + v[3] * w0.w + v[4] * w1.x + v[5] * w1.y + v[6] * w1.z + v[7] * w1.w;
         }
@@ -351,9 +358,16 @@ __global__ void __launch_bounds__(kThreads, 2) head_loss_rows_kernel(const __gri
       const int b = b0 + q * nwarps;
       const __nv_bfloat162* zr = reinterpret_cast<const __nv_bfloat162*>(H + (size_t)b * ldh);
 #pragma unroll
-      for (int i = 0; i < kPairs; ++i) z[q][i] = b < B && 64 * i + 2 * lane < ldh ? zr[32 * i + lane] : __floats2bfloat162_rn(0.f, 0.f);
+      for (int i = 0; i < kPairs; ++i) z[q][i] = b < B && 64 * i + 2 * lane < NH ? zr[32 * i + lane] : __floats2bfloat162_rn(0.f, 0.f);
 #pragma unroll
       for (int i = 0; i < kLin; ++i) lv[q][i] = b < B && lane + 32 * i < NL ? L[(size_t)b * NL + lane + 32 * i] : 0.f;
+    }
+    if (NH & 1) {                                                 // the last column's neighbour
+#pragma unroll
+      for (int q = 0; q < kR; ++q)
+#pragma unroll
+        for (int i = 0; i < kPairs; ++i)
+          if (64 * i + 2 * lane == NH - 1) z[q][i].y = __float2bfloat16(0.f);
     }
     const int mine = b0 + lane * nwarps;                          // lane q looks after row q
     const bool own = lane < kR && mine < B;

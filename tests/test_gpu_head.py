@@ -82,6 +82,31 @@ def test_head_score(B, nh, widths):
     assert bool(((got.view(-1).double() - z @ w.double()).abs() <= bound).all())
 
 
+@pytest.mark.parametrize("B,nh,widths", [(1, 8, ()), (17, 75, (39, 1)), (700, 60, (1,)), (33, 257, (33,)), (2999, 75, (39, 1)), (1185, 256, (200,)),
+                                         (300, 512, (1632,)), (40, 1017, (3064, 1)), (5000, 401, (26, 1))])
+@pytest.mark.parametrize("relu", [True, False])
+def test_what_lies_behind_a_pieces_columns_is_left_out(B, nh, widths, relu):
+    """Infinities and NaN there change nothing, to the bit."""
+    tn.core.init()
+    gen = torch.Generator(device="cuda").manual_seed(B)
+    pieces, ks = _pieces(B, nh, widths, gen, False), [nh, *widths]
+    w = (torch.randn(sum(ks) + 1, generator=gen, device="cuda") / sum(ks) ** 0.5).requires_grad_()
+    y = (torch.rand(B, generator=gen, device="cuda") < 0.3).float()
+    got = []
+    for fill in (0.0, float("nan"), float("inf")):
+        h = pieces[0].clone()
+        h[:, nh:] = fill
+        h.requires_grad_()
+        w.grad = torch.zeros_like(w)
+        pred = torch.empty(B, device="cuda")
+        F.head_loss([h, *pieces[1:]], ks, w, y, torch.zeros(4, device="cuda"), F.head_scratch(ks, "cuda"), relu, pred).backward()
+        # (the weight's gradient is a sum of blocks in no fixed order)
+        got.append((pred, h.grad, F.head_score([h.detach(), *pieces[1:]], ks, w), w.grad.clone()))
+    for other in got[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(got[0][:3], other[:3]))
+        assert torch.allclose(got[0][3], other[3], rtol=1e-4, atol=1e-6)
+
+
 @pytest.mark.parametrize("B,K", [(1, 8), (32, 260), (33, 42), (70, 127), (500, 319), (2048, 500)])
 @pytest.mark.parametrize("relu", [False, True])
 def test_small_head_is_the_layer_to_the_bit(B, K, relu):
