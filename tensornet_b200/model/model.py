@@ -717,12 +717,14 @@ class Model(nn.Module):
             side = F._side_stream(rt.device)
             opt = self.optimizer
             side.wait_stream(main)
-            if opt.table.initialized and type(opt).step is Optimizer.step and "step" not in vars(opt):
+            if (opt.table.initialized and type(opt).step is Optimizer.step and "step" not in vars(opt)
+                    and type(self).backwards is Model.backwards and "backwards" not in vars(self)):
                 with torch.cuda.stream(side):
                     opt.step()
                 self.backwards()
-            else:                                   # a step of the user's stays on the caller's stream
+            else:      # a step of the user's stays on the caller's stream; `backwards` comes before it and finds the gradients whole
                 self._late_grads.join()
+                side.wait_stream(main)
                 with torch.cuda.stream(side):
                     self.backwards()
                 opt.step()

@@ -97,6 +97,32 @@ def test_a_step_of_the_users_runs_behind_the_gradients(tn_gpu, status_ok):
     assert norms[0] > 0 and abs(norms[0] - norms[1]) <= 1e-6 * norms[0]
 
 
+@pytest.mark.parametrize("how", ["subclass", "instance"])
+def test_backwards_of_the_users_finds_the_gradients(tn_gpu, status_ok, how):
+    """``Model.backwards`` replaced: called between the backward pass and the update, on a stream behind the weights' gradients."""
+    tn = tn_gpu
+    seen = []
+
+    def look(m, *a):
+        seen.append((m.optimizer.table.G.double().norm().item(), m.optimizer.iterations))
+        return tn.models.DeepFM.backwards(m, *a)
+    m = _model(tn, "DeepFM")
+    f, y = _batch(tn, 1000)
+    m.train_on_batch(f, y)                                       # (the gradients' memory is there)
+    ref = _model(tn, "DeepFM")
+    ref.train_on_batch(f, y)
+    ref.optimizer.table.ctx, ctx = _Spy(ref.optimizer.table, want := []), ref.optimizer.table.ctx
+    ref.optimizer.table.ctx.real = ctx
+    ref.train_on_batch(f, y)
+    if how == "subclass":
+        m.__class__ = type("Own", (type(m),), {"backwards": look})
+    else:
+        m.backwards = lambda *a: look(m, *a)
+    m.train_on_batch(f, y)
+    (norm, before), = seen
+    assert before == 1 and m.optimizer.iterations == 2 and abs(norm - want[0]) <= 1e-6 * want[0] and want[0] > 0
+
+
 class _Spy:
     def __init__(self, table, out):
         self.table, self.out = table, out
