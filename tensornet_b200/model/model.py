@@ -473,7 +473,7 @@ class Model(nn.Module):
         self._graphs: Dict[Any, _GraphPair] = {}     # batch signature -> the two captures of the step
         self._rings: Dict[Any, _GraphRing] = {}      # same, for callers that name the following batch
         self._ring_refused = False
-        self._flat_cache = None                      # (batch object, its flattened form) of the batch named as next
+        self._flat_cache = None                      # (batch object, its flattened form) of the batch named as next at the last call
         self._fronts_now = ()                        # (layer, next ids) of the step being issued
         self._loss_out = None                        # where the step being captured leaves its loss
         self._loss_stream = None                     # the stream that copies it there
@@ -852,11 +852,18 @@ class Model(nn.Module):
         captured path its sparse ids are deduplicated and sent to their owners on a second stream while this step
         runs, so the next step's pull only probes and returns rows.  ``fit`` passes it by itself."""
         flat = None
+        d = self.__dict__                            # plain attributes: nn.Module's bookkeeping costs microseconds per write
+        promised, d["_flat_cache"] = self._flat_cache, None      # holds for the call after the one that named the batch, no longer
         if next_data is not None and self._use_graph and self._front_ahead_on():
-            flat = self._flat(data)
+            if promised is not None and promised[0] is data:
+                flat = promised[1]
+            else:
+                flat, promised = self._flat(data), None
             loss = self._ring_step(flat, next_data)
             if loss is not None:
                 return loss
+            if promised is not None:                 # not the ring's step after all: the batch as it is now
+                flat = None
         features, labels = data
         if not self.training:
             self.train()
@@ -881,7 +888,6 @@ class Model(nn.Module):
             key = (spec, tuple([(t.shape, t.dtype) for t in leaves]))
         what = "eager" if key is None else graph_decision(rt.world, key in self._graphs, static, held, self._max_graphs,
                                                           self._eager_steps, self._graph_warmup)
-        d = self.__dict__                            # plain attributes: nn.Module's bookkeeping costs microseconds per write
         if kind is not None and not kind.hold:       # (a kind held off captures is not to be captured at its exact lengths either)
             d["_uncaptured"] = self._uncaptured + 1 if key is None else 0
         if what == "eager":
@@ -970,11 +976,7 @@ class Model(nn.Module):
         ring.sig[i] = sig
 
     def _flat(self, batch):
-        """(spec, leaves, shapes, addresses) of a batch; the batch named as ``next_data`` at the previous call is
-        looked up instead of being walked again."""
-        c = self._flat_cache
-        if c is not None and c[0] is batch:
-            return c[1]
+        """(spec, leaves, shapes, addresses) of a batch."""
         leaves: List[torch.Tensor] = []
         spec = _flatten(batch, leaves)
         if not _is_static(spec):
@@ -987,17 +989,16 @@ class Model(nn.Module):
         spec, leaves, shapes, sig = flat
         if shapes is None:       # ragged
             return None
+        key = (spec, shapes)
+        ring = self._rings.get(key)
+        if ring is None and (self._rings or self._ring_refused or self._eager_steps < self._graph_warmup or key in self._graphs):
+            return None          # one ring per model, captured right after the warm-up steps on every rank alike
         nflat = self._flat(next_data)
         nspec, nleaves, nshapes, nsig = nflat
         if nspec != spec or nshapes != shapes:
             return None          # the following batch has another shape (a shorter last batch): no run-ahead for it
-        d = self.__dict__        # plain attributes: nn.Module's bookkeeping costs microseconds per write
-        d["_flat_cache"] = (next_data, nflat)
-        key = (spec, shapes)
-        ring = self._rings.get(key)
+        d = self.__dict__
         if ring is None:
-            if self._rings or self._ring_refused or self._eager_steps < self._graph_warmup or key in self._graphs:
-                return None      # one ring per model, captured right after the warm-up steps on every rank alike
             if not self.training:
                 self.train()
             ring = self._capture_ring(spec, leaves, nleaves, key)
@@ -1010,6 +1011,7 @@ class Model(nn.Module):
             self._status_poll.tick()
         main = torch.cuda.current_stream()
         cur = ring.turn
+        d["_flat_cache"] = (next_data, nflat)
         warm = ring.sig[cur] == sig and all(lk._front is _FRONT_IN_GRAPH for lk in ring.links)
         if not warm:
             # (re)start: whatever front is pending belongs to another batch

@@ -258,3 +258,24 @@ def test_pull_front_run_ahead_in_the_captured_ring_matches_the_plain_path(tn_gpu
     for a, b in zip(la, lb):
         assert abs(a - b) < 5e-2 * max(1.0, abs(a)), (la, lb)
     assert la[-1] < 0.8 * la[0]
+
+
+@pytest.mark.parametrize("ring", [True, False])
+def test_a_batch_that_was_named_as_next_may_change_before_it_is_used(tn_gpu, status_ok, ring):
+    """What a step trains on is the batch it gets.  What was noted of a batch when it was named as the following one holds for the
+    next call alone, and only where that one is captured with the fronts run ahead."""
+    tn = tn_gpu
+    m, slots = _make(tn, graph=True)
+    data = _batches(tn, slots, 512, 4)
+    if not ring:                                    # ids whose pulls are not started ahead: one tensor per slot, 32 bits wide
+        data = [({**{s: f[tn.data.PACKED_KEY].ids[k].int() for k, s in enumerate(slots)}, "dense": f["dense"]}, y) for f, y in data]
+    for k in range(6):
+        m.train_step(data[k % 4], data[(k + 1) % 4])
+    assert bool(m._rings) == ring
+    m.train_step(data[2], data[3])
+    if ring:
+        m.train_step(data[0])
+    data[3][0]["dense"] = new = torch.full((512, 5), 0.25)
+    m.train_step(data[3], data[0])
+    torch.cuda.synchronize()
+    assert any(t.shape == new.shape and torch.equal(t.cpu(), new) for t in m._static_leaves)
