@@ -60,6 +60,8 @@ class MLP(nn.Module):
 class DenseHead(nn.Module):
     """``Dense(1)`` on a padded bf16 operand: returns fp32 logits ``[B, 1]``."""
 
+    _scratch = None          # of the head kernels; no part of a saved or copied layer
+
     def __init__(self, in_dim: int):
         super().__init__()
         self.in_dim = int(in_dim)
@@ -67,7 +69,9 @@ class DenseHead(nn.Module):
         limit = math.sqrt(6.0 / (in_dim + 1))
         w[:in_dim].uniform_(-limit, limit)
         self.weight = nn.Parameter(w)
-        self._scratch = None
+
+    def __getstate__(self):
+        return {k: v for k, v in self.__dict__.items() if k != "_scratch"}
 
     def forward(self, z: torch.Tensor) -> torch.Tensor:
         return F.head(z, self.weight)

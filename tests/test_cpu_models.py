@@ -94,3 +94,22 @@ def test_interrupted_save_keeps_previous_done_file(tmp_path):
     assert m2.load_weights(root, mode="bin")
     got = torch.as_tensor(m2.predict_on_batch(f)).reshape(-1)
     assert torch.allclose(got, want, atol=1e-5)
+
+
+def test_scratch_of_the_head_kernels_is_no_part_of_a_saved_layer():
+    """A layer pickled as a whole before there was any has none and loads; one that has trained does not take it along (a layer
+    moved to the host would otherwise ask for a GPU where it is loaded)."""
+    import copy
+    import io
+
+    for trained in (False, True):
+        head = tn.layers.DenseHead(6)
+        head.__dict__.pop("_scratch", None)
+        if trained:
+            head._scratch = ((8, head.weight.device), torch.zeros(4))
+        buf = io.BytesIO()
+        torch.save(head, buf)
+        buf.seek(0)
+        for other in (torch.load(buf, weights_only=False), copy.deepcopy(head)):
+            assert "_scratch" not in other.__dict__ and other._scratch is None
+            assert torch.equal(other(torch.ones(2, 7)), head(torch.ones(2, 7)))
