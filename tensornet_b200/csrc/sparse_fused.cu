@@ -1624,20 +1624,21 @@ cudaError_t launch_sparse_pull_local_rows(const PullArgs& args, cudaStream_t str
   return launch_pdl(pull_local_rows_kernel, dim3(want > 148 * 8 ? 148 * 8 : want < 1 ? 1 : (int)want), dim3(kLocalThreads), 0, stream, args);
 }
 
-// Fronts run beside the backward pass, whose GEMMs leave room on an SM for three blocks of 128 threads and have priority.  A grid
-// of larger blocks that takes the whole chip keeps the GEMMs out until it has run: the two then come one behind the other.  These
-// grids take longer by themselves (24 + 13 us -> 58 + 20), but beside the GEMMs.  Sixteen steps of DeepFM at 8192, 213 K ids:
-// 4 057 us with up to four blocks of 256 threads per SM and GEMMs of 96 registers, 3 870 now (GEMMs of 64 registers with the
-// old grids: 4 065; without their priority 1 to 2 % more).  Eight steps with two tables of 117 K ids each: 2 020 -> 1 930; with
-// both tables' fronts in one launch 1 950.
+// Fronts run beside the backward pass, whose GEMMs leave room on an SM for one block of 256 threads and have priority.  A grid
+// that fills the chip keeps the GEMMs out until it has run; one that is too small outlasts the backward pass, and the step ends
+// with it.  Two blocks per SM as long as a thread has at most two ids, three beyond.  Over 160 workloads (DeepFM, Wide&Deep,
+// Deep&Cross, DCN-v2; 20 K to 790 K single-hot ids; towers from 64-32 to 1024-512-256) three take 0.2 % less per step than the
+// pull's own grid of up to four; two take 0.1 to 0.2 % less than three up to 151 K ids, 0.6 to 1 % more beyond 300 K.  Two tables of
+// 2999 x 39 ids beside 300-150-75: 147.4 us with two, 149.4 with three, 154 with four; 8192 x 26 beside 64-32: 146, 142, 141.  Blocks
+// of 128 threads, of which more fit beside a GEMM, four per SM (two for the second kernel): 1.7 to 2.5 % more than four of 256 on
+// the mean, and where the tower is short up to a quarter (7753 x 46 beside 128-128: 218 -> 270 us).
 cudaError_t launch_sparse_pull_local_front(const PullArgs& args, cudaStream_t stream) {
-  constexpr int kBlock = 128;
   PullArgsOf<1> batch;
   batch.a[0] = args;
-  const dim3 block(kBlock);
-  const int probe = local_grid(args, false) * (kLocalThreads / kBlock), resolve = local_grid(args, true) * (kLocalThreads / kBlock);
-  const cudaError_t e = launch_pdl(pull_local_probe_kernel<1>, dim3(min(probe, 148 * 4)), block, 0, stream, batch);
-  return e != cudaSuccess ? e : launch_pdl(pull_local_resolve_kernel, dim3(min(resolve, 148 * 2)), block, 0, stream, args);
+  const dim3 block(kLocalThreads);
+  const int most = args.n_ids <= 2 * 2 * 148 * kLocalThreads ? 148 * 2 : 148 * 3;
+  const cudaError_t e = launch_pdl(pull_local_probe_kernel<1>, dim3(min(local_grid(args, false), most)), block, 0, stream, batch);
+  return e != cudaSuccess ? e : launch_pdl(pull_local_resolve_kernel, dim3(min(local_grid(args, true), most)), block, 0, stream, args);
 }
 
 cudaError_t launch_sparse_pull(const PullArgs& args, int work_items, cudaStream_t stream) {
