@@ -46,9 +46,10 @@ constexpr int kEpiWarps = 4 * kEpiSubs;
 constexpr int kGemmThreads = 32 * (2 + kEpiWarps);   // warp0 TMA, warp1 MMA + TMEM owner, the rest epilogue
 constexpr int kEpiBytesPerWarp = gemm_epi::kBytesPerWarp;
 
-// 64 registers for what a training step runs: an SM's four register files take five warps of this kernel and then have room for
-// three of another one, so that a block of 128 threads (the lookup of the next batch) can run beside it.  At 72, for none of 256
-// threads, at 96 for none.  Nothing is spilled; kernel times are the same.
+// 64 registers for what a training step runs: each of an SM's four register files takes up to five warps of this kernel and then
+// has room for two more of 64 registers, so that a block of 256 threads (the lookup of the next batch) can run beside it; at 96
+// there is none.  With 96, DeepFM steps of 8192 x 26 ids 187 -> 195 us, 2999 x 39 148 -> 151, DCN-v2 8192 x 39 346 -> 357.  Nothing is
+// spilled, kernel times are the same.  (The pair kernel's epilogue does not fit in as few.)
 template <int kStages, int kHalves, gemm_epi::Kinds kKinds>
 __global__ void __maxnreg__(kKinds == kAny || kHalves == 2 ? 96 : 64)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -341,9 +342,16 @@ const char* gemm_bf16_pair(const GemmDesc& d, const GemmParams& p, int raster_gr
 double gemm_splitk_plan(const GemmDesc& d, int* best_bn, int* best_s);
 const char* gemm_bf16_splitk(const GemmDesc& d, GemmParams p, int BN, int S, cudaStream_t stream);
 
-static int highest_priority() {
+// Launches inside a capture go before what the captured step runs beside them, the next batch's lookup: 160 workloads with such a
+// lookup take 0 to 1.1 % less per step (DCN-v2, 8192 x 39 ids: 360 -> 347 us).  Elsewhere nothing of the package runs beside them,
+// and a caller's streams keep the order that the caller gave them.  (The pair and split-K kernels have no priority: with it, 0.1 %
+// on the mean of 13 workloads.)
+static bool highest_priority(cudaStream_t stream, int* priority) {
   static const int p = []() { int lo = 0, hi = 0; return cudaDeviceGetStreamPriorityRange(&lo, &hi) == cudaSuccess ? hi : 0; }();
-  return p;
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &s) != cudaSuccess) { cudaGetLastError(); return false; }
+  *priority = p;
+  return s == cudaStreamCaptureStatusActive;
 }
 
 const char* gemm_bf16(const GemmDesc& d, cudaStream_t stream) {
@@ -495,12 +503,14 @@ const char* gemm_bf16(const GemmDesc& d, cudaStream_t stream) {
   cfg.blockDim = dim3(kGemmThreads);
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  attr[0].id = cudaLaunchAttributePriority;            // before what runs beside them, such as the next batch's lookup
-  attr[0].val.priority = highest_priority();
+  unsigned n_attrs = 0;
+  if (use_pdl) {
+    attr[n_attrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n_attrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (highest_priority(stream, &attr[n_attrs].val.priority)) attr[n_attrs++].id = cudaLaunchAttributePriority;
   cfg.attrs = attr;
-  cfg.numAttrs = use_pdl ? 2 : 1;
+  cfg.numAttrs = n_attrs;
   // Plain bf16 outputs (forward products) have instances of their own.  With all epilogues in one kernel the plain one takes
   // 0.2 to 0.5 us longer where its instructions are at hand (512 x 512 x 1025 8.9 -> 9.1, 8192 x 400 x 401 9.8 -> 10.3,
   // launch to launch) and 2 us where the kernel runs once between others, as in a request of 512 examples (a pass 93.5 ->
