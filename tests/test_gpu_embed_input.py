@@ -41,7 +41,7 @@ CASES = [(4, 8, False, 32, 2, 0), (1, 1, False, 1, 1, 0), (39, 10, False, 301, 1
 
 
 @pytest.mark.parametrize("S,dim,cvm,B,bags,Dd", CASES)
-@pytest.mark.parametrize("combiner", ["sum", "mean"])
+@pytest.mark.parametrize("combiner", ["sum", "mean", "sqrtn"])
 @pytest.mark.parametrize("staged", [False, True])
 def test_against_the_layers(S, dim, cvm, B, bags, Dd, combiner, staged, monkeypatch):
     tn.core.init()
@@ -104,3 +104,36 @@ def test_linear_weights_in_the_rows(S, D, B, bags):
     assert torch.allclose(lin, both[:, :, D].detach(), rtol=1e-6, atol=1e-7) and torch.allclose(fm, F.fm(deep.detach(), S, D), rtol=1e-4, atol=1e-4)
     torch.autograd.backward([x0, lin], [gx, gl])
     assert float((_grads(layer.link) - g_want).norm()) <= 1e-5 * float(g_want.norm())
+
+
+@pytest.mark.parametrize("kind", ["wide_deep", "deepfm", "deep_cross", "dcn_v2"])
+@pytest.mark.parametrize("dim,frozen", [(132, ()), (8, ("head",)), (8, ("mlp",)), (132, ("head", "mlp"))])
+def test_own_steps_that_the_kernels_do_not_take_whole(kind, dim, frozen):
+    """Slots wider than the kernel's columns are pooled, a frozen head or tower goes through the layers: the same steps as one by one,
+    and what is frozen stays as it is."""
+    tn.core.init()
+    S, B, slots, runs = 3, 40, ["0", "1", "2"], []
+    for fused in (True, False):
+        torch.manual_seed(2)
+        kw = dict(dnn_hidden_units=(32, 16), embedding_dim=dim, dense_dim=3, bucket_size=B, table_rows=1 << 12)
+        cls = {"wide_deep": tn.models.WideDeep, "deepfm": tn.models.DeepFM, "deep_cross": tn.models.DeepCross, "dcn_v2": tn.models.DCNv2}[kind]
+        with torch.device("cuda"):
+            m = cls(*([slots, slots] if kind in ("wide_deep", "deepfm") else [slots]), **kw)
+        for part in frozen:
+            for p in getattr(m.sub_model, part).parameters():
+                p.requires_grad_(False)
+        kept = [p.detach().clone() for part in frozen for p in getattr(m.sub_model, part).parameters()]
+        m.compile(optimizer=tn.optimizer.Optimizer(tn.core.AdaGrad(learning_rate=0.05)), cuda_graph=False)
+        m.use_fused = fused
+        assert m.deep_emb.gives_operand() == (m.deep_emb.out_dim <= 128)
+        g = torch.Generator().manual_seed(5)
+        losses = []
+        for _ in range(3):
+            f = {tn.data.PACKED_KEY: tn.data.PackedFeatures(slots, ids=torch.randint(0, 90, (S, B), generator=g)), "dense": torch.randn(B, 3, generator=g)}
+            losses.append(float(m.train_on_batch(f, (torch.rand(B, generator=g) < 0.4).float())))
+        now = [p.detach() for part in frozen for p in getattr(m.sub_model, part).parameters()]
+        assert all(torch.equal(a, b) for a, b in zip(kept, now))
+        runs.append((losses, torch.cat([p.detach().flatten() for p in m.sub_model.parameters()])))
+        tn.core.runtime().check_status()
+    assert runs[0][0] == pytest.approx(runs[1][0], rel=5e-3)
+    assert float((runs[0][1] - runs[1][1]).norm()) <= 1e-2 * float(runs[1][1].norm())

@@ -46,6 +46,37 @@ def test_rows_are_those_of_the_pull(n, dim, cvm, monkeypatch):
     tn.core.runtime().check_status()
 
 
+@pytest.mark.parametrize("n", [1, 33, 5000])
+@pytest.mark.parametrize("dim,cvm,kind", [(8, False, "adagrad"), (10, True, "adagrad"), (3, False, "adam"), (64, False, "ftrl"), (128, False, "adam")])
+@pytest.mark.parametrize("zeros", [False, True])
+def test_a_new_row_starts_as_the_one_a_pull_makes(n, dim, cvm, kind, zeros):
+    """Two layers of one optimizer: the new signs of a batch, several times over, get their rows by lookup in one and by a pull in
+    the other.  Values depend on key and column alone (a table in inference mode starts rows at zero), so whole rows agree, the
+    optimizer's state included."""
+    tn.core.init()
+    opts = {"adagrad": tn.core.AdaGrad(learning_rate=0.01, initial_g2sum=0.1, initial_scale=0.3), "adam": tn.core.Adam(initial_scale=0.3),
+            "ftrl": tn.core.Ftrl(initial_scale=0.3)}
+    g = torch.Generator().manual_seed(n + dim)
+    pool = torch.cat([torch.randint(0, 1 << 62, (max(1, n // 2),), generator=g), torch.tensor([0, -1])])
+    ids = pool[torch.randint(0, pool.numel(), (n,), generator=g)].cuda()
+    got = []
+    for by_lookup in (True, False):
+        layer = _layer(dim, 1, n, cvm=cvm, opt=opts[kind])
+        layer.table.set_training(not zeros)
+        with torch.no_grad():
+            if by_lookup:
+                found = layer.link.lookup_in_place(ids).long()
+            else:
+                layer.link.pull_in_place(ids, training=False)
+        at = layer.table.lookup_rows(torch.unique(ids)).long()
+        assert int(at.min()) >= 0 and layer.table.n_rows == at.numel()
+        if by_lookup:
+            assert torch.equal(found, layer.table.lookup_rows(ids).long())
+        got.append(layer.table.rows[at].clone())
+    assert torch.equal(*got) and bool((got[0][:, :dim] != 0).any()) != zeros
+    tn.core.runtime().check_status()
+
+
 def test_two_tables_in_one_launch_and_a_front_that_waits():
     tn.core.init()
     g = torch.Generator().manual_seed(1)
