@@ -1,7 +1,7 @@
 """Small, self-contained launches of the hot kernels, for timing with CUDA events and for capturing
 with Nsight Compute (one GPU, a few launches, a few hundred MB on the device).
 
-    python benchmarks/kernel_cases.py gemm_fwd|gemm_dgrad|gemm_wgrad|gemm_big|sparse|deepfm|dense|small_ops  [--iters N]
+    python benchmarks/kernel_cases.py gemm_fwd|gemm_dgrad|gemm_wgrad|gemm_big|sparse|deepfm|deepfm_head|embed_input|lookup|bn_join|dense|small_ops  [--iters N]
 
 Each case prints the per-launch device time (CUDA events around N back-to-back launches after warm-up,
 inputs larger than L2 for the sparse cases) and the algorithmic bytes / FLOPs so a roofline fraction
@@ -44,7 +44,7 @@ def peaks():
 
 def main():
     ap = argparse.ArgumentParser()
-    ap.add_argument("case", choices=["gemm_fwd", "gemm_dgrad", "gemm_wgrad", "gemm_big", "sparse", "sparse_front", "deepfm", "deepfm_head", "mlp_chain", "dense", "small_ops"])
+    ap.add_argument("case", choices=["gemm_fwd", "gemm_dgrad", "gemm_wgrad", "gemm_big", "sparse", "sparse_front", "deepfm", "deepfm_head", "embed_input", "lookup", "bn_join", "mlp_chain", "dense", "small_ops"])
     ap.add_argument("--iters", type=int, default=20)
     ap.add_argument("--batch", type=int, default=8192)
     a = ap.parse_args()
@@ -155,10 +155,50 @@ def main():
         lin, fm = torch.randn(B, NL, device=dev) * 0.1, torch.randn(B, device=dev) * 0.1
         w = torch.nn.Parameter(torch.randn(NH + NL + 2, device=dev) * 0.05)
         y = (torch.rand(B, device=dev) < 0.25).float()
-        sums = torch.zeros(4, device=dev)
-        us = timed(lambda: F.deepfm_head_loss(h, lin, fm, w, y, sums, NH), a.iters)
+        pieces, widths = [h, lin, fm.view(-1, 1)], [NH, NL, 1]
+        grads, loss, sums, w.grad = [torch.empty_like(p) for p in pieces], torch.empty((), device=dev), torch.zeros(4, device=dev), torch.zeros_like(w)
+        scratch = F.head_scratch(widths, dev)                   # kept between calls, as a layer does
+        us = timed(lambda: ext.head_loss(pieces, widths, w.detach(), y, grads, True, w.grad, sums, loss, scratch, None), a.iters)
         nbytes = B * 408 * 2 * 2 + B * NL * 4 * 2 + B * 12
         out.update(us=us, min_bytes=nbytes, GBps=nbytes / us / 1e3, frac_of_hbm=nbytes / us / 1e3 / pk["hbm_gbs"], peak=tag)
+    elif a.case in ("embed_input", "lookup"):
+        # the operand of the first layer straight from the rows, and its gradient into them; the rows of a batch that is scored
+        import bench
+        B, S, D = a.batch, 26, 16
+        slots = [str(i) for i in range(S)]
+        cols = [tn.feature_column.embedding_column(tn.feature_column.category_column(key=k, bucket_size=B), D + 4, "sum") for k in slots]
+        layer = tn.layers.EmbeddingFeatures(cols, tn.core.Adam(learning_rate=1e-3, initial_scale=0.1), name="emb", is_concat=True, rows=1 << 22)
+        data = [b[0] for b in bench.make_batches(8, B, 3846154, dev, 5)]
+        feats = [{tn.data.PACKED_KEY: tn.data.PackedFeatures(slots, ids=i)} for i in data]
+        dense = torch.randn(B, 13, device=dev)
+        k = [0]
+        def both():
+            k[0] += 1
+            x0, fm, lin, _ = layer.operand(feats[k[0] % 8], True, dense, True, D, D)
+            if k[0] <= 1:
+                g[:] = [torch.randn_like(t) for t in (x0, fm, lin)]
+            torch.autograd.backward([x0, fm, lin], g)
+            layer.backwards()
+        def score():
+            k[0] += 1
+            with torch.no_grad():
+                layer.link.lookup_in_place(data[k[0] % 8].reshape(-1))
+        g = []
+        for _ in range(16):
+            both()
+        us = timed(score if a.case == "lookup" else both, a.iters)
+        out.update(us=us, what="three launches" if a.case == "lookup" else "pull, input, its gradient, push; eager", ids=B * S)
+    elif a.case == "bn_join":
+        # batch norm of a training step between tower and head, and its gradient
+        res = {}
+        for rows, nh, nx in ((32, 256, 4), (1024, 32, 10), (2048, 256, 26)):
+            bn = tn.layers.TNBatchNormalization(nh + nx, name="bn%d" % rows).to(dev).train()
+            h = torch.randn(rows, (nh + 8) // 8 * 8, device=dev).relu().bfloat16().requires_grad_()
+            x = torch.randn(rows, nx, device=dev).requires_grad_()
+            z = bn.join_operand(h, nh, x, masked=True)
+            gz = torch.randn_like(z)
+            res["%d x %d" % (rows, nh + nx)] = timed(lambda: bn.join_operand(h, nh, x, masked=True).backward(gz), a.iters)
+        out.update(us_eager=res)
     elif a.case == "mlp_chain":
         # the DeepFM tower 429-400-400-400 as one kernel per direction against the three GEMM launches it replaces
         from tensornet_b200.layers import MLP

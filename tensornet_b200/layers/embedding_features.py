@@ -18,7 +18,7 @@ from typing import Dict, Optional, Sequence
 import torch
 from torch import nn
 
-from .. import core
+from .. import _build, core
 from ..data.features import PACKED_KEY, adjacent_columns, gather_columns, padded_columns
 from ..feature_column import EmbeddingColumn
 from ..ops import functional as F
@@ -148,8 +148,8 @@ class EmbeddingFeatures(nn.Module):
 
     def gives_operand(self, width: Optional[int] = None) -> bool:
         """Whether :meth:`operand` may stand in for a call of this layer: on a GPU, with nobody looking on."""
-        return (core.runtime().on_gpu and type(self) is EmbeddingFeatures and self.is_concat and (width or self.out_dim) <= 128
-                and unobserved(self, backward=True))
+        return (core.runtime().on_gpu and type(self) is EmbeddingFeatures and self.is_concat
+                and (width or self.out_dim) <= _build.cuda_ext().EMBED_INPUT_COLUMNS and unobserved(self, backward=True))
 
     def operand(self, features: Dict, training: bool, dense: Optional[torch.Tensor] = None, fm: bool = False, width: Optional[int] = None,
                 lin_col: int = -1, pooled: bool = False):

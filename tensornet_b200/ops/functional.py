@@ -697,11 +697,3 @@ def head_score(pieces, widths, w) -> torch.Tensor:
     out = torch.empty((pieces[0].shape[0], 1), dtype=torch.float32, device=w.device)
     _ext().head_score([p.detach() for p in pieces], list(widths), w.detach(), out)
     return out
-
-
-def deepfm_head_loss(h, lin, fm, w, label, sums, n_hidden):
-    """:func:`head_loss` over ``[h[:, :n_hidden] | lin | fm]`` as ``(loss, prediction)``."""
-    pieces = [h] + ([lin.contiguous()] if lin is not None else []) + [fm.reshape(-1, 1)]
-    widths = [n_hidden] + [int(p.shape[1]) for p in pieces[1:]]
-    pred = torch.empty(h.shape[0], dtype=torch.float32, device=h.device)
-    return head_loss(pieces, widths, w, label.contiguous().view(-1).float(), sums, head_scratch(widths, h.device), True, pred), pred
