@@ -71,7 +71,7 @@ __device__ __forceinline__ float4 load_bf16(const __nv_bfloat16* p, int n) {
 // `wpe` warps (a power of two) share an example, each takes a run of its slots; they meet in shared memory for the FM term.  A
 // warp first fetches the row numbers of up to 32 slots, a lane each (or the bounds of their bags), hands them to the groups of
 // G lanes that read the rows, kFlight at a time: the chain of dependent loads is walked once per 32 slots.
-// Bound by the latency of those loads.  8192 x 26 slots of 16 with their linear weights 17.8 us.  In place of pooling, FM term
+// Bound by the latency of those loads (L2 and memory at 22 and 15 % of their rates).  8192 x 26 slots of 16 with their linear weights 17.8 us.  In place of pooling, FM term
 // and concatenation: 2999 x 39 slots of 10, 8.2 us for 18 (and three launches more); 4096 x 20 bags of three ids and 10 columns 24
 // for 22.6; 8192 x 100 bags of five ids and 64 columns 330 for 375.  More blocks of fewer registers per SM (five, six, eight):
 // 8 to 40 % slower; sixty-four warps per SM by splitting examples: 7 to 50 % slower.
@@ -204,7 +204,8 @@ __global__ void __launch_bounds__(kThreads, 4) embed_input_fwd_kernel(const RowS
 
 // One group of G lanes per bag, example after example, so that the operand's gradient and the pooled columns are read as they
 // lie; kFlight bags on the way at once when every bag holds one id.  The field sums of the FM term come from the forward pass: no
-// bag waits for another.  Columns from `dim` on (show / click) carry no gradient.  Bound by the reductions into the rows.
+// bag waits for another.  Columns from `dim` on (show / click) carry no gradient.  Bound by the latency of its loads (for which a
+// warp waits ten of its fifteen cycles per instruction; L2 at 22 % of its rate, memory at 28 %): reductions into the rows are not waited for.
 // 8192 x 26 slots of 16 with their linear weights 15.1 us (a warp per example 14.6).  In place of split, FM backward, additions and
 // pooling backward: 2999 x 39 slots of 10, 8.4 us for 27 and four launches more; 4096 x 20 bags of three ids and 10 columns 9.9 for
 // 14.5; 8192 x 100 bags of five ids and 64 columns 422 for 492.

@@ -310,7 +310,8 @@ __global__ void __launch_bounds__(kThreads) head_score_kernel(const __grid_const
 // side in one lane per row, gradients of the weights are summed in registers, and warps meet in shared memory with plain
 // stores (a float add to shared memory is a compare-and-swap loop).
 //
-// 8192 x [400 | 26 | 1] 8.1 us, 4096 x [256 | 200] 7.0, 2999 x [75 | 39 | 1] 6.0, 1024 x 42 3.6, 32 x 260 3.5.  As kernels of
+// Bound by latency: a quarter of the warps an SM can hold (128 registers), memory at 7 % of its rate.
+// 8192 x [400 | 26 | 1] 8.2 us, 4096 x [256 | 200] 7.0, 2999 x [75 | 39 | 1] 5.6, 1024 x 42 3.8, 32 x 260 3.3.  As kernels of
 // their own (operand assembled, dot products, loss, gradients, and the copies and fills between them) the last four took
 // 36, 47, 12 and 12 us of a step's critical path, seven to eleven launches.
 template <int kPairs, int kLin, bool kMask>
@@ -590,7 +591,9 @@ __global__ void __launch_bounds__(kThreads, 2) head_loss_small_kernel(const __gr
   if (!alone && threadIdx.x == 0) publish_loss(a);
 }
 
-// The instance for a head, or null where none takes it.
+// The instance for a head, or null where none takes it.  By powers of two, but for the padded rows of 256 to 312 units, which would
+// fall to the widest one: five pairs (ten columns) a lane in place of eight (17) take 7.03 in place of 7.43 us at 4096 x [256 | 200],
+// 4.9 in place of 5.6 at 500 x 256, 3.3 in place of 4.1 at 32 x 260.
 using HeadKernel = void (*)(HeadArgs);
 template <int kPairs>
 HeadKernel rows_kernel_lin(int lin, bool mask) {
