@@ -440,11 +440,11 @@ const void* mapped_host_ptr(const at::Tensor& t) {
   if (cudaPointerGetAttributes(&at, p) != cudaSuccess) { cudaGetLastError(); return nullptr; }
   const char* d = static_cast<const char*>(at.devicePointer);
   if (at.type != cudaMemoryTypeHost || d == nullptr) return nullptr;
-  // Memory that was registered by somebody, not allocated page-locked: its last byte too.  No more than the pages that it begins
-  // in may be known to the driver, and a kernel would read on behind them.
-  static const c10::DeleterFnPtr allocated = at::getHostAllocator(at::kCUDA)->allocate(1).get_deleter();
-  if (t.storage().data_ptr().get_deleter() == allocated) return d;
-  if (cudaPointerGetAttributes(&at, p + t.nbytes() - 1) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+  // Its last byte too, where that lies on another page: somebody may have registered no more than the pages that it begins in, and
+  // a kernel would read on behind them.
+  const char* last = p + t.nbytes() - 1;
+  if (reinterpret_cast<uintptr_t>(p) >> 12 == reinterpret_cast<uintptr_t>(last) >> 12) return d;
+  if (cudaPointerGetAttributes(&at, last) != cudaSuccess) { cudaGetLastError(); return nullptr; }
   return at.type == cudaMemoryTypeHost && at.devicePointer == d + t.nbytes() - 1 ? d : nullptr;
 }
 
